@@ -3423,8 +3423,8 @@ namespace {
 struct HmData {
   HmPlan plan;
   std::shared_ptr<MeshData::HmPlanCache> pc;  // the mesh's plan (perm, iperm on the device)
-  Buf leaf_lo, leaf_ptr, leaf_ent, dn, D1, D2, vt_items, lb_items;
-  int32_t n_vt = 0, n_lb = 0;
+  Buf leaf_lo, leaf_ptr, leaf_ent, dn, D1, D2, vt_items, lb_items, db_items;
+  int32_t n_vt = 0, n_lb = 0, n_db = 0;
   Buf lr[2], U[2], V[2];
   int32_t n_lr = 0, n_dense = 0, n_leaf = 0;
   int64_t tstride = 0, pstride = 0;
@@ -3441,7 +3441,7 @@ struct HmData {
   bemgpu_hmatrix_stats st{};
   size_t bytes() const {
     size_t b = leaf_lo.bytes + leaf_ptr.bytes + leaf_ent.bytes + dn.bytes + D1.bytes +
-               D2.bytes + vt_items.bytes + lb_items.bytes;
+               D2.bytes + vt_items.bytes + lb_items.bytes + db_items.bytes;
     for (int o = 0; o < 2; ++o) b += lr[o].bytes + U[o].bytes + V[o].bytes;
     b += ny_pinv.bytes + ny_nbptr.bytes + ny_nbel.bytes + ny_woff.bytes + ny_w.bytes;
     return b;
@@ -3470,6 +3470,8 @@ struct HmData {
     A.lb_items = lb_items.as<HmItem>();
     A.n_vt = n_vt;
     A.n_lb = n_lb;
+    A.db_items = db_items.as<HmItem>();
+    A.n_db = n_db;
     A.T = T;
     A.tstride = tstride;
     A.P = static_cast<char*>(s) + (size_t)nr * tstride * 16;
@@ -3749,6 +3751,26 @@ int hm_build(bemgpu_ctx* c, MeshData* m, const bemgpu_problem& p, int kind,
   H->n_dense = (int32_t)dn.size();
   H->n_lr = (int32_t)lblk.size();
   TRY(upload(c, dn, &H->dn));
+  // row chunks of the full blocks for the products (those of wide blocks, the longest, first)
+  // and column chunks for their evaluation
+  std::vector<HmItem> dbi, dei;
+  for (size_t b = 0; b < dn.size(); ++b) {
+    const int32_t m_ = dn[b].m, n_ = dn[b].n;
+    const int32_t rows = n_ > kHmNarrow ? kHmWideRows : kHmDenseRows;
+    for (int32_t r0 = 0; r0 < m_; r0 += rows)
+      dbi.push_back(HmItem{(int32_t)b, r0, std::min(rows, m_ - r0), 0});
+    const int32_t step = std::max(1, kHmDenseChunk / std::max(1, m_));
+    for (int32_t c0 = 0; c0 < n_; c0 += step)
+      dei.push_back(HmItem{(int32_t)b, c0, std::min(step, n_ - c0), 0});
+  }
+  std::stable_sort(dbi.begin(), dbi.end(), [&](const HmItem& a, const HmItem& b) {
+    const int32_t na = dn[(size_t)a.blk].n, nb = dn[(size_t)b.blk].n;
+    return (na > kHmNarrow ? na : 0) > (nb > kHmNarrow ? nb : 0);
+  });
+  H->n_db = (int32_t)dbi.size();
+  TRY(upload(c, dbi, &H->db_items));
+  Buf d_dei;
+  TRY(upload(c, dei, &d_dei));
   TRY(alloc(c, (size_t)std::max<int64_t>(1, off) * es, &H->D1));
   TRY(alloc(c, (size_t)std::max<int64_t>(1, off) * es, &H->D2));
   // U and V were allocated at the rank cap: move the ranks reached into tight pools
@@ -3779,7 +3801,7 @@ int hm_build(bemgpu_ctx* c, MeshData* m, const bemgpu_problem& p, int kind,
   for (int op = 0; op < 2; ++op) TRY(upload(c, keep[op], &H->lr[op]));
   {
     Prof pr(c, "hm_dense");
-    launch_hm_dense(L, H->dn.as<HmDense>(), H->n_dense, H->D1.p, H->D2.p, recs, H->f32,
+    launch_hm_dense(L, H->dn.as<HmDense>(), d_dei.as<HmItem>(), (int32_t)dei.size(), H->D1.p, H->D2.p, recs, H->f32,
                     H->pc->perm.as<int32_t>(), kind, k, a_re, a_im);
   }
   // near pairs (the mesh's list, same order) into their full leaf blocks

@@ -329,19 +329,20 @@ void launch_hm_compact(const Launch& L, const HmCopy* d, int32_t count, const vo
 
 // ------------------------------------------------------------------ full blocks
 template <typename R, int KIND>
-__global__ void __launch_bounds__(256) k_hm_dense(const HmDense* __restrict__ dn, void* D1,
+__global__ void __launch_bounds__(256) k_hm_dense(const HmDense* __restrict__ dn,
+                                                  const HmItem* __restrict__ items, void* D1,
                                                   void* D2, const R* __restrict__ recs,
                                                   const int32_t* __restrict__ perm, double k_,
                                                   double a_re, double a_im) {
   constexpr int kRec = Prec<R>::kRec;
-  const HmDense B = dn[blockIdx.x];
-  const int64_t cnt = (int64_t)B.m * B.n;
+  const HmItem it = items[blockIdx.x];  // columns [lo, lo + cnt) of a block
+  const HmDense B = dn[it.blk];
+  const int64_t e0 = (int64_t)B.m * it.lo, e1 = e0 + (int64_t)B.m * it.cnt;
   const cx<R> al = {(R)a_re, (R)a_im};
   const R k = (R)k_;
   cx<R>* o1 = static_cast<cx<R>*>(D1) + B.off;
   cx<R>* o2 = static_cast<cx<R>*>(D2) + B.off;
-  for (int64_t e = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; e < cnt;
-       e += (int64_t)blockDim.x * gridDim.y) {
+  for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
     const int i = (int)(e % B.m), j = (int)(e / B.m);
     const int32_t pi = perm[B.rlo + i], pj = perm[B.clo + j];
     if (pi == pj) continue;  // self pair: near kernel
@@ -360,23 +361,23 @@ __global__ void __launch_bounds__(256) k_hm_dense(const HmDense* __restrict__ dn
   }
 }
 
-void launch_hm_dense(const Launch& L, const HmDense* dn, int32_t n_dense, void* D1, void* D2,
-                     const void* recs, bool f32, const int32_t* perm, int kind, double k,
+void launch_hm_dense(const Launch& L, const HmDense* dn, const HmItem* items, int32_t n_items,
+                     void* D1, void* D2, const void* recs, bool f32, const int32_t* perm, int kind, double k,
                      double a_re, double a_im) {
-  if (n_dense <= 0) return;
-  dim3 g((unsigned)n_dense, 4);
+  if (n_items <= 0) return;
+  const unsigned g = (unsigned)n_items;
   const float* rf = static_cast<const float*>(recs);
   const double* rd = static_cast<const double*>(recs);
   if (f32) {
     if (kind == kAsmBM)
-      k_hm_dense<float, kAsmBM><<<g, 256, 0, L.stream>>>(dn, D1, D2, rf, perm, k, a_re, a_im);
+      k_hm_dense<float, kAsmBM><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rf, perm, k, a_re, a_im);
     else
-      k_hm_dense<float, kAsmCBIE><<<g, 256, 0, L.stream>>>(dn, D1, D2, rf, perm, k, a_re, a_im);
+      k_hm_dense<float, kAsmCBIE><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rf, perm, k, a_re, a_im);
   } else {
     if (kind == kAsmBM)
-      k_hm_dense<double, kAsmBM><<<g, 256, 0, L.stream>>>(dn, D1, D2, rd, perm, k, a_re, a_im);
+      k_hm_dense<double, kAsmBM><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rd, perm, k, a_re, a_im);
     else
-      k_hm_dense<double, kAsmCBIE><<<g, 256, 0, L.stream>>>(dn, D1, D2, rd, perm, k, a_re, a_im);
+      k_hm_dense<double, kAsmCBIE><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rd, perm, k, a_re, a_im);
   }
   count_launch(1);
 }
@@ -401,6 +402,7 @@ __device__ __forceinline__ bool group_on(const GmState* st, int r0, int rb, int 
 // Coefficients of one column chunk of a compressed block: T[toff + c kmax + l] =
 // sum over the chunk of V[j, l] x[clo + j]; one warp per l, four independent accumulators
 // per lane and right-hand side (added in a fixed order).
+constexpr int kVtU = 4, kVtN = 3;  // coefficients per warp and values per lane in flight
 template <typename R, int RB>
 __global__ void __launch_bounds__(256) k_hm_vt(HmOp A, const void* __restrict__ X, int64_t ldx,
                                                int32_t nr, const GmState* st, int mode,
@@ -418,6 +420,45 @@ __global__ void __launch_bounds__(256) k_hm_vt(HmOp A, const void* __restrict__ 
   for (int q = 0; q < RB; ++q)
     x[q] = static_cast<const C*>(X) + (int64_t)min(r0 + q, nr - 1) * ldx + B.clo;
   const int j0 = it.lo, j1 = it.lo + it.cnt;
+  if (it.cnt <= 32 * kVtN) {
+    // short chunks (most blocks have about 40 columns): kVtU coefficients per warp at a time,
+    // all their values in flight (82 -> 45 us a product of 20480 panels); per coefficient the
+    // order is that of the general loop's remainder, which takes all of such a chunk
+    for (int l0 = wid; l0 < B.rank; l0 += 8 * kVtU) {
+      C v[kVtU][kVtN];
+#pragma unroll
+      for (int e = 0; e < kVtU; ++e)
+#pragma unroll
+        for (int u = 0; u < kVtN; ++u) {
+          const int l = l0 + 8 * e, j = j0 + lane + 32 * u;
+          v[e][u] = l < B.rank && j < j1 ? V[(int64_t)l * B.n + j] : C{0, 0};
+        }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        C xv[kVtN];
+#pragma unroll
+        for (int u = 0; u < kVtN; ++u) {
+          const int j = j0 + lane + 32 * u;
+          xv[u] = j < j1 ? x[q][j] : C{0, 0};
+        }
+#pragma unroll
+        for (int e = 0; e < kVtU; ++e) {
+          const int l = l0 + 8 * e;
+          if (l >= B.rank) break;  // uniform per warp
+          C s = {0, 0};
+#pragma unroll
+          for (int u = 0; u < kVtN; ++u)
+            if (j0 + lane + 32 * u < j1) s += v[e][u] * xv[u];
+          const C t = cwarp_sum(s);
+          if (lane == 0 && r0 + q < nr) {
+            double* T = A.T + 2 * ((int64_t)(r0 + q) * A.tstride + B.toff + (int64_t)it.c * B.kmax);
+            stc(T, l, cd{(double)t.x, (double)t.y});
+          }
+        }
+      }
+    }
+    return;
+  }
   for (int l = wid; l < B.rank; l += 8) {
     const C* v = V + (int64_t)l * B.n;
     C s[RB][4];
@@ -453,8 +494,17 @@ __global__ void __launch_bounds__(256) k_hm_vt(HmOp A, const void* __restrict__ 
 constexpr int kLeafRows = 64;
 constexpr int kLeafSlices = 4;
 
-// Partial rows of every full block: P[poff + i] = sum_j D[i, j] x[clo + j] (64 rows x 4
-// column slices per pass, slices added in a fixed order), RB right-hand sides per CTA.
+// Partial rows of the full blocks: P[poff + i] = sum_j D[i, j] x[clo + j], one CTA per row
+// item of a block, RB right-hand sides per CTA.  Bound by memory latency: beside the leaf
+// blocks (about 40 x 40) a densified block can have thousands of rows and columns, so the
+// rows are spread over items (one CTA per block took 9 ms a product of 20480 panels with a
+// 10240-column densified block), the wide blocks' items come first in the list, and a thread
+// keeps all or kDblkU of its loads in flight.  A row is the sum of eight column chains
+// j = c + 8 t, in the order (0 + 4) + (1 + 5) + (2 + 6) + (3 + 7); for 64 x 64 blocks of four
+// chains j = c + 4 t.  Narrow blocks (at most kHmNarrow columns): 64 rows, a thread takes
+// chains c and c + 4 at once.  Wide ones: 32 rows, a thread takes one chain.
+template <typename R>
+constexpr int kDblkU = sizeof(R) == 4 ? 16 : 8;
 template <typename R, int RB>
 __global__ void __launch_bounds__(kLeafRows * kLeafSlices) k_hm_dblk(
     HmOp A, const void* __restrict__ X, int64_t ldx, int32_t nr, const GmState* st, int mode,
@@ -463,60 +513,101 @@ __global__ void __launch_bounds__(kLeafRows * kLeafSlices) k_hm_dblk(
   const int r0 = blockIdx.y * RB;
   if (!group_on(st, r0, RB, nr, mode)) return;
   if (jptr) X = static_cast<const C*>(X) + (int64_t)*jptr * jstride;
-  const HmDense& B = A.dn[blockIdx.x];
-  const int row = threadIdx.x % kLeafRows, s = threadIdx.x / kLeafRows;
-  __shared__ C part[RB][kLeafSlices][kLeafRows];
-  const C* D = static_cast<const C*>(A.D) + B.off;
+  const HmItem it = A.db_items[blockIdx.x];
+  const HmDense B = A.dn[it.blk];
+  __shared__ C part[RB][kLeafSlices * kLeafRows];
+  const int64_t m = B.m;
+  const int n = B.n;
   const C* x[RB];
 #pragma unroll
   for (int q = 0; q < RB; ++q)
     x[q] = static_cast<const C*>(X) + (int64_t)min(r0 + q, nr - 1) * ldx + B.clo;
-  auto store = [&](int i) {
+  const bool wide = n > kHmNarrow;
+  const int rows = wide ? kHmWideRows : kLeafRows;
+  const int row = threadIdx.x % rows, ch = threadIdx.x / rows;
+  const C* D = static_cast<const C*>(A.D) + B.off + it.lo + row;
+  if (wide) {
+    constexpr int U = kDblkU<R>;
+    C a[RB];
+#pragma unroll
+    for (int q = 0; q < RB; ++q) a[q] = C{0, 0};
+    if (row < it.cnt)
+      for (int j0 = ch; j0 < n; j0 += 8 * U) {
+        C d[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int j = j0 + 8 * u;
+          d[u] = j < n ? D[(int64_t)j * m] : C{0, 0};
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int j = j0 + 8 * u;
+#pragma unroll
+          for (int q = 0; q < RB; ++q)
+            if (j < n) a[q] += d[u] * x[q][j];
+        }
+      }
+#pragma unroll
+    for (int q = 0; q < RB; ++q) part[q][threadIdx.x] = a[q];
+    __syncthreads();
+    if (ch < kLeafSlices) {
+#pragma unroll
+      for (int q = 0; q < RB; ++q) a[q] = part[q][threadIdx.x] + part[q][threadIdx.x + 4 * kHmWideRows];
+    }
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < RB; ++q)
-      if (r0 + q < nr)
-        static_cast<C*>(A.P)[(int64_t)(r0 + q) * A.pstride + B.poff + i] =
-            ((part[q][0][row] + part[q][1][row]) + part[q][2][row]) + part[q][3][row];
-  };
-  if (B.m == kLeafRows && B.n == kLeafRows) {  // leaf x leaf block: all loads in flight
+      if (ch < kLeafSlices) part[q][threadIdx.x] = a[q];
+  } else if (m == kLeafRows && n == kLeafRows) {
     constexpr int kPer = kLeafRows / kLeafSlices;
     C d[kPer];
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) d[u] = D[row + (int64_t)(s + u * kLeafSlices) * kLeafRows];
+    for (int u = 0; u < kPer; ++u) d[u] = D[(int64_t)(ch + u * kLeafSlices) * kLeafRows];
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
-      C a = d[0] * x[q][s];
+      C a = d[0] * x[q][ch];
 #pragma unroll
-      for (int u = 1; u < kPer; ++u) a += d[u] * x[q][s + u * kLeafSlices];
-      part[q][s][row] = a;
+      for (int u = 1; u < kPer; ++u) a += d[u] * x[q][ch + u * kLeafSlices];
+      part[q][threadIdx.x] = a;
     }
-    __syncthreads();
-    if (s == 0) store(row);
-    return;
-  }
-  for (int rr = 0; rr < B.m; rr += kLeafRows) {
-    const int i = rr + row;
+  } else {
+    constexpr int kPer = kHmNarrow / 8;
+    C d0[kPer], d1[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int j = ch + 8 * u;
+      d0[u] = row < it.cnt && j < n ? D[(int64_t)j * m] : C{0, 0};
+      d1[u] = row < it.cnt && j + 4 < n ? D[(int64_t)(j + 4) * m] : C{0, 0};
+    }
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
       C a0 = {0, 0}, a1 = {0, 0};
-      if (i < B.m) {
-        int j = s;
-        for (; j + kLeafSlices < B.n; j += 2 * kLeafSlices) {
-          a0 += D[i + (int64_t)j * B.m] * x[q][j];
-          a1 += D[i + (int64_t)(j + kLeafSlices) * B.m] * x[q][j + kLeafSlices];
-        }
-        for (; j < B.n; j += kLeafSlices) a0 += D[i + (int64_t)j * B.m] * x[q][j];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int j = ch + 8 * u;
+        if (j < n) a0 += d0[u] * x[q][j];
+        if (j + 4 < n) a1 += d1[u] * x[q][j + 4];
       }
-      part[q][s][row] = a0 + a1;
+      part[q][threadIdx.x] = a0 + a1;
     }
-    __syncthreads();
-    if (s == 0 && i < B.m) store(i);
-    __syncthreads();
+  }
+  __syncthreads();
+  if (ch == 0 && row < it.cnt) {
+#pragma unroll
+    for (int q = 0; q < RB; ++q)
+      if (r0 + q < nr)
+        static_cast<C*>(A.P)[(int64_t)(r0 + q) * A.pstride + B.poff + it.lo + row] =
+            ((part[q][row] + part[q][row + rows]) + part[q][row + 2 * rows]) +
+            part[q][row + 3 * rows];
   }
 }
 
 // Partial rows of one row chunk of a compressed block: P[poff + i] = sum_l U[i, l] t[l],
-// t = the block's coefficient chunks added in order; RB right-hand sides per CTA.
+// t = the block's coefficient chunks added in order; RB right-hand sides per CTA.  Bound by
+// memory latency (descriptor, coefficients and U values are dependent loads, and most blocks
+// have about 40 rows): CTAs of 64 threads keep 32 blocks in flight per SM, and the U values
+// of the next eight ranks are loaded ahead.
+constexpr int kLbU = 8;
 template <typename R, int RB>
 __global__ void __launch_bounds__(kHmRowChunk) k_hm_lblk(HmOp A, int32_t nr, const GmState* st,
                                                         int mode) {
@@ -526,7 +617,15 @@ __global__ void __launch_bounds__(kHmRowChunk) k_hm_lblk(HmOp A, int32_t nr, con
   const HmItem it = A.lb_items[blockIdx.x];
   const HmLR B = A.lr[it.blk];
   __shared__ C t[RB][kHmMaxRank];
-  if (threadIdx.x < B.rank) {
+  static_assert(kHmRowChunk >= kHmMaxRank, "one coefficient per thread");
+  const int rank = B.rank, rank4 = rank & ~3;
+  const bool on = threadIdx.x < it.cnt;
+  const int64_t m = B.m;
+  const C* U = static_cast<const C*>(A.U) + B.uoff + it.lo + threadIdx.x;
+  C u[kLbU];
+#pragma unroll
+  for (int e = 0; e < kLbU; ++e) u[e] = on && e < rank4 ? U[(int64_t)e * m] : C{0, 0};
+  if (threadIdx.x < rank) {
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
       const double* T = A.T + 2 * ((int64_t)min(r0 + q, nr - 1) * A.tstride + B.toff);
@@ -536,33 +635,33 @@ __global__ void __launch_bounds__(kHmRowChunk) k_hm_lblk(HmOp A, int32_t nr, con
     }
   }
   __syncthreads();
-  const int i = it.lo + threadIdx.x;
-  if (threadIdx.x >= it.cnt) return;
-  const C* U = static_cast<const C*>(A.U) + B.uoff + i;
+  if (!on) return;
   C a[RB][4];
 #pragma unroll
   for (int q = 0; q < RB; ++q) a[q][0] = a[q][1] = a[q][2] = a[q][3] = C{0, 0};
-  int l = 0;
-  for (; l + 3 < B.rank; l += 4) {
-    const C u0 = U[(int64_t)l * B.m], u1 = U[(int64_t)(l + 1) * B.m],
-            u2 = U[(int64_t)(l + 2) * B.m], u3 = U[(int64_t)(l + 3) * B.m];
+  for (int l = 0; l < rank4; l += kLbU) {
+    C nx[kLbU];
 #pragma unroll
-    for (int q = 0; q < RB; ++q) {
-      a[q][0] += u0 * t[q][l];
-      a[q][1] += u1 * t[q][l + 1];
-      a[q][2] += u2 * t[q][l + 2];
-      a[q][3] += u3 * t[q][l + 3];
+    for (int e = 0; e < kLbU; ++e)
+      nx[e] = l + kLbU + e < rank4 ? U[(int64_t)(l + kLbU + e) * m] : C{0, 0};
+#pragma unroll
+    for (int e = 0; e < kLbU; ++e) {
+      if (l + e < rank4) {
+#pragma unroll
+        for (int q = 0; q < RB; ++q) a[q][e & 3] += u[e] * t[q][l + e];
+      }
+      u[e] = nx[e];
     }
   }
-  for (; l < B.rank; ++l) {
-    const C u0 = U[(int64_t)l * B.m];
+  for (int l = rank4; l < rank; ++l) {
+    const C u0 = U[(int64_t)l * m];
 #pragma unroll
     for (int q = 0; q < RB; ++q) a[q][0] += u0 * t[q][l];
   }
 #pragma unroll
   for (int q = 0; q < RB; ++q)
     if (r0 + q < nr)
-      static_cast<C*>(A.P)[(int64_t)(r0 + q) * A.pstride + B.poff + i] =
+      static_cast<C*>(A.P)[(int64_t)(r0 + q) * A.pstride + B.poff + it.lo + threadIdx.x] =
           ((a[q][0] + a[q][1]) + a[q][2]) + a[q][3];
 }
 
@@ -625,7 +724,7 @@ void launch_hm_matvec(const Launch& L, const HmOp& A, const double* X, int64_t l
   constexpr int kRB = 4;  // right-hand sides per CTA of the block products
   const int rb = nr >= kRB ? kRB : 1;
   const unsigned ng = (unsigned)((nr + rb - 1) / rb);
-  const dim3 gv((unsigned)A.n_vt, ng), gb((unsigned)A.n_lb, ng), gd((unsigned)A.n_dense, ng),
+  const dim3 gv((unsigned)A.n_vt, ng), gb((unsigned)A.n_lb, ng), gd((unsigned)A.n_db, ng),
       gl((unsigned)A.n_leaf, (unsigned)nr);
   constexpr int TL = kLeafRows * kLeafSlices;
   int launches = 1;

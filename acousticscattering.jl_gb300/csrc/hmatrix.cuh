@@ -25,10 +25,13 @@ struct HmLR {
   int64_t poff;        // offset of the block's m partial rows in the row scratch
 };
 
-// Work items of the compressed-block products: a column chunk of V^T x (c: chunk index)
-// or a row chunk of U t.
+// Work items of the block products: a column chunk of V^T x (c: chunk index), a row chunk
+// of U t or of a full block.
 constexpr int kHmColChunk = 256;
-constexpr int kHmRowChunk = 256;
+constexpr int kHmRowChunk = 64;
+constexpr int kHmNarrow = 64;     // full blocks of at most this many columns are narrow
+constexpr int kHmDenseRows = 64;  // rows of a product item of a narrow full block,
+constexpr int kHmWideRows = 32;   // of a wide one
 struct HmItem {
   int32_t blk, lo, cnt, c;
 };
@@ -53,7 +56,8 @@ struct HmOp {
   int32_t n_lr, n_dense, n_leaf, f32;
   const HmItem* vt_items;   // column chunks of every compressed block
   const HmItem* lb_items;   // row chunks of every compressed block
-  int32_t n_vt, n_lb;
+  const HmItem* db_items;   // row chunks of every full block, wide blocks first
+  int32_t n_vt, n_lb, n_db;
   double* T;                // coefficient scratch: per right-hand side tstride complex128
   int64_t tstride;
   void* P;                  // partial-row scratch: per right-hand side pstride complex
@@ -115,8 +119,11 @@ void launch_hm_compact(const Launch& L, const HmCopy* d, int32_t count, const vo
                        void* dst);
 // Regular-rule entries of the full blocks of both operators (self pairs left to the near
 // kernel, which writes them through AsmInst.near_dst), precision as launch_hm_aca.
-void launch_hm_dense(const Launch& L, const HmDense* dn, int32_t n_dense, void* D1, void* D2,
-                     const void* recs, bool f32, const int32_t* perm, int kind, double k,
+// items: column chunks of the blocks (lo: first column, cnt: columns), about kHmDenseChunk
+// entries each.
+constexpr int kHmDenseChunk = 1024;
+void launch_hm_dense(const Launch& L, const HmDense* dn, const HmItem* items, int32_t n_items,
+                     void* D1, void* D2, const void* recs, bool f32, const int32_t* perm, int kind, double k,
                      double a_re, double a_im);
 // Y[:, r] = sb B[:, r] + sa (A X)[:, r] for every right-hand side r < nr with
 // (act == null or act[r].active), the operands in permuted order.
