@@ -3360,10 +3360,13 @@ int bemgpu_far_field(bemgpu_solution* sol, int32_t rhs, int64_t ndir, const doub
     }
   }
   if (ndir == 0) return BEMGPU_OK;
-  Buf dd, dout, dw;
-  TRY(upload(c, d, &dd));
+  Buf dd, dout;
   TRY(alloc(c, (size_t)ndir * 16, &dout));
   WaveInst w{};
+  if (ndir == 1)
+    std::copy(d.begin(), d.end(), w.dir1);
+  else
+    TRY(upload(c, d, &dd));
   w.panels = s->mesh->panels.as<double>();
   w.n = s->mesh->n;
   w.k = s->k;
@@ -3377,11 +3380,9 @@ int bemgpu_far_field(bemgpu_solution* sol, int32_t rhs, int64_t ndir, const doub
   Buf dpart;
   TRY(alloc(c, far_field_scratch(w.n, (int32_t)ndir, 1), &dpart));
   w.part = dpart.as<double>();
-  std::vector<WaveInst> wv{w};
-  TRY(upload(c, wv, &dw));
   {
     Prof p(c, "far_field");
-    launch_far_field(c->launch(), dw.as<WaveInst>(), 1, 1, (int32_t)ndir, w.n);
+    launch_far_field_one(c->launch(), w);
   }
   CUDA_TRY(c, cudaGetLastError());
   CUDA_TRY(c, cudaMemcpyAsync(out, dout.p, (size_t)ndir * 16, cudaMemcpyDeviceToHost, c->stream));

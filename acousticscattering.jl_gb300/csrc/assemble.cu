@@ -360,98 +360,255 @@ void launch_incident(const Launch& L, const WaveInst* d_inst, int ninst, int64_t
 
 // ------------------------------------------------------------------ far field
 // f(xh) = -(1/4pi) sum_j area_j (ik xh.n_j p_j + q_j) sum_g W_g e^{-ik xh.y_jg}
-// (solvers/bem/full.jl:509-519).  The panels are split into chunks of kFarChunk, one CTA
-// (one panel per thread) per (chunk, direction, rhs, instance), so the FP64 phase work
-// of one direction is spread over the GPU; a second kernel sums the chunk partials in
-// chunk order.  Every sum has a fixed order, so the result does not depend on what else
-// runs on the GPU.
-constexpr int kFarChunk = 128;
+// (solvers/bem/full.jl:509-519).
+//
+// Bound by FP64 issue (two FMAs per clock and SM), so the work per (panel, direction) is
+// what counts.  The seven phases of a panel are one sine / cosine at the centroid times a
+// power series: the Gauss points of the 7-point rule lie on the lines from the centroid c to
+// the vertices, y - c = lambda (v_m - c), so with t_m = k xh.(y_{4+m} - c), t_0 + t_1 + t_2 = 0,
+//   sum_g W_g e^{-ik xh.(y_g - c)} = sum_n c_n (-i)^n P_n,  P_n = t_0^n + t_1^n + t_2^n,
+// where c_n = (W_1 rho^n + W_4) / n! (rho: ratio of the two orbits' lambda) and the power
+// sums obey P_n = m_2 P_{n-2} + e_3 P_{n-3} (Newton's identities without e_1).  Terms up to
+// n = 11 (|t| <= 0.232) or 17 (|t| <= 0.743) leave a remainder below 3e-17; longer panels
+// take six more sines and cosines.  Per pair about 80 FP64 instructions instead of about
+// 230: 6000 directions of 5120 panels 13.0 -> 5.6 ms on a GB300, one direction of 1280
+// panels 20 -> 9 us.
+//
+// Many directions (>= kFarMany): thread = direction, the panels of a chunk staged in shared
+// memory and read by broadcast, no reductions.  Few: thread = panel, one warp per 32 panels,
+// which spreads one direction over more SMs.  The lines' crossover is not critical: at 32
+// directions both take about the same time.  A second kernel adds the chunk sums.  Every
+// sum has a fixed order, so the result does not depend on what else runs on the GPU.
+constexpr int kFarChunk = 128;  // panels per chunk, thread = direction
+constexpr int kFarFew = 32;     // panels per chunk, thread = panel
+constexpr int kFarMany = 32;    // directions from which a thread takes a direction
+constexpr int kFarThreads = 128;
+constexpr double kFarT11 = 0.232, kFarT17 = 0.743;
 
 size_t far_field_scratch(int64_t n, int32_t ndir, int32_t nrhs) {
-  const int64_t chunks = (n + kFarChunk - 1) / kFarChunk;
+  const int64_t per = ndir >= kFarMany ? kFarChunk : kFarFew;
+  const int64_t chunks = (n + per - 1) / per;
   return (size_t)chunks * (size_t)ndir * (size_t)nrhs * 2 * sizeof(double);
 }
 
-__global__ void __launch_bounds__(kFarChunk) k_far_field(const WaveInst* __restrict__ insts) {
-  const WaveInst& W = insts[blockIdx.z];
-  const int64_t dr = blockIdx.x;
-  const int64_t chunk = blockIdx.y;
-  const int64_t nchunks = (W.n + kFarChunk - 1) / kFarChunk;
-  if (dr >= (int64_t)W.ndir * W.nrhs || chunk >= nchunks) return;
-  const int r = (int)(dr / W.ndir), d = (int)(dr % W.ndir);
-  const double* xh = W.dirs + 3 * ((int64_t)r * W.ndir + d);
-  const double k = W.k;
-  const double x0 = xh[0], x1 = xh[1], x2 = xh[2];
-  double ar = 0.0, ai = 0.0;
-  const int64_t j = chunk * kFarChunk + threadIdx.x;
-  if (j < W.n) {
-    const double* rec = W.panels + j * kPanelDoubles;
-    const int64_t o = 2 * (j + r * W.ldp);
-    const double pr = W.p[o], pi = W.p[o + 1];
-    const double qr = W.q[o], qi = W.q[o + 1];
-    const double kxn = k * (x0 * rec[3] + x1 * rec[4] + x2 * rec[5]);
-    // a = i kxn p + q
-    const double a_r = -kxn * pi + qr, a_i = kxn * pr + qi;
-    double sr = 0.0, si = 0.0;
+// c_n of the panel phase series, sign of (-i)^n included (even: real, odd: imaginary part)
+constexpr double far_coef(int n) {
+  // 1 - 3 b of the two orbits (b: the repeated barycentric coordinate)
+  constexpr double l1 = 1.0 - 3.0 * kRuleB[1][1], l2 = 1.0 - 3.0 * kRuleB[4][1];
+  double r = 1.0, f = 1.0;
+  for (int i = 1; i <= n; ++i) {
+    r *= l1 / l2;
+    f *= (double)i;
+  }
+  const double s = (n % 4 == 0 || n % 4 == 3) ? 1.0 : -1.0;
+  return s * (kRuleW[1] * r + kRuleW[4]) / f;
+}
+
+__constant__ double dFarCoef[18] = {
+    far_coef(0),  far_coef(1),  far_coef(2),  far_coef(3),  far_coef(4),  far_coef(5),
+    far_coef(6),  far_coef(7),  far_coef(8),  far_coef(9),  far_coef(10), far_coef(11),
+    far_coef(12), far_coef(13), far_coef(14), far_coef(15), far_coef(16), far_coef(17)};
+
+// One panel's values staged for all directions of a chunk (areas folded into p and q).
+struct FarPanel {
+  double c[3], n[3], e0[3], e1[3];  // k c, k n, k (y_4 - c), k (y_5 - c)
+  double pr, pi, qr, qi;
+};
+
+__device__ __forceinline__ void far_panel(const WaveInst& W, int r, int64_t j, FarPanel& F,
+                                          double& tmax) {
+  const double* rec = W.panels + j * kPanelDoubles;
+  const double k = W.k, area = rec[6];
+  double m[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int g = 0; g < 7; ++g) {
-      const double ph = -k * (x0 * rec[8 + 3 * g] + x1 * rec[9 + 3 * g] + x2 * rec[10 + 3 * g]);
-      double sn, cs;
-      sincos(ph, &sn, &cs);
-      sr += dRuleW[g] * cs;
-      si += dRuleW[g] * sn;
+  for (int a = 0; a < 3; ++a) {
+    F.c[a] = k * rec[a];
+    F.n[a] = k * rec[3 + a];
+    const double d0 = k * (rec[8 + 12 + a] - rec[a]), d1 = k * (rec[8 + 15 + a] - rec[a]);
+    F.e0[a] = d0;
+    F.e1[a] = d1;
+    m[0] += d0 * d0;
+    m[1] += d1 * d1;
+    m[2] += (d0 + d1) * (d0 + d1);
+  }
+  tmax = fmax(m[0], fmax(m[1], m[2]));  // squared bound of |t_m| over all directions
+  const int64_t o = 2 * (j + r * W.ldp);
+  F.pr = area * W.p[o];
+  F.pi = area * W.p[o + 1];
+  F.qr = area * W.q[o];
+  F.qi = area * W.q[o + 1];
+}
+
+// Adds the panel's contribution for the unit direction x; N: last term of the series, 0: by
+// sines and cosines.
+template <int N>
+__device__ __forceinline__ void far_add(const FarPanel& F, const double x[3], double& ar,
+                                        double& ai) {
+  const double ph = x[0] * F.c[0] + x[1] * F.c[1] + x[2] * F.c[2];
+  const double kxn = x[0] * F.n[0] + x[1] * F.n[1] + x[2] * F.n[2];
+  const double t0 = x[0] * F.e0[0] + x[1] * F.e0[1] + x[2] * F.e0[2];
+  const double t1 = x[0] * F.e1[0] + x[1] * F.e1[1] + x[2] * F.e1[2];
+  double fr = 1.0, fi = 0.0;
+  if (N > 0) {
+    const double s = t0 + t1, m2 = t0 * s + t1 * t1, e3 = -(t0 * t1) * s;
+    double pa = 0.0, pb = 2.0 * m2, pc = 3.0 * e3;  // P_{n-3}, P_{n-2}, P_{n-1} before n = 4
+    fr += dFarCoef[2] * pb;
+    fi += dFarCoef[3] * pc;
+#pragma unroll
+    for (int n = 4; n <= N; ++n) {
+      const double pn = n == 4 ? m2 * pb : m2 * pb + e3 * pa;
+      if (n % 2 == 0)
+        fr += dFarCoef[n] * pn;
+      else
+        fi += dFarCoef[n] * pn;
+      pa = pb;
+      pb = pc;
+      pc = pn;
     }
-    const double area = rec[6];
-    ar = area * (a_r * sr - a_i * si);
-    ai = area * (a_r * si + a_i * sr);
+  } else {
+    constexpr double rho = (1.0 - 3.0 * kRuleB[1][1]) / (1.0 - 3.0 * kRuleB[4][1]);
+    constexpr double w0 = kRuleW[0], w1 = kRuleW[1], w4 = kRuleW[4];
+    fr = w0;
+#pragma unroll 1
+    for (int m = 0; m < 3; ++m) {
+      const double t = m == 0 ? t0 : m == 1 ? t1 : -(t0 + t1);
+      double s1, c1, s2, c2;
+      sincos(rho * t, &s1, &c1);
+      sincos(t, &s2, &c2);
+      fr += w1 * c1 + w4 * c2;
+      fi -= w1 * s1 + w4 * s2;
+    }
+  }
+  double sn, cs;
+  sincos(ph, &sn, &cs);
+  // (i kxn p + q) f e^{-i ph}
+  const double br = F.qr - kxn * F.pi, bi = F.qi + kxn * F.pr;
+  const double gr = br * fr - bi * fi, gi = br * fi + bi * fr;
+  ar += gr * cs + gi * sn;
+  ai += gi * cs - gr * sn;
+}
+
+// thread = direction: grid (directions / 128, chunks, instance x rhs)
+__global__ void __launch_bounds__(kFarThreads) k_far_field_many(WaveInst w0,
+                                                                const WaveInst* insts,
+                                                                int max_rhs) {
+  const WaveInst& W = insts ? insts[blockIdx.z / max_rhs] : w0;
+  const int r = (int)(blockIdx.z % max_rhs);
+  const int64_t nchunks = (W.n + kFarChunk - 1) / kFarChunk, chunk = blockIdx.y;
+  const int64_t d0 = (int64_t)blockIdx.x * kFarThreads;
+  if (r >= W.nrhs || chunk >= nchunks || d0 >= W.ndir) return;  // uniform over the CTA
+  __shared__ FarPanel sp[kFarChunk];
+  const int64_t j0 = chunk * kFarChunk;
+  const int cnt = (int)min((int64_t)kFarChunk, W.n - j0);
+  double tm = 0.0;
+  if (threadIdx.x < cnt) far_panel(W, r, j0 + threadIdx.x, sp[threadIdx.x], tm);
+  const bool over11 = __syncthreads_or(!(tm <= kFarT11 * kFarT11));
+  const bool over17 = __syncthreads_or(!(tm <= kFarT17 * kFarT17));
+  const int64_t d = d0 + threadIdx.x;
+  if (d >= W.ndir) return;
+  const double* xh = W.dirs + 3 * ((int64_t)r * W.ndir + d);
+  const double x[3] = {xh[0], xh[1], xh[2]};
+  double ar = 0.0, ai = 0.0;
+  if (!over11)
+    for (int j = 0; j < cnt; ++j) far_add<11>(sp[j], x, ar, ai);
+  else if (!over17)
+    for (int j = 0; j < cnt; ++j) far_add<17>(sp[j], x, ar, ai);
+  else
+    for (int j = 0; j < cnt; ++j) far_add<0>(sp[j], x, ar, ai);
+  double* o = W.part + 2 * (((int64_t)r * W.ndir + d) * nchunks + chunk);
+  o[0] = ar;
+  o[1] = ai;
+}
+
+// thread = panel: grid (direction x rhs, groups of 4 chunks, instance), a warp per chunk
+__global__ void __launch_bounds__(kFarThreads) k_far_field_few(WaveInst w0,
+                                                               const WaveInst* insts) {
+  const WaveInst& W = insts ? insts[blockIdx.z] : w0;
+  const int64_t dr = blockIdx.x;
+  const int64_t nchunks = (W.n + kFarFew - 1) / kFarFew;
+  const int64_t chunk = (int64_t)blockIdx.y * (kFarThreads / 32) + (threadIdx.x >> 5);
+  if (dr >= (int64_t)W.ndir * W.nrhs || chunk >= nchunks) return;  // uniform per warp
+  const int r = (int)(dr / W.ndir);
+  const double* xh = W.dirs ? W.dirs + 3 * dr : W.dir1;
+  const double x[3] = {xh[0], xh[1], xh[2]};
+  const int lane = threadIdx.x & 31;
+  const int64_t j = chunk * kFarFew + lane;
+  double ar = 0.0, ai = 0.0, tm = 0.0;
+  FarPanel F;
+  if (j < W.n) far_panel(W, r, j, F, tm);
+  const bool over11 = __any_sync(0xffffffffu, !(tm <= kFarT11 * kFarT11));
+  const bool over17 = __any_sync(0xffffffffu, !(tm <= kFarT17 * kFarT17));
+  if (j < W.n) {
+    if (!over11)
+      far_add<11>(F, x, ar, ai);
+    else if (!over17)
+      far_add<17>(F, x, ar, ai);
+    else
+      far_add<0>(F, x, ar, ai);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     ar += __shfl_down_sync(0xffffffffu, ar, off);
     ai += __shfl_down_sync(0xffffffffu, ai, off);
   }
-  __shared__ double red[2][kFarChunk / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) {
-    red[0][wid] = ar;
-    red[1][wid] = ai;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tr = 0.0, ti = 0.0;
-    for (int w = 0; w < kFarChunk / 32; ++w) {
-      tr += red[0][w];
-      ti += red[1][w];
-    }
     double* o = W.part + 2 * (dr * nchunks + chunk);
-    o[0] = tr;
-    o[1] = ti;
+    o[0] = ar;
+    o[1] = ai;
   }
 }
 
-__global__ void k_far_field_finish(const WaveInst* __restrict__ insts) {
-  const WaveInst& W = insts[blockIdx.z];
-  const int64_t dr = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// one warp per (direction, rhs): its chunk sums, lane-strided, then a shuffle tree
+__global__ void __launch_bounds__(kFarThreads) k_far_field_finish(WaveInst w0,
+                                                                  const WaveInst* insts, int per) {
+  const WaveInst& W = insts ? insts[blockIdx.z] : w0;
+  const int64_t dr = (int64_t)blockIdx.x * (kFarThreads / 32) + (threadIdx.x >> 5);
   if (dr >= (int64_t)W.ndir * W.nrhs) return;
-  const int64_t nchunks = (W.n + kFarChunk - 1) / kFarChunk;
+  const int64_t nchunks = (W.n + per - 1) / per;
+  const double2* part = reinterpret_cast<const double2*>(W.part) + dr * nchunks;
   double tr = 0.0, ti = 0.0;
-  for (int64_t c = 0; c < nchunks; ++c) {
-    tr += W.part[2 * (dr * nchunks + c)];
-    ti += W.part[2 * (dr * nchunks + c) + 1];
+  for (int64_t c = threadIdx.x & 31; c < nchunks; c += 32) {
+    const double2 v = part[c];
+    tr += v.x;
+    ti += v.y;
   }
-  W.out[2 * dr] = -tr * kInv4Pi;
-  W.out[2 * dr + 1] = -ti * kInv4Pi;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    tr += __shfl_down_sync(0xffffffffu, tr, off);
+    ti += __shfl_down_sync(0xffffffffu, ti, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    W.out[2 * dr] = -tr * kInv4Pi;
+    W.out[2 * dr + 1] = -ti * kInv4Pi;
+  }
+}
+
+static void far_field(const Launch& L, const WaveInst& w0, const WaveInst* d_inst, int ninst,
+                      int32_t max_rhs, int32_t max_dirs, int64_t max_n) {
+  if (ninst <= 0 || max_dirs <= 0 || max_rhs <= 0 || max_n <= 0) return;
+  const int64_t dr = (int64_t)max_dirs * max_rhs;
+  const bool many = max_dirs >= kFarMany;
+  const int per = many ? kFarChunk : kFarFew;
+  const int64_t chunks = (max_n + per - 1) / per;
+  if (many)
+    k_far_field_many<<<dim3((unsigned)((max_dirs + kFarThreads - 1) / kFarThreads),
+                            (unsigned)chunks, (unsigned)(ninst * max_rhs)),
+                       kFarThreads, 0, L.stream>>>(w0, d_inst, max_rhs);
+  else
+    k_far_field_few<<<dim3((unsigned)dr, (unsigned)((chunks + 3) / 4), (unsigned)ninst),
+                      kFarThreads, 0, L.stream>>>(w0, d_inst);
+  k_far_field_finish<<<dim3((unsigned)((dr + 3) / 4), 1, (unsigned)ninst), kFarThreads, 0,
+                       L.stream>>>(w0, d_inst, per);
+  count_launch(2);
 }
 
 void launch_far_field(const Launch& L, const WaveInst* d_inst, int ninst, int32_t max_rhs,
                       int32_t max_dirs, int64_t max_n) {
-  if (ninst <= 0 || max_dirs <= 0 || max_rhs <= 0 || max_n <= 0) return;
-  const int64_t dr = (int64_t)max_dirs * max_rhs;
-  dim3 grid((unsigned)dr, (unsigned)((max_n + kFarChunk - 1) / kFarChunk), (unsigned)ninst);
-  k_far_field<<<grid, kFarChunk, 0, L.stream>>>(d_inst);
-  k_far_field_finish<<<dim3((unsigned)((dr + 127) / 128), 1, (unsigned)ninst), 128, 0, L.stream>>>(
-      d_inst);
-  count_launch(2);
+  far_field(L, WaveInst{}, d_inst, ninst, max_rhs, max_dirs, max_n);
+}
+
+void launch_far_field_one(const Launch& L, const WaveInst& w) {
+  far_field(L, w, nullptr, 1, w.nrhs, w.ndir, w.n);
 }
 
 }  // namespace bemgpu

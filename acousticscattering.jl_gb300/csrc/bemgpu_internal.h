@@ -127,9 +127,11 @@ struct WaveInst {
   double* out;             // complex128 results
   int64_t ldp;             // leading dimension of p / q
   double* part;            // far field: per-chunk partial sums (far_field_scratch bytes)
+  double dir1[3];          // far field: the direction when dirs is null (ndir = nrhs = 1)
 };
 
-// bytes of WaveInst.part for a far-field launch over n panels, ndir directions, nrhs
+// bytes of WaveInst.part for a far-field launch over n panels, ndir directions, nrhs; the
+// instances of one launch agree on ndir
 size_t far_field_scratch(int64_t n, int32_t ndir, int32_t nrhs);
 
 // Dense-matrix instance for the batched factor / solve kernels.
@@ -222,6 +224,8 @@ void launch_incident(const Launch& L, const WaveInst* d_inst, int ninst, int64_t
                      int32_t max_rhs);
 void launch_far_field(const Launch& L, const WaveInst* d_inst, int ninst, int32_t max_rhs,
                       int32_t max_dirs, int64_t max_n);
+// one instance, its descriptor passed by value
+void launch_far_field_one(const Launch& L, const WaveInst& w);
 #endif
 
 }  // namespace bemgpu
