@@ -28,6 +28,7 @@
 #include "nystrom.cuh"
 #include "refine.cuh"
 #include "condition.cuh"
+#include "gemm_oz.cuh"
 #include "gemm_tc.cuh"
 #include "hmatrix.cuh"
 #include "hmatrix_plan.h"
@@ -1664,6 +1665,123 @@ int getrf_tc(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<MatI
   return BEMGPU_OK;
 }
 
+// Complex128 LU in 128-column blocks of four 32-column SIMT panels; the updates inside a
+// block (K = 32), the U12 solve (through -(L11^{-1} - I)) and the trailing update (K = 128)
+// run on the tensor cores from integer digit slices (gemm_oz.cu).
+int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax) {
+  const Launch L = c->launch();
+  const int ni = (int)mi.size();
+  constexpr int B = kOzK;
+  constexpr int kInner = B / kPanelNB - 1;  // panels of a block with columns to their right
+  std::vector<Buf> apack(ni), bpack(ni), npack(ni), negn(ni), aexp(ni), bexp(ni), nexp(ni);
+  std::vector<double2*> np(ni);
+  for (int t = 0; t < ni; ++t) {
+    const int64_t n = mi[t].n;
+    TRY(alloc(c, oz_pack_bytes(n, B, kOzA), &apack[t]));
+    TRY(alloc(c, oz_pack_bytes(n, B, kOzB), &bpack[t]));
+    TRY(alloc(c, oz_pack_bytes(B, B, kOzA), &npack[t]));
+    TRY(alloc(c, (size_t)B * B * 16, &negn[t]));
+    TRY(alloc(c, oz_exps(n, kOzA) * 4, &aexp[t]));
+    TRY(alloc(c, oz_exps(n, kOzB) * 4, &bexp[t]));
+    TRY(alloc(c, oz_exps(B, kOzA) * 4, &nexp[t]));
+    np[t] = negn[t].as<double2>();
+  }
+  // descriptors of every update, uploaded once: per block and inner panel, then the U12
+  // solve and the trailing update
+  enum { kU12 = kInner, kTrail, kPhases };
+  const int64_t blocks = (nmax + B - 1) / B;
+  const size_t count = (size_t)blocks * kPhases * ni;
+  std::vector<OzPackInst> pa(count), pb(count);
+  std::vector<OzGemmInst> ge(count);
+  std::vector<int64_t> tiles(count), ra((size_t)blocks * kPhases, 0), rb((size_t)blocks * kPhases, 0);
+  for (int64_t b = 0; b < blocks; ++b)
+    for (int ph = 0; ph < kPhases; ++ph)
+      for (int t = 0; t < ni; ++t) {
+        const int64_t n = mi[t].n, K0 = b * B, end = std::min<int64_t>(K0 + B, n);
+        // K range [k0, k0 + kk), rows [r0, r1) and columns [c0, c1) of the update
+        int64_t k0 = K0, r0 = end, r1 = n, c0 = end, c1 = n;
+        int kk = (int)std::max<int64_t>(0, end - K0);
+        if (ph < kInner) {
+          k0 = K0 + (int64_t)ph * kPanelNB;
+          kk = kPanelNB;
+          r0 = c0 = k0 + kPanelNB;
+          c1 = end;
+        } else if (ph == kU12) {
+          r0 = K0;
+          r1 = end;
+        }
+        const bool on = kk > 0 && r1 > r0 && c1 > c0;
+        const size_t q = ((size_t)b * kPhases + ph) * ni + t;
+        const bool u12 = ph == kU12;
+        OzPackInst& a = pa[q];
+        a = OzPackInst{u12 ? negn[t].p : mi[t].a, u12 ? (int64_t)B : mi[t].lda, u12 ? 0 : r0,
+                       u12 ? 0 : k0, on ? r1 - r0 : 0, on ? kk : 0, 0,
+                       u12 ? npack[t].p : apack[t].p,
+                       u12 ? nexp[t].as<int32_t>() : aexp[t].as<int32_t>()};
+        pb[q] = OzPackInst{mi[t].a, mi[t].lda, c0, k0, on ? c1 - c0 : 0, on ? kk : 0, 0,
+                           bpack[t].p, bexp[t].as<int32_t>()};
+        ge[q] = OzGemmInst{a.out, bpack[t].p, a.exps, bexp[t].as<int32_t>(), mi[t].a, mi[t].lda,
+                           r0, c0, on ? r1 - r0 : 0, on ? c1 - c0 : 0, on ? kk : 0, 0};
+        tiles[q] = on ? oz_tiles(r1 - r0, c1 - c0) : 0;
+        int64_t& ma = ra[(size_t)b * kPhases + ph];
+        int64_t& mb = rb[(size_t)b * kPhases + ph];
+        ma = std::max(ma, a.rows);
+        mb = std::max(mb, pb[q].rows);
+      }
+  Buf dpa, dpb, dge, dnp;
+  TRY(to_device(c, pa, &dpa));
+  TRY(to_device(c, pb, &dpb));
+  TRY(to_device(c, ge, &dge));
+  TRY(to_device(c, np, &dnp));
+  const MatInst* dm = d.as<MatInst>();
+  auto update = [&](int64_t b, int ph) {
+    const size_t q = (size_t)b * kPhases + ph;
+    if (ra[q] <= 0 || rb[q] <= 0) return;
+    {
+      Prof pr(c, "oz_pack");
+      launch_oz_pack(L, dpa.as<OzPackInst>() + q * ni, ni, ra[q], kOzA);
+      launch_oz_pack(L, dpb.as<OzPackInst>() + q * ni, ni, rb[q], kOzB);
+    }
+    Prof pr(c, ph == kTrail ? "gemm_c128" : "gemm_oz");
+    launch_oz_gemm(L, dge.as<OzGemmInst>() + q * ni, ni, &tiles[q * ni]);
+  };
+  for (int64_t b = 0; b < blocks; ++b) {
+    const int64_t K0 = b * B, K1 = K0 + B;
+    for (int q = 0; q <= kInner; ++q) {
+      const int64_t k0 = K0 + (int64_t)q * kPanelNB;
+      if (k0 >= nmax) break;
+      {
+        Prof pr(c, "getf2");
+        launch_getf2(L, dm, ni, k0, kPanelNB, 0);
+      }
+      {
+        Prof pr(c, "laswp");
+        launch_laswp(L, dm, ni, k0, kPanelNB, K0, K1, k0, k0 + kPanelNB, 0);
+      }
+      if (q == kInner) break;
+      {
+        Prof pr(c, "trsm");
+        launch_trsm_panel(L, dm, ni, k0, kPanelNB, k0 + kPanelNB, K1, 0);
+      }
+      update(b, q);
+    }
+    {
+      Prof pr(c, "laswp");
+      launch_laswp(L, dm, ni, K0, B, 0, nmax, K0, K1, 0);
+    }
+    if (ra[(size_t)b * kPhases + kTrail] <= 0) continue;
+    {
+      Prof pr(c, "trsm");
+      launch_linv_neg_c128(L, dm, ni, K0, dnp.as<double2* const>());
+    }
+    update(b, kU12);
+    update(b, kTrail);
+  }
+  CUDA_TRY(c, cudaGetLastError());
+  TRY(check_device_error(c));
+  return BEMGPU_OK;
+}
+
 // LU of a batch of same-precision factors (prec 1: complex64 in LU, 0: complex128).
 int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool promoted) {
   if (fs.empty()) return BEMGPU_OK;
@@ -1690,6 +1808,8 @@ int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool prom
   TRY(to_device(c, mi, &d));
   if (prec == 1 && c->tensor_lu) {
     TRY(getrf_tc(c, fs, mi, d, nmax));
+  } else if (prec == 0 && c->tensor_lu) {
+    TRY(getrf_oz(c, mi, d, nmax));
   } else {
     // right-looking blocked LU, 32-column panels; each kernel family timed on its own
     const MatInst* dm = d.as<MatInst>();

@@ -490,12 +490,13 @@ __global__ void __launch_bounds__(kSwpWarps * 32) k_laswp(const MatInst* __restr
 // U12 = L11^{-1} A12 for the columns [c_lo, min(c_hi, n)); L11 = unit lower nbe x nbe
 // block at (k0, k0), staged once per CTA in shared memory; each warp solves TrsmCols<R>
 // columns (column = warp + kTrsmWarps * t), lane r holding rows r, r + 32, ...
-// complex128 takes fewer columns per warp: its FP64 solve is about 8x slower per column,
-// and more CTAs spread the few trailing columns of small orders over the SMs.
+// complex128 takes one column per warp: it solves the at most 96 columns to the right of a
+// 32-column panel inside a 128-column block, 8 per CTA, so that the FP64 work (two FMAs per
+// clock and SM) spreads over a dozen SMs.
 constexpr int kTrsmWarps = 8;
 template <typename R>
 struct TrsmCols {
-  static constexpr int value = sizeof(R) == 4 ? 16 : 2;
+  static constexpr int value = sizeof(R) == 4 ? 16 : 1;
 };
 
 template <typename R, int NB>
@@ -885,6 +886,71 @@ void launch_linv_neg(const Launch& L, const MatInst* d, int ninst, int64_t k0, f
     cudaFuncSetAttribute(k_linv_neg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   k_linv_neg<<<ninst, 256, smem, L.stream>>>(d, k0, outs);
+  count_launch(1);
+}
+
+// The same for complex128 factors (out: complex128): the strict lower triangle of L11 packed
+// by columns in shared memory (127 KB), one warp per column of the inverse, the columns of a
+// CTA spread over the triangle for balance.  Bound by FP64 issue and the 128 dependent steps
+// of a column: about 10 us with kLinvCtas CTAs per instance, against 0.4 ms with one.
+constexpr int kLinvCtas = 32;
+__global__ void __launch_bounds__(kLinvB / kLinvCtas * 32) k_linv_neg_c128(
+    const MatInst* __restrict__ insts, int64_t k0, double2* const* outs) {
+  const MatInst& M = insts[blockIdx.y];
+  const int64_t n = M.n;
+  if (!M.active || k0 >= n) return;
+  const int nbe = (int)min((int64_t)kLinvB, n - k0);
+  const int64_t lda = M.lda;
+  extern __shared__ __align__(16) unsigned char linv_smem[];
+  cx<double>* sL = reinterpret_cast<cx<double>*>(linv_smem);
+  // column c: rows c + 1 .. kLinvB - 1 at c (2 kLinvB - c - 1) / 2
+  auto at = [](int r, int c) { return c * (2 * kLinvB - c - 1) / 2 + r - c - 1; };
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  constexpr int kWarps = kLinvB / kLinvCtas;
+  for (int c = wid; c < nbe; c += kWarps)
+    for (int r = c + 1 + lane; r < nbe; r += 32) sL[at(r, c)] = ld<double>(M.a, (k0 + r) + (k0 + c) * lda);
+  __syncthreads();
+  const int j = blockIdx.x + kLinvCtas * wid;
+  constexpr int kPer = kLinvB / 32;
+  cx<double> x[kPer];
+#pragma unroll
+  for (int t = 0; t < kPer; ++t) x[t] = cx<double>{lane + 32 * t == j ? 1.0 : 0.0, 0.0};
+  if (j < nbe) {
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      for (int cl = 0; cl < 32; ++cl) {
+        const int c = 32 * t + cl;
+        if (c >= nbe) break;
+        if (c < j) continue;
+        cx<double> xc;
+        xc.x = __shfl_sync(0xffffffffu, x[t].x, cl);
+        xc.y = __shfl_sync(0xffffffffu, x[t].y, cl);
+#pragma unroll
+        for (int u = t; u < kPer; ++u) {
+          const int r = lane + 32 * u;
+          if (r > c && r < nbe) x[u] -= sL[at(r, c)] * xc;
+        }
+      }
+    }
+  }
+  double2* out = outs[blockIdx.y];
+#pragma unroll
+  for (int t = 0; t < kPer; ++t) {
+    const int r = lane + 32 * t;
+    const bool strict = r > j && r < nbe && j < nbe;
+    out[r + (int64_t)j * kLinvB] = strict ? make_double2(-x[t].x, -x[t].y) : make_double2(0.0, 0.0);
+  }
+}
+
+void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t k0,
+                          double2* const* outs) {
+  const size_t smem = (size_t)kLinvB * (kLinvB - 1) / 2 * sizeof(cx<double>);
+  static PerDeviceOnce attr;
+  attr.call([&] {
+    cudaFuncSetAttribute(k_linv_neg_c128, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
+  k_linv_neg_c128<<<dim3(kLinvCtas, (unsigned)ninst), kLinvB / kLinvCtas * 32, smem, L.stream>>>(
+      d, k0, outs);
   count_launch(1);
 }
 

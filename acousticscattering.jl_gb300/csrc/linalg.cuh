@@ -32,6 +32,9 @@ void launch_getrs(const Launch& L, const MatInst* d, int ninst, int64_t nmax, in
 // out[i] (kLinvB x kLinvB complex64, column-major) = -(L11^{-1} - I) of the unit lower
 // block at (k0, k0) of instance i (complex64 factors).
 void launch_linv_neg(const Launch& L, const MatInst* d, int ninst, int64_t k0, float2* const* outs);
+// The same for complex128 factors.
+void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t k0,
+                          double2* const* outs);
 // Row permutation of each factor from its pivots (one CTA per instance).
 void launch_make_perm(const Launch& L, const MatInst* d, int ninst, int64_t nmax);
 
