@@ -1269,6 +1269,18 @@ int estimate_rcond(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
 //   P5: U12bot = L11b^{-1} A12bot            P6: A22 -= L21 U12 (K = kk0 + kk1)
 }  // namespace
 
+// Factors the 32-column panel at k0; returns the end of the columns [k0, .) whose
+// interchanges it has applied itself (k0: none).
+namespace {
+int64_t panel(bemgpu_ctx* c, const Launch& L, const std::vector<MatInst>& mi, const MatInst* dm,
+              int64_t nmax, int64_t k0, int prec) {
+  int nact = 0;
+  for (const MatInst& m : mi) nact += m.n > k0;
+  Prof pr(c, "getf2");
+  return launch_getf2(L, dm, (int)mi.size(), nact, nmax, k0, kPanelNB, prec) ? k0 + kPanelNB : k0;
+}
+}  // namespace
+
 // A captured launch sequence of the tensor-core LU for one exact batch shape, with the
 // descriptor arrays its kernels take as arguments (rewritten before every replay).
 struct LuGraph {
@@ -1552,17 +1564,10 @@ int getrf_tc(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<MatI
     const int64_t st = H / SB;
     const int h = (int)((H % SB) / HB);
     for (int64_t k0 = H; k0 < H + HB && k0 < nmax; k0 += kPanelNB) {
-      {
-        // cluster size by the batch-size rule: timing the candidates on the first panels
-        // of a shape class (in place, in the order 2 4 8 8 4 2 to cancel the panels' work
-        // trend) chose sizes that were slower over the whole batch (184 vs 132 ms of
-        // panels per 64 x 10240 factorisation), as did timing them on scratch copies
-        Prof pr(c, "getf2");
-        launch_getf2(L, dm, ni, k0, kPanelNB, 1, 0);
-      }
+      const int64_t skip = panel(c, L, mi, dm, nmax, k0, 1);
       {
         Prof pr(c, "laswp");
-        launch_laswp(L, dm, ni, k0, kPanelNB, H, H + HB, k0, k0 + kPanelNB, 1);
+        launch_laswp(L, dm, ni, k0, kPanelNB, H, H + HB, k0, skip, 1);
       }
       {
         Prof pr(c, "trsm");
@@ -1750,13 +1755,10 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
     for (int q = 0; q <= kInner; ++q) {
       const int64_t k0 = K0 + (int64_t)q * kPanelNB;
       if (k0 >= nmax) break;
-      {
-        Prof pr(c, "getf2");
-        launch_getf2(L, dm, ni, k0, kPanelNB, 0);
-      }
+      const int64_t skip = panel(c, L, mi, dm, nmax, k0, 0);
       {
         Prof pr(c, "laswp");
-        launch_laswp(L, dm, ni, k0, kPanelNB, K0, K1, k0, k0 + kPanelNB, 0);
+        launch_laswp(L, dm, ni, k0, kPanelNB, K0, K1, k0, skip, 0);
       }
       if (q == kInner) break;
       {
@@ -1815,13 +1817,10 @@ int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool prom
     const MatInst* dm = d.as<MatInst>();
     const int ni = (int)fs.size();
     for (int64_t k0 = 0; k0 < nmax; k0 += kPanelNB) {
-      {
-        Prof pr(c, "getf2");
-        launch_getf2(L, dm, ni, k0, kPanelNB, prec);
-      }
+      const int64_t skip = panel(c, L, mi, dm, nmax, k0, prec);
       {
         Prof pr(c, "laswp");
-        launch_laswp(L, dm, ni, k0, kPanelNB, 0, nmax, k0, k0 + kPanelNB, prec);
+        launch_laswp(L, dm, ni, k0, kPanelNB, 0, nmax, k0, skip, prec);
       }
       {
         Prof pr(c, "trsm");

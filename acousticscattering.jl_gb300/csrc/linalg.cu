@@ -7,7 +7,7 @@
 //
 // LU: right-looking blocked partial pivoting (LAPACK zgetrf semantics: pivot = first
 // row of largest |re| + |im| in the column, P A = L U with unit lower L):
-//   getf2   panel of kPanelNB columns, one CTA per instance, column by column;
+//   getf2   panel of kPanelNB columns, one thread-block cluster per instance;
 //   laswp   the panel's row interchanges applied to the columns outside it;
 //   trsm    U12 = L11^{-1} A12, one warp per column of A12;
 //   gemm    A22 -= L21 U12 (SIMT tile kernel; the complex64 factor of the mixed path
@@ -57,118 +57,6 @@ __device__ __forceinline__ cx<R> cinv(cx<R> a) {
 template <typename R>
 __device__ __forceinline__ cx<R> cconj(cx<R> a) {
   return {a.x, -a.y};
-}
-
-// ------------------------------------------------------------------ getf2 (panel)
-// One CTA per instance factors the nbe-column panel at k0 column by column.  The panel
-// lives in global memory (L2); every pass issues independent loads in groups (4 rows
-// in the pivot search, 8 columns in the update) before any dependent store, so each
-// thread keeps several requests in flight.
-template <typename R>
-struct Getf2Cfg;
-template <>
-struct Getf2Cfg<float> {
-  static constexpr int kThreads = 1024;
-};
-template <>
-struct Getf2Cfg<double> {
-  static constexpr int kThreads = 512;
-};
-
-template <typename R>
-__global__ void __launch_bounds__(Getf2Cfg<R>::kThreads) k_getf2(const MatInst* __restrict__ insts,
-                                                                int64_t k0, int nb) {
-  constexpr int T = Getf2Cfg<R>::kThreads;
-  const MatInst& M = insts[blockIdx.x];
-  const int64_t n = M.n;
-  if (!M.active || k0 >= n) return;
-  const int nbe = (int)min((int64_t)nb, n - k0);
-  const int64_t lda = M.lda;
-  void* A = M.a;
-  __shared__ R s_val[T / 32];
-  __shared__ int64_t s_idx[T / 32];
-  __shared__ cx<R> s_u[kPanelNB];
-  __shared__ int64_t s_piv;
-  __shared__ R s_pmax;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (int c = 0; c < nbe; ++c) {
-    const int64_t col = k0 + c;
-    const void* colp = static_cast<const cx<R>*>(A) + col * lda;
-    // pivot search: largest |re|+|im|, first index on ties
-    R best = (R)-1;
-    int64_t bidx = col;
-    for (int64_t r = col + tid; r < n; r += 4 * T) {
-      R v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t rr = r + (int64_t)u * T;
-        v[u] = rr < n ? cabs1(ld<R>(colp, rr)) : (R)-1;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (v[u] > best) {
-          best = v[u];
-          bidx = r + (int64_t)u * T;
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      R ov = __shfl_down_sync(0xffffffffu, best, off);
-      int64_t oi = __shfl_down_sync(0xffffffffu, bidx, off);
-      if (ov > best || (ov == best && oi < bidx)) {
-        best = ov;
-        bidx = oi;
-      }
-    }
-    if (lane == 0) {
-      s_val[wid] = best;
-      s_idx[wid] = bidx;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      R bv = s_val[0];
-      int64_t bi = s_idx[0];
-      for (int w = 1; w < T / 32; ++w)
-        if (s_val[w] > bv || (s_val[w] == bv && s_idx[w] < bi)) {
-          bv = s_val[w];
-          bi = s_idx[w];
-        }
-      s_piv = bi;
-      s_pmax = bv;
-      M.ipiv[col] = (int32_t)bi;
-      if (!(bv > (R)0) && *M.info == 0) *M.info = (int32_t)(col + 1);
-    }
-    __syncthreads();
-    const int64_t piv = s_piv;
-    const bool nonzero = s_pmax > (R)0;
-    if (nonzero && piv != col && tid < nbe) {
-      const int64_t cc = k0 + tid;
-      cx<R> a = ld<R>(A, col + cc * lda), b = ld<R>(A, piv + cc * lda);
-      st<R>(A, col + cc * lda, b);
-      st<R>(A, piv + cc * lda, a);
-    }
-    __syncthreads();
-    if (tid < nbe) s_u[tid] = ld<R>(A, col + (k0 + tid) * lda);
-    __syncthreads();
-    const cx<R> inv = nonzero ? cinv(s_u[c]) : cx<R>{(R)1, (R)0};
-    for (int64_t r = col + 1 + tid; r < n; r += T) {
-      cx<R> l = ld<R>(A, r + col * lda);
-      if (nonzero) {
-        l = l * inv;
-        st<R>(A, r + col * lda, l);
-      }
-      for (int cc0 = c + 1; cc0 < nbe; cc0 += 8) {
-        cx<R> a[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (cc0 + e < nbe) a[e] = ld<R>(A, r + (k0 + cc0 + e) * lda);
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (cc0 + e < nbe) st<R>(A, r + (k0 + cc0 + e) * lda, a[e] - l * s_u[cc0 + e]);
-      }
-    }
-    __syncthreads();
-  }
 }
 
 // ------------------------------------------------------------------ getf2, left-looking
@@ -388,6 +276,283 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
   int64_t r = k0 + g;
   if (r <= colL) r += ((colL + 1 - r + stride - 1) / stride) * stride;
   for (; r < n; r += stride) st<R>(A, r + colL * lda, ld<R>(A, r + colL * lda) * inv_prev);
+}
+
+// ------------------------------------------------------------------ getf2, in registers
+// The panel factorisation of both precisions up to kRegRows rows per thread: a cluster of
+// CTAs holds the panel's rows in registers, W columns at a time (a sub-panel), and never
+// moves them: a row keeps its place and remembers its position under the interchanges
+// (implicit pivoting; the launcher's caller applies the interchanges to the panel's columns
+// with everybody else's).  Bound by the latency of a column step, so a step has one CTA
+// barrier and one cluster barrier: the CTA's candidate (value, position, reciprocal and the
+// row's remaining entries) is pushed by its owner's warp into every CTA's shared memory
+// before the cluster barrier, after which each CTA picks the winner among the copies it
+// holds and updates its rows from registers.  Sub-panels are left-looking: the rows' finished
+// L values come back from global memory (L2) and the pivot rows' U values are solved by every
+// CTA.  Every entry takes its updates a -= l_j u_j one by one in the order of j with the same
+// four FMAs whatever W, the cluster size and the rows per thread, so factors do not depend
+// on the batch.  Measured, one instance of 8960 unknowns, complex64: 7.0 us a column with the
+// streaming kernel above, see the launcher for this one's; complex128 (FP64 issue: two FMAs
+// per clock and SM beside the latency) of 5760 unknowns: 27 us a column before.
+constexpr int kRegT = 512;      // threads per CTA at most
+constexpr int kRegMaxCS = 16;   // CTAs per cluster at most
+
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void st_peer_b32(uint32_t a, uint32_t v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// x -= a b, the one form every kernel path of the panel uses
+__device__ __forceinline__ void cfnma(cx<float>& x, cx<float> a, cx<float> b) {
+  x.x = __fmaf_rn(a.y, b.y, __fmaf_rn(-a.x, b.x, x.x));
+  x.y = __fmaf_rn(-a.y, b.x, __fmaf_rn(-a.x, b.y, x.y));
+}
+__device__ __forceinline__ void cfnma(cx<double>& x, cx<double> a, cx<double> b) {
+  x.x = __fma_rn(a.y, b.y, __fma_rn(-a.x, b.x, x.x));
+  x.y = __fma_rn(-a.y, b.x, __fma_rn(-a.x, b.y, x.y));
+}
+// reciprocal with one division: scaled by a power of two so that the squares neither
+// overflow nor vanish
+__device__ __forceinline__ cx<double> cinv_fast(cx<double> a) {
+  const int e = (max(__double2hiint(a.x) & 0x7FFFFFFF, __double2hiint(a.y) & 0x7FFFFFFF)) >> 20;
+  if (e < 2 || e > 2044) return cinv(a);
+  const double sc = __hiloint2double((2046 - e) << 20, 0);
+  const double x = a.x * sc, y = a.y * sc;
+  const double q = sc / (x * x + y * y);
+  return {x * q, -y * q};
+}
+__device__ __forceinline__ cx<float> cinv_fast(cx<float> a) { return cinv(a); }
+
+// Ordered key of a pivot candidate: |re| + |im| as bits, 0 for a NaN (never a candidate).
+struct PivKey {
+  uint32_t hi, lo;   // value bits (lo: 0 for complex64)
+  int32_t pos;       // position under the interchanges, INT32_MAX: no candidate
+  int32_t phys;      // row
+};
+__device__ __forceinline__ void key_of(cx<float> a, uint32_t& hi, uint32_t& lo) {
+  hi = __float_as_uint(cabs1(a));
+  lo = 0u;
+}
+__device__ __forceinline__ void key_of(cx<double> a, uint32_t& hi, uint32_t& lo) {
+  const double v = cabs1(a);
+  hi = (uint32_t)__double2hiint(v);
+  lo = (uint32_t)__double2loint(v);
+}
+__device__ __forceinline__ bool key_nan(const PivKey& k, float) { return k.hi > 0x7F800000u; }
+__device__ __forceinline__ bool key_nan(const PivKey& k, double) {
+  return k.hi > 0x7FF00000u || (k.hi == 0x7FF00000u && k.lo != 0u);
+}
+__device__ __forceinline__ bool key_better(const PivKey& a, const PivKey& b) {
+  if (a.pos == INT32_MAX) return false;
+  if (b.pos == INT32_MAX) return true;
+  if (a.hi != b.hi) return a.hi > b.hi;
+  if (a.lo != b.lo) return a.lo > b.lo;
+  return a.pos < b.pos;
+}
+// best candidate of a warp, in every lane; returns the lane that holds it (-1: none)
+template <typename R>
+__device__ __forceinline__ int warp_best(PivKey& k) {
+  const bool cand = k.pos != INT32_MAX;
+  const uint32_t any = __ballot_sync(0xffffffffu, cand);
+  if (!any) return -1;
+  uint32_t h = cand ? k.hi : 0u;
+  const uint32_t mh = __reduce_max_sync(0xffffffffu, h);
+  bool in = cand && k.hi == mh;
+  if (sizeof(R) == 8) {
+    const uint32_t ml = __reduce_max_sync(0xffffffffu, in ? k.lo : 0u);
+    in = in && k.lo == ml;
+    k.lo = ml;
+  }
+  k.hi = mh;
+  const int32_t mp = __reduce_min_sync(0xffffffffu, in ? k.pos : INT32_MAX);
+  const int src = __ffs(__ballot_sync(0xffffffffu, in && k.pos == mp)) - 1;
+  k.pos = mp;
+  k.phys = __shfl_sync(0xffffffffu, k.phys, src);
+  return src;
+}
+__device__ __forceinline__ cx<float> shfl_c(cx<float> v, int src) {
+  return {__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
+}
+__device__ __forceinline__ cx<double> shfl_c(cx<double> v, int src) {
+  return {__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
+}
+__device__ __forceinline__ void st_peer_c(uint32_t a, cx<float> v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_peer_c(uint32_t a, cx<double> v) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+
+template <typename R, int W>
+struct alignas(16) PivSlot {
+  PivKey key;
+  cx<R> inv;
+  cx<R> row[W];
+};
+
+template <typename R, int W, int RPT>
+__global__ void __launch_bounds__(kRegT) k_getf2_reg(const MatInst* __restrict__ insts, int64_t k0,
+                                                     int nb) {
+  using C = cx<R>;
+  const unsigned rank = cluster_rank(), cs = cluster_size();
+  const MatInst& M = insts[blockIdx.x / cs];
+  const int64_t n = M.n;
+  if (!M.active || k0 >= n) return;  // the whole cluster (one instance) leaves together
+  const int nbe = (int)min((int64_t)nb, n - k0);
+  const int64_t lda = M.lda;
+  void* A = M.a;
+  __shared__ PivSlot<R, W> slot[2][kRegMaxCS];
+  __shared__ PivKey s_key[kRegT / 32];
+  __shared__ C sL[kPanelNB][kPanelNB + 1];  // L rows of the pivots of finished sub-panels
+  __shared__ C sU[W][kPanelNB];             // U rows of this sub-panel's columns
+  __shared__ int32_t s_phys[kPanelNB];      // row of every pivot
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int T = blockDim.x, nw = T >> 5;
+  const int64_t stride = (int64_t)cs * T;
+  const int64_t g = k0 + (int64_t)rank * T + tid;
+  int32_t pos[RPT], fz[RPT];  // position; step at which the row became a pivot (nb: not yet)
+#pragma unroll
+  for (int t = 0; t < RPT; ++t) {
+    pos[t] = (int32_t)(g + t * stride);
+    fz[t] = g + t * stride < n ? kPanelNB : -1;  // -1: no row
+  }
+  for (int s0 = 0; s0 < nbe; s0 += W) {
+    const int wn = min(W, nbe - s0);
+    C a[RPT][W];
+#pragma unroll
+    for (int t = 0; t < RPT; ++t)
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        a[t][w] = fz[t] >= 0 && w < wn ? ld<R>(A, (g + t * stride) + (k0 + s0 + w) * lda) : C{0, 0};
+    if (s0 > 0) {
+      // U rows of the finished pivots in these columns
+      for (int e = tid; e < s0 * s0; e += T) {
+        const int j = e % s0, i = e / s0;
+        if (i < j) sL[j][i] = ld<R>(A, s_phys[j] + (k0 + i) * lda);
+      }
+      for (int w = wid; w < wn; w += nw) {
+        if (lane < s0) sU[w][lane] = ld<R>(A, s_phys[lane] + (k0 + s0 + w) * lda);
+      }
+      __syncthreads();
+      for (int w = wid; w < wn; w += nw) {
+        C x = lane < s0 ? sU[w][lane] : C{0, 0};
+        for (int i = 0; i + 1 < s0; ++i) {
+          const C ui = shfl_c(x, i);
+          if (lane > i && lane < s0) cfnma(x, sL[lane][i], ui);
+        }
+        __syncwarp();
+        if (lane < s0) sU[w][lane] = x;
+      }
+      __syncthreads();
+      constexpr int kB = sizeof(R) == 4 ? 8 : 4;  // L values in flight (s0 is a multiple)
+#pragma unroll
+      for (int t = 0; t < RPT; ++t) {
+        const int lim = min(fz[t], s0);
+        for (int j0 = 0; j0 < lim; j0 += kB) {
+          C l[kB];
+#pragma unroll
+          for (int e = 0; e < kB; ++e)
+            if (j0 + e < lim) l[e] = ld<R>(A, (g + t * stride) + (k0 + j0 + e) * lda);
+#pragma unroll
+          for (int e = 0; e < kB; ++e)
+            if (j0 + e < lim) {
+#pragma unroll
+              for (int w = 0; w < W; ++w)
+                if (w < wn) cfnma(a[t][w], l[e], sU[w][j0 + e]);
+            }
+        }
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      if (w >= wn) break;  // uniform over the cluster
+      const int c = s0 + w;
+      const int32_t col = (int32_t)(k0 + c);
+      PivSlot<R, W>* sl = slot[c & 1];
+      // this thread's, the warp's and the CTA's candidate
+      PivKey best = {0u, 0u, INT32_MAX, 0};
+#pragma unroll
+      for (int t = 0; t < RPT; ++t) {
+        PivKey k;
+        key_of(a[t][w], k.hi, k.lo);
+        k.pos = fz[t] == kPanelNB ? pos[t] : INT32_MAX;
+        k.phys = (int32_t)(g + t * stride);
+        if (!key_nan(k, R{}) && key_better(k, best)) best = k;
+      }
+      warp_best<R>(best);
+      if (lane == 0) s_key[wid] = best;
+      __syncthreads();
+      best = lane < nw ? s_key[lane] : PivKey{0u, 0u, INT32_MAX, 0};
+      const int bw = warp_best<R>(best);  // warp of the CTA's candidate
+      // its owner's warp pushes it to every CTA, lane i to CTA i
+      if (wid == max(bw, 0)) {
+        int own = -1;  // this thread's row that is the candidate
+#pragma unroll
+        for (int t = 0; t < RPT; ++t)
+          if (bw >= 0 && fz[t] == kPanelNB && pos[t] == best.pos) own = t;
+        const uint32_t who = __ballot_sync(0xffffffffu, own >= 0);
+        const int src = who ? __ffs(who) - 1 : 0;
+        const uint32_t dst = peer_smem(&sl[rank], (unsigned)min(lane, (int)cs - 1));
+        const bool send = lane < (int)cs;
+        if (send) {
+          st_peer_b32(dst, best.hi);
+          st_peer_b32(dst + 4, best.lo);
+          st_peer_b32(dst + 8, (uint32_t)best.pos);
+          st_peer_b32(dst + 12, (uint32_t)best.phys);
+        }
+#pragma unroll
+        for (int q = w; q < W; ++q) {
+          C v = a[0][q];
+#pragma unroll
+          for (int t = 1; t < RPT; ++t)
+            if (own == t) v = a[t][q];
+          v = shfl_c(v, src);
+          if (q == w) v = (best.hi | best.lo) != 0u && bw >= 0 ? cinv_fast(v) : C{(R)1, (R)0};
+          if (send) st_peer_c(dst + 16 + (q == w ? 0 : 1 + q) * (uint32_t)sizeof(C), v);
+        }
+      }
+      cluster_sync_all();
+      // the cluster's pivot; the slots of step c are free again after the barrier of c + 1
+      best = lane < (int)cs ? sl[lane].key : PivKey{0u, 0u, INT32_MAX, 0};
+      const int win = max(warp_best<R>(best), 0);
+      // no candidate (only NaNs): the row at the diagonal position, marked singular
+      const int32_t piv = best.pos == INT32_MAX ? col : best.pos;
+      const bool nonzero = best.pos != INT32_MAX && (best.hi | best.lo) != 0u;
+      const C inv = sl[win].inv;
+      if (rank == 0 && tid == 0) {
+        M.ipiv[col] = piv;
+        if (!nonzero && *M.info == 0) *M.info = col + 1;
+      }
+      if (tid == 0) s_phys[c] = best.pos != INT32_MAX ? best.phys : col;
+#pragma unroll
+      for (int t = 0; t < RPT; ++t) {
+        if (fz[t] == kPanelNB) {
+          if (pos[t] == piv) {
+            fz[t] = c;
+            pos[t] = col;
+          } else {
+            if (pos[t] == col) pos[t] = piv;
+            const C l = a[t][w] * inv;
+            a[t][w] = l;
+#pragma unroll
+            for (int q = w + 1; q < W; ++q)
+              if (q < wn) cfnma(a[t][q], l, sl[win].row[q]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < RPT; ++t)
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (fz[t] >= 0 && w < wn) st<R>(A, (g + t * stride) + (k0 + s0 + w) * lda, a[t][w]);
+    // the stores before the other CTAs' reads of the pivot rows, and no CTA leaves while a
+    // peer can still write to its shared memory
+    cluster_sync_all();
+  }
 }
 
 // ------------------------------------------------------------------ laswp
@@ -1282,15 +1447,6 @@ __global__ void __launch_bounds__(256) k_make_perm(const MatInst* __restrict__ i
 // ------------------------------------------------------------------ launch wrappers
 static int prec_is_single(int prec) { return prec == 1; }
 
-// CTAs per instance of the left-looking panel kernel: as many as keep the batch on the
-// SMs in one wave (a power of two, 2..8: the portable cluster limit).
-static int getf2_cluster(int ninst) {
-  const int sms = device_sm_count();
-  int cs = 2;
-  while (cs < 8 && (int64_t)ninst * cs * 2 <= sms) cs *= 2;
-  return cs;
-}
-
 // complex64: 1024 threads, 16 L values in flight per row; complex128: 512 threads and 8
 // (the 64-register budget of 1024 threads would spill the FP64 values)
 template <typename R>
@@ -1299,41 +1455,67 @@ struct LLCfg {
   static constexpr int kBatch = sizeof(R) == 4 ? kLLBatch : kLLBatch / 2;
 };
 
-template <typename R, int CS>
-static void getf2_ll_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb) {
+template <typename K>
+static void cluster_launch(const Launch& L, K kernel, int ninst, int cs, int threads,
+                           const MatInst* d, int64_t k0, int nb) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ninst * CS));
-  cfg.blockDim = dim3(LLCfg<R>::kT);
+  cfg.gridDim = dim3((unsigned)(ninst * cs));
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = L.stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CS;
+  at[0].val.clusterDim.x = (unsigned)cs;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_getf2_ll<R, CS, LLCfg<R>::kT, LLCfg<R>::kBatch>, d, k0, nb);
+  cudaLaunchKernelEx(&cfg, kernel, d, k0, nb);
+  count_launch(1);
 }
 
-void launch_getf2(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int prec,
-                  int cs) {
-  // left-looking, one thread-block cluster per instance
-  const int csel = cs > 0 ? cs : getf2_cluster(ninst);
-  if (prec_is_single(prec)) {
-    switch (csel) {
-      case 8: getf2_ll_t<float, 8>(L, d, ninst, k0, nb); break;
-      case 4: getf2_ll_t<float, 4>(L, d, ninst, k0, nb); break;
-      default: getf2_ll_t<float, 2>(L, d, ninst, k0, nb); break;
-    }
+template <typename R, int W, int RPT>
+static void getf2_reg_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int cs,
+                        int threads) {
+  static PerDeviceOnce attr;
+  attr.call([] {  // clusters of 16 are beyond the portable size
+    cudaFuncSetAttribute(k_getf2_reg<R, W, RPT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  cluster_launch(L, k_getf2_reg<R, W, RPT>, ninst, cs, threads, d, k0, nb);
+}
+
+// The panel kernel's shape.  Cluster size: the batch in one wave of CTAs (at most 8 clusters
+// of 16 are resident, one per GPC), no more CTAs than give each kRegRows* rows; complex128
+// takes fewer rows per CTA since its FP64 work, not the barriers, sets the step.  Columns in
+// registers: as many as the rows per thread leave room for.
+bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_t nmax, int64_t k0,
+                  int nb, int prec) {
+  const bool single = prec_is_single(prec);
+  const int64_t rows = nmax - k0;
+  const int sms = device_sm_count();
+  const int per = single ? 256 : 64;
+  int cs = 1;
+  while (cs < kRegMaxCS && (int64_t)nact * cs * 2 <= sms && (cs < 8 || nact <= 8) &&
+         (int64_t)cs * per < rows)
+    cs *= 2;
+  const int64_t share = (rows + cs - 1) / cs;  // rows per CTA
+  const int threads = (int)std::min<int64_t>(kRegT, std::max<int64_t>(32, (share + 31) / 32 * 32));
+  const int64_t q = (share + threads - 1) / threads;  // rows per thread
+  if (single) {
+    if (q <= 1) return getf2_reg_t<float, 16, 1>(L, d, ninst, k0, nb, cs, threads), false;
+    if (q <= 2) return getf2_reg_t<float, 16, 2>(L, d, ninst, k0, nb, cs, threads), false;
+    if (q <= 5) return getf2_reg_t<float, 8, 5>(L, d, ninst, k0, nb, cs, threads), false;
+    if (q <= 10) return getf2_reg_t<float, 4, 10>(L, d, ninst, k0, nb, cs, threads), false;
+    cluster_launch(L, k_getf2_ll<float, 2, LLCfg<float>::kT, LLCfg<float>::kBatch>, ninst, 2,
+                   LLCfg<float>::kT, d, k0, nb);
   } else {
-    switch (csel) {
-      case 8: getf2_ll_t<double, 8>(L, d, ninst, k0, nb); break;
-      case 4: getf2_ll_t<double, 4>(L, d, ninst, k0, nb); break;
-      default: getf2_ll_t<double, 2>(L, d, ninst, k0, nb); break;
-    }
+    if (q <= 1) return getf2_reg_t<double, 8, 1>(L, d, ninst, k0, nb, cs, threads), false;
+    if (q <= 2) return getf2_reg_t<double, 8, 2>(L, d, ninst, k0, nb, cs, threads), false;
+    if (q <= 5) return getf2_reg_t<double, 4, 5>(L, d, ninst, k0, nb, cs, threads), false;
+    cluster_launch(L, k_getf2_ll<double, 2, LLCfg<double>::kT, LLCfg<double>::kBatch>, ninst, 2,
+                   LLCfg<double>::kT, d, k0, nb);
   }
-  count_launch(1);
+  return true;
 }
 
 void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int64_t c_lo,
@@ -1616,17 +1798,6 @@ void launch_getrs(const Launch& L, const MatInst* d, int ninst, int64_t nmax, in
       trsv_t<double, false, true, true>(L, d, ninst, nmax, max_rhs);
     }
     if (swaps) launch_rhs_swap(L, d, ninst, max_rhs, 1, prec);
-  }
-}
-
-// Full SIMT LU of a batch (used by the complex128 path and by the complex64 path when
-// the tensor-core trailing update is not selected).
-void launch_getrf_simt(const Launch& L, const MatInst* d, int ninst, int64_t nmax, int prec) {
-  for (int64_t k0 = 0; k0 < nmax; k0 += kPanelNB) {
-    launch_getf2(L, d, ninst, k0, kPanelNB, prec);
-    launch_laswp(L, d, ninst, k0, kPanelNB, 0, nmax, k0, k0 + kPanelNB, prec);
-    launch_trsm_panel(L, d, ninst, k0, kPanelNB, k0 + kPanelNB, nmax, prec);
-    launch_gemm_update(L, d, ninst, k0, kPanelNB, nmax, k0 + kPanelNB, nmax, prec);
   }
 }
 

@@ -9,10 +9,11 @@ namespace bemgpu {
 constexpr int kPanelNB = 32;  // LU panel width (columns factored per getf2 launch)
 constexpr int kTrsvNB = 64;   // triangular-solve block (rows per diagonal block)
 
-// cs: CTAs per instance of the complex64 panel kernel (2, 4 or 8; 0 = the batch-size
-// rule); the factor is identical for every choice
-void launch_getf2(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int prec,
-                  int cs = 0);
+// Factors the panel [k0, k0 + nb) of every instance; nmax: largest order, nact: instances
+// with rows left (the launch shape; the factor does not depend on it).  Returns whether the
+// interchanges were applied to the panel's own columns (if not, they are the caller's).
+bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_t nmax, int64_t k0,
+                  int nb, int prec);
 // row interchanges k0 .. k0 + nb - 1 on columns [c_lo, c_hi) \ [s_lo, s_hi)
 void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int64_t c_lo,
                   int64_t c_hi, int64_t s_lo, int64_t s_hi, int prec);
@@ -37,7 +38,5 @@ void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t 
                           double2* const* outs);
 // Row permutation of each factor from its pivots (one CTA per instance).
 void launch_make_perm(const Launch& L, const MatInst* d, int ninst, int64_t nmax);
-
-void launch_getrf_simt(const Launch& L, const MatInst* d, int ninst, int64_t nmax, int prec);
 
 }  // namespace bemgpu
