@@ -793,6 +793,7 @@ struct FactorData {
   Buf region_tab;          // kAsmRegion: RegionTable
   Buf outer;               // kAsmRegion: panel borders the exterior (int8)
   bool region_cbie = false;
+  Buf dinv;                        // inverted diagonal blocks of the current factor
   Buf LU, ipiv, info, perm;        // working factor (complex64 when single)
   Buf LU64, ipiv64, info64, perm64;  // complex128 factor after promotion
   Buf rows, cols, rowsum, cols_inv, rows_inv, cols_inv32;
@@ -814,7 +815,7 @@ struct FactorData {
   int32_t* info_ptr() const { return single ? info.as<int32_t>() : (mixed ? info64.as<int32_t>() : info.as<int32_t>()); }
   int32_t* perm_ptr() const { return single ? perm.as<int32_t>() : (mixed ? perm64.as<int32_t>() : perm.as<int32_t>()); }
   size_t bytes() const {
-    return A.bytes + dnear.bytes + dnear_rhs.bytes + Mrhs.bytes + LU.bytes + LU64.bytes + ipiv.bytes +
+    return A.bytes + dinv.bytes + dnear.bytes + dnear_rhs.bytes + Mrhs.bytes + LU.bytes + LU64.bytes + ipiv.bytes +
            ipiv64.bytes + rows.bytes + cols.bytes + rowsum.bytes;
   }
 };
@@ -1206,6 +1207,7 @@ int estimate_rcond(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
     m.info = fs[t]->info.as<int32_t>();
     m.x = work.as<float2>() + off[t];
     m.y = work2.as<float2>() + off[t];
+    m.dinv = fs[t]->dinv.p;
     m.ldx = fs[t]->N;
     m.nrhs = 1;
     m.active = 0;
@@ -1213,7 +1215,6 @@ int estimate_rcond(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
   TRY(upload(c, st, &d_st));
   TRY(upload(c, mi, &d_m1));
   TRY(upload(c, mi, &d_m2));
-  TrsvWork tw{1};
   Lacn2Dev* ds = d_st.as<Lacn2Dev>();
   MatInst* m1 = d_m1.as<MatInst>();
   MatInst* m2 = d_m2.as<MatInst>();
@@ -1229,7 +1230,7 @@ int estimate_rcond(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
     if (any1) {
       {
         Prof pr(c, "getrs");
-        launch_getrs(L, m1, (int)F, nmax, 1, 1, 1, 0, &tw);
+        launch_getrs(L, m1, (int)F, nmax, 1, 1, 1, 0, false);
       }
       launch_lacn2(L, ds, (int)F, work.as<float2>(), m1, m2, 1);
       any2 = true;  // those instances usually ask for the other product next
@@ -1237,7 +1238,7 @@ int estimate_rcond(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
     if (any2) {
       {
         Prof pr(c, "getrs");
-        launch_getrs(L, m2, (int)F, nmax, 1, 0, 1, 0, &tw);
+        launch_getrs(L, m2, (int)F, nmax, 1, 0, 1, 0, false);
       }
       launch_lacn2(L, ds, (int)F, work.as<float2>(), m1, m2, 2);
     }
@@ -1802,6 +1803,8 @@ int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool prom
     Buf& pb = promoted ? f->perm64 : f->perm;
     TRY(alloc(c, (size_t)f->N * 4, &pb));
     m.perm = pb.as<int32_t>();
+    TRY(alloc(c, tri_inv_bytes(f->N, prec), &f->dinv));
+    m.dinv = f->dinv.p;
     m.active = 1;
     CUDA_TRY(c, cudaMemsetAsync(m.info, 0, sizeof(int32_t), c->stream));
     nmax = std::max(nmax, f->N);
@@ -1833,6 +1836,10 @@ int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool prom
     }
   }
   launch_make_perm(L, d.as<MatInst>(), (int)fs.size(), nmax);
+  {
+    Prof pr(c, "tri_inv");
+    launch_tri_inv(L, d.as<MatInst>(), (int)fs.size(), nmax, prec);
+  }
   CUDA_TRY(c, cudaGetLastError());
   for (size_t t = 0; t < fs.size(); ++t) {
     int32_t h = 0;
@@ -2240,12 +2247,14 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
     rmax = std::max(rmax, s->R);
   }
   launch_corr_prep(L, d.as<VecInst>(), (int)vi.size(), nmax, rmax);
-  for (int prec : {1, 0}) {
+  for (int pass = 0; pass < 4; ++pass) {  // precision, few or many right-hand sides
+    const int prec = pass < 2 ? 1 : 0;
+    const bool many = (pass & 1) != 0;
     std::vector<MatInst> mi;
     int64_t pn = 0;
     int32_t pr = 0;
     for (SolveInst* s : who) {
-      if ((s->f->single ? 1 : 0) != prec) continue;
+      if ((s->f->single ? 1 : 0) != prec || many_rhs(s->R) != many) continue;
       MatInst m{};
       m.a = s->f->factor_ptr();
       m.n = s->f->N;
@@ -2256,6 +2265,7 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
       m.x = s->work.p;
       m.y = s->work2.p;
       m.perm = s->f->perm_ptr();
+      m.dinv = s->f->dinv.p;
       m.ldx = s->f->N;
       m.nrhs = s->R;
       m.active = 1;
@@ -2266,9 +2276,8 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
     if (mi.empty()) continue;
     Buf dm;
     TRY(to_device(c, mi, &dm));
-    TrsvWork tw{1};
     Prof p(c, "getrs");
-    launch_getrs(L, dm.as<MatInst>(), (int)mi.size(), pn, pr, 0, prec, 1, &tw);
+    launch_getrs(L, dm.as<MatInst>(), (int)mi.size(), pn, pr, 0, prec, 1, many);
   }
   launch_corr_apply(L, d.as<VecInst>(), (int)vi.size(), nmax, rmax, mode);
   CUDA_TRY(c, cudaGetLastError());

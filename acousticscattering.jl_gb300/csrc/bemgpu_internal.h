@@ -147,11 +147,7 @@ struct MatInst {
   int32_t active;
   int32_t* perm;    // row permutation of the factor: (P b)[i] = b[perm[i]]
   void* y;          // second vector buffer of the triangular solves (n x nrhs, ld ldx)
-};
-
-// Selects the blocked triangular solves (MatInst.y / MatInst.perm provided).
-struct TrsvWork {
-  int32_t blocked;
+  void* dinv;       // inverses of the factor's diagonal blocks (tri_inv_bytes)
 };
 
 // ------------------------------------------------------------------ launch wrappers

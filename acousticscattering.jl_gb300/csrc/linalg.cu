@@ -12,9 +12,7 @@
 //   trsm    U12 = L11^{-1} A12, one warp per column of A12;
 //   gemm    A22 -= L21 U12 (SIMT tile kernel; the complex64 factor of the mixed path
 //           uses the tensor-core kernel in gemm_tc.cu instead).
-// getrs: row interchanges, then blocked triangular solves: a diagonal-block solve
-// (one CTA per instance and right-hand side) followed by a rank-update of the rows
-// still to solve, for L, U, U^H and L^H (the last two for condition estimation).
+// The triangular solves are in trsv.cu.
 #include <cfloat>
 #include <cstdio>
 
@@ -54,11 +52,6 @@ __device__ __forceinline__ cx<R> cinv(cx<R> a) {
   R d = (ar * ar + ai * ai) * s;
   return {ar / d, -ai / d};
 }
-template <typename R>
-__device__ __forceinline__ cx<R> cconj(cx<R> a) {
-  return {a.x, -a.y};
-}
-
 // ------------------------------------------------------------------ getf2, left-looking
 // Complex64 panel factorisation for the LU driver: column c is brought up to date only
 // when it is reached (U[0:c, c] by one warp from the finished L11 rows cached in shared
@@ -294,9 +287,7 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
 // on the batch.  Measured, one instance of 8960 unknowns, complex64: 7.0 us a column with the
 // streaming kernel above, see the launcher for this one's; complex128 (FP64 issue: two FMAs
 // per clock and SM beside the latency) of 5760 unknowns: 27 us a column before.
-constexpr int kRegT = 512;      // threads per CTA at most
 constexpr int kRegMaxCS = 16;   // CTAs per cluster at most
-
 __device__ __forceinline__ unsigned cluster_size() {
   unsigned r;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
@@ -393,8 +384,10 @@ struct alignas(16) PivSlot {
   cx<R> row[W];
 };
 
-template <typename R, int W, int RPT>
-__global__ void __launch_bounds__(kRegT) k_getf2_reg(const MatInst* __restrict__ insts, int64_t k0,
+// T: threads per CTA at most (complex128 sub-panels of 16 columns need the registers of a
+// CTA of 256)
+template <typename R, int W, int RPT, int T_>
+__global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ insts, int64_t k0,
                                                      int nb) {
   using C = cx<R>;
   const unsigned rank = cluster_rank(), cs = cluster_size();
@@ -405,7 +398,7 @@ __global__ void __launch_bounds__(kRegT) k_getf2_reg(const MatInst* __restrict__
   const int64_t lda = M.lda;
   void* A = M.a;
   __shared__ PivSlot<R, W> slot[2][kRegMaxCS];
-  __shared__ PivKey s_key[kRegT / 32];
+  __shared__ PivKey s_key[T_ / 32];
   __shared__ C sL[kPanelNB][kPanelNB + 1];  // L rows of the pivots of finished sub-panels
   __shared__ C sU[W][kPanelNB];             // U rows of this sub-panel's columns
   __shared__ int32_t s_phys[kPanelNB];      // row of every pivot
@@ -789,203 +782,6 @@ __global__ void __launch_bounds__(kGThreads) k_gemm_update(const MatInst* __rest
     }
 }
 
-// ------------------------------------------------------------------ getrs pieces
-// Row interchanges on the right-hand sides (forward: ipiv in order; back: reverse).
-template <typename R>
-__global__ void k_rhs_swap(const MatInst* __restrict__ insts, int reverse) {
-  const MatInst& M = insts[blockIdx.y];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!M.active || r >= M.nrhs) return;
-  const int64_t n = M.n;
-  void* X = M.x;
-  const int64_t off = (int64_t)r * M.ldx;
-  if (!reverse) {
-    for (int64_t i = 0; i < n; ++i) {
-      int64_t p = M.ipiv[i];
-      if (p != i) {
-        cx<R> a = ld<R>(X, off + i), b = ld<R>(X, off + p);
-        st<R>(X, off + i, b);
-        st<R>(X, off + p, a);
-      }
-    }
-  } else {
-    for (int64_t i = n - 1; i >= 0; --i) {
-      int64_t p = M.ipiv[i];
-      if (p != i) {
-        cx<R> a = ld<R>(X, off + i), b = ld<R>(X, off + p);
-        st<R>(X, off + i, b);
-        st<R>(X, off + p, a);
-      }
-    }
-  }
-}
-
-// element (r, c) of op(A): A or A^H
-template <typename R, bool TRANS>
-__device__ __forceinline__ cx<R> opel(const void* A, int64_t lda, int64_t r, int64_t c) {
-  if (TRANS) return cconj(ld<R>(A, c + r * lda));
-  return ld<R>(A, r + c * lda);
-}
-
-// Diagonal block solve: rows [r0, r0 + nbs) of op(T) x = x, op(T) lower when
-// EFF_LOWER.  One CTA (kTrsvNB threads) per (rhs, instance).
-template <typename R, bool EFF_LOWER, bool TRANS, bool UNIT>
-__global__ void __launch_bounds__(kTrsvNB) k_trsv_block(const MatInst* __restrict__ insts,
-                                                        int64_t r0) {
-  const MatInst& M = insts[blockIdx.y];
-  const int rhs = blockIdx.x;
-  const int64_t n = M.n;
-  if (!M.active || rhs >= M.nrhs || r0 >= n) return;
-  const int nbs = (int)min((int64_t)kTrsvNB, n - r0);
-  const int64_t lda = M.lda, off = (int64_t)rhs * M.ldx;
-  __shared__ cx<R> sx[kTrsvNB];
-  const int t = threadIdx.x;
-  if (t < nbs) sx[t] = ld<R>(M.x, off + r0 + t);
-  __syncthreads();
-  if (EFF_LOWER) {
-    for (int c = 0; c < nbs; ++c) {
-      if (!UNIT && t == c) sx[c] = sx[c] * cinv(opel<R, TRANS>(M.a, lda, r0 + c, r0 + c));
-      __syncthreads();
-      if (t > c && t < nbs) sx[t] -= opel<R, TRANS>(M.a, lda, r0 + t, r0 + c) * sx[c];
-      __syncthreads();
-    }
-  } else {
-    for (int c = nbs - 1; c >= 0; --c) {
-      if (!UNIT && t == c) sx[c] = sx[c] * cinv(opel<R, TRANS>(M.a, lda, r0 + c, r0 + c));
-      __syncthreads();
-      if (t < c) sx[t] -= opel<R, TRANS>(M.a, lda, r0 + t, r0 + c) * sx[c];
-      __syncthreads();
-    }
-  }
-  if (t < nbs) st<R>(M.x, off + r0 + t, sx[t]);
-}
-
-// Update of the unsolved rows by the solved block [r0, r0 + nbs): thread per row.
-template <typename R, bool EFF_LOWER, bool TRANS>
-__global__ void __launch_bounds__(256) k_trsv_update(const MatInst* __restrict__ insts,
-                                                     int64_t r0) {
-  const MatInst& M = insts[blockIdx.z];
-  const int rhs = blockIdx.y;
-  const int64_t n = M.n;
-  if (!M.active || rhs >= M.nrhs || r0 >= n) return;
-  const int nbs = (int)min((int64_t)kTrsvNB, n - r0);
-  const int64_t lda = M.lda, off = (int64_t)rhs * M.ldx;
-  __shared__ cx<R> sx[kTrsvNB];
-  if (threadIdx.x < nbs) sx[threadIdx.x] = ld<R>(M.x, off + r0 + threadIdx.x);
-  __syncthreads();
-  int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (EFF_LOWER)
-    row += r0 + nbs;
-  if (EFF_LOWER ? row >= n : row >= r0) return;
-  cx<R> acc = {0, 0};
-  for (int c = 0; c < nbs; ++c) acc += opel<R, TRANS>(M.a, lda, row, r0 + c) * sx[c];
-  st<R>(M.x, off + row, ld<R>(M.x, off + row) - acc);
-}
-
-// Whole triangular solve in one launch: one CTA per (rhs, instance) holds the
-// right-hand side in shared memory, walks the 32-row diagonal blocks (warp 0 solves a
-// block with shuffles) and lets all threads update the unsolved rows after each block.
-// SWAP 1: LAPACK's forward row interchanges before the solve; 2: the reverse
-// interchanges after it (the P^T of A^H x = b); 0: none.
-constexpr int kTrsvThreads = 512;
-
-template <typename R, bool EFF_LOWER, bool TRANS, bool UNIT, int SWAP>
-__global__ void __launch_bounds__(kTrsvThreads) k_trsv_full(const MatInst* __restrict__ insts) {
-  const MatInst& M = insts[blockIdx.y];
-  const int rhs = blockIdx.x;
-  if (!M.active || rhs >= M.nrhs) return;
-  const int64_t n = M.n, lda = M.lda, off = (int64_t)rhs * M.ldx;
-  extern __shared__ __align__(16) unsigned char trsv_smem[];
-  cx<R>* sx = reinterpret_cast<cx<R>*>(trsv_smem);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int64_t i = tid; i < n; i += kTrsvThreads) sx[i] = ld<R>(M.x, off + i);
-  __syncthreads();
-  if (SWAP == 1 && tid == 0) {
-    for (int64_t i = 0; i < n; ++i) {
-      const int64_t p = M.ipiv[i];
-      if (p != i) {
-        cx<R> t = sx[i];
-        sx[i] = sx[p];
-        sx[p] = t;
-      }
-    }
-  }
-  __syncthreads();
-  const int64_t nblk = (n + 31) / 32;
-  for (int64_t bb = 0; bb < nblk; ++bb) {
-    const int64_t b = EFF_LOWER ? bb : nblk - 1 - bb;
-    const int64_t r0 = b * 32;
-    const int nb = (int)min((int64_t)32, n - r0);
-    if (warp == 0) {
-      cx<R> x = lane < nb ? sx[r0 + lane] : cx<R>{0, 0};
-      if (EFF_LOWER) {
-        for (int c = 0; c < nb; ++c) {
-          if (!UNIT && lane == c) x = x * cinv(opel<R, TRANS>(M.a, lda, r0 + c, r0 + c));
-          cx<R> xc;
-          xc.x = __shfl_sync(0xffffffffu, x.x, c);
-          xc.y = __shfl_sync(0xffffffffu, x.y, c);
-          if (lane > c && lane < nb) x -= opel<R, TRANS>(M.a, lda, r0 + lane, r0 + c) * xc;
-        }
-      } else {
-        for (int c = nb - 1; c >= 0; --c) {
-          if (!UNIT && lane == c) x = x * cinv(opel<R, TRANS>(M.a, lda, r0 + c, r0 + c));
-          cx<R> xc;
-          xc.x = __shfl_sync(0xffffffffu, x.x, c);
-          xc.y = __shfl_sync(0xffffffffu, x.y, c);
-          if (lane < c) x -= opel<R, TRANS>(M.a, lda, r0 + lane, r0 + c) * xc;
-        }
-      }
-      if (lane < nb) sx[r0 + lane] = x;
-    }
-    __syncthreads();
-    const int64_t lo = EFF_LOWER ? r0 + nb : 0, hi = EFF_LOWER ? n : r0;
-    for (int64_t r = lo + tid; r < hi; r += kTrsvThreads) {
-      cx<R> acc = {0, 0};
-#pragma unroll
-      for (int h = 0; h < 32; h += 16) {
-        cx<R> lv[16];  // 16 independent loads in flight per thread
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          lv[c] = (h + c < nb) ? opel<R, TRANS>(M.a, lda, r, r0 + h + c) : cx<R>{0, 0};
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          if (h + c < nb) acc += lv[c] * sx[r0 + h + c];
-      }
-      sx[r] -= acc;
-    }
-    __syncthreads();
-  }
-  if (SWAP == 2 && tid == 0) {
-    for (int64_t i = n - 1; i >= 0; --i) {
-      const int64_t p = M.ipiv[i];
-      if (p != i) {
-        cx<R> t = sx[i];
-        sx[i] = sx[p];
-        sx[p] = t;
-      }
-    }
-  }
-  __syncthreads();
-  for (int64_t i = tid; i < n; i += kTrsvThreads) st<R>(M.x, off + i, sx[i]);
-}
-
-template <typename R, bool EL, bool TR, bool UN, int SW>
-static void trsv_full_t(const Launch& L, const MatInst* d, int ninst, int64_t nmax,
-                        int32_t max_rhs) {
-  const size_t smem = (size_t)nmax * sizeof(cx<R>);
-  static PerDeviceOnce attr;
-  attr.call([] {
-    cudaFuncSetAttribute(k_trsv_full<R, EL, TR, UN, SW>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  });
-  k_trsv_full<R, EL, TR, UN, SW><<<dim3((unsigned)max_rhs, (unsigned)ninst), kTrsvThreads, smem,
-                                   L.stream>>>(d);
-  count_launch(1);
-}
-
-// largest order whose right-hand side fits the shared memory of one CTA
-static int64_t trsv_full_max(int prec) { return (int64_t)(220 * 1024) / (prec == 1 ? 8 : 16); }
-
 // ------------------------------------------------------------------ -(L11^{-1} - I)
 // For the tensor-core U12 solve: with L11^{-1} = I + N (N strictly lower),
 // U12 = L11^{-1} A12 = A12 - (-N) A12.  One CTA per instance stages the unit lower
@@ -1119,308 +915,6 @@ void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t 
   count_launch(1);
 }
 
-// ------------------------------------------------------------------ blocked solves
-// Two-level triangular solve: diagonal blocks of kBigB rows are solved by one CTA per
-// (rhs, instance) holding the block's slice of the vector in shared memory; the rows
-// outside the block are then updated by a full-GPU product kernel.  About 2 n / kBigB
-// launches per triangle.
-//
-// Inside a diagonal block the 32 x 32 triangle of each sub-block is staged in shared
-// memory (double-buffered: the next sub-block's triangle is fetched while warp 0 solves
-// the current one from shared memory with shuffles), then all warps update the rest of
-// the block.  op(A) = A^H reads A along its columns in both phases (a warp per row,
-// lanes along the column), so every global access is coalesced.
-constexpr int kBigB = 512;
-constexpr int kDiagThreads = 512;
-constexpr int kTilePad = 33;
-constexpr int kPre = 32;  // prefetched update operands per thread
-static_assert(kBigB - 32 <= kDiagThreads, "one update row per thread");
-static_assert((kBigB - 32 + (kDiagThreads / 32) * 4 - 1) / ((kDiagThreads / 32) * 4) * 4 <= kPre,
-              "transposed update rows per lane");
-
-template <typename R>
-constexpr size_t diag_smem_bytes() {
-  return sizeof(cx<R>) * (kBigB + 2 * 32 * kTilePad + 2 * 32);
-}
-
-template <typename R, bool EFF_LOWER, bool TRANS, bool UNIT>
-__global__ void __launch_bounds__(kDiagThreads) k_trsv_diag(const MatInst* __restrict__ insts,
-                                                            int64_t r0) {
-  const MatInst& M = insts[blockIdx.y];
-  const int rhs = blockIdx.x;
-  if (!M.active || rhs >= M.nrhs || r0 >= M.n) return;
-  const int64_t n = M.n, lda = M.lda, off = (int64_t)rhs * M.ldx;
-  const int nbs = (int)min((int64_t)kBigB, n - r0);
-  extern __shared__ __align__(16) unsigned char diag_smem[];
-  cx<R>* sx = reinterpret_cast<cx<R>*>(diag_smem);
-  cx<R>* tiles = sx + kBigB;  // [2][32][kTilePad], tile[i][j] = op(A)[s0 + i, s0 + j]
-  cx<R>* dinv = tiles + 2 * 32 * kTilePad;  // [2][32] reciprocals of the tiles' diagonals
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nsub = (nbs + 31) / 32;
-  auto sub_of = [&](int bb) { return EFF_LOWER ? bb : nsub - 1 - bb; };
-  // stage the triangle of sub-block b in tile buffer buf (threads [t0, kDiagThreads))
-  auto stage = [&](int buf, int b, int t0) {
-    const int s0 = b * 32, nb = min(32, nbs - s0);
-    cx<R>* T = tiles + buf * 32 * kTilePad;
-    for (int e = tid - t0; e < 1024; e += kDiagThreads - t0) {
-      const int p = e & 31, q = e >> 5;  // physical A[s0 + p, s0 + q], coalesced in p
-      cx<R> v = {0, 0};
-      if (p < nb && q < nb) v = ld<R>(M.a, (r0 + s0 + p) + (r0 + s0 + q) * lda);
-      if (TRANS)
-        T[q * kTilePad + p] = cconj(v);
-      else
-        T[p * kTilePad + q] = v;
-      if (!UNIT && p == q && p < nb) dinv[buf * 32 + p] = cinv(TRANS ? cconj(v) : v);
-    }
-  };
-  for (int i = tid; i < nbs; i += kDiagThreads) sx[i] = ld<R>(M.x, off + r0 + i);
-  stage(0, sub_of(0), 0);
-  __syncthreads();
-  for (int bb = 0; bb < nsub; ++bb) {
-    const int b = sub_of(bb);
-    const int s0 = b * 32;
-    const int nb = min(32, nbs - s0);
-    const cx<R>* T = tiles + (bb & 1) * 32 * kTilePad;
-    const cx<R>* DI = dinv + (bb & 1) * 32;
-    // this sub-block's update operands, loaded before the solve so that their memory
-    // latency overlaps it (one row of 32 values per thread, or 32 column values per
-    // lane for op(A) = A^H)
-    constexpr int kP = sizeof(R) == 4 ? kPre : kPre / 2;  // FP64: half, rest on demand
-    cx<R> pre[kP];
-    {
-      const int lo = EFF_LOWER ? s0 + nb : 0, hi = EFF_LOWER ? nbs : s0;
-      if (!TRANS) {
-        const int r = lo + tid;
-#pragma unroll
-        for (int c = 0; c < kP; ++c)
-          pre[c] = (r < hi && c < nb) ? ld<R>(M.a, (r0 + r) + (r0 + s0 + c) * lda) : cx<R>{0, 0};
-      } else {
-#pragma unroll
-        for (int q = 0; q < kP; ++q) {
-          const int r = lo + warp * 4 + (q & 3) + (q >> 2) * (kDiagThreads / 32) * 4;
-          pre[q] = (r < hi && lane < nb) ? ld<R>(M.a, (r0 + s0 + lane) + (r0 + r) * lda)
-                                         : cx<R>{0, 0};
-        }
-      }
-    }
-    if (warp == 0) {
-      cx<R> x = lane < nb ? sx[s0 + lane] : cx<R>{0, 0};
-      if (EFF_LOWER) {
-        for (int c = 0; c < nb; ++c) {
-          if (!UNIT && lane == c) x = x * DI[c];
-          cx<R> xc;
-          xc.x = __shfl_sync(0xffffffffu, x.x, c);
-          xc.y = __shfl_sync(0xffffffffu, x.y, c);
-          if (lane > c && lane < nb) x -= T[lane * kTilePad + c] * xc;
-        }
-      } else {
-        for (int c = nb - 1; c >= 0; --c) {
-          if (!UNIT && lane == c) x = x * DI[c];
-          cx<R> xc;
-          xc.x = __shfl_sync(0xffffffffu, x.x, c);
-          xc.y = __shfl_sync(0xffffffffu, x.y, c);
-          if (lane < c) x -= T[lane * kTilePad + c] * xc;
-        }
-      }
-      if (lane < nb) sx[s0 + lane] = x;
-    } else if (bb + 1 < nsub) {
-      stage((bb + 1) & 1, sub_of(bb + 1), 32);
-    }
-    __syncthreads();
-    const int lo = EFF_LOWER ? s0 + nb : 0, hi = EFF_LOWER ? nbs : s0;
-    if (!TRANS) {
-      // one row per thread (the block's rows outside the sub-block fit in kDiagThreads)
-      const int r = lo + tid;
-      if (r < hi) {
-        cx<R> acc = {0, 0};
-#pragma unroll
-        for (int c = 0; c < kP; ++c)
-          if (c < nb) acc += pre[c] * sx[s0 + c];
-#pragma unroll
-        for (int c = kP; c < 32; ++c)
-          if (c < nb) acc += ld<R>(M.a, (r0 + r) + (r0 + s0 + c) * lda) * sx[s0 + c];
-        sx[r] -= acc;
-      }
-    } else {
-      // op(A)[r, s0 + c] = conj(A[s0 + c, r]): lanes along c, 4 rows per warp pass
-      const cx<R> xv = lane < nb ? sx[s0 + lane] : cx<R>{0, 0};
-#pragma unroll
-      for (int q = 0; q < kPre; ++q) {
-        const cx<R> av =
-            q < kP ? pre[q < kP ? q : 0]
-                   : [&] {
-                       const int rr = lo + warp * 4 + (q & 3) + (q >> 2) * (kDiagThreads / 32) * 4;
-                       return (rr < hi && lane < nb) ? ld<R>(M.a, (r0 + s0 + lane) + (r0 + rr) * lda)
-                                                     : cx<R>{0, 0};
-                     }();
-        cx<R> t = cconj(av) * xv;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-          t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
-        }
-        const int r = lo + warp * 4 + (q & 3) + (q >> 2) * (kDiagThreads / 32) * 4;
-        if (lane == 0 && r < hi) sx[r] -= t;
-      }
-    }
-    __syncthreads();
-  }
-  for (int i = tid; i < nbs; i += kDiagThreads) st<R>(M.x, off + r0 + i, sx[i]);
-}
-
-// Rows outside the solved block [r0, r0 + kBigB): x_r -= sum_c op(A)[r, c] x_c, one
-// thread per row, the block's solution in shared memory (op(A) = A, coalesced along r).
-// RG right-hand sides per CTA share every matrix element a thread loads, so a sweep's
-// many right-hand sides read the factor once per group instead of once each.
-template <typename R, int RG>
-constexpr size_t upd_smem_bytes() {
-  return sizeof(cx<R>) * (size_t)RG * kBigB;
-}
-
-// Rows [lo, hi) (absolute, clamped to the instance: beyond its block for the lower solve,
-// before it for the upper one) are updated from the solution of block [r0, r0 + kBigB).
-template <typename R, bool EFF_LOWER, bool TRANS, int RG>
-__global__ void __launch_bounds__(256) k_trsv_big_update(const MatInst* __restrict__ insts,
-                                                         int64_t r0, int64_t lo, int64_t hi) {
-  const MatInst& M = insts[blockIdx.z];
-  const int rg0 = blockIdx.y * RG;
-  const int64_t n = M.n;
-  if (!M.active || rg0 >= M.nrhs || r0 >= n) return;
-  const int nr = min(RG, M.nrhs - rg0);
-  const int nbs = (int)min((int64_t)kBigB, n - r0);
-  const int64_t lda = M.lda, ldx = M.ldx;
-  extern __shared__ __align__(16) unsigned char upd_smem[];
-  cx<R>* sx = reinterpret_cast<cx<R>*>(upd_smem);  // [RG][kBigB]
-  for (int r = 0; r < nr; ++r)
-    for (int i = threadIdx.x; i < nbs; i += blockDim.x)
-      sx[r * kBigB + i] = ld<R>(M.x, (int64_t)(rg0 + r) * ldx + r0 + i);
-  __syncthreads();
-  const int64_t row = lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= hi || (EFF_LOWER ? (row < r0 + nbs || row >= n) : row >= r0)) return;
-  cx<R> acc[RG];
-#pragma unroll
-  for (int r = 0; r < RG; ++r) acc[r] = cx<R>{0, 0};
-  for (int c0 = 0; c0 < nbs; c0 += 8) {
-    cx<R> lv[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-      lv[c] = (c0 + c < nbs) ? opel<R, TRANS>(M.a, lda, row, r0 + c0 + c) : cx<R>{0, 0};
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      if (c0 + c < nbs) {
-#pragma unroll
-        for (int r = 0; r < RG; ++r)
-          if (r < nr) acc[r] += lv[c] * sx[r * kBigB + c0 + c];
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < RG; ++r) {
-    if (r < nr) {
-      const int64_t o = (int64_t)(rg0 + r) * ldx + row;
-      st<R>(M.x, o, ld<R>(M.x, o) - acc[r]);
-    }
-  }
-}
-
-// The same update for op(A) = A^H: x_r -= sum_c conj(A[c, r]) x_c reads column r of A,
-// so a warp takes 4 rows with its lanes along c (coalesced), then reduces by shuffles.
-constexpr int kTrUpRows = 32;  // rows per 256-thread CTA (8 warps x 4)
-template <typename R, bool EFF_LOWER, int RG>
-__global__ void __launch_bounds__(256) k_trsv_big_update_h(const MatInst* __restrict__ insts,
-                                                           int64_t r0, int64_t lo, int64_t hi) {
-  const MatInst& M = insts[blockIdx.z];
-  const int rg0 = blockIdx.y * RG;
-  const int64_t n = M.n;
-  if (!M.active || rg0 >= M.nrhs || r0 >= n) return;
-  const int nr = min(RG, M.nrhs - rg0);
-  const int nbs = (int)min((int64_t)kBigB, n - r0);
-  const int64_t lda = M.lda, ldx = M.ldx;
-  extern __shared__ __align__(16) unsigned char upd_smem[];
-  cx<R>* sx = reinterpret_cast<cx<R>*>(upd_smem);  // [RG][kBigB]
-  for (int r = 0; r < nr; ++r)
-    for (int i = threadIdx.x; i < nbs; i += blockDim.x)
-      sx[r * kBigB + i] = ld<R>(M.x, (int64_t)(rg0 + r) * ldx + r0 + i);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row0 = lo + (int64_t)blockIdx.x * kTrUpRows + warp * 4;
-  const int64_t lim = min(hi, EFF_LOWER ? n : r0);
-  if (row0 >= lim || (EFF_LOWER && row0 < r0 + nbs)) return;  // lo is a multiple of 4 rows
-  cx<R> acc[4][RG];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int r = 0; r < RG; ++r) acc[u][r] = cx<R>{0, 0};
-  for (int c = lane; c < nbs; c += 32) {
-    cx<R> v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      v[u] = (row0 + u < lim) ? cconj(ld<R>(M.a, (r0 + c) + (row0 + u) * lda)) : cx<R>{0, 0};
-#pragma unroll
-    for (int r = 0; r < RG; ++r) {
-      if (r < nr) {
-        const cx<R> xv = sx[r * kBigB + c];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u][r] += v[u] * xv;
-      }
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-#pragma unroll
-    for (int r = 0; r < RG; ++r) {
-      if (r < nr) {
-        cx<R> t = acc[u][r];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-          t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
-        }
-        if (lane == 0 && row0 + u < lim) {
-          const int64_t o2 = (int64_t)(rg0 + r) * ldx + row0 + u;
-          st<R>(M.x, o2, ld<R>(M.x, o2) - t);
-        }
-      }
-    }
-  }
-}
-
-// x[i] = y[perm[i]] (forward interchanges as one gather; y holds a copy of x)
-template <typename R>
-__global__ void k_gather_perm(const MatInst* __restrict__ insts) {
-  const MatInst& M = insts[blockIdx.z];
-  const int rhs = blockIdx.y;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (!M.active || rhs >= M.nrhs || i >= M.n) return;
-  const int64_t off = (int64_t)rhs * M.ldx;
-  st<R>(M.x, off + i, ld<R>(M.y, off + M.perm[i]));
-}
-
-// (P^T w): x[perm[i]] = y[i] for every stream, then the caller's x holds the result.
-template <typename R>
-__global__ void k_scatter_perm(const MatInst* __restrict__ insts, int max_rhs) {
-  const MatInst& M = insts[blockIdx.z];
-  const int rhs = blockIdx.y;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (!M.active || rhs >= M.nrhs || i >= M.n) return;
-  const int64_t off = (int64_t)rhs * M.ldx;
-  st<R>(M.x, off + M.perm[i], ld<R>(M.y, off + i));
-}
-
-// x -> y copy (both ld ldx)
-template <typename R>
-__global__ void k_copy_xy(const MatInst* __restrict__ insts, int to_y) {
-  const MatInst& M = insts[blockIdx.z];
-  const int rhs = blockIdx.y;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (!M.active || rhs >= M.nrhs || i >= M.n) return;
-  const int64_t off = (int64_t)rhs * M.ldx;
-  if (to_y)
-    st<R>(M.y, off + i, ld<R>(M.x, off + i));
-  else
-    st<R>(M.x, off + i, ld<R>(M.y, off + i));
-}
-
 // perm from LAPACK pivots: apply the interchanges in order to the identity, in shared
 // memory (SMEM, orders up to the shared-memory capacity) or in place in global memory.
 template <bool SMEM>
@@ -1474,14 +968,14 @@ static void cluster_launch(const Launch& L, K kernel, int ninst, int cs, int thr
   count_launch(1);
 }
 
-template <typename R, int W, int RPT>
+template <typename R, int W, int RPT, int T = 512>
 static void getf2_reg_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int cs,
                         int threads) {
   static PerDeviceOnce attr;
   attr.call([] {  // clusters of 16 are beyond the portable size
-    cudaFuncSetAttribute(k_getf2_reg<R, W, RPT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k_getf2_reg<R, W, RPT, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   });
-  cluster_launch(L, k_getf2_reg<R, W, RPT>, ninst, cs, threads, d, k0, nb);
+  cluster_launch(L, k_getf2_reg<R, W, RPT, T>, ninst, cs, threads, d, k0, nb);
 }
 
 // The panel kernel's shape.  Cluster size: the batch in one wave of CTAs (at most 8 clusters
@@ -1499,7 +993,9 @@ bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_
          (int64_t)cs * per < rows)
     cs *= 2;
   const int64_t share = (rows + cs - 1) / cs;  // rows per CTA
-  const int threads = (int)std::min<int64_t>(kRegT, std::max<int64_t>(32, (share + 31) / 32 * 32));
+  // complex128: at least eight warps, which solve the U rows of a sub-panel's columns
+  const int threads =
+      (int)std::min<int64_t>(512, std::max<int64_t>(single ? 64 : 256, (share + 31) / 32 * 32));
   const int64_t q = (share + threads - 1) / threads;  // rows per thread
   if (single) {
     if (q <= 1) return getf2_reg_t<float, 16, 1>(L, d, ninst, k0, nb, cs, threads), false;
@@ -1509,6 +1005,8 @@ bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_
     cluster_launch(L, k_getf2_ll<float, 2, LLCfg<float>::kT, LLCfg<float>::kBatch>, ninst, 2,
                    LLCfg<float>::kT, d, k0, nb);
   } else {
+    if (threads <= 256 && q <= 1)
+      return getf2_reg_t<double, 16, 1, 256>(L, d, ninst, k0, nb, cs, threads), false;
     if (q <= 1) return getf2_reg_t<double, 8, 1>(L, d, ninst, k0, nb, cs, threads), false;
     if (q <= 2) return getf2_reg_t<double, 8, 2>(L, d, ninst, k0, nb, cs, threads), false;
     if (q <= 5) return getf2_reg_t<double, 4, 5>(L, d, ninst, k0, nb, cs, threads), false;
@@ -1581,141 +1079,6 @@ void launch_gemm_update(const Launch& L, const MatInst* d, int ninst, int64_t k0
   count_launch(1);
 }
 
-void launch_rhs_swap(const Launch& L, const MatInst* d, int ninst, int32_t max_rhs, int reverse,
-                     int prec) {
-  dim3 grid((unsigned)((max_rhs + 63) / 64), (unsigned)ninst);
-  if (prec_is_single(prec))
-    k_rhs_swap<float><<<grid, 64, 0, L.stream>>>(d, reverse);
-  else
-    k_rhs_swap<double><<<grid, 64, 0, L.stream>>>(d, reverse);
-  count_launch(1);
-}
-
-template <typename R, bool EL, bool TR, bool UN>
-static void trsv_t(const Launch& L, const MatInst* d, int ninst, int64_t nmax, int32_t max_rhs) {
-  const int64_t nblk = (nmax + kTrsvNB - 1) / kTrsvNB;
-  for (int64_t b = 0; b < nblk; ++b) {
-    const int64_t blk = EL ? b : nblk - 1 - b;
-    const int64_t r0 = blk * kTrsvNB;
-    k_trsv_block<R, EL, TR, UN><<<dim3((unsigned)max_rhs, (unsigned)ninst), kTrsvNB, 0,
-                                  L.stream>>>(d, r0); count_launch(1);
-    const int64_t rows = EL ? (nmax - r0 - kTrsvNB) : r0;
-    if (rows > 0) {
-      k_trsv_update<R, EL, TR><<<dim3((unsigned)((rows + 255) / 256), (unsigned)max_rhs,
-                                      (unsigned)ninst),
-                                 256, 0, L.stream>>>(d, r0);
-      count_launch(1);
-    }
-  }
-}
-
-template <typename R, bool EL, bool TR, bool UN>
-static void trsv_big_t(const Launch& L, const MatInst* d, int ninst, int64_t nmax,
-                       int32_t max_rhs) {
-  constexpr size_t smem = diag_smem_bytes<R>();
-  static PerDeviceOnce attr;
-  attr.call([&] {
-    cudaFuncSetAttribute(k_trsv_diag<R, EL, TR, UN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-  });
-  // right-hand sides per update CTA: one, or a group sharing the matrix loads
-  constexpr int RG = sizeof(R) == 4 ? 8 : 4;
-  static PerDeviceOnce uattr;
-  uattr.call([] {
-    cudaFuncSetAttribute(k_trsv_big_update<R, EL, TR, RG>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)upd_smem_bytes<R, RG>());
-    cudaFuncSetAttribute(k_trsv_big_update_h<R, EL, RG>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)upd_smem_bytes<R, RG>());
-  });
-  const int64_t nblk = (nmax + kBigB - 1) / kBigB;
-  const unsigned gy = max_rhs >= 4 ? (unsigned)((max_rhs + RG - 1) / RG) : (unsigned)max_rhs;
-  auto diag = [&](cudaStream_t s, int64_t r0) {
-    k_trsv_diag<R, EL, TR, UN><<<dim3((unsigned)max_rhs, (unsigned)ninst), kDiagThreads, smem, s>>>(
-        d, r0);
-    count_launch(1);
-  };
-  auto update = [&](cudaStream_t s, int64_t r0, int64_t lo, int64_t hi) {  // rows [lo, hi)
-    if (hi <= lo) return;
-    const int64_t rows = hi - lo;
-    if (TR) {
-      const dim3 g((unsigned)((rows + kTrUpRows - 1) / kTrUpRows), gy, (unsigned)ninst);
-      if (max_rhs >= 4)
-        k_trsv_big_update_h<R, EL, RG><<<g, 256, upd_smem_bytes<R, RG>(), s>>>(d, r0, lo, hi);
-      else
-        k_trsv_big_update_h<R, EL, 1><<<g, 256, upd_smem_bytes<R, 1>(), s>>>(d, r0, lo, hi);
-    } else {
-      const dim3 g((unsigned)((rows + 255) / 256), gy, (unsigned)ninst);
-      if (max_rhs >= 4)
-        k_trsv_big_update<R, EL, TR, RG><<<g, 256, upd_smem_bytes<R, RG>(), s>>>(d, r0, lo, hi);
-      else
-        k_trsv_big_update<R, EL, TR, 1><<<g, 256, upd_smem_bytes<R, 1>(), s>>>(d, r0, lo, hi);
-    }
-    count_launch(1);
-  };
-  auto block_row = [&](int64_t b) { return (EL ? b : nblk - 1 - b) * kBigB; };
-  if (!L.side || nblk < 3 || L.n_events < 2 * (int)nblk + 1) {
-    for (int64_t b = 0; b < nblk; ++b) {
-      const int64_t r0 = block_row(b);
-      diag(L.stream, r0);
-      if (EL)
-        update(L.stream, r0, r0 + kBigB, nmax);
-      else
-        update(L.stream, r0, 0, r0);
-    }
-    return;
-  }
-  // Look-ahead: the main stream updates only the next block's rows and solves that block
-  // while the side stream updates every later row from the same solved block.  Both write
-  // x by read-modify-write, so the main stream's next-block update waits for the side
-  // stream's previous update (which also covered those rows), and the side stream's update
-  // waits for the block it reads.
-  cudaEvent_t* ev = L.events;
-  cudaEventRecord(ev[0], L.stream);  // the side stream starts after the main stream's work
-  cudaStreamWaitEvent(L.side, ev[0], 0);
-  diag(L.stream, block_row(0));
-  for (int64_t b = 0; b < nblk; ++b) {
-    const int64_t r0 = block_row(b);
-    cudaEvent_t e_diag = ev[1 + 2 * b], e_big = ev[2 + 2 * b];
-    cudaEventRecord(e_diag, L.stream);
-    if (b + 1 < nblk) {
-      const int64_t rn = block_row(b + 1);  // the next block in solve order
-      if (b > 0) cudaStreamWaitEvent(L.stream, ev[2 + 2 * (b - 1)], 0);
-      update(L.stream, r0, rn, rn + kBigB);
-      diag(L.stream, rn);
-    }
-    cudaStreamWaitEvent(L.side, e_diag, 0);
-    if (EL)
-      update(L.side, r0, r0 + 2 * kBigB, nmax);
-    else
-      update(L.side, r0, 0, r0 - kBigB);
-    cudaEventRecord(e_big, L.side);
-  }
-  cudaStreamWaitEvent(L.stream, ev[2 + 2 * (nblk - 1)], 0);  // join before returning
-}
-
-template <typename R>
-static void getrs_big_t(const Launch& L, const MatInst* d, int ninst, int64_t nmax,
-                        int32_t max_rhs, int trans, int swaps) {
-  dim3 g((unsigned)((nmax + 255) / 256), (unsigned)max_rhs, (unsigned)ninst);
-  if (!trans) {
-    if (swaps) {
-      k_copy_xy<R><<<g, 256, 0, L.stream>>>(d, 1);
-      k_gather_perm<R><<<g, 256, 0, L.stream>>>(d);
-      count_launch(2);
-    }
-    trsv_big_t<R, true, false, true>(L, d, ninst, nmax, max_rhs);
-    trsv_big_t<R, false, false, false>(L, d, ninst, nmax, max_rhs);
-  } else {
-    trsv_big_t<R, true, true, false>(L, d, ninst, nmax, max_rhs);
-    trsv_big_t<R, false, true, true>(L, d, ninst, nmax, max_rhs);
-    if (swaps) {
-      k_copy_xy<R><<<g, 256, 0, L.stream>>>(d, 1);
-      k_scatter_perm<R><<<g, 256, 0, L.stream>>>(d, max_rhs);
-      count_launch(2);
-    }
-  }
-}
-
 void launch_make_perm(const Launch& L, const MatInst* d, int ninst, int64_t nmax) {
   constexpr size_t kMaxSmem = 227 * 1024;
   const size_t smem = (size_t)nmax * sizeof(int32_t);
@@ -1731,74 +1094,6 @@ void launch_make_perm(const Launch& L, const MatInst* d, int ninst, int64_t nmax
   });
   k_make_perm<true><<<ninst, 256, smem, L.stream>>>(d);
   count_launch(1);
-}
-
-// Solve op(LU) x = b in place on MatInst.x.  trans = 0: A x = b; trans = 1: A^H x = b.
-// swaps = 0 leaves out the row interchanges (the (LU)^{-1} and (LU)^{-H} products that
-// LAPACK's condition estimator applies).
-void launch_getrs(const Launch& L, const MatInst* d, int ninst, int64_t nmax, int32_t max_rhs,
-                  int trans, int prec, int swaps, const TrsvWork* work) {
-  if (nmax <= 0 || ninst <= 0 || max_rhs <= 0) return;
-  if (work) {  // blocked two-level solve; needs MatInst.y and MatInst.perm
-    if (prec_is_single(prec))
-      getrs_big_t<float>(L, d, ninst, nmax, max_rhs, trans, swaps);
-    else
-      getrs_big_t<double>(L, d, ninst, nmax, max_rhs, trans, swaps);
-    return;
-  }
-  if (nmax <= trsv_full_max(prec)) {
-    const bool sp = prec_is_single(prec);
-    if (!trans) {
-      if (sp) {
-        if (swaps)
-          trsv_full_t<float, true, false, true, 1>(L, d, ninst, nmax, max_rhs);
-        else
-          trsv_full_t<float, true, false, true, 0>(L, d, ninst, nmax, max_rhs);
-        trsv_full_t<float, false, false, false, 0>(L, d, ninst, nmax, max_rhs);
-      } else {
-        if (swaps)
-          trsv_full_t<double, true, false, true, 1>(L, d, ninst, nmax, max_rhs);
-        else
-          trsv_full_t<double, true, false, true, 0>(L, d, ninst, nmax, max_rhs);
-        trsv_full_t<double, false, false, false, 0>(L, d, ninst, nmax, max_rhs);
-      }
-    } else {
-      if (sp) {
-        trsv_full_t<float, true, true, false, 0>(L, d, ninst, nmax, max_rhs);
-        if (swaps)
-          trsv_full_t<float, false, true, true, 2>(L, d, ninst, nmax, max_rhs);
-        else
-          trsv_full_t<float, false, true, true, 0>(L, d, ninst, nmax, max_rhs);
-      } else {
-        trsv_full_t<double, true, true, false, 0>(L, d, ninst, nmax, max_rhs);
-        if (swaps)
-          trsv_full_t<double, false, true, true, 2>(L, d, ninst, nmax, max_rhs);
-        else
-          trsv_full_t<double, false, true, true, 0>(L, d, ninst, nmax, max_rhs);
-      }
-    }
-    return;
-  }
-  if (!trans) {
-    if (swaps) launch_rhs_swap(L, d, ninst, max_rhs, 0, prec);
-    if (prec_is_single(prec)) {
-      trsv_t<float, true, false, true>(L, d, ninst, nmax, max_rhs);
-      trsv_t<float, false, false, false>(L, d, ninst, nmax, max_rhs);
-    } else {
-      trsv_t<double, true, false, true>(L, d, ninst, nmax, max_rhs);
-      trsv_t<double, false, false, false>(L, d, ninst, nmax, max_rhs);
-    }
-  } else {
-    // A^H = U^H L^H P: solve U^H (lower, non-unit), then L^H (upper, unit), then P^T.
-    if (prec_is_single(prec)) {
-      trsv_t<float, true, true, false>(L, d, ninst, nmax, max_rhs);
-      trsv_t<float, false, true, true>(L, d, ninst, nmax, max_rhs);
-    } else {
-      trsv_t<double, true, true, false>(L, d, ninst, nmax, max_rhs);
-      trsv_t<double, false, true, true>(L, d, ninst, nmax, max_rhs);
-    }
-    if (swaps) launch_rhs_swap(L, d, ninst, max_rhs, 1, prec);
-  }
 }
 
 }  // namespace bemgpu

@@ -7,7 +7,6 @@
 namespace bemgpu {
 
 constexpr int kPanelNB = 32;  // LU panel width (columns factored per getf2 launch)
-constexpr int kTrsvNB = 64;   // triangular-solve block (rows per diagonal block)
 
 // Factors the panel [k0, k0 + nb) of every instance; nmax: largest order, nact: instances
 // with rows left (the launch shape; the factor does not depend on it).  Returns whether the
@@ -23,13 +22,17 @@ void launch_trsm_panel(const Launch& L, const MatInst* d, int ninst, int64_t k0,
 // rows [k0 + nb, n) x columns [c_lo, c_hi) -= L21 U12 (SIMT)
 void launch_gemm_update(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb,
                         int64_t nmax, int64_t c_lo, int64_t c_hi, int prec);
-void launch_rhs_swap(const Launch& L, const MatInst* d, int ninst, int32_t max_rhs, int reverse,
-                     int prec);
-// Solve with the LU factor in place on MatInst.x (trans 1: A^H x = b; swaps 0 leaves
-// out the row interchanges).  With work != null the flag-synchronised block solve is
-// two-level blocked solve is used (needs MatInst.y and, for swaps, MatInst.perm).
+// Triangular solves (trsv.cu).  Bytes of the inverted diagonal blocks of a factor
+// (MatInst.dinv), and their computation.
+size_t tri_inv_bytes(int64_t n, int prec);
+void launch_tri_inv(const Launch& L, const MatInst* d, int ninst, int64_t nmax, int prec);
+// Solves with the factor in place on MatInst.x; MatInst.y is a second buffer.  trans 0:
+// A x = b, swaps 0 leaving out the row interchanges (MatInst.perm otherwise); trans 1:
+// (LU)^H x = b, without interchanges.  The instances of one launch agree on many =
+// many_rhs(nrhs), which selects the path by each system's own right-hand sides.
+bool many_rhs(int32_t nrhs);
 void launch_getrs(const Launch& L, const MatInst* d, int ninst, int64_t nmax, int32_t max_rhs,
-                  int trans, int prec, int swaps, const TrsvWork* work = nullptr);
+                  int trans, int prec, int swaps, bool many);
 // out[i] (kLinvB x kLinvB complex64, column-major) = -(L11^{-1} - I) of the unit lower
 // block at (k0, k0) of instance i (complex64 factors).
 void launch_linv_neg(const Launch& L, const MatInst* d, int ninst, int64_t k0, float2* const* outs);
