@@ -1745,8 +1745,8 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
     if (ra[q] <= 0 || rb[q] <= 0) return;
     {
       Prof pr(c, "oz_pack");
-      launch_oz_pack(L, dpa.as<OzPackInst>() + q * ni, ni, ra[q], kOzA);
-      launch_oz_pack(L, dpb.as<OzPackInst>() + q * ni, ni, rb[q], kOzB);
+      launch_oz_pack(L, dpa.as<OzPackInst>() + q * ni, ni, ra[q], B, kOzA);
+      launch_oz_pack(L, dpb.as<OzPackInst>() + q * ni, ni, rb[q], B, kOzB);
     }
     Prof pr(c, ph == kTrail ? "gemm_c128" : "gemm_oz");
     launch_oz_gemm(L, dge.as<OzGemmInst>() + q * ni, ni, &tiles[q * ni]);
@@ -2284,6 +2284,83 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
   return BEMGPU_OK;
 }
 
+// y = A x (mode 0) or y = b - A x with den = |b| + |A||x| (mode 1) of one system with many
+// right-hand sides: the vectors and the matrix, in row panels, are cut into digit slices and
+// multiplied on the tensor cores (gemm_oz.cu), the near corrections and the denominators are
+// added by their own kernels.  The row-wise products spend about 44 FP32 instructions per
+// complex product whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 34 ms (of
+// which 16 the products, 5 the slices of the matrix, 11 the denominators).
+int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
+  const Launch L = c->launch();
+  const int64_t n = v.n, kb = (n + kOzK - 1) / kOzK;
+  const int32_t R = v.nrhs;
+  Buf xp, xe, ap, ae;
+  TRY(alloc(c, oz_pack_bytes(R, (int)n, kOzB), &xp));
+  TRY(alloc(c, (size_t)kb * oz_exps(R, kOzB) * 4, &xe));
+  // row panels: about 8 GB of slices, at most a quarter of what the budget leaves
+  const size_t tile = oz_pack_bytes(128, (int)n, kOzA);
+  const uint64_t used = total_live(c), budget = root_of(c)->budget;
+  const uint64_t room = std::min<uint64_t>(8ull << 30, budget > used ? (budget - used) / 4 : 0);
+  const int64_t tiles = std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, (int64_t)(room / tile)));
+  const int64_t rows = tiles * 128;
+  TRY(alloc(c, tile * (size_t)tiles, &ap));
+  TRY(alloc(c, (size_t)kb * (size_t)rows * 4, &ae));
+  std::vector<OzPackInst> pk;
+  std::vector<OzGemmInst> ge;
+  pk.push_back(OzPackInst{v.x, v.ldx, 0, 0, R, (int32_t)n, 0, xp.p, xe.as<int32_t>()});
+  for (int64_t r0 = 0; r0 < n; r0 += rows) {
+    const int64_t m = std::min(rows, n - r0);
+    pk.push_back(OzPackInst{v.A, v.lda, r0, 0, m, (int32_t)n, v.a32, ap.p, ae.as<int32_t>()});
+    ge.push_back(OzGemmInst{ap.p, xp.p, ae.as<int32_t>(), xe.as<int32_t>(), v.y, v.ldy, r0, 0, m, R,
+                            (int32_t)n, 1});
+  }
+  Buf dpk, dge;
+  TRY(to_device(c, pk, &dpk));
+  TRY(to_device(c, ge, &dge));
+  if (mode == 1) {
+    CUDA_TRY(c, cudaMemcpy2DAsync(v.y, (size_t)v.ldy * 16, v.b, (size_t)v.ldb * 16, (size_t)n * 16,
+                                  (size_t)R, cudaMemcpyDeviceToDevice, c->stream));
+    Buf xa;
+    TRY(alloc(c, (size_t)n * R * 4, &xa));
+    launch_wide_abs(L, v, xa.as<float>());
+  } else {
+    CUDA_TRY(c, cudaMemset2DAsync(v.y, (size_t)v.ldy * 16, 0, (size_t)n * 16, (size_t)R, c->stream));
+  }
+  launch_oz_pack(L, dpk.as<OzPackInst>(), 1, R, (int)n, kOzB);
+  for (size_t p = 0; p < ge.size(); ++p) {
+    launch_oz_pack(L, dpk.as<OzPackInst>() + 1 + p, 1, ge[p].m, (int)n, kOzA, v.a32 != 0);
+    const int64_t t = oz_tiles(ge[p].m, R);
+    launch_oz_gemm(L, dge.as<OzGemmInst>() + p, 1, &t);
+  }
+  launch_wide_finish(L, v, mode);
+  CUDA_TRY(c, cudaGetLastError());
+  return BEMGPU_OK;
+}
+
+// Products of every instance: those with kWideRhs right-hand sides or more one by one on the
+// tensor cores, the others batched.  rows: as launch_gemv.  A system's path follows from its
+// own right-hand sides, so its results do not depend on the batch.
+int products(bemgpu_ctx* c, const std::vector<VecInst>& all, int mode, int rows) {
+  std::vector<VecInst> few;
+  int64_t nmax = 0;
+  int32_t rmax = 0;
+  for (const VecInst& v : all) {
+    if (v.nrhs >= kWideRhs && c->tensor_lu) {
+      TRY(wide_product(c, v, mode));
+      continue;
+    }
+    few.push_back(v);
+    nmax = std::max(nmax, v.n);
+    rmax = std::max(rmax, v.nrhs);
+  }
+  if (few.empty()) return BEMGPU_OK;
+  Buf d;
+  TRY(to_device(c, few, &d));
+  launch_gemv(c->launch(), d.as<VecInst>(), (int)few.size(), nmax, rmax, mode, rows);
+  CUDA_TRY(c, cudaGetLastError());
+  return BEMGPU_OK;
+}
+
 // residual y = b - A x, den, statistics for all rhs of the given instances
 int residual_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss,
                   std::vector<std::vector<double>>* stats) {
@@ -2302,18 +2379,28 @@ int residual_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss,
     Prof p(c, "residual");
     // rows per thread of the compact products, measured on the live pass (idempotent: the
     // last candidate's outputs are the pass's outputs)
-    bool any32 = false;
-    for (auto* s : ss) any32 |= s->f->a32;
-    const std::string key = "gemv/" + std::to_string(vi.size()) + "/" +
-                            std::to_string(log2_bucket(nmax)) + "/" + std::to_string(rmax > 1);
-    const int rows = any32 ? tune_pick(c, key, {2, 1},
-                                       [&](int r) {
-                                         launch_gemv(L, d.as<VecInst>(), (int)vi.size(), nmax,
-                                                     rmax, 1, r);
-                                       },
-                                       [] {})
-                           : 2;
-    launch_gemv(L, d.as<VecInst>(), (int)vi.size(), nmax, rmax, 1, rows);
+    std::vector<VecInst> few;
+    int64_t fn = 0;
+    int32_t fr = 0;
+    for (const VecInst& v : vi)
+      if (v.a32 && v.nrhs < kWideRhs) {
+        few.push_back(v);
+        fn = std::max(fn, v.n);
+        fr = std::max(fr, v.nrhs);
+      }
+    const std::string key = "gemv/" + std::to_string(few.size()) + "/" +
+                            std::to_string(log2_bucket(fn)) + "/" + std::to_string(fr > 1);
+    int rows = 2;
+    if (!few.empty()) {
+      Buf df;
+      TRY(to_device(c, few, &df));
+      rows = tune_pick(c, key, {2, 1},
+                       [&](int r) {
+                         launch_gemv(L, df.as<VecInst>(), (int)few.size(), fn, fr, 1, r);
+                       },
+                       [] {});
+    }
+    TRY(products(c, vi, 1, rows));
     launch_resid_stats(L, d.as<VecInst>(), (int)vi.size(), rmax);
   }
   stats->resize(ss.size());
@@ -2466,14 +2553,13 @@ int solve_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<i
       }
     }
     Prof p(c, "forcing");
-    Buf d1, d2, d3;
+    Buf d1, d3;
     if (!stack.empty()) {
       TRY(to_device(c, stack, &d1));
       launch_stack(L, d1.as<TraceInst>(), (int)stack.size(), nmax, rmax);
     }
     if (!gv.empty()) {
-      TRY(to_device(c, gv, &d2));
-      launch_gemv(L, d2.as<VecInst>(), (int)gv.size(), nmax, rmax, 0);
+      TRY(products(c, gv, 0, 2));
     }
     if (!cbie.empty()) {
       TRY(to_device(c, cbie, &d3));

@@ -1,4 +1,4 @@
-// Complex128 trailing update on the bfloat16 tensor cores: C -= A B, K <= 128.
+// Complex128 products on the bfloat16 tensor cores: C -= A B, in K-blocks of at most 128.
 //
 // The FP64 pipe of this part issues two FMAs per clock and SM (about 1.2 TFLOP/s over the
 // GPU), the bfloat16 tensor cores 1.9 PFLOP/s.  The update is therefore computed from
@@ -46,6 +46,7 @@ namespace bemgpu {
 
 constexpr int kOzM = 128, kOzN = 32;        // tile of C
 constexpr int kOzKC = 16;                   // K per chunk
+constexpr int kOzBlockChunks = kOzK / kOzKC;
 constexpr int kOzSlices = 7;
 constexpr int kOzLevels = 8;                // digit products p + q = 2..9
 constexpr int kOzABlock = kOzM * 64;        // one slice of a chunk, 64-byte rows
@@ -72,6 +73,25 @@ __device__ __forceinline__ long long oz_fixed(double x, int erow) {
   m = s >= 0 ? m << s : (m + (1LL << (-s - 1))) >> -s;
   return b < 0 ? -m : m;
 }
+__device__ __forceinline__ long long oz_fixed(float x, int erow) {  // zero when subnormal
+  const uint32_t b = __float_as_uint(x);
+  const int ex = (int)((b >> 23) & 0xFF);
+  long long m = (long long)((b & 0x7FFFFFu) | 0x800000u) << 29;
+  const int s = ex + 896 - erow + 2;  // exponent field of the same value in FP64
+  if (ex == 0 || s < -53) return 0;
+  m = s >= 0 ? m << s : (m + (1LL << (-s - 1))) >> -s;
+  return (int32_t)b < 0 ? -m : m;
+}
+// FP64 exponent field of the larger of two magnitudes (0: none)
+__device__ __forceinline__ int oz_expo(double2 v) {
+  return (int)(max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu,
+                   (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu) >> 20);
+}
+__device__ __forceinline__ int oz_expo(float2 v) {
+  const int e = (int)(max(__float_as_uint(v.x) & 0x7FFFFFFFu,
+                          __float_as_uint(v.y) & 0x7FFFFFFFu) >> 23);
+  return e == 0 ? 0 : e == 0xFF ? 0x7FF : e + 896;
+}
 // bfloat16 bits of two digits (biased by 128, 0..256)
 __device__ __forceinline__ uint32_t oz_bf16x2(uint32_t d0, uint32_t d1) {
   const float f0 = __uint_as_float(0x4B000000u | d0) - 8388736.0f;
@@ -79,43 +99,44 @@ __device__ __forceinline__ uint32_t oz_bf16x2(uint32_t d0, uint32_t d1) {
   return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
 
-// One CTA per R rows of an operand tile of T rows, all K: the rows' exponents, then the
+// One CTA per R rows of an operand tile of T rows and K-block: the rows' exponents, then the
 // slices, eight K values of one row per work item (14 vector stores of eight digits).  Integer
 // work on small pieces: R is a quarter of the tile so that an operand of a few thousand rows
 // fills the GPU.
-template <int T, int R, bool TRANS>
+template <class V2, int T, int R, bool TRANS>
 __global__ void __launch_bounds__(256) k_oz_pack(const OzPackInst* __restrict__ insts) {
   const OzPackInst& P = insts[blockIdx.y];
+  if ((P.single != 0) != (sizeof(V2) == sizeof(float2))) return;
   const int64_t row0 = (int64_t)blockIdx.x * R;
   // rows beyond the operand up to the end of its last tile are packed as zeros
-  if (row0 >= (P.rows + T - 1) / T * T || P.kk <= 0) return;
+  const int kb = (int)blockIdx.z * kOzK, kk = min(kOzK, P.kk - kb);
+  if (row0 >= (P.rows + T - 1) / T * T || kk <= 0) return;
+  const int64_t k0 = P.k0 + kb;
   constexpr int kBlock = T * 64, kChunk = kOzSlices * kBlock;
   constexpr int kPer = 256 / R;  // threads per row in the exponent pass
   __shared__ int s_exp[R];
-  const double2* A = static_cast<const double2*>(P.a);
+  const V2* A = static_cast<const V2*>(P.a);
   const int tid = threadIdx.x;
   for (int r = tid; r < R; r += 256) s_exp[r] = 0;
   __syncthreads();
   {
     const int r = TRANS ? tid / kPer : tid % R, g = TRANS ? tid % kPer : tid / R;
     const int64_t gr = row0 + r;
-    uint32_t mx = 0;
+    int mx = 0;
     if (gr < P.rows)
-      for (int k = g; k < P.kk; k += kPer) {
-        const double2 v = A[TRANS ? (P.k0 + k) + (P.r0 + gr) * P.lda
-                                  : (P.r0 + gr) + (P.k0 + k) * P.lda];
-        mx = max(mx, max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu,
-                         (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu));
-      }
-    atomicMax(&s_exp[r], (int)(mx >> 20));
+      for (int k = g; k < kk; k += kPer)
+        mx = max(mx, oz_expo(A[TRANS ? (k0 + k) + (P.r0 + gr) * P.lda
+                                     : (P.r0 + gr) + (k0 + k) * P.lda]));
+    atomicMax(&s_exp[r], mx);
   }
   __syncthreads();
+  int32_t* exps = P.exps + (int64_t)blockIdx.z * ((P.rows + T - 1) / T * T);
   for (int r = tid; r < R; r += 256) {
     const int e = s_exp[r];
-    P.exps[row0 + r] = e == 0x7FF ? kOzNaN : e - 1021;
+    exps[row0 + r] = e == 0x7FF ? kOzNaN : e - 1021;
   }
-  const int chunks = (P.kk + kOzKC - 1) / kOzKC;
-  uint8_t* out = static_cast<uint8_t*>(P.out) + (size_t)(row0 / T) * chunks * kChunk;
+  const int all = (P.kk + kOzKC - 1) / kOzKC, chunks = (kk + kOzKC - 1) / kOzKC;
+  uint8_t* out = static_cast<uint8_t*>(P.out) + ((size_t)(row0 / T) * all + kb / kOzKC) * kChunk;
   const int rt = (int)(row0 % T);  // first row inside the tile
   const int groups = chunks * 2;  // eight K values each
   for (int item = tid; item < R * groups; item += 256) {
@@ -126,9 +147,9 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackInst* __restrict__ 
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int k = g * 8 + e;
-      double2 v = make_double2(0.0, 0.0);
-      if (gr < P.rows && k < P.kk)
-        v = A[TRANS ? (P.k0 + k) + (P.r0 + gr) * P.lda : (P.r0 + gr) + (P.k0 + k) * P.lda];
+      V2 v = V2{0, 0};
+      if (gr < P.rows && k < kk)
+        v = A[TRANS ? (k0 + k) + (P.r0 + gr) * P.lda : (P.r0 + gr) + (k0 + k) * P.lda];
       // digits + 128 in the bytes (byte 6 keeps a carry into bit 8)
       zr[e] = (unsigned long long)(oz_fixed(v.x, erow) + 0x0080808080808080LL);
       zi[e] = (unsigned long long)(oz_fixed(v.y, erow) + 0x0080808080808080LL);
@@ -192,10 +213,16 @@ __device__ __forceinline__ void oz_coords(const OzShared& S, const OzGemmInst* i
       hi = mid - 1;
   }
   const int64_t local = t - (int64_t)S.prefix[lo];
-  const int64_t mtiles = (insts[lo].m + kOzM - 1) / kOzM;
   *inst = lo;
-  *mt = local % mtiles;
-  *nt = local / mtiles;
+  if (insts[lo].n_first) {
+    const int64_t ntiles = (insts[lo].n + kOzN - 1) / kOzN;
+    *nt = local % ntiles;
+    *mt = local / ntiles;
+  } else {
+    const int64_t mtiles = (insts[lo].m + kOzM - 1) / kOzM;
+    *mt = local % mtiles;
+    *nt = local / mtiles;
+  }
 }
 
 // 2^(e - 28), exact (subnormal at the lower end); NaN for a row with a NaN or an infinity
@@ -294,10 +321,15 @@ __global__ void __launch_bounds__(kOzThreads, 1)
         int64_t mt, nt;
         oz_coords(S, insts, ninst, t, &inst, &mt, &nt);
         const int chunks = (insts[inst].kk + kOzKC - 1) / kOzKC;
-        if (!tc_wait(&S.tempty, tphase ^ 1, err, abort_flag)) break;
-        tc_fence_after();
         bool ok = true;
         for (int c = 0; c < chunks; ++c) {
+          if (c % kOzBlockChunks == 0) {  // a K-block begins with empty accumulators
+            if (!tc_wait(&S.tempty, tphase ^ 1, err, abort_flag)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+          }
           if (!tc_wait(&S.full[stage], phase, err, abort_flag)) {
             ok = false;
             break;
@@ -319,7 +351,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             mma_bf16(dr, a_im, b_im, neg, 1u);
             mma_bf16(di, a_im, b_re, pos, 1u);
           };
-          if (c == 0) {  // slice 2 starts levels 3..9, the leading digits' product level 2
+          if (c % kOzBlockChunks == 0) {  // slice 2 starts levels 3..9, the leading digits' product level 2
             products(1, 0, kOzSlices, 0u);
             products(0, 0, 1, 0u);
             products(0, 1, kOzSlices, 1u);
@@ -334,10 +366,12 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             stage = 0;
             phase ^= 1;
           }
+          if (c % kOzBlockChunks == kOzBlockChunks - 1 || c + 1 == chunks) {
+            mma_commit(&S.tfull);
+            tphase ^= 1;
+          }
         }
         if (!ok) break;
-        mma_commit(&S.tfull);
-        tphase ^= 1;
       }
     }
   } else {
@@ -356,50 +390,60 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       const int64_t gr = mt * kOzM + row;
       const int64_t gc = nt * kOzN + half * 16;
       const int ncol = gr < G.m ? (int)max((int64_t)0, min((int64_t)16, G.n - gc)) : 0;
-      const double sr = gr < G.m ? oz_scale(G.aexp[gr]) : 0.0;
       double2* C = static_cast<double2*>(G.c) + (G.c_r0 + gr) + (G.c_c0 + gc) * G.ldc;
-      const bool ok = tc_wait(&S.tfull, tphase, err, abort_flag);
-      if (!__all_sync(0xffffffffu, ok)) break;
-      tc_fence_after();
-      tphase ^= 1;
-      long long v[2][16];
+      const int64_t as = (G.m + kOzM - 1) / kOzM * kOzM, bs = (G.n + kOzN - 1) / kOzN * kOzN;
+      const int blocks = (G.kk + kOzK - 1) / kOzK;
+      bool gone = false;
+      for (int kb = 0; kb < blocks; ++kb) {
+        const double sr = gr < G.m ? oz_scale(G.aexp[kb * as + gr]) : 0.0;
+        const int32_t* be = G.bexp + kb * bs;
+        const bool ok = tc_wait(&S.tfull, tphase, err, abort_flag);
+        if (!__all_sync(0xffffffffu, ok)) {
+          gone = true;
+          break;
+        }
+        tc_fence_after();
+        tphase ^= 1;
+        long long v[2][16];
 #pragma unroll
-      for (int part = 0; part < 2; ++part)
+        for (int part = 0; part < 2; ++part)
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          float f[kOzLevels][8];
+          for (int g = 0; g < 2; ++g) {
+            float f[kOzLevels][8];
 #pragma unroll
-          for (int d = 0; d < kOzLevels; ++d)
-            tmem_ld8(tl + part * kOzIm + (uint32_t)(d * kOzN + g * 8), f[d]);
-          tmem_wait_ld();
+            for (int d = 0; d < kOzLevels; ++d)
+              tmem_ld8(tl + part * kOzIm + (uint32_t)(d * kOzN + g * 8), f[d]);
+            tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            // levels 2..4 in units of 2^-32, levels 5..9 in units of 2^-64, sum in 2^-56
-            const long long h = (long long)__float2int_rn(f[0][j]) * 65536 +
-                                (long long)__float2int_rn(f[1][j]) * 256 +
-                                (long long)__float2int_rn(f[2][j]);
-            const long long l = (long long)__float2int_rn(f[3][j]) * 16777216 +
-                                (long long)__float2int_rn(f[4][j]) * 65536 +
-                                (long long)__float2int_rn(f[5][j]) * 256 +
-                                (long long)(__float2int_rn(f[6][j]) +
-                                            ((__float2int_rn(f[7][j]) + 128) >> 8));
-            v[part][g * 8 + j] = (h << 24) + ((l + 128) >> 8);
+            for (int j = 0; j < 8; ++j) {
+              // levels 2..4 in units of 2^-32, levels 5..9 in units of 2^-64, sum in 2^-56
+              const long long h = (long long)__float2int_rn(f[0][j]) * 65536 +
+                                  (long long)__float2int_rn(f[1][j]) * 256 +
+                                  (long long)__float2int_rn(f[2][j]);
+              const long long l = (long long)__float2int_rn(f[3][j]) * 16777216 +
+                                  (long long)__float2int_rn(f[4][j]) * 65536 +
+                                  (long long)__float2int_rn(f[5][j]) * 256 +
+                                  (long long)(__float2int_rn(f[6][j]) +
+                                              ((__float2int_rn(f[7][j]) + 128) >> 8));
+              v[part][g * 8 + j] = (h << 24) + ((l + 128) >> 8);
+            }
           }
-        }
-      tc_fence_before();
-      mbar_arrive(&S.tempty);
-      double2 x[16];  // every load in flight before the first store
+        tc_fence_before();
+        mbar_arrive(&S.tempty);
+        double2 x[16];  // every load in flight before the first store
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (j < ncol) x[j] = C[(int64_t)j * G.ldc];
+        for (int j = 0; j < 16; ++j)
+          if (j < ncol) x[j] = C[(int64_t)j * G.ldc];
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (j < ncol) {
-          const double sc = sr * oz_scale(G.bexp[gc + j]);  // 2^(e + f - 56)
-          x[j].x -= (double)v[0][j] * sc;
-          x[j].y -= (double)v[1][j] * sc;
-          C[(int64_t)j * G.ldc] = x[j];
-        }
+        for (int j = 0; j < 16; ++j)
+          if (j < ncol) {
+            const double sc = sr * oz_scale(be[gc + j]);  // 2^(e + f - 56)
+            x[j].x -= (double)v[0][j] * sc;
+            x[j].y -= (double)v[1][j] * sc;
+            C[(int64_t)j * G.ldc] = x[j];
+          }
+      }
+      if (gone) break;
     }
   }
   tc_fence_before();
@@ -427,15 +471,20 @@ int64_t oz_tiles(int64_t m, int64_t n) {
   return m > 0 && n > 0 ? ((m + kOzM - 1) / kOzM) * ((n + kOzN - 1) / kOzN) : 0;
 }
 
-void launch_oz_pack(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows,
-                    OzSide side) {
-  if (ninst <= 0 || max_rows <= 0) return;
+void launch_oz_pack(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows, int max_kk,
+                    OzSide side, bool single) {
+  if (ninst <= 0 || max_rows <= 0 || max_kk <= 0) return;
   const int64_t t = side == kOzA ? kOzM : kOzN;
-  const dim3 grid((unsigned)((max_rows + t - 1) / t * 4), (unsigned)ninst);
-  if (side == kOzA)
-    k_oz_pack<kOzM, kOzM / 4, false><<<grid, 256, 0, L.stream>>>(d);
-  else
-    k_oz_pack<kOzN, kOzN / 4, true><<<grid, 256, 0, L.stream>>>(d);
+  const dim3 grid((unsigned)((max_rows + t - 1) / t * 4), (unsigned)ninst,
+                  (unsigned)((max_kk + kOzK - 1) / kOzK));
+  if (side == kOzA) {
+    if (single)
+      k_oz_pack<float2, kOzM, kOzM / 4, false><<<grid, 256, 0, L.stream>>>(d);
+    else
+      k_oz_pack<double2, kOzM, kOzM / 4, false><<<grid, 256, 0, L.stream>>>(d);
+  } else {
+    k_oz_pack<double2, kOzN, kOzN / 4, true><<<grid, 256, 0, L.stream>>>(d);
+  }
   count_launch(1);
 }
 

@@ -5,7 +5,7 @@
 
 namespace bemgpu {
 
-constexpr int kOzK = 128;        // largest K of one update (exact accumulation, gemm_oz.cu)
+constexpr int kOzK = 128;        // K of one exact accumulation (gemm_oz.cu); longer K in blocks
 constexpr int kOzMaxInst = 256;  // instances per GEMM launch (more are split by the wrapper)
 
 // One operand panel to cut into digit slices.
@@ -15,10 +15,11 @@ struct OzPackInst {
   int64_t r0;      // first operand row (side A: matrix row; side B: matrix column)
   int64_t k0;      // first K index (side A: matrix column; side B: matrix row)
   int64_t rows;    // operand rows (M or N extent); 0: nothing to do
-  int32_t kk;      // K extent, at most kOzK
-  int32_t pad;
+  int32_t kk;      // K extent
+  int32_t single;  // 1: complex64 matrix
   void* out;       // slice images, oz_pack_bytes(rows, kk, side)
-  int32_t* exps;   // exponent of every operand row (oz_exps(rows, side) values)
+  int32_t* exps;   // exponent of every operand row and block of kOzK columns, block by block:
+                   // oz_exps(rows, side) values each
 };
 
 // One C -= A B update: C block rows [c_r0, c_r0 + m), columns [c_c0, c_c0 + n).
@@ -32,7 +33,7 @@ struct OzGemmInst {
   int64_t c_r0, c_c0;
   int64_t m, n;    // 0: nothing to do
   int32_t kk;
-  int32_t pad;
+  int32_t n_first;  // 1: neighbouring CTAs take neighbouring columns (A larger than L2)
 };
 
 enum OzSide { kOzA = 0, kOzB = 1 };
@@ -41,9 +42,10 @@ size_t oz_exps(int64_t rows, OzSide side);
 int64_t oz_tiles(int64_t m, int64_t n);  // tiles of one update
 
 #ifdef __CUDACC__
-// side A: element (r, k) at r + k lda; side B: at k + r lda
-void launch_oz_pack(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows,
-                    OzSide side);
+// side A: element (r, k) at r + k lda, single: the complex64 instances (the others are
+// skipped); side B: at k + r lda, complex128
+void launch_oz_pack(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows, int max_kk,
+                    OzSide side, bool single = false);
 // tiles[i]: oz_tiles of instance i (host array), for the grid of each launch
 void launch_oz_gemm(const Launch& L, const OzGemmInst* d, int ninst, const int64_t* tiles);
 #endif

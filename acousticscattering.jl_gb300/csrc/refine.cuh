@@ -56,6 +56,12 @@ void launch_scale_copy(const Launch& L, const VecInst* d, int ninst, int64_t nma
 // the compact-storage product (1 or 2; results identical)
 void launch_gemv(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int32_t max_rhs,
                  int mode, int rows = 2);
+// Products of one system with many vectors (api.cu:wide_product): den = |b| + |A||x|, and the
+// end of a product whose sum the tensor-core kernel left in y (mode 0: y = -A x without the
+// near corrections, mode 1: y = b - A x without them).
+constexpr int kWideRhs = 16;  // right-hand sides of a system from which they are used
+void launch_wide_abs(const Launch& L, const VecInst& v, float* xa);  // xa: n x nrhs scratch
+void launch_wide_finish(const Launch& L, const VecInst& v, int mode);
 // compact instances: out (complex128, ld n) += the near corrections, each scaled by
 // 1 / (rows_i cols_j) (unit_scales = 0) or unscaled (unit_scales = 1)
 void launch_near_add(const Launch& L, const VecInst* d, int ninst, int64_t max_near,
