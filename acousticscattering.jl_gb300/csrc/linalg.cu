@@ -1018,6 +1018,9 @@ bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_
 
 void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int64_t c_lo,
                   int64_t c_hi, int64_t s_lo, int64_t s_hi, int prec) {
+  // the excluded block may reach past the last column
+  s_lo = std::min(s_lo, c_hi);
+  s_hi = std::min(s_hi, c_hi);
   const int64_t cols = (c_hi - c_lo) - (s_hi - s_lo);
   if (cols <= 0) return;
   dim3 grid((unsigned)((cols + kSwpCols - 1) / kSwpCols), (unsigned)ninst);
