@@ -4932,7 +4932,7 @@ int bemgpu_pressure_region(bemgpu_solution* sol, int32_t rhs, int64_t npts, cons
   if (s->mesh->nystrom) return nystrom_pressure(c, s, rhs, npts, points, field, out);
   std::vector<double> pts(points, points + 3 * npts);
   std::vector<double> dir(s->dirs.begin() + 3 * rhs, s->dirs.begin() + 3 * rhs + 3);
-  Buf dp, dd, dout, dreg;
+  Buf dp, dd, dout, dreg, dint;
   TRY(upload(c, pts, &dp));
   TRY(upload(c, dir, &dd));
   TRY(alloc(c, (size_t)npts * 16, &dout));
@@ -4954,6 +4954,11 @@ int bemgpu_pressure_region(bemgpu_solution* sol, int32_t rhs, int64_t npts, cons
   P.eta = s->mesh->eta;
   P.field = field;
   P.fluid = fluid ? 1 : 0;
+  if (fluid && !s->region) {
+    TRY(alloc(c, (size_t)s->mesh->n * 32, &dint));
+    P.pi = dint.as<double>();
+    P.qi = dint.as<double>() + 2 * (size_t)s->mesh->n;
+  }
   if (s->region) {  // coupled regions: the union's surfaces and the solved unknowns
     const int32_t count = (int32_t)s->parents.size();
     P.nsurf = count;

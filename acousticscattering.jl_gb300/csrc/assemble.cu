@@ -46,7 +46,7 @@ __device__ __forceinline__ void store_n(void* base, bool c64, double* dnear, int
 
 template <typename R, int KIND>
 __global__ void __launch_bounds__(kAsmRows) k_assemble_regular(const AsmInst* __restrict__ insts,
-                                                               int* err) {
+                                                               int cols, int* err) {
   constexpr int kCols = Prec<R>::kCols;
   constexpr int kRec = Prec<R>::kRec;
   __shared__ alignas(128) R srec[kCols * kRec];
@@ -54,9 +54,9 @@ __global__ void __launch_bounds__(kAsmRows) k_assemble_regular(const AsmInst* __
   const AsmInst& I = insts[blockIdx.z];
   const int64_t n = I.n;
   const int64_t i0 = (int64_t)blockIdx.x * kAsmRows;
-  const int64_t j0 = (int64_t)blockIdx.y * kCols;
+  const int64_t j0 = (int64_t)blockIdx.y * cols;
   if (i0 >= n || j0 >= n) return;  // uniform over the CTA
-  const int cnt = (int)min((int64_t)kCols, n - j0);
+  const int cnt = (int)min((int64_t)cols, n - j0);
   const R* recs = Prec<R>::recs(I);
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -133,8 +133,7 @@ __global__ void __launch_bounds__(kAsmRows) k_assemble_regular(const AsmInst* __
       e.S = e.D = e.K = e.H = cx<R>{0, 0};
       t = e;
       constexpr bool kh = (KIND == kAsmMuller);
-      regular_panel<R, kh>(rec, x, nx, ke, e);
-      regular_panel<R, kh>(rec, x, nx, ki, t);
+      regular_panel2<R, kh>(rec, x, nx, ke, ki, e, t);
       // block combinations in the quadrature precision (no FP64 work on the FP32 path)
       const R g = (R)I.g, ginv = (R)(1.0 / I.g);
       cx<R> a11, a12, a21, a22;
@@ -287,15 +286,20 @@ void launch_near_laplace(const Launch& L, const double* panels, const double* ve
 template <typename R>
 static void launch_regular_t(const Launch& L, const AsmInst* d, int ninst, int64_t nmax,
                              int kind) {
-  constexpr int kCols = Prec<R>::kCols;
-  dim3 grid((unsigned)((nmax + kAsmRows - 1) / kAsmRows), (unsigned)((nmax + kCols - 1) / kCols),
-            (unsigned)ninst);
+  // source panels per CTA: the staging buffer's, halved until the grid has about four CTAs per
+  // SM (a 320-panel body in 64-column CTAs of FP64 is 15 CTAs: 1.16 ms, 0.14 ms in
+  // 4-column CTAs)
+  int cols = Prec<R>::kCols;
+  const int64_t row_tiles = (nmax + kAsmRows - 1) / kAsmRows;
+  while (cols > 4 && row_tiles * ((nmax + cols - 1) / cols) * ninst < 4 * (int64_t)device_sm_count())
+    cols /= 2;
+  dim3 grid((unsigned)row_tiles, (unsigned)((nmax + cols - 1) / cols), (unsigned)ninst);
   switch (kind) {
-    case kAsmBM: k_assemble_regular<R, kAsmBM><<<grid, kAsmRows, 0, L.stream>>>(d, L.err_flag); count_launch(1); break;
-    case kAsmCBIE: k_assemble_regular<R, kAsmCBIE><<<grid, kAsmRows, 0, L.stream>>>(d, L.err_flag); count_launch(1); break;
-    case kAsmMuller: k_assemble_regular<R, kAsmMuller><<<grid, kAsmRows, 0, L.stream>>>(d, L.err_flag); count_launch(1); break;
-    case kAsmRegion: k_assemble_regular<R, kAsmRegion><<<grid, kAsmRows, 0, L.stream>>>(d, L.err_flag); count_launch(1); break;
-    default: k_assemble_regular<R, kAsmFluidCBIE><<<grid, kAsmRows, 0, L.stream>>>(d, L.err_flag); count_launch(1); break;
+    case kAsmBM: k_assemble_regular<R, kAsmBM><<<grid, kAsmRows, 0, L.stream>>>(d, cols, L.err_flag); count_launch(1); break;
+    case kAsmCBIE: k_assemble_regular<R, kAsmCBIE><<<grid, kAsmRows, 0, L.stream>>>(d, cols, L.err_flag); count_launch(1); break;
+    case kAsmMuller: k_assemble_regular<R, kAsmMuller><<<grid, kAsmRows, 0, L.stream>>>(d, cols, L.err_flag); count_launch(1); break;
+    case kAsmRegion: k_assemble_regular<R, kAsmRegion><<<grid, kAsmRows, 0, L.stream>>>(d, cols, L.err_flag); count_launch(1); break;
+    default: k_assemble_regular<R, kAsmFluidCBIE><<<grid, kAsmRows, 0, L.stream>>>(d, cols, L.err_flag); count_launch(1); break;
   }
 }
 

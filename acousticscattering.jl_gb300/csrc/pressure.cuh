@@ -11,6 +11,8 @@ struct PressureInst {
   int64_t n;             // panels
   const double* p;       // scattered pressure trace of one rhs (complex128, n)
   const double* q;       // scattered normal-derivative trace (complex128, n)
+  double* pi;            // scratch for a fluid body's interior traces (complex128, n each)
+  double* qi;
   const double* dir;     // incidence direction (3)
   const double* points;  // 3 x npts
   int64_t npts;
