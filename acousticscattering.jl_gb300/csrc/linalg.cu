@@ -388,7 +388,7 @@ struct alignas(16) PivSlot {
 // CTA of 256)
 template <typename R, int W, int RPT, int T_>
 __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ insts, int64_t k0,
-                                                     int nb) {
+                                                     int nb, int share) {
   using C = cx<R>;
   const unsigned rank = cluster_rank(), cs = cluster_size();
   const MatInst& M = insts[blockIdx.x / cs];
@@ -404,13 +404,14 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
   __shared__ int32_t s_phys[kPanelNB];      // row of every pivot
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int T = blockDim.x, nw = T >> 5;
-  const int64_t stride = (int64_t)cs * T;
-  const int64_t g = k0 + (int64_t)rank * T + tid;
+  // this CTA's rows: share of them from k0 + rank share on, T at a time
+  const int64_t stride = T;
+  const int64_t g = k0 + (int64_t)rank * share + tid;
   int32_t pos[RPT], fz[RPT];  // position; step at which the row became a pivot (nb: not yet)
 #pragma unroll
   for (int t = 0; t < RPT; ++t) {
     pos[t] = (int32_t)(g + t * stride);
-    fz[t] = g + t * stride < n ? kPanelNB : -1;  // -1: no row
+    fz[t] = tid + t * T < share && g + t * stride < n ? kPanelNB : -1;  // -1: no row
   }
   for (int s0 = 0; s0 < nbe; s0 += W) {
     const int wn = min(W, nbe - s0);
@@ -557,14 +558,13 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
 // warp barrier and stores them at their destinations.
 constexpr int kSwpMaxNb = 128;   // interchanges per launch
 constexpr int kSwpWarps = 8;
-constexpr int kSwpCols = 128;    // columns per CTA
 constexpr int kSwpHash = 512;    // open-addressing table of touched rows beyond the block
 
 template <typename R>
 __global__ void __launch_bounds__(kSwpWarps * 32) k_laswp(const MatInst* __restrict__ insts,
                                                          int64_t k0, int nb, int64_t c_lo,
                                                          int64_t c_hi, int64_t s_lo,
-                                                         int64_t s_hi) {
+                                                         int64_t s_hi, int cols) {
   const MatInst& M = insts[blockIdx.y];
   const int64_t n = M.n;
   if (!M.active || k0 >= n) return;
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kSwpWarps * 32) k_laswp(const MatInst* __restr
     if (j >= s_lo) j += skip;
     return (j >= n || j >= c_hi) ? (int64_t)-1 : j;
   };
-  const int64_t q0 = (int64_t)blockIdx.x * kSwpCols;
+  const int64_t q0 = (int64_t)blockIdx.x * cols;
   if (column(q0) < 0) return;  // uniform per CTA
   __shared__ int32_t piv[kSwpMaxNb];
   __shared__ int32_t pos[2 * kSwpMaxNb], src[2 * kSwpMaxNb];  // slot: row, its source row
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(kSwpWarps * 32) k_laswp(const MatInst* __restr
   const int lane = tid & 31, wid = tid >> 5;
   const int64_t lda = M.lda;
   constexpr int kPer = 2 * kSwpMaxNb / 32;
-  for (int q = wid; q < kSwpCols; q += kSwpWarps) {
+  for (int q = wid; q < cols; q += kSwpWarps) {
     const int64_t j = column(q0 + q);
     if (j < 0) break;
     cx<R> v[kPer];
@@ -646,29 +646,24 @@ __global__ void __launch_bounds__(kSwpWarps * 32) k_laswp(const MatInst* __restr
 
 // ------------------------------------------------------------------ trsm (U12)
 // U12 = L11^{-1} A12 for the columns [c_lo, min(c_hi, n)); L11 = unit lower nbe x nbe
-// block at (k0, k0), staged once per CTA in shared memory; each warp solves TrsmCols<R>
-// columns (column = warp + kTrsmWarps * t), lane r holding rows r, r + 32, ...
-// complex128 takes one column per warp: it solves the at most 96 columns to the right of a
-// 32-column panel inside a 128-column block, 8 per CTA, so that the FP64 work (two FMAs per
-// clock and SM) spreads over a dozen SMs.
+// block at (k0, k0), staged once per CTA in shared memory; each warp solves per_warp columns
+// (column = warp + kTrsmWarps * t), lane r holding rows r, r + 32, ...
+// The columns are the at most 96 to the right of a 32-column panel inside a 128-column block.
+// A warp takes per_warp of them, one after the other (32 dependent steps each): few for one
+// system, where 16 made one CTA do all the work (8 us a launch, 2 us with two), 16 in a large
+// batch, whose CTAs then stage the block once (see the launcher).
 constexpr int kTrsmWarps = 8;
-template <typename R>
-struct TrsmCols {
-  static constexpr int value = sizeof(R) == 4 ? 16 : 1;
-};
-
 template <typename R, int NB>
 __global__ void __launch_bounds__(kTrsmWarps * 32) k_trsm_panel(const MatInst* __restrict__ insts,
                                                                int64_t k0, int64_t c_lo,
-                                                               int64_t c_hi) {
-  constexpr int kTrsmCols = TrsmCols<R>::value;
+                                                               int64_t c_hi, int per_warp) {
   const MatInst& M = insts[blockIdx.y];
   const int64_t n = M.n;
   if (!M.active || k0 >= n) return;
   const int nbe = (int)min((int64_t)NB, n - k0);
   const int64_t lda = M.lda;
   const int64_t c_end = min(c_hi, n);
-  const int64_t cta0 = c_lo + (int64_t)blockIdx.x * kTrsmWarps * kTrsmCols;
+  const int64_t cta0 = c_lo + (int64_t)blockIdx.x * kTrsmWarps * per_warp;
   if (cta0 >= c_end) return;  // uniform per CTA
   extern __shared__ __align__(16) unsigned char trsm_smem[];
   cx<R>* sL = reinterpret_cast<cx<R>*>(trsm_smem);  // [NB][NB + 1]
@@ -679,7 +674,7 @@ __global__ void __launch_bounds__(kTrsmWarps * 32) k_trsm_panel(const MatInst* _
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   constexpr int kPer = NB / 32;
-  for (int tcol = 0; tcol < kTrsmCols; ++tcol) {
+  for (int tcol = 0; tcol < per_warp; ++tcol) {
     const int64_t j = cta0 + wid + (int64_t)kTrsmWarps * tcol;
     if (j >= c_end) break;
     cx<R> x[kPer];
@@ -789,9 +784,19 @@ __global__ void __launch_bounds__(kGThreads) k_gemm_update(const MatInst* __rest
 // column j (one warp per column); out (ld kLinvB, complex64) receives -N.
 constexpr int kLinvB = 128;
 
-__global__ void __launch_bounds__(256) k_linv_neg(const MatInst* __restrict__ insts, int64_t k0,
-                                                  float2* const* outs) {
-  const MatInst& M = insts[blockIdx.x];
+// gridDim.x CTAs per instance take the columns j = blockIdx.x + gridDim.x i (spread over the
+// triangle for balance), a warp one column after the other.  One CTA per instance took 32 us a
+// launch (16 columns per warp); 32 CTAs take 5, but each stages the block, so a batch uses
+// fewer (linv_ctas).
+constexpr int kLinvWarps = 8;
+static int linv_ctas(int ninst) {
+  int n = 32;
+  while (n > 1 && (int64_t)n * ninst > 2 * (int64_t)device_sm_count()) n /= 2;
+  return n;
+}
+__global__ void __launch_bounds__(kLinvWarps * 32) k_linv_neg(
+    const MatInst* __restrict__ insts, int64_t k0, float2* const* outs) {
+  const MatInst& M = insts[blockIdx.y];
   const int64_t n = M.n;
   if (!M.active || k0 >= n) return;
   const int nbe = (int)min((int64_t)kLinvB, n - k0);
@@ -803,10 +808,10 @@ __global__ void __launch_bounds__(256) k_linv_neg(const MatInst* __restrict__ in
     sL[r * (kLinvB + 1) + c] = ld<float>(M.a, (k0 + r) + (k0 + c) * lda);
   }
   __syncthreads();
-  float2* out = outs[blockIdx.x];
+  float2* out = outs[blockIdx.y];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   constexpr int kPer = kLinvB / 32;
-  for (int j = wid; j < kLinvB; j += 8) {
+  for (int j = blockIdx.x + gridDim.x * wid; j < kLinvB; j += gridDim.x * (blockDim.x >> 5)) {
     cx<float> x[kPer];
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
@@ -846,16 +851,16 @@ void launch_linv_neg(const Launch& L, const MatInst* d, int ninst, int64_t k0, f
   attr.call([&] {
     cudaFuncSetAttribute(k_linv_neg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
-  k_linv_neg<<<ninst, 256, smem, L.stream>>>(d, k0, outs);
+  const int ctas = linv_ctas(ninst);
+  k_linv_neg<<<dim3((unsigned)ctas, (unsigned)ninst), std::min(kLinvWarps, kLinvB / ctas) * 32, smem,
+               L.stream>>>(d, k0, outs);
   count_launch(1);
 }
 
 // The same for complex128 factors (out: complex128): the strict lower triangle of L11 packed
-// by columns in shared memory (127 KB), one warp per column of the inverse, the columns of a
-// CTA spread over the triangle for balance.  Bound by FP64 issue and the 128 dependent steps
-// of a column: about 10 us with kLinvCtas CTAs per instance, against 0.4 ms with one.
-constexpr int kLinvCtas = 32;
-__global__ void __launch_bounds__(kLinvB / kLinvCtas * 32) k_linv_neg_c128(
+// by columns in shared memory (127 KB).  Bound by FP64 issue and the 128 dependent steps of a
+// column: about 10 us with 32 CTAs per instance, against 0.4 ms with one.
+__global__ void __launch_bounds__(kLinvWarps * 32) k_linv_neg_c128(
     const MatInst* __restrict__ insts, int64_t k0, double2* const* outs) {
   const MatInst& M = insts[blockIdx.y];
   const int64_t n = M.n;
@@ -867,39 +872,40 @@ __global__ void __launch_bounds__(kLinvB / kLinvCtas * 32) k_linv_neg_c128(
   // column c: rows c + 1 .. kLinvB - 1 at c (2 kLinvB - c - 1) / 2
   auto at = [](int r, int c) { return c * (2 * kLinvB - c - 1) / 2 + r - c - 1; };
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int kWarps = kLinvB / kLinvCtas;
-  for (int c = wid; c < nbe; c += kWarps)
+  const int warps = blockDim.x >> 5;
+  for (int c = wid; c < nbe; c += warps)
     for (int r = c + 1 + lane; r < nbe; r += 32) sL[at(r, c)] = ld<double>(M.a, (k0 + r) + (k0 + c) * lda);
   __syncthreads();
-  const int j = blockIdx.x + kLinvCtas * wid;
   constexpr int kPer = kLinvB / 32;
-  cx<double> x[kPer];
+  double2* out = outs[blockIdx.y];
+  for (int j = blockIdx.x + gridDim.x * wid; j < kLinvB; j += gridDim.x * warps) {
+    cx<double> x[kPer];
 #pragma unroll
-  for (int t = 0; t < kPer; ++t) x[t] = cx<double>{lane + 32 * t == j ? 1.0 : 0.0, 0.0};
-  if (j < nbe) {
+    for (int t = 0; t < kPer; ++t) x[t] = cx<double>{lane + 32 * t == j ? 1.0 : 0.0, 0.0};
+    if (j < nbe) {
 #pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      for (int cl = 0; cl < 32; ++cl) {
-        const int c = 32 * t + cl;
-        if (c >= nbe) break;
-        if (c < j) continue;
-        cx<double> xc;
-        xc.x = __shfl_sync(0xffffffffu, x[t].x, cl);
-        xc.y = __shfl_sync(0xffffffffu, x[t].y, cl);
+      for (int t = 0; t < kPer; ++t) {
+        for (int cl = 0; cl < 32; ++cl) {
+          const int c = 32 * t + cl;
+          if (c >= nbe) break;
+          if (c < j) continue;
+          cx<double> xc;
+          xc.x = __shfl_sync(0xffffffffu, x[t].x, cl);
+          xc.y = __shfl_sync(0xffffffffu, x[t].y, cl);
 #pragma unroll
-        for (int u = t; u < kPer; ++u) {
-          const int r = lane + 32 * u;
-          if (r > c && r < nbe) x[u] -= sL[at(r, c)] * xc;
+          for (int u = t; u < kPer; ++u) {
+            const int r = lane + 32 * u;
+            if (r > c && r < nbe) x[u] -= sL[at(r, c)] * xc;
+          }
         }
       }
     }
-  }
-  double2* out = outs[blockIdx.y];
 #pragma unroll
-  for (int t = 0; t < kPer; ++t) {
-    const int r = lane + 32 * t;
-    const bool strict = r > j && r < nbe && j < nbe;
-    out[r + (int64_t)j * kLinvB] = strict ? make_double2(-x[t].x, -x[t].y) : make_double2(0.0, 0.0);
+    for (int t = 0; t < kPer; ++t) {
+      const int r = lane + 32 * t;
+      const bool strict = r > j && r < nbe && j < nbe;
+      out[r + (int64_t)j * kLinvB] = strict ? make_double2(-x[t].x, -x[t].y) : make_double2(0.0, 0.0);
+    }
   }
 }
 
@@ -910,8 +916,9 @@ void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t 
   attr.call([&] {
     cudaFuncSetAttribute(k_linv_neg_c128, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
-  k_linv_neg_c128<<<dim3(kLinvCtas, (unsigned)ninst), kLinvB / kLinvCtas * 32, smem, L.stream>>>(
-      d, k0, outs);
+  const int ctas = linv_ctas(ninst);
+  k_linv_neg_c128<<<dim3((unsigned)ctas, (unsigned)ninst), std::min(kLinvWarps, kLinvB / ctas) * 32,
+                    smem, L.stream>>>(d, k0, outs);
   count_launch(1);
 }
 
@@ -949,9 +956,9 @@ struct LLCfg {
   static constexpr int kBatch = sizeof(R) == 4 ? kLLBatch : kLLBatch / 2;
 };
 
-template <typename K>
+template <typename K, typename... Args>
 static void cluster_launch(const Launch& L, K kernel, int ninst, int cs, int threads,
-                           const MatInst* d, int64_t k0, int nb) {
+                           const MatInst* d, int64_t k0, int nb, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(ninst * cs));
   cfg.blockDim = dim3((unsigned)threads);
@@ -964,52 +971,70 @@ static void cluster_launch(const Launch& L, K kernel, int ninst, int cs, int thr
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, d, k0, nb);
+  cudaLaunchKernelEx(&cfg, kernel, d, k0, nb, args...);
   count_launch(1);
 }
 
 template <typename R, int W, int RPT, int T = 512>
 static void getf2_reg_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int cs,
-                        int threads) {
+                        int threads, int share) {
   static PerDeviceOnce attr;
   attr.call([] {  // clusters of 16 are beyond the portable size
     cudaFuncSetAttribute(k_getf2_reg<R, W, RPT, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   });
-  cluster_launch(L, k_getf2_reg<R, W, RPT, T>, ninst, cs, threads, d, k0, nb);
+  cluster_launch(L, k_getf2_reg<R, W, RPT, T>, ninst, cs, threads, d, k0, nb, share);
 }
 
-// The panel kernel's shape.  Cluster size: the batch in one wave of CTAs (at most 8 clusters
-// of 16 are resident, one per GPC), no more CTAs than give each kRegRows* rows; complex128
-// takes fewer rows per CTA since its FP64 work, not the barriers, sets the step.  Columns in
-// registers: as many as the rows per thread leave room for.
+// The panel kernel's cluster size.  A column step costs about 1.5 us of barriers and exchanges
+// plus the CTA's rows: 1.25 ns a row in complex64 (measured: 1.9, 2.2 and 3.2 us a column with
+// 160, 560 and 1280 rows per CTA; half as much again when more than 5 rows per thread force
+// sub-panels of 4 columns), 17 ns in complex128 (16 updates of 4 FMAs on average, two per
+// clock).  A batch takes as many waves as its clusters need, one CTA per SM, and at most 8
+// clusters of 16 or 18 of 8 fit the GPU's processing clusters.  64 systems of 10240 unknowns:
+// 138 ms of panels with two CTAs each in one wave, 109 with four, see the launcher's choice.
+static int panel_cluster(int nact, int64_t rows, bool single) {
+  const int sms = device_sm_count();
+  int best = 1;
+  double best_cost = 1e300;
+  for (int cs = 1; cs <= kRegMaxCS; cs *= 2) {
+    const int resident = std::max(1, cs == 16 ? sms / 19 : cs == 8 ? sms / 19 * 9 / 4 : sms / cs);
+    const double waves = (double)((nact + resident - 1) / resident);
+    const double share = (double)((rows + cs - 1) / cs);
+    const double row = single ? (share > 5 * 512 ? 1.9e-3 : 1.25e-3) : 17e-3;
+    double cost = waves * (1.5 + 0.02 * cs + row * share);
+    if (share > (single ? 10 : 5) * 512) cost *= 2.0;  // the streaming kernel
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = cs;
+    }
+  }
+  return best;
+}
+
+// Columns in registers: as many as the rows per thread leave room for.
 bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_t nmax, int64_t k0,
                   int nb, int prec) {
   const bool single = prec_is_single(prec);
   const int64_t rows = nmax - k0;
-  const int sms = device_sm_count();
-  const int per = single ? 256 : 64;
-  int cs = 1;
-  while (cs < kRegMaxCS && (int64_t)nact * cs * 2 <= sms && (cs < 8 || nact <= 8) &&
-         (int64_t)cs * per < rows)
-    cs *= 2;
-  const int64_t share = (rows + cs - 1) / cs;  // rows per CTA
+  const int cs = panel_cluster(std::max(1, nact), rows, single);
+  const int share = (int)(((rows + cs - 1) / cs + 31) / 32 * 32);  // rows per CTA
   // complex128: at least eight warps, which solve the U rows of a sub-panel's columns
   const int threads =
-      (int)std::min<int64_t>(512, std::max<int64_t>(single ? 64 : 256, (share + 31) / 32 * 32));
-  const int64_t q = (share + threads - 1) / threads;  // rows per thread
+      std::min(512, std::max(single ? 64 : 256, share));
+  const int q = (share + threads - 1) / threads;  // rows per thread
   if (single) {
-    if (q <= 1) return getf2_reg_t<float, 16, 1>(L, d, ninst, k0, nb, cs, threads), false;
-    if (q <= 2) return getf2_reg_t<float, 16, 2>(L, d, ninst, k0, nb, cs, threads), false;
-    if (q <= 5) return getf2_reg_t<float, 8, 5>(L, d, ninst, k0, nb, cs, threads), false;
-    if (q <= 10) return getf2_reg_t<float, 4, 10>(L, d, ninst, k0, nb, cs, threads), false;
+    if (q <= 1) return getf2_reg_t<float, 16, 1>(L, d, ninst, k0, nb, cs, threads, share), false;
+    if (q <= 2) return getf2_reg_t<float, 16, 2>(L, d, ninst, k0, nb, cs, threads, share), false;
+    if (q <= 5) return getf2_reg_t<float, 8, 5>(L, d, ninst, k0, nb, cs, threads, share), false;
+    if (q <= 10) return getf2_reg_t<float, 4, 10>(L, d, ninst, k0, nb, cs, threads, share), false;
     cluster_launch(L, k_getf2_ll<float, 2, LLCfg<float>::kT, LLCfg<float>::kBatch>, ninst, 2,
                    LLCfg<float>::kT, d, k0, nb);
   } else {
     if (threads <= 256 && q <= 1)
-      return getf2_reg_t<double, 16, 1, 256>(L, d, ninst, k0, nb, cs, threads), false;
-    if (q <= 1) return getf2_reg_t<double, 8, 1>(L, d, ninst, k0, nb, cs, threads), false;
-    if (q <= 2) return getf2_reg_t<double, 8, 2>(L, d, ninst, k0, nb, cs, threads), false;
-    if (q <= 5) return getf2_reg_t<double, 4, 5>(L, d, ninst, k0, nb, cs, threads), false;
+      return getf2_reg_t<double, 16, 1, 256>(L, d, ninst, k0, nb, cs, threads, share), false;
+    if (q <= 1) return getf2_reg_t<double, 8, 1>(L, d, ninst, k0, nb, cs, threads, share), false;
+    if (q <= 2) return getf2_reg_t<double, 8, 2>(L, d, ninst, k0, nb, cs, threads, share), false;
+    if (q <= 5) return getf2_reg_t<double, 4, 5>(L, d, ninst, k0, nb, cs, threads, share), false;
     cluster_launch(L, k_getf2_ll<double, 2, LLCfg<double>::kT, LLCfg<double>::kBatch>, ninst, 2,
                    LLCfg<double>::kT, d, k0, nb);
   }
@@ -1023,15 +1048,20 @@ void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int 
   s_hi = std::min(s_hi, c_hi);
   const int64_t cols = (c_hi - c_lo) - (s_hi - s_lo);
   if (cols <= 0) return;
-  dim3 grid((unsigned)((cols + kSwpCols - 1) / kSwpCols), (unsigned)ninst);
+  // columns per CTA: 128, halved down to 16 while the grid has less than two CTAs per SM (each
+  // warp moves its columns one after the other, at memory latency: 24 us a launch for 8960
+  // columns in 70 CTAs)
+  int per = 128;
+  while (per > 16 && (cols + per - 1) / per * ninst < 2 * (int64_t)device_sm_count()) per /= 2;
+  dim3 grid((unsigned)((cols + per - 1) / per), (unsigned)ninst);
   for (int b0 = 0; b0 < nb; b0 += kSwpMaxNb) {  // sequential chunks of interchanges
     const int nbc = std::min(kSwpMaxNb, nb - b0);
     if (prec_is_single(prec))
       k_laswp<float><<<grid, kSwpWarps * 32, 0, L.stream>>>(d, k0 + b0, nbc, c_lo, c_hi, s_lo,
-                                                              s_hi);
+                                                              s_hi, per);
     else
       k_laswp<double><<<grid, kSwpWarps * 32, 0, L.stream>>>(d, k0 + b0, nbc, c_lo, c_hi, s_lo,
-                                                               s_hi);
+                                                               s_hi, per);
     count_launch(1);
   }
 }
@@ -1046,9 +1076,11 @@ static void trsm_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int
       cudaFuncSetAttribute(k_trsm_panel<R, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem);
     });
-  const int64_t per = (int64_t)kTrsmWarps * TrsmCols<R>::value;
+  // complex128 columns are FP64-bound: one per warp in a small batch
+  const int per_warp = ninst >= 32 ? 16 : sizeof(R) == 4 ? 2 : 1;
+  const int64_t per = (int64_t)kTrsmWarps * per_warp;
   dim3 grid((unsigned)((c_hi - c_lo + per - 1) / per), (unsigned)ninst);
-  k_trsm_panel<R, NB><<<grid, kTrsmWarps * 32, smem, L.stream>>>(d, k0, c_lo, c_hi);
+  k_trsm_panel<R, NB><<<grid, kTrsmWarps * 32, smem, L.stream>>>(d, k0, c_lo, c_hi, per_warp);
   count_launch(1);
 }
 
