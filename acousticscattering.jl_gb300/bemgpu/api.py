@@ -120,7 +120,7 @@ class Context:
         _check(C.lib().bemgpu_ctx_synchronize(self.handle), self.handle)
 
     def set_autotune(self, enable: bool = True):
-        """Measured launch shapes (panel cluster size, residual rows per thread); every
+        """Measured launch shapes (panel cluster size, residual CTA size); every
         choice gives bit-identical results."""
         _check(C.lib().bemgpu_ctx_set_autotune(self.handle, int(enable)), self.handle)
 

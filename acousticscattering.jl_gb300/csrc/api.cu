@@ -2071,7 +2071,7 @@ int factorize_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
     TRY(alloc(c, (size_t)f->N * 8, &f->cols_inv));
     TRY(alloc(c, (size_t)f->N * 4, &f->rows_inv));
     TRY(alloc(c, (size_t)f->N * 4, &f->cols_inv32));
-    TRY(alloc(c, (size_t)kChunks * f->N * 2 * 8, &part[t]));
+    TRY(alloc(c, (size_t)vec_chunks(f->N) * f->N * 2 * 8, &part[t]));
     TRY(alloc(c, (size_t)f->N * f->N * (f->single ? 8 : 16), &f->LU));
     TRY(alloc(c, (size_t)f->N * 4, &f->ipiv));
     TRY(alloc(c, 4, &f->info));
@@ -2142,7 +2142,7 @@ int factorize_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs) {
   std::vector<Buf> ppart;
   for (FactorData* f : prom) {
     Buf b;
-    TRY(alloc(c, (size_t)kChunks * f->N * 2 * 8, &b));
+    TRY(alloc(c, (size_t)vec_chunks(f->N) * f->N * 2 * 8, &b));
     ppart.push_back(std::move(b));
   }
   TRY(promote(c, prom, ppart));
@@ -2377,7 +2377,7 @@ int residual_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss,
   TRY(to_device(c, vi, &d));
   {
     Prof p(c, "residual");
-    // rows per thread of the compact products, measured on the live pass (idempotent: the
+    // CTA size of the compact products, measured on the live pass (idempotent: the
     // last candidate's outputs are the pass's outputs)
     std::vector<VecInst> few;
     int64_t fn = 0;
@@ -2478,12 +2478,12 @@ int solve_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<i
     TRY(alloc(c, (size_t)N * s.R * 16, &s.y));
     TRY(alloc(c, (size_t)N * s.R * 8, &s.den));
     if (f->a32) {
-      TRY(alloc(c, (size_t)N * s.R * 16, &s.xs));
+      TRY(alloc(c, (size_t)N * s.R * 32, &s.xs));
       TRY(alloc(c, (size_t)N * s.R * 4, &s.xa));
     }
     TRY(alloc(c, (size_t)N * s.R * 16, &s.work));
     TRY(alloc(c, (size_t)kStats * s.R * 8, &s.stats));
-    TRY(alloc(c, (size_t)std::max<int64_t>(kChunks * (int64_t)s.R * N * 3, kChunks * N * 2) * 8,
+    TRY(alloc(c, (size_t)vec_chunks(N) * (int64_t)s.R * N * 3 * 8,
               &s.part));
     TRY(alloc(c, (size_t)s.R * 4, &s.active));
     TRY(alloc(c, (size_t)s.R * 4, &s.changed));
@@ -2634,7 +2634,7 @@ int solve_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<i
       std::vector<Buf> ppart;
       for (FactorData* f : to_promote) {
         Buf b;
-        TRY(alloc(c, (size_t)kChunks * f->N * 2 * 8, &b));
+        TRY(alloc(c, (size_t)vec_chunks(f->N) * f->N * 2 * 8, &b));
         ppart.push_back(std::move(b));
       }
       TRY(promote(c, to_promote, ppart));
@@ -2671,7 +2671,7 @@ int solve_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<i
       if (!stag.empty()) {
         std::vector<Buf> ppart;
         Buf b;
-        TRY(alloc(c, (size_t)kChunks * s.f->N * 2 * 8, &b));
+        TRY(alloc(c, (size_t)vec_chunks(s.f->N) * s.f->N * 2 * 8, &b));
         ppart.push_back(std::move(b));
         TRY(promote(c, stag, ppart));
         std::vector<SolveInst*> one{&s};
@@ -2844,7 +2844,7 @@ int64_t order_of(const ServerReq& r) {
 size_t solve_bytes(const ServerReq& r) {
   const size_t N = (size_t)order_of(r);
   const size_t R = (size_t)r.nangles;
-  const size_t b = N * R * (16 * 6 + 8) + (size_t)kChunks * R * N * 3 * 8;
+  const size_t b = N * R * (16 * 6 + 8) + (size_t)vec_chunks((int64_t)N) * R * N * 3 * 8;
   return b + b / 20;
 }
 
@@ -5178,7 +5178,7 @@ int bemgpu_dense_solve(bemgpu_ctx* c, int64_t n, const double* A, int32_t nrhs, 
   TRY(alloc(c, (size_t)n * nrhs * 8, &s.den));
   TRY(alloc(c, (size_t)n * nrhs * 16, &s.work));
   TRY(alloc(c, (size_t)kStats * nrhs * 8, &s.stats));
-  TRY(alloc(c, (size_t)std::max<int64_t>(kChunks * (int64_t)nrhs * n * 3, kChunks * n * 2) * 8,
+  TRY(alloc(c, (size_t)vec_chunks(n) * (int64_t)nrhs * n * 3 * 8,
             &s.part));
   TRY(alloc(c, (size_t)nrhs * 4, &s.active));
   TRY(alloc(c, (size_t)nrhs * 4, &s.changed));
@@ -5231,7 +5231,7 @@ int bemgpu_dense_solve(bemgpu_ctx* c, int64_t n, const double* A, int32_t nrhs, 
       if (prom) {
         std::vector<Buf> pp;
         Buf b;
-        TRY(alloc(c, (size_t)kChunks * n * 2 * 8, &b));
+        TRY(alloc(c, (size_t)vec_chunks(n) * n * 2 * 8, &b));
         pp.push_back(std::move(b));
         TRY(promote(c, fs, pp));
       }
@@ -5250,7 +5250,7 @@ int bemgpu_dense_solve(bemgpu_ctx* c, int64_t n, const double* A, int32_t nrhs, 
             f->reason = BEMGPU_REASON_STAGNATION;
             std::vector<Buf> pp;
             Buf b;
-            TRY(alloc(c, (size_t)kChunks * n * 2 * 8, &b));
+            TRY(alloc(c, (size_t)vec_chunks(n) * n * 2 * 8, &b));
             pp.push_back(std::move(b));
             TRY(promote(c, fs, pp));
             s.rs[r].previous = INFINITY;

@@ -785,12 +785,12 @@ __global__ void __launch_bounds__(kGThreads) k_gemm_update(const MatInst* __rest
 constexpr int kLinvB = 128;
 
 // gridDim.x CTAs per instance take the columns j = blockIdx.x + gridDim.x i (spread over the
-// triangle for balance), a warp one column after the other.  One CTA per instance took 32 us a
-// launch (16 columns per warp); 32 CTAs take 5, but each stages the block, so a batch uses
-// fewer (linv_ctas).
+// triangle for balance), a warp one column after the other.  A launch for one instance took 68 us
+// with 32 CTAs whose loads waited for one another and takes 23 with 16; each CTA stages the block, so
+// a batch uses fewer (linv_ctas).
 constexpr int kLinvWarps = 8;
 static int linv_ctas(int ninst) {
-  int n = 32;
+  int n = 16;
   while (n > 1 && (int64_t)n * ninst > 2 * (int64_t)device_sm_count()) n /= 2;
   return n;
 }
@@ -803,9 +803,22 @@ __global__ void __launch_bounds__(kLinvWarps * 32) k_linv_neg(
   const int64_t lda = M.lda;
   extern __shared__ __align__(16) unsigned char linv_smem[];
   cx<float>* sL = reinterpret_cast<cx<float>*>(linv_smem);  // [kLinvB][kLinvB + 1]
-  for (int t = threadIdx.x; t < nbe * nbe; t += blockDim.x) {
-    int r = t % nbe, c = t / nbe;
-    sL[r * (kLinvB + 1) + c] = ld<float>(M.a, (k0 + r) + (k0 + c) * lda);
+  {  // a column per 128 threads, kFly of them in flight
+    constexpr int kFly = 16;
+    const int r = threadIdx.x % kLinvB, c0 = threadIdx.x / kLinvB, cols = blockDim.x / kLinvB;
+    for (int cb = c0; cb < nbe; cb += cols * kFly) {
+      cx<float> v[kFly];
+#pragma unroll
+      for (int e = 0; e < kFly; ++e) {
+        const int c = cb + cols * e;
+        v[e] = r < nbe && c < r ? ld<float>(M.a, (k0 + r) + (k0 + c) * lda) : cx<float>{0, 0};
+      }
+#pragma unroll
+      for (int e = 0; e < kFly; ++e) {
+        const int c = cb + cols * e;
+        if (c < r) sL[r * (kLinvB + 1) + c] = v[e];
+      }
+    }
   }
   __syncthreads();
   float2* out = outs[blockIdx.y];
@@ -852,14 +865,14 @@ void launch_linv_neg(const Launch& L, const MatInst* d, int ninst, int64_t k0, f
     cudaFuncSetAttribute(k_linv_neg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   const int ctas = linv_ctas(ninst);
-  k_linv_neg<<<dim3((unsigned)ctas, (unsigned)ninst), std::min(kLinvWarps, kLinvB / ctas) * 32, smem,
+  k_linv_neg<<<dim3((unsigned)ctas, (unsigned)ninst), kLinvWarps * 32, smem,
                L.stream>>>(d, k0, outs);
   count_launch(1);
 }
 
 // The same for complex128 factors (out: complex128): the strict lower triangle of L11 packed
 // by columns in shared memory (127 KB).  Bound by FP64 issue and the 128 dependent steps of a
-// column: about 10 us with 32 CTAs per instance, against 0.4 ms with one.
+// column: 95 us with 16 CTAs per instance, against 0.4 ms with one.
 __global__ void __launch_bounds__(kLinvWarps * 32) k_linv_neg_c128(
     const MatInst* __restrict__ insts, int64_t k0, double2* const* outs) {
   const MatInst& M = insts[blockIdx.y];
@@ -873,8 +886,23 @@ __global__ void __launch_bounds__(kLinvWarps * 32) k_linv_neg_c128(
   auto at = [](int r, int c) { return c * (2 * kLinvB - c - 1) / 2 + r - c - 1; };
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
-  for (int c = wid; c < nbe; c += warps)
-    for (int r = c + 1 + lane; r < nbe; r += 32) sL[at(r, c)] = ld<double>(M.a, (k0 + r) + (k0 + c) * lda);
+  {  // a column per 128 threads, kFly of them in flight
+    constexpr int kFly = 8;
+    const int r = threadIdx.x % kLinvB, c0 = threadIdx.x / kLinvB, cols = blockDim.x / kLinvB;
+    for (int cb = c0; cb < nbe; cb += cols * kFly) {
+      cx<double> v[kFly];
+#pragma unroll
+      for (int e = 0; e < kFly; ++e) {
+        const int c = cb + cols * e;
+        v[e] = r < nbe && c < r ? ld<double>(M.a, (k0 + r) + (k0 + c) * lda) : cx<double>{0, 0};
+      }
+#pragma unroll
+      for (int e = 0; e < kFly; ++e) {
+        const int c = cb + cols * e;
+        if (r < nbe && c < r) sL[at(r, c)] = v[e];
+      }
+    }
+  }
   __syncthreads();
   constexpr int kPer = kLinvB / 32;
   double2* out = outs[blockIdx.y];
@@ -917,32 +945,43 @@ void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t 
     cudaFuncSetAttribute(k_linv_neg_c128, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
   const int ctas = linv_ctas(ninst);
-  k_linv_neg_c128<<<dim3((unsigned)ctas, (unsigned)ninst), std::min(kLinvWarps, kLinvB / ctas) * 32,
+  k_linv_neg_c128<<<dim3((unsigned)ctas, (unsigned)ninst), kLinvWarps * 32,
                     smem, L.stream>>>(d, k0, outs);
   count_launch(1);
 }
 
-// perm from LAPACK pivots: apply the interchanges in order to the identity, in shared
-// memory (SMEM, orders up to the shared-memory capacity) or in place in global memory.
-template <bool SMEM>
+// perm from LAPACK pivots (position i holds row perm[i] after the interchanges).  One thread
+// carrying out n interchanges waits for shared memory twice in each (52 us for 1280 unknowns,
+// 323 us for 8960), so every row follows its own position instead: interchange i concerns it
+// only if it stands at i or at ipiv[i], which is tested for kPermGroup interchanges at once
+// (25 and 156 us); a group that holds one is gone through in order.
+constexpr int kPermGroup = 16, kPermTile = 2048;
 __global__ void __launch_bounds__(256) k_make_perm(const MatInst* __restrict__ insts) {
-  const MatInst& M = insts[blockIdx.x];
+  const MatInst& M = insts[blockIdx.y];
   if (!M.active || !M.perm) return;
-  extern __shared__ int32_t sperm_smem[];
-  int32_t* sperm = SMEM ? sperm_smem : M.perm;
-  const int64_t n = M.n;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) sperm[i] = (int32_t)i;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int64_t i = 0; i < n; ++i) {
-      const int32_t p = M.ipiv[i];
-      const int32_t t = sperm[i];
-      sperm[i] = sperm[p];
-      sperm[p] = t;
+  __shared__ alignas(16) int32_t piv[kPermTile];
+  const int n = (int)M.n, e = blockIdx.x * 256 + threadIdx.x;
+  if ((int)blockIdx.x * 256 >= n) return;
+  int pos = e;  // threads past the last row stand where no interchange reaches
+  for (int t0 = 0; t0 < n; t0 += kPermTile) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < kPermTile; i += 256)
+      piv[i] = t0 + i < n ? M.ipiv[t0 + i] : t0 + i;
+    __syncthreads();
+    const int end = min(kPermTile, n - t0);
+    for (int g = 0; g < end; g += kPermGroup) {
+      const int i0 = t0 + g;
+      bool hit = (unsigned)(pos - i0) < (unsigned)kPermGroup;
+#pragma unroll
+      for (int q = 0; q < kPermGroup; ++q) hit = hit || piv[g + q] == pos;
+      if (hit)
+        for (int q = 0; q < kPermGroup; ++q) {
+          const int p = piv[g + q];
+          pos = pos == i0 + q ? p : pos == p ? i0 + q : pos;
+        }
     }
-  __syncthreads();
-  if (SMEM)
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) M.perm[i] = sperm[i];
+  }
+  if (e < n) M.perm[pos] = e;
 }
 
 // ------------------------------------------------------------------ launch wrappers
@@ -1115,19 +1154,7 @@ void launch_gemm_update(const Launch& L, const MatInst* d, int ninst, int64_t k0
 }
 
 void launch_make_perm(const Launch& L, const MatInst* d, int ninst, int64_t nmax) {
-  constexpr size_t kMaxSmem = 227 * 1024;
-  const size_t smem = (size_t)nmax * sizeof(int32_t);
-  if (smem > kMaxSmem) {  // beyond 58112 unknowns: interchanges in global memory
-    k_make_perm<false><<<ninst, 256, 0, L.stream>>>(d);
-    count_launch(1);
-    return;
-  }
-  static PerDeviceOnce attr;
-  attr.call([] {
-    cudaFuncSetAttribute(k_make_perm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kMaxSmem);
-  });
-  k_make_perm<true><<<ninst, 256, smem, L.stream>>>(d);
+  k_make_perm<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)ninst), 256, 0, L.stream>>>(d);
   count_launch(1);
 }
 

@@ -5,7 +5,7 @@
 // fluid_system.jl:229-239.
 //
 // Column-major matrices are swept with one thread per row (consecutive threads read
-// consecutive rows of a column: coalesced), and the columns are split into kChunks
+// consecutive rows of a column: coalesced), and the columns are split into vec_chunks(n)
 // chunks whose partial results are combined by a second kernel in a fixed order, so
 // every reduction here is deterministic.
 #include <cfloat>
@@ -25,10 +25,20 @@ __device__ __forceinline__ void stc(void* base, int64_t idx, cd v) {
   reinterpret_cast<double2*>(base)[idx] = make_double2(v.x, v.y);
 }
 __device__ __forceinline__ double cabs(cd a) { return hypot(a.x, a.y); }
+// The nearest float of a (ties away from zero; below the normal range 0), by integer
+// instructions: a conversion instruction of a double takes a turn of the FP64 pipe, and four of
+// them per entry were half of the pipe's work in the products of complex128 systems.
+__device__ __forceinline__ float near_float(double a) {
+  const uint32_t hi = (uint32_t)__double2hiint(a) & 0x7fffffffu, lo = (uint32_t)__double2loint(a);
+  if (hi < 0x38100000u) return 0.f;                       // |a| < 2^-126
+  if (hi >= 0x47f00000u)                                  // |a| >= 2^128, infinity, NaN
+    return hi > 0x7ff00000u || (hi == 0x7ff00000u && lo) ? NAN : INFINITY;
+  return __uint_as_float(__funnelshift_l(lo, hi - 0x38000000u, 3) + ((lo >> 28) & 1u));
+}
 // Magnitude for scales, norms and componentwise denominators: single precision is
 // ample there (relative 1e-7), and GB300 issues FP64 at a small fraction of FP32.
 __device__ __forceinline__ float fabs_c(cd a) {
-  const float x = (float)a.x, y = (float)a.y;
+  const float x = near_float(a.x), y = near_float(a.y);
   return sqrtf(fmaf(x, x, y * y));
 }
 
@@ -43,12 +53,20 @@ __device__ __forceinline__ float2 ldf(const void* base, int64_t idx) {
   return reinterpret_cast<const float2*>(base)[idx];
 }
 template <bool A32>
+struct Entry {
+  using T = cd;
+  static __device__ __forceinline__ T at(const VecInst& V, int64_t idx) { return ldc(V.A, idx); }
+  static __device__ __forceinline__ float mag(T a) { return fabs_c(a); }
+};
+template <>
+struct Entry<true> {
+  using T = float2;
+  static __device__ __forceinline__ T at(const VecInst& V, int64_t idx) { return ldf(V.A, idx); }
+  static __device__ __forceinline__ float mag(T a) { return sqrtf(fmaf(a.x, a.x, a.y * a.y)); }
+};
+template <bool A32>
 __device__ __forceinline__ float mag_at(const VecInst& V, int64_t idx) {
-  if (A32) {
-    const float2 a = ldf(V.A, idx);
-    return sqrtf(fmaf(a.x, a.x, a.y * a.y));
-  }
-  return fabs_c(ldc(V.A, idx));
+  return Entry<A32>::mag(Entry<A32>::at(V, idx));
 }
 
 // ---------------------------------------------------------------- equilibration
@@ -57,25 +75,30 @@ __device__ __forceinline__ void rowstats_body(const VecInst& V) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.n) return;
   int64_t j0, j1;
-  chunk_range(V.n, blockIdx.y, kChunks, &j0, &j1);
-  float mx = 0.f;
+  if (blockIdx.y >= vec_chunks(V.n)) return;
+  chunk_range(V.n, blockIdx.y, vec_chunks(V.n), &j0, &j1);
+  using E = Entry<A32>;
+  float mx = 0.f, sm32 = 0.f;
   double sm = 0.0;
-  constexpr int kB = 16;
+  auto take = [&](typename E::T v) {
+    const float a = E::mag(v);
+    mx = fmaxf(mx, a);
+    sm32 += a;
+  };
+  constexpr int kB = A32 ? 16 : 8;  // columns loaded before the first is used
   for (int64_t jf = j0; jf < j1; jf += 256) {  // fold into FP64 every 256 terms
-    float sm32 = 0.f;
     const int64_t jf1 = min(j1, jf + 256);
-    for (int64_t jb = jf; jb < jf1; jb += kB) {
-      const int cnt = (int)min((int64_t)kB, jf1 - jb);
-      float a[kB];
+    int64_t j = jf;
+    for (; j + kB <= jf1; j += kB) {
+      typename E::T a[kB];
 #pragma unroll
-      for (int q = 0; q < kB; ++q) a[q] = q < cnt ? mag_at<A32>(V, i + (jb + q) * V.lda) : 0.f;
+      for (int q = 0; q < kB; ++q) a[q] = E::at(V, i + (j + q) * V.lda);
 #pragma unroll
-      for (int q = 0; q < kB; ++q) {
-        mx = fmaxf(mx, a[q]);
-        sm32 += a[q];
-      }
+      for (int q = 0; q < kB; ++q) take(a[q]);
     }
+    for (; j < jf1; ++j) take(E::at(V, i + j * V.lda));
     sm += sm32;
+    sm32 = 0.f;
   }
   V.part[2 * (blockIdx.y * V.n + i)] = mx;
   V.part[2 * (blockIdx.y * V.n + i) + 1] = sm;
@@ -93,7 +116,9 @@ __global__ void k_rowstats_finish(const VecInst* __restrict__ insts) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.n) return;
   double mx = 0.0, sm = 0.0;
-  for (int c = 0; c < kChunks; ++c) {
+  const int chunks = vec_chunks(V.n);
+#pragma unroll 8
+  for (int c = 0; c < chunks; ++c) {
     mx = fmax(mx, V.part[2 * (c * V.n + i)]);
     sm += V.part[2 * (c * V.n + i) + 1];
   }
@@ -112,15 +137,17 @@ __device__ __forceinline__ void colmax_body(const VecInst& V) {
   float mx = 0.f;
   const int64_t n = V.n, base = j * V.lda;
   int64_t i = lane;
-  for (; i + 96 < n; i += 128) {
-    float a[4], w[4];
+  constexpr int kB = 8;
+  for (; i + 32 * (kB - 1) < n; i += 32 * kB) {
+    typename Entry<A32>::T a[kB];
+    float w[kB];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      a[q] = mag_at<A32>(V, base + i + 32 * q);
+    for (int q = 0; q < kB; ++q) {
+      a[q] = Entry<A32>::at(V, base + i + 32 * q);
       w[q] = V.rows_inv[i + 32 * q];
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) mx = fmaxf(mx, a[q] * w[q]);
+    for (int q = 0; q < kB; ++q) mx = fmaxf(mx, Entry<A32>::mag(a[q]) * w[q]);
   }
   for (; i < n; i += 32) mx = fmaxf(mx, mag_at<A32>(V, base + i) * V.rows_inv[i]);
 #pragma unroll
@@ -156,7 +183,8 @@ __device__ __forceinline__ void scale_copy_body(const VecInst& V) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V.n) return;
   int64_t j0, j1;
-  chunk_range(V.n, blockIdx.y, kChunks, &j0, &j1);
+  if (blockIdx.y >= vec_chunks(V.n)) return;
+  chunk_range(V.n, blockIdx.y, vec_chunks(V.n), &j0, &j1);
   double sm = 0.0;
   float sm32 = 0.f;
   int cnt = 0;
@@ -225,20 +253,23 @@ __global__ void k_scale_copy(const VecInst* __restrict__ insts) {
 }
 
 // stats[0] = max_i rowsum_i (||A||_inf), stats[1] = max_i sum_c part (||scaled||_inf)
-__global__ void k_norms_finish(const VecInst* __restrict__ insts) {
+constexpr int kNormT = 1024;
+__global__ void __launch_bounds__(kNormT) k_norms_finish(const VecInst* __restrict__ insts) {
   const VecInst& V = insts[blockIdx.x];
-  __shared__ double s0[256], s1[256];
+  __shared__ double s0[kNormT], s1[kNormT];
   double m0 = 0.0, m1 = 0.0;
-  for (int64_t i = threadIdx.x; i < V.n; i += 256) {
+  const int chunks = vec_chunks(V.n);
+  for (int64_t i = threadIdx.x; i < V.n; i += kNormT) {
     double t = 0.0;
-    for (int c = 0; c < kChunks; ++c) t += V.part[c * V.n + i];
+#pragma unroll 8
+    for (int c = 0; c < chunks; ++c) t += V.part[c * V.n + i];
     m0 = fmax(m0, V.rowsum[i]);
     m1 = fmax(m1, t);
   }
   s0[threadIdx.x] = m0;
   s1[threadIdx.x] = m1;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
+  for (int s = kNormT / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) {
       s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + s]);
       s1[threadIdx.x] = fmax(s1[threadIdx.x], s1[threadIdx.x + s]);
@@ -277,7 +308,8 @@ __global__ void k_expand_a32(const VecInst* __restrict__ insts) {
   }
 }
 
-// x split for the compact products: hi = fl32(x), lo = fl32(x - hi)
+// x split for the compact products: hi = fl32(x), lo = fl32(x - hi), every part twice (the paired
+// instructions take it for two rows)
 __global__ void k_split_x(const VecInst* __restrict__ insts) {
   const VecInst& V = insts[blockIdx.z];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -286,7 +318,9 @@ __global__ void k_split_x(const VecInst* __restrict__ insts) {
   const cd x = ldc(V.x, i + (int64_t)r * V.ldx);
   const float hr = (float)x.x, hi = (float)x.y;
   const float lr = (float)(x.x - (double)hr), li = (float)(x.y - (double)hi);
-  V.xs[i + (int64_t)r * V.n] = make_float4(hr, hi, lr, li);
+  float4* xs = V.xs + 2 * (i + (int64_t)r * V.n);
+  xs[0] = make_float4(hr, hr, hi, hi);
+  xs[1] = make_float4(lr, lr, li, li);
   V.xa[i + (int64_t)r * V.n] = sqrtf(fmaf(hr, hr, hi * hi));
 }
 
@@ -302,29 +336,42 @@ __global__ void k_split_x(const VecInst* __restrict__ insts) {
 // operation emulation on the CPU), under the refinement's 1e-13 acceptance, at a small
 // fraction of the FP64 instruction count of the complex128 path.  The intrinsics keep the
 // compiler from contracting or reassociating the error-free steps.
+// Two rows go through the paired FP32 instructions, which round each half as the single ones do.
+// a - b and -a through products with -1, which are exact: one instruction each.
+__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ float2 f2_neg(float2 a) {
+  return __fmul2_rn(a, make_float2(-1.f, -1.f));
+}
 struct FPair {
-  float s, t;
+  float2 s, t;
 };
-__device__ __forceinline__ void pair_add_prod(FPair& a, float u, float v) {
-  const float p = __fmul_rn(u, v);
-  const float e = __fmaf_rn(u, v, -p);
-  const float s = __fadd_rn(a.s, p);
-  const float bb = __fsub_rn(s, a.s);
-  const float err = __fadd_rn(__fsub_rn(a.s, __fsub_rn(s, bb)), __fsub_rn(p, bb));
+// a += u v, nu = -u
+__device__ __forceinline__ void pair_add_prod(FPair& a, float2 u, float2 nu, float2 v) {
+  const float2 p = __fmul2_rn(u, v);
+  const float2 e = __ffma2_rn(nu, v, p);  // -(the product's error)
+  const float2 s = __fadd2_rn(a.s, p);
+  const float2 bb = f2_sub(s, a.s);
+  const float2 err = __fadd2_rn(f2_sub(a.s, f2_sub(s, bb)), f2_sub(p, bb));
   a.s = s;
-  a.t = __fadd_rn(a.t, __fadd_rn(err, e));
+  a.t = __fadd2_rn(a.t, f2_sub(err, e));
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 
-template <bool A32, int NR>
+template <int NR>
 __device__ __forceinline__ void gemv_body(const VecInst& V, int with_abs) {
   constexpr int kGemvR = NR;  // right-hand sides per pass of this instantiation
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int ch = blockIdx.y % kChunks, grp = blockIdx.y / kChunks;
+  const int ch = blockIdx.y % kMaxChunks, grp = blockIdx.y / kMaxChunks;
+  if (ch >= vec_chunks(V.n)) return;
   const int r0 = grp * kGemvR;
   if (i >= V.n || r0 >= V.nrhs) return;
   const int nr = min(kGemvR, V.nrhs - r0);
   int64_t j0, j1;
-  chunk_range(V.n, ch, kChunks, &j0, &j1);
+  chunk_range(V.n, ch, vec_chunks(V.n), &j0, &j1);
   cd acc[kGemvR];
   float aacc[kGemvR];
 #pragma unroll
@@ -332,62 +379,25 @@ __device__ __forceinline__ void gemv_body(const VecInst& V, int with_abs) {
     acc[r] = cd{0.0, 0.0};
     aacc[r] = 0.f;
   }
-  if (A32) {
-    // fold into FP64 every kFold columns; columns loaded kBatch at a time so each
-    // thread keeps kBatch independent requests in flight
-    constexpr int kFold = 32, kBatch = NR == 1 ? 16 : 8;
-    const float2* Acol = reinterpret_cast<const float2*>(V.A) + i;
-    const int64_t lda = V.lda, ldxs = V.n;
-    for (int64_t jf = j0; jf < j1; jf += kFold) {
-      FPair re[kGemvR], im[kGemvR];
+  constexpr int kBatch = 4;  // columns loaded before the first is used
+  for (int64_t jb = j0; jb < j1; jb += kBatch) {
+    const int cnt = (int)min((int64_t)kBatch, j1 - jb);
+    cd a[kBatch];
 #pragma unroll
-      for (int r = 0; r < kGemvR; ++r) re[r] = im[r] = FPair{0.f, 0.f};
-      const int64_t jf1 = min(j1, jf + kFold);
-      for (int64_t jb = jf; jb < jf1; jb += kBatch) {
-        const int cnt = (int)min((int64_t)kBatch, jf1 - jb);
-        float2 a[kBatch];
+    for (int q = 0; q < kBatch; ++q)
+      a[q] = q < cnt ? ldc(V.A, i + (jb + q) * V.lda) : cd{0.0, 0.0};
 #pragma unroll
-        for (int q = 0; q < kBatch; ++q)
-          a[q] = q < cnt ? Acol[(jb + q) * lda] : make_float2(0.f, 0.f);
+    for (int q = 0; q < kBatch; ++q) {
+      if (q < cnt) {
+        const float aa = with_abs ? fabs_c(a[q]) : 0.f;
 #pragma unroll
-        for (int q = 0; q < kBatch; ++q) {
-          if (q < cnt) {
-            const float aa = with_abs ? sqrtf(fmaf(a[q].x, a[q].x, a[q].y * a[q].y)) : 0.f;
-#pragma unroll
-            for (int r = 0; r < kGemvR; ++r) {
-              if (r < nr) {
-                const int64_t xo = jb + q + (int64_t)(r0 + r) * ldxs;
-                const float4 x = V.xs[xo];
-                // re += a.x x.re - a.y x.im ; im += a.x x.im + a.y x.re
-                pair_add_prod(re[r], a[q].x, x.x);
-                pair_add_prod(re[r], -a[q].y, x.y);
-                pair_add_prod(im[r], a[q].x, x.y);
-                pair_add_prod(im[r], a[q].y, x.x);
-                re[r].t = __fmaf_rn(a[q].x, x.z, __fmaf_rn(-a[q].y, x.w, re[r].t));
-                im[r].t = __fmaf_rn(a[q].x, x.w, __fmaf_rn(a[q].y, x.z, im[r].t));
-                if (with_abs) aacc[r] = fmaf(aa, V.xa[xo], aacc[r]);
-              }
-            }
+        for (int r = 0; r < kGemvR; ++r) {
+          if (r < nr) {
+            const cd x = ldc(V.x, jb + q + (int64_t)(r0 + r) * V.ldx);
+            acc[r].x = fma(a[q].x, x.x, fma(-a[q].y, x.y, acc[r].x));
+            acc[r].y = fma(a[q].x, x.y, fma(a[q].y, x.x, acc[r].y));
+            if (with_abs) aacc[r] = fmaf(aa, fabs_c(x), aacc[r]);
           }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < kGemvR; ++r) {
-        acc[r].x += (double)re[r].s + (double)re[r].t;
-        acc[r].y += (double)im[r].s + (double)im[r].t;
-      }
-    }
-  } else {
-    for (int64_t j = j0; j < j1; ++j) {
-      cd a = ldc(V.A, i + j * V.lda);
-      const float aa = with_abs ? fabs_c(a) : 0.f;
-#pragma unroll
-      for (int r = 0; r < kGemvR; ++r) {
-        if (r < nr) {
-          cd x = ldc(V.x, j + (int64_t)(r0 + r) * V.ldx);
-          acc[r].x = fma(a.x, x.x, fma(-a.y, x.y, acc[r].x));
-          acc[r].y = fma(a.x, x.y, fma(a.y, x.x, acc[r].y));
-          if (with_abs) aacc[r] = fmaf(aa, fabs_c(x), aacc[r]);
         }
       }
     }
@@ -404,99 +414,142 @@ __device__ __forceinline__ void gemv_body(const VecInst& V, int with_abs) {
   }
 }
 
-// Compact instances: ROWS rows per thread (i, i + 256, ..., all coalesced), so every x
-// value loaded serves ROWS rows and each thread carries 2 ROWS independent pair-sum chains
-// per right-hand side.  Columns are loaded kBatch at a time, folded into FP64 every
-// kFold columns.  ROWS (1 or 2) is a launch shape of the autotuner; it does not change
-// any row's arithmetic.
-template <int NR, int ROWS>
-__device__ __forceinline__ void gemv_a32_body(const VecInst& V, int with_abs) {
-  constexpr int kA32Rows = ROWS;
-  constexpr int kFold = 32, kBatch = NR == 1 ? 8 : 4;
-  const int64_t n = V.n;
-  const int64_t i0 = (int64_t)blockIdx.x * (256 * kA32Rows) + threadIdx.x;
-  const int ch = blockIdx.y % kChunks, grp = blockIdx.y / kChunks;
+// Compact instances: a thread takes two rows (T apart: coalesced) as the halves of the paired
+// instructions.  Its columns come through a ring of its own in shared memory, kA32Stages groups of
+// kA32Cols ahead by asynchronous copies, so that no thread waits for another one: with the loads in
+// registers the kernel waited for them half of the time, 1.69 ms for four systems of 10240
+// unknowns (3.4 GB, 0.53 ms of reading); now 1.23 ms, of which the issue of about 54 instructions
+// per entry (14 of them for |A||x|) is half.  The sums are folded into FP64 every kFold columns.
+// T (64 or 128) is a launch shape of the autotuner; it does not change any row's arithmetic.
+constexpr int kA32Cols = 4, kA32Stages = 4;
+constexpr int a32_smem(int threads) { return kA32Stages * kA32Cols * 2 * 8 * threads; }
+
+template <int NR, bool ABS, int T>
+__global__ void __launch_bounds__(T, (NR == 1 ? 640 : 512) / T) k_gemv_a32(const VecInst* __restrict__ insts) {
+  constexpr int kFold = 32, kRows = 2;
+  const VecInst& V = insts[blockIdx.z];
+  if (!V.a32) return;
+  extern __shared__ __align__(16) unsigned char a32_ring[];
+  const int64_t n = V.n, lda = V.lda;
+  const int64_t i0 = (int64_t)blockIdx.x * (kRows * T) + threadIdx.x;
+  const int ch = blockIdx.y % kMaxChunks, grp = blockIdx.y / kMaxChunks;
+  if (ch >= vec_chunks(n)) return;
   const int r0 = grp * NR;
   if (i0 >= n || r0 >= V.nrhs) return;
   const int nr = min(NR, V.nrhs - r0);
-  const bool ok1 = i0 + 256 < n;
   int64_t j0, j1;
-  chunk_range(n, ch, kChunks, &j0, &j1);
-  const float2* A0 = reinterpret_cast<const float2*>(V.A) + i0;
-  const float2* A1 = (ROWS > 1 && ok1) ? A0 + 256 : A0;
-  const int64_t lda = V.lda;
+  chunk_range(n, ch, vec_chunks(n), &j0, &j1);
+  const int cols = (int)(j1 - j0), groups = cols / kA32Cols;  // whole groups
+  const float2* A[kRows];  // rows past the last: the first one again
+#pragma unroll
+  for (int h = 0; h < kRows; ++h)
+    A[h] = reinterpret_cast<const float2*>(V.A) + (i0 + T * h < n ? i0 + T * h : i0) + j0 * lda;
+  // column q, row h of group g: ring[((g % kA32Stages) kA32Cols + q) kRows + h][thread]
+  float2* ring = reinterpret_cast<float2*>(a32_ring) + threadIdx.x;
+  const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring);
+  constexpr uint32_t kGroup = kA32Cols * kRows * T;  // entries
+  int fetched = 0;
+  uint32_t to = 0, from = 0;
+  auto fetch = [&]() {
+    if (fetched < groups) {
+      const uint32_t at = ring_at + to * 8;
+#pragma unroll
+      for (int q = 0; q < kA32Cols; ++q)
+#pragma unroll
+        for (int h = 0; h < kRows; ++h) {
+          cp_async8(at + (kRows * q + h) * T * 8, A[h]);
+          A[h] += lda;
+        }
+    }
+    ++fetched;
+    to = to == (kA32Stages - 1) * kGroup ? 0 : to + kGroup;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int g = 0; g < kA32Stages - 1; ++g) fetch();
   const float4* xs[NR];
   const float* xa[NR];
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
-    const int64_t rr = (int64_t)(r0 + (r < nr ? r : 0)) * n;
-    xs[r] = V.xs + rr;
+    const int64_t rr = (int64_t)(r0 + (r < nr ? r : 0)) * n + j0;
+    xs[r] = V.xs + 2 * rr;
     xa[r] = V.xa + rr;
   }
-  cd acc[kA32Rows][NR];
-  float aacc[kA32Rows][NR];
+  cd acc[kRows][NR];
+  float aacc[kRows][NR];
 #pragma unroll
-  for (int h = 0; h < kA32Rows; ++h)
+  for (int h = 0; h < kRows; ++h)
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       acc[h][r] = cd{0.0, 0.0};
       aacc[h][r] = 0.f;
     }
-  for (int64_t jf = j0; jf < j1; jf += kFold) {
-    FPair re[kA32Rows][NR], im[kA32Rows][NR];
+  FPair re[NR], im[NR];
 #pragma unroll
-    for (int h = 0; h < kA32Rows; ++h)
-#pragma unroll
-      for (int r = 0; r < NR; ++r) re[h][r] = im[h][r] = FPair{0.f, 0.f};
-    const int64_t jf1 = min(j1, jf + kFold);
-    for (int64_t jb = jf; jb < jf1; jb += kBatch) {
-      const int cnt = (int)min((int64_t)kBatch, jf1 - jb);
-      float2 a[kA32Rows][kBatch];
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        a[0][q] = q < cnt ? A0[(jb + q) * lda] : make_float2(0.f, 0.f);
-        if (ROWS > 1) a[ROWS - 1][q] = q < cnt ? A1[(jb + q) * lda] : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        if (q < cnt) {
-          float aa[kA32Rows];
-#pragma unroll
-          for (int h = 0; h < kA32Rows; ++h)
-            aa[h] = with_abs ? sqrtf(fmaf(a[h][q].x, a[h][q].x, a[h][q].y * a[h][q].y)) : 0.f;
-#pragma unroll
-          for (int r = 0; r < NR; ++r) {
-            const float4 x = xs[r][jb + q];
-            const float xm = with_abs ? xa[r][jb + q] : 0.f;
-#pragma unroll
-            for (int h = 0; h < kA32Rows; ++h) {
-              const float2 av = a[h][q];
-              // re += a.x x.re - a.y x.im ; im += a.x x.im + a.y x.re
-              pair_add_prod(re[h][r], av.x, x.x);
-              pair_add_prod(re[h][r], -av.y, x.y);
-              pair_add_prod(im[h][r], av.x, x.y);
-              pair_add_prod(im[h][r], av.y, x.x);
-              re[h][r].t = __fmaf_rn(av.x, x.z, __fmaf_rn(-av.y, x.w, re[h][r].t));
-              im[h][r].t = __fmaf_rn(av.x, x.w, __fmaf_rn(av.y, x.z, im[h][r].t));
-              aacc[h][r] = fmaf(aa[h], xm, aacc[h][r]);
-            }
-          }
-        }
-      }
+  for (int r = 0; r < NR; ++r) re[r] = im[r] = FPair{};
+  // column c past xs and xa
+  auto column = [&](float2 a0, float2 a1, int c) {
+    const float2 ax = make_float2(a0.x, a1.x), ay = make_float2(a0.y, a1.y);
+    const float2 nax = f2_neg(ax), nay = f2_neg(ay);
+    float m0 = 0.f, m1 = 0.f;
+    if (ABS) {
+      m0 = sqrtf(fmaf(a0.x, a0.x, a0.y * a0.y));
+      m1 = sqrtf(fmaf(a1.x, a1.x, a1.y * a1.y));
     }
 #pragma unroll
-    for (int h = 0; h < kA32Rows; ++h)
-#pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        acc[h][r].x += (double)re[h][r].s + (double)re[h][r].t;
-        acc[h][r].y += (double)im[h][r].s + (double)im[h][r].t;
+    for (int r = 0; r < NR; ++r) {
+      const float4 hi = xs[r][2 * c], lo = xs[r][2 * c + 1];  // (re re, im im)
+      const float2 hr = make_float2(hi.x, hi.y), hm = make_float2(hi.z, hi.w);
+      const float2 lr = make_float2(lo.x, lo.y), lm = make_float2(lo.z, lo.w);
+      // re += a.x x.re - a.y x.im ; im += a.x x.im + a.y x.re
+      pair_add_prod(re[r], ax, nax, hr);
+      pair_add_prod(re[r], nay, ay, hm);
+      pair_add_prod(im[r], ax, nax, hm);
+      pair_add_prod(im[r], ay, nay, hr);
+      re[r].t = __ffma2_rn(ax, lr, __ffma2_rn(nay, lm, re[r].t));
+      im[r].t = __ffma2_rn(ax, lm, __ffma2_rn(ay, lr, im[r].t));
+      if (ABS) {
+        const float xm = xa[r][c];
+        aacc[0][r] = fmaf(m0, xm, aacc[0][r]);
+        aacc[1][r] = fmaf(m1, xm, aacc[1][r]);
       }
+    }
+  };
+  auto fold = [&]() {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      acc[0][r].x += (double)re[r].s.x + (double)re[r].t.x;
+      acc[0][r].y += (double)im[r].s.x + (double)im[r].t.x;
+      acc[1][r].x += (double)re[r].s.y + (double)re[r].t.y;
+      acc[1][r].y += (double)im[r].s.y + (double)im[r].t.y;
+      re[r] = im[r] = FPair{};
+    }
+  };
+  for (int g = 0; g < groups; ++g) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kA32Stages - 2) : "memory");
+    const float2* at = ring + from;
+    from = from == (kA32Stages - 1) * kGroup ? 0 : from + kGroup;
+#pragma unroll
+    for (int q = 0; q < kA32Cols; ++q) column(at[(2 * q) * T], at[(2 * q + 1) * T], q);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      xs[r] += 2 * kA32Cols;
+      xa[r] += kA32Cols;
+    }
+    fetch();  // into the group read before this one
+    if ((g + 1) % (kFold / kA32Cols) == 0) fold();
   }
+  for (int c = 0; c < cols - groups * kA32Cols; ++c) {  // A stands behind the whole groups
+    column(*A[0], *A[1], c);
+    A[0] += lda;
+    A[1] += lda;
+  }
+  fold();
   // part layout: [chunk][rhs][row] x (re, im, abs)
 #pragma unroll
-  for (int h = 0; h < kA32Rows; ++h) {
-    const int64_t i = i0 + 256 * h;
-    if (h == 1 && !ok1) break;
+  for (int h = 0; h < kRows; ++h) {
+    const int64_t i = i0 + T * h;
+    if (i >= n) break;
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       if (r < nr) {
@@ -509,57 +562,87 @@ __device__ __forceinline__ void gemv_a32_body(const VecInst& V, int with_abs) {
   }
 }
 
-template <int NR, int ROWS>
-__global__ void __launch_bounds__(256, 2) k_gemv_a32(const VecInst* __restrict__ insts, int with_abs) {
-  const VecInst& V = insts[blockIdx.z];
-  if (!V.a32) return;
-  gemv_a32_body<NR, ROWS>(V, with_abs);
+template <int NR, bool ABS, int T>
+void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int groups) {
+  static PerDeviceOnce attr;
+  attr.call([] {
+    cudaFuncSetAttribute(k_gemv_a32<NR, ABS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         a32_smem(T));
+  });
+  constexpr int rows = 2 * T;
+  k_gemv_a32<NR, ABS, T><<<dim3((unsigned)((nmax + rows - 1) / rows),
+                                (unsigned)(kMaxChunks * groups), (unsigned)ninst),
+                           T, a32_smem(T), L.stream>>>(d);
+}
+template <int NR, bool ABS>
+void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int groups, int rows) {
+  if (rows == 1)
+    gemv_a32<NR, ABS, 64>(L, d, ninst, nmax, groups);
+  else
+    gemv_a32<NR, ABS, 128>(L, d, ninst, nmax, groups);
 }
 
 // partial y = A x (and |A||x|) over a column chunk, up to kGemvR right-hand sides
-// per pass (rhs group = blockIdx.y / kChunks).
-template <bool A32, int NR>
+// per pass (rhs group = blockIdx.y / kMaxChunks).
+template <int NR>
 __global__ void __launch_bounds__(256) k_gemv_part(const VecInst* __restrict__ insts, int with_abs) {
   const VecInst& V = insts[blockIdx.z];
-  if ((V.a32 != 0) != A32) return;
-  gemv_body<A32, NR>(V, with_abs);
+  if (V.a32) return;
+  gemv_body<NR>(V, with_abs);
 }
 
-// the row's near corrections (FP64, fixed CSR order) times x
-__device__ __forceinline__ cd near_product(const VecInst& V, int64_t i, int r, cd s) {
+// Lane s of the eight threads of a row: its share of the row's near corrections (FP64, every
+// eighth pair) times x, added to t.
+__device__ __forceinline__ void near_product(const VecInst& V, int64_t i, int r, int s, cd& t) {
   const int br = i >= V.n_mesh ? 1 : 0;
   const int64_t im_ = i - br * V.n_mesh;
-  for (int32_t p = V.near_ptr[im_]; p < V.near_ptr[im_ + 1]; ++p) {
+  const int32_t p1 = V.near_ptr[im_ + 1];
+  for (int32_t p = V.near_ptr[im_] + s; p < p1; p += 8) {
     const int64_t j = V.near_j[p];
     for (int bc = 0; bc < V.nbc; ++bc) {
       const cd d = ldc(V.dnear, (int64_t)(br * V.nbc + bc) * V.n_near + p);
       const cd x = ldc(V.x, j + bc * V.n_mesh + (int64_t)r * V.ldx);
-      s.x = fma(d.x, x.x, fma(-d.y, x.y, s.x));
-      s.y = fma(d.x, x.y, fma(d.y, x.x, s.y));
+      t.x = fma(d.x, x.x, fma(-d.y, x.y, t.x));
+      t.y = fma(d.x, x.y, fma(d.y, x.x, t.y));
     }
   }
-  return s;
+}
+__device__ __forceinline__ double row8_sum(double v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// mode 0: y = A x.  mode 1: y = b - A x, den = |b| + |A||x|.  Compact instances add the
-// near corrections of the row (FP64, fixed CSR order).
+// mode 0: y = A x.  mode 1: y = b - A x, den = |b| + |A||x|.  Compact instances add the near
+// corrections of the row.  Eight threads per row (a chunk sum and a list of about 30 pairs is a
+// chain of dependent loads: 41 us for 1280 rows with one thread, 12 us with eight), their
+// shares added by a fixed tree.
 __global__ void k_gemv_finish(const VecInst* __restrict__ insts, int mode) {
   const VecInst& V = insts[blockIdx.z];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y;
-  if (i >= V.n || r >= V.nrhs) return;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int r = blockIdx.y, s = threadIdx.x & 7;
+  if (r >= V.nrhs) return;
+  const bool on = i < V.n;
   double re = 0.0, im = 0.0, ab = 0.0;
-  for (int c = 0; c < kChunks; ++c) {
-    int64_t o = 3 * (((int64_t)c * V.nrhs + r) * V.n + i);
-    re += V.part[o];
-    im += V.part[o + 1];
-    ab += V.part[o + 2];
+  if (on) {
+    const int chunks = vec_chunks(V.n);
+    for (int c = s; c < chunks; c += 8) {
+      const int64_t o = 3 * (((int64_t)c * V.nrhs + r) * V.n + i);
+      re += V.part[o];
+      im += V.part[o + 1];
+      ab += V.part[o + 2];
+    }
+    if (V.a32) {
+      cd t = {re, im};
+      near_product(V, i, r, s, t);
+      re = t.x;
+      im = t.y;
+    }
   }
-  if (V.a32) {
-    const cd s = near_product(V, i, r, cd{re, im});
-    re = s.x;
-    im = s.y;
-  }
+  re = row8_sum(re);
+  im = row8_sum(im);
+  ab = row8_sum(ab);
+  if (!on || s != 0) return;
   const int64_t yo = i + (int64_t)r * V.ldy;
   if (mode == 0) {
     stc(V.y, yo, cd{re, im});
@@ -656,33 +739,47 @@ void launch_wide_abs(const Launch& L, const VecInst& v, float* xa) {
 }
 
 __global__ void k_wide_finish(const VecInst V, int mode) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y;
-  if (i >= V.n) return;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int r = blockIdx.y, s = threadIdx.x & 7;
+  const bool on = i < V.n;
+  cd t = {0.0, 0.0};
+  if (on && V.a32) near_product(V, i, r, s, t);
+  t.x = row8_sum(t.x);
+  t.y = row8_sum(t.y);
+  if (!on || s != 0) return;
   const int64_t yo = i + (int64_t)r * V.ldy;
-  cd y = ldc(V.y, yo);
-  const cd nearp = V.a32 ? near_product(V, i, r, cd{0.0, 0.0}) : cd{0.0, 0.0};
-  y = y - nearp;
+  const cd y = ldc(V.y, yo) - t;
   stc(V.y, yo, mode == 0 ? cd{-y.x, -y.y} : y);
 }
 
 void launch_wide_finish(const Launch& L, const VecInst& v, int mode) {
-  k_wide_finish<<<dim3((unsigned)((v.n + 255) / 256), (unsigned)v.nrhs), 256, 0, L.stream>>>(v, mode);
+  k_wide_finish<<<dim3((unsigned)((v.n + 31) / 32), (unsigned)v.nrhs), 256, 0, L.stream>>>(v, mode);
   count_launch(1);
 }
 
 // Per right-hand side statistics of a residual r (in y), denominators den, solution x,
 // rhs b and row scales:  [0] max|r|  [1] max |r|/den (0/0 = 0, r/0 = inf)  [2] max|x|
 // [3] max|b|  [4] sum|r|^2  [5] sum|b|^2  [6] sum|r/rows|^2  [7] sum|b/rows|^2
-// [8] nonfinite flag.  One CTA per (rhs, instance).
+// [8] nonfinite flag.  The hypots make it FP64-bound (about 250 instructions a row), so the
+// rows of a right-hand side are shared by stat_split(n) CTAs whose results, left in the products'
+// scratch, the second kernel combines in order: 0.6 ms a pass for one system of 8960 unknowns
+// with one CTA, 32 us so.
+constexpr int kMaxStatSplit = 16;
+__host__ __device__ inline int stat_split(int64_t n) {
+  return n < 512 ? 1 : n >= 256 * kMaxStatSplit ? kMaxStatSplit : (int)(n / 256);
+}
+__device__ __forceinline__ bool stat_is_sum(int t) { return t >= 4 && t <= 7; }
+
 __global__ void __launch_bounds__(256) k_resid_stats(const VecInst* __restrict__ insts) {
   const VecInst& V = insts[blockIdx.y];
-  const int r = blockIdx.x;
-  if (r >= V.nrhs) return;
+  const int r = blockIdx.x, split = stat_split(V.n), z = blockIdx.z;
+  if (r >= V.nrhs || z >= split) return;
+  int64_t j0, j1;
+  chunk_range(V.n, z, split, &j0, &j1);
   double v[kStats];
 #pragma unroll
   for (int t = 0; t < kStats; ++t) v[t] = 0.0;
-  for (int64_t i = threadIdx.x; i < V.n; i += 256) {
+  for (int64_t i = j0 + threadIdx.x; i < j1; i += 256) {
     const int64_t o = i + (int64_t)r * V.ldy;
     cd rr = ldc(V.y, o);
     cd bb = ldc(V.b, i + (int64_t)r * V.ldb);
@@ -711,23 +808,41 @@ __global__ void __launch_bounds__(256) k_resid_stats(const VecInst* __restrict__
 #pragma unroll
       for (int t = 0; t < kStats; ++t) {
         double a = sh[t][threadIdx.x], b = sh[t][threadIdx.x + s];
-        sh[t][threadIdx.x] = (t == 4 || t == 5 || t == 6 || t == 7) ? a + b : fmax(a, b);
+        sh[t][threadIdx.x] = stat_is_sum(t) ? a + b : fmax(a, b);
       }
     }
     __syncthreads();
   }
-  if (threadIdx.x < kStats) V.stats[(int64_t)r * kStats + threadIdx.x] = sh[threadIdx.x][0];
+  if (threadIdx.x < kStats)
+    V.part[((int64_t)r * split + z) * kStats + threadIdx.x] = sh[threadIdx.x][0];
 }
 
 // ---------------------------------------------------------------- correction steps
-// stats[r * kStats] = max_i |v_i / rows_i| for the vectors in y (v = b or residual)
+
+__global__ void k_stats_finish(const VecInst* __restrict__ insts) {
+  const VecInst& V = insts[blockIdx.y];
+  const int r = blockIdx.x, t = threadIdx.x, split = stat_split(V.n);
+  if (r >= V.nrhs || t >= kStats) return;
+  double v = 0.0;
+  for (int z = 0; z < split; ++z) {
+    const double a = V.part[((int64_t)r * split + z) * kStats + t];
+    v = stat_is_sum(t) ? v + a : fmax(v, a);
+  }
+  V.stats[(int64_t)r * kStats + t] = v;
+}
+
+// The maxima of |v_i / rows_i| over each CTA's rows of the vectors in y (v = b or residual); NaN
+// where one isn't finite.  Split as the statistics, for the same reason: 88 us for one system of
+// 8960 unknowns with one CTA, 11 us so.
 __global__ void __launch_bounds__(256) k_scaled_absmax(const VecInst* __restrict__ insts) {
   const VecInst& V = insts[blockIdx.y];
-  const int r = blockIdx.x;
-  if (r >= V.nrhs) return;
+  const int r = blockIdx.x, split = stat_split(V.n), z = blockIdx.z;
+  if (r >= V.nrhs || z >= split) return;
+  int64_t j0, j1;
+  chunk_range(V.n, z, split, &j0, &j1);
   double m = 0.0;
   bool bad = false;
-  for (int64_t i = threadIdx.x; i < V.n; i += 256) {
+  for (int64_t i = j0 + threadIdx.x; i < j1; i += 256) {
     cd a = ldc(V.y, i + (int64_t)r * V.ldy);
     double s = V.rows ? V.rows[i] : 1.0;
     double t = hypot(a.x / s, a.y / s);
@@ -735,26 +850,33 @@ __global__ void __launch_bounds__(256) k_scaled_absmax(const VecInst* __restrict
     m = fmax(m, t);
   }
   __shared__ double sh[256];
-  __shared__ int sb;
-  if (threadIdx.x == 0) sb = 0;
-  __syncthreads();
-  if (bad) sb = 1;
+  bad = __syncthreads_or(bad);
   sh[threadIdx.x] = m;
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) {
     if (threadIdx.x < s) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + s]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) V.stats[(int64_t)r * kStats] = sb ? NAN : sh[0];
+  if (threadIdx.x == 0) V.part[(int64_t)r * split + z] = bad ? NAN : sh[0];
 }
 
-// work (getrs input, complex64 or complex128, ld n) = (v / rows) / mag
+// work (getrs input, complex64 or complex128, ld n) = (v / rows) / mag, mag the largest of
+// k_scaled_absmax's maxima
 __global__ void k_corr_prep(const VecInst* __restrict__ insts) {
   const VecInst& V = insts[blockIdx.z];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y;
   if (i >= V.n || r >= V.nrhs) return;
-  const double mag = V.stats[(int64_t)r * kStats];
+  const int split = stat_split(V.n);
+  double mag = 0.0;
+  bool bad = false;
+  for (int z = 0; z < split; ++z) {
+    const double m = V.part[(int64_t)r * split + z];
+    bad = bad || isnan(m);
+    mag = fmax(mag, m);
+  }
+  if (bad) mag = NAN;
+  if (i == 0) V.stats[(int64_t)r * kStats] = mag;  // for the way back
   cd a = ldc(V.y, i + (int64_t)r * V.ldy);
   double s = V.rows ? V.rows[i] : 1.0;
   cd w = {0.0, 0.0};
@@ -804,7 +926,7 @@ __global__ void k_corr_apply(const VecInst* __restrict__ insts, int mode) {
 
 // ---------------------------------------------------------------- launch wrappers
 void launch_equilibrate(const Launch& L, const VecInst* d, int ninst, int64_t nmax) {
-  dim3 g1((unsigned)((nmax + 255) / 256), kChunks, (unsigned)ninst);
+  dim3 g1((unsigned)((nmax + 255) / 256), kMaxChunks, (unsigned)ninst);
   k_rowstats<<<g1, 256, 0, L.stream>>>(d); count_launch(1);
   k_rowstats_finish<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)ninst), 256, 0, L.stream>>>(d); count_launch(1);
   k_colmax<<<dim3((unsigned)((nmax + 7) / 8), (unsigned)ninst), 256, 0, L.stream>>>(d); count_launch(1);
@@ -813,9 +935,9 @@ void launch_equilibrate(const Launch& L, const VecInst* d, int ninst, int64_t nm
 void launch_scale_copy(const Launch& L, const VecInst* d, int ninst, int64_t nmax) {
   k_cols_inv<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)ninst), 256, 0, L.stream>>>(d);
   count_launch(1);
-  dim3 g1((unsigned)((nmax + 255) / 256), kChunks, (unsigned)ninst);
+  dim3 g1((unsigned)((nmax + 255) / 256), kMaxChunks, (unsigned)ninst);
   k_scale_copy<<<g1, 256, 0, L.stream>>>(d); count_launch(1);
-  k_norms_finish<<<ninst, 256, 0, L.stream>>>(d); count_launch(1);
+  k_norms_finish<<<ninst, kNormT, 0, L.stream>>>(d); count_launch(1);
 }
 
 void launch_gemv(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int32_t max_rhs,
@@ -826,25 +948,22 @@ void launch_gemv(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int
   const int groups = (max_rhs + nr - 1) / nr;
   dim3 g0((unsigned)((nmax + 255) / 256), (unsigned)max_rhs, (unsigned)ninst);
   k_split_x<<<g0, 256, 0, L.stream>>>(d); count_launch(1);
-  dim3 g1((unsigned)((nmax + 255) / 256), (unsigned)(kChunks * groups), (unsigned)ninst);
-  const int rw = rows == 1 ? 1 : 2;
-  dim3 ga((unsigned)((nmax + 256 * rw - 1) / (256 * rw)), (unsigned)(kChunks * groups),
-          (unsigned)ninst);
+  dim3 g1((unsigned)((nmax + 255) / 256), (unsigned)(kMaxChunks * groups), (unsigned)ninst);
   if (nr == 1) {
-    if (rw == 1)
-      k_gemv_a32<1, 1><<<ga, 256, 0, L.stream>>>(d, mode == 1);
+    if (mode == 1)
+      gemv_a32<1, true>(L, d, ninst, nmax, groups, rows);
     else
-      k_gemv_a32<1, 2><<<ga, 256, 0, L.stream>>>(d, mode == 1);
-    k_gemv_part<false, 1><<<g1, 256, 0, L.stream>>>(d, mode == 1);
+      gemv_a32<1, false>(L, d, ninst, nmax, groups, rows);
+    k_gemv_part<1><<<g1, 256, 0, L.stream>>>(d, mode == 1);
   } else {
-    if (rw == 1)
-      k_gemv_a32<kGemvR, 1><<<ga, 256, 0, L.stream>>>(d, mode == 1);
+    if (mode == 1)
+      gemv_a32<kGemvR, true>(L, d, ninst, nmax, groups, rows);
     else
-      k_gemv_a32<kGemvR, 2><<<ga, 256, 0, L.stream>>>(d, mode == 1);
-    k_gemv_part<false, kGemvR><<<g1, 256, 0, L.stream>>>(d, mode == 1);
+      gemv_a32<kGemvR, false>(L, d, ninst, nmax, groups, rows);
+    k_gemv_part<kGemvR><<<g1, 256, 0, L.stream>>>(d, mode == 1);
   }
   count_launch(2);
-  dim3 g2((unsigned)((nmax + 255) / 256), (unsigned)max_rhs, (unsigned)ninst);
+  dim3 g2((unsigned)((nmax + 31) / 32), (unsigned)max_rhs, (unsigned)ninst);
   k_gemv_finish<<<g2, 256, 0, L.stream>>>(d, mode); count_launch(1);
 }
 
@@ -863,12 +982,14 @@ void launch_expand_a32(const Launch& L, const VecInst* d, int ninst, int64_t nma
 }
 
 void launch_resid_stats(const Launch& L, const VecInst* d, int ninst, int32_t max_rhs) {
-  k_resid_stats<<<dim3((unsigned)max_rhs, (unsigned)ninst), 256, 0, L.stream>>>(d); count_launch(1);
+  k_resid_stats<<<dim3((unsigned)max_rhs, (unsigned)ninst, kMaxStatSplit), 256, 0, L.stream>>>(d);
+  k_stats_finish<<<dim3((unsigned)max_rhs, (unsigned)ninst), 32, 0, L.stream>>>(d);
+  count_launch(2);
 }
 
 void launch_corr_prep(const Launch& L, const VecInst* d, int ninst, int64_t nmax,
                       int32_t max_rhs) {
-  k_scaled_absmax<<<dim3((unsigned)max_rhs, (unsigned)ninst), 256, 0, L.stream>>>(d); count_launch(1);
+  k_scaled_absmax<<<dim3((unsigned)max_rhs, (unsigned)ninst, kMaxStatSplit), 256, 0, L.stream>>>(d); count_launch(1);
   k_corr_prep<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)max_rhs, (unsigned)ninst), 256, 0,
                 L.stream>>>(d); count_launch(1);
 }

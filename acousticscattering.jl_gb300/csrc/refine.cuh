@@ -5,7 +5,11 @@
 
 namespace bemgpu {
 
-constexpr int kChunks = 8;   // column chunks of the row-wise sweeps
+// Column chunks of the row-wise sweeps, by the system's own order: a thread takes a row, so
+// small systems need more chunks to fill the GPU (1280 unknowns: 24 CTAs with 8 chunks, 76 us
+// a residual; 19 us with 32).
+constexpr int kMaxChunks = 32;
+__host__ __device__ inline int vec_chunks(int64_t n) { return n <= 2560 ? 32 : n <= 5120 ? 16 : 8; }
 constexpr int kGemvR = 4;    // right-hand sides per gemv pass
 constexpr int kStats = 9;    // residual statistics per right-hand side
 
@@ -18,7 +22,7 @@ struct VecInst {
   double* rowsum;    // row sums of |A| (n)
   double* cols_inv;  // 1 / cols (n), filled by the scaled-copy launch
   float* rows_inv;   // 1 / rows (n), filled by the row-statistics launch
-  double* part;      // scratch: kChunks * nrhs * n * 3 doubles (>= kChunks * n * 2)
+  double* part;      // scratch: vec_chunks(n) * nrhs * n * 3 doubles (>= vec_chunks(n) * n * 2)
   void* out;         // scaled copy / correction work buffer (ld n)
   int32_t out_single;
   int32_t nrhs;
@@ -43,7 +47,7 @@ struct VecInst {
   const int32_t* near_i;
   const int32_t* near_j;
   const double* dnear;       // corrections, complex128 [block][n_near], block = nbc br + bc
-  float4* xs;                // x split as FP32 (hi.re, hi.im, lo.re, lo.im), n x nrhs
+  float4* xs;                // x split as FP32, every part twice: (hi.re, hi.im), (lo.re, lo.im)
   float* xa;                 // |x| in FP32, n x nrhs
   float* cols_inv32;         // 1 / cols in FP32 (n)
   double norm_floor;         // equilibration: lower bound of the row and column scales
@@ -52,8 +56,8 @@ struct VecInst {
 #ifdef __CUDACC__
 void launch_equilibrate(const Launch& L, const VecInst* d, int ninst, int64_t nmax);
 void launch_scale_copy(const Launch& L, const VecInst* d, int ninst, int64_t nmax);
-// mode 0: y = A x; mode 1: y = b - A x and den = |b| + |A||x|.  rows: rows per thread of
-// the compact-storage product (1 or 2; results identical)
+// mode 0: y = A x; mode 1: y = b - A x and den = |b| + |A||x|.  rows: CTAs of 128 (1) or
+// 256 (2) rows in the compact-storage product (results identical)
 void launch_gemv(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int32_t max_rhs,
                  int mode, int rows = 2);
 // Products of one system with many vectors (api.cu:wide_product): den = |b| + |A||x|, and the

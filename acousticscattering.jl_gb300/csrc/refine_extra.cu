@@ -144,6 +144,11 @@ __device__ int lac_imax(const float2* x, int n, double* sv, int* si) {
   return bi;
 }
 
+// |z| of a complex64 value: its squares neither overflow nor vanish in FP64
+__device__ __forceinline__ double mag(float2 z) {
+  return sqrt((double)z.x * z.x + (double)z.y * z.y);
+}
+
 __global__ void __launch_bounds__(kLacT) k_lacn2(Lacn2Dev* __restrict__ st, float2* __restrict__ work,
                                                 MatInst* __restrict__ mi1,
                                                 MatInst* __restrict__ mi2, int want) {
@@ -158,13 +163,13 @@ __global__ void __launch_bounds__(kLacT) k_lacn2(Lacn2Dev* __restrict__ st, floa
   double est = S.est;
   auto sum1 = [&]() {
     double t = 0.0;
-    for (int i = threadIdx.x; i < n; i += kLacT) t += hypot((double)x[i].x, (double)x[i].y);
+    for (int i = threadIdx.x; i < n; i += kLacT) t += mag(x[i]);
     return lac_sum(t, sh);
   };
   auto normalise = [&]() {
     const double safmin = 2.2250738585072014e-308;
     for (int i = threadIdx.x; i < n; i += kLacT) {
-      const double re = x[i].x, im = x[i].y, a = hypot(re, im);
+      const double re = x[i].x, im = x[i].y, a = mag(x[i]);
       x[i] = a > safmin ? make_float2((float)(re / a), (float)(im / a)) : make_float2(1.f, 0.f);
     }
   };

@@ -498,7 +498,7 @@ int bemgpu_hmatrix_apply(bemgpu_ctx *ctx, const bemgpu_mesh *mesh, const bemgpu_
 
 /*
  * Launch-shape autotuner (default on): the first time a batch shape is met, the compact
- * residual's rows per thread are chosen by timing the candidates.  Every candidate
+ * residual's CTA size is chosen by timing the candidates.  Every candidate
  * computes bit-identical results.  enable = 0 switches it off and forgets the measured
  * choices (fixed rules are used).  No reference counterpart.
  */
