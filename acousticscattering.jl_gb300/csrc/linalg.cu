@@ -390,6 +390,10 @@ template <typename R, int W, int RPT, int T_>
 __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ insts, int64_t k0,
                                                      int nb, int share) {
   using C = cx<R>;
+  // Columns whose code is unrolled.  All 16 of a sub-panel are 80 KB of instructions that run twice
+  // in a launch: a quarter of the cycles waited for them.  Four at a time: 74 to 58 us a panel of
+  // 1280 rows.  With more than two rows per thread the registers that take turns cost more.
+  constexpr int kU = RPT > 2 || W <= 4 ? W : 4;
   const unsigned rank = cluster_rank(), cs = cluster_size();
   const MatInst& M = insts[blockIdx.x / cs];
   const int64_t n = M.n;
@@ -460,81 +464,101 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
         }
       }
     }
+    // kU columns at a time, after which the columns move up by kU places (back where they were
+    // after W of them)
+#pragma unroll 1
+    for (int w0 = 0; w0 < W; w0 += kU) {
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      if (w >= wn) break;  // uniform over the cluster
-      const int c = s0 + w;
-      const int32_t col = (int32_t)(k0 + c);
-      PivSlot<R, W>* sl = slot[c & 1];
-      // this thread's, the warp's and the CTA's candidate
-      PivKey best = {0u, 0u, INT32_MAX, 0};
+      for (int w = 0; w < kU; ++w) {
+        if (w0 + w >= wn) break;  // uniform over the cluster
+        const int c = s0 + w0 + w;
+        const int32_t col = (int32_t)(k0 + c);
+        PivSlot<R, W>* sl = slot[c & 1];
+        // this thread's, the warp's and the CTA's candidate
+        PivKey best = {0u, 0u, INT32_MAX, 0};
 #pragma unroll
-      for (int t = 0; t < RPT; ++t) {
-        PivKey k;
-        key_of(a[t][w], k.hi, k.lo);
-        k.pos = fz[t] == kPanelNB ? pos[t] : INT32_MAX;
-        k.phys = (int32_t)(g + t * stride);
-        if (!key_nan(k, R{}) && key_better(k, best)) best = k;
-      }
-      warp_best<R>(best);
-      if (lane == 0) s_key[wid] = best;
-      __syncthreads();
-      best = lane < nw ? s_key[lane] : PivKey{0u, 0u, INT32_MAX, 0};
-      const int bw = warp_best<R>(best);  // warp of the CTA's candidate
-      // its owner's warp pushes it to every CTA, lane i to CTA i
-      if (wid == max(bw, 0)) {
-        int own = -1;  // this thread's row that is the candidate
-#pragma unroll
-        for (int t = 0; t < RPT; ++t)
-          if (bw >= 0 && fz[t] == kPanelNB && pos[t] == best.pos) own = t;
-        const uint32_t who = __ballot_sync(0xffffffffu, own >= 0);
-        const int src = who ? __ffs(who) - 1 : 0;
-        const uint32_t dst = peer_smem(&sl[rank], (unsigned)min(lane, (int)cs - 1));
-        const bool send = lane < (int)cs;
-        if (send) {
-          st_peer_b32(dst, best.hi);
-          st_peer_b32(dst + 4, best.lo);
-          st_peer_b32(dst + 8, (uint32_t)best.pos);
-          st_peer_b32(dst + 12, (uint32_t)best.phys);
+        for (int t = 0; t < RPT; ++t) {
+          PivKey k;
+          key_of(a[t][w], k.hi, k.lo);
+          k.pos = fz[t] == kPanelNB ? pos[t] : INT32_MAX;
+          k.phys = (int32_t)(g + t * stride);
+          if (!key_nan(k, R{}) && key_better(k, best)) best = k;
         }
+        warp_best<R>(best);
+        if (lane == 0) s_key[wid] = best;
+        __syncthreads();
+        best = lane < nw ? s_key[lane] : PivKey{0u, 0u, INT32_MAX, 0};
+        const int bw = warp_best<R>(best);  // warp of the CTA's candidate
+        // its owner's warp pushes it to every CTA, lane i to CTA i
+        if (wid == max(bw, 0)) {
+          int own = -1;  // this thread's row that is the candidate
 #pragma unroll
-        for (int q = w; q < W; ++q) {
-          C v = a[0][q];
-#pragma unroll
-          for (int t = 1; t < RPT; ++t)
-            if (own == t) v = a[t][q];
-          v = shfl_c(v, src);
-          if (q == w) v = (best.hi | best.lo) != 0u && bw >= 0 ? cinv_fast(v) : C{(R)1, (R)0};
-          if (send) st_peer_c(dst + 16 + (q == w ? 0 : 1 + q) * (uint32_t)sizeof(C), v);
-        }
-      }
-      cluster_sync_all();
-      // the cluster's pivot; the slots of step c are free again after the barrier of c + 1
-      best = lane < (int)cs ? sl[lane].key : PivKey{0u, 0u, INT32_MAX, 0};
-      const int win = max(warp_best<R>(best), 0);
-      // no candidate (only NaNs): the row at the diagonal position, marked singular
-      const int32_t piv = best.pos == INT32_MAX ? col : best.pos;
-      const bool nonzero = best.pos != INT32_MAX && (best.hi | best.lo) != 0u;
-      const C inv = sl[win].inv;
-      if (rank == 0 && tid == 0) {
-        M.ipiv[col] = piv;
-        if (!nonzero && *M.info == 0) *M.info = col + 1;
-      }
-      if (tid == 0) s_phys[c] = best.pos != INT32_MAX ? best.phys : col;
-#pragma unroll
-      for (int t = 0; t < RPT; ++t) {
-        if (fz[t] == kPanelNB) {
-          if (pos[t] == piv) {
-            fz[t] = c;
-            pos[t] = col;
-          } else {
-            if (pos[t] == col) pos[t] = piv;
-            const C l = a[t][w] * inv;
-            a[t][w] = l;
-#pragma unroll
-            for (int q = w + 1; q < W; ++q)
-              if (q < wn) cfnma(a[t][q], l, sl[win].row[q]);
+          for (int t = 0; t < RPT; ++t)
+            if (bw >= 0 && fz[t] == kPanelNB && pos[t] == best.pos) own = t;
+          const uint32_t who = __ballot_sync(0xffffffffu, own >= 0);
+          const int src = who ? __ffs(who) - 1 : 0;
+          const uint32_t dst = peer_smem(&sl[rank], (unsigned)min(lane, (int)cs - 1));
+          const bool send = lane < (int)cs;
+          if (send) {
+            st_peer_b32(dst, best.hi);
+            st_peer_b32(dst + 4, best.lo);
+            st_peer_b32(dst + 8, (uint32_t)best.pos);
+            st_peer_b32(dst + 12, (uint32_t)best.phys);
           }
+#pragma unroll
+          for (int q = w; q < W; ++q) {
+            if (q / kU * kU >= wn - w0) break;  // columns that are left, rounded up to kU
+            C v = a[0][q];
+#pragma unroll
+            for (int t = 1; t < RPT; ++t)
+              if (own == t) v = a[t][q];
+            v = shfl_c(v, src);
+            if (q == w) v = (best.hi | best.lo) != 0u && bw >= 0 ? cinv_fast(v) : C{(R)1, (R)0};
+            if (send) st_peer_c(dst + 16 + (q == w ? 0 : 1 + q) * (uint32_t)sizeof(C), v);
+          }
+        }
+        cluster_sync_all();
+        // the cluster's pivot; the slots of step c are free again after the barrier of c + 1
+        best = lane < (int)cs ? sl[lane].key : PivKey{0u, 0u, INT32_MAX, 0};
+        const int win = max(warp_best<R>(best), 0);
+        // no candidate (only NaNs): the row at the diagonal position, marked singular
+        const int32_t piv = best.pos == INT32_MAX ? col : best.pos;
+        const bool nonzero = best.pos != INT32_MAX && (best.hi | best.lo) != 0u;
+        const C inv = sl[win].inv;
+        if (rank == 0 && tid == 0) {
+          M.ipiv[col] = piv;
+          if (!nonzero && *M.info == 0) *M.info = col + 1;
+        }
+        if (tid == 0) s_phys[c] = best.pos != INT32_MAX ? best.phys : col;
+#pragma unroll
+        for (int t = 0; t < RPT; ++t) {
+          if (fz[t] == kPanelNB) {
+            if (pos[t] == piv) {
+              fz[t] = c;
+              pos[t] = col;
+            } else {
+              if (pos[t] == col) pos[t] = piv;
+              const C l = a[t][w] * inv;
+              a[t][w] = l;
+#pragma unroll
+              for (int q = w + 1; q < W; ++q) {
+                if (q / kU * kU >= wn - w0) break;
+                cfnma(a[t][q], l, sl[win].row[q]);
+              }
+            }
+          }
+        }
+      }
+      if (W > kU) {
+#pragma unroll
+        for (int t = 0; t < RPT; ++t) {
+          C first[kU];
+#pragma unroll
+          for (int w = 0; w < kU; ++w) first[w] = a[t][w];
+#pragma unroll
+          for (int w = 0; w + kU < W; ++w) a[t][w] = a[t][w + kU];
+#pragma unroll
+          for (int w = 0; w < kU; ++w) a[t][W - kU + w] = first[w];
         }
       }
     }
