@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
       if (e < nr * NB && r < n)
         bv[o] = ldv<R>(src, (int64_t)(r0g + e / NB) * ldx + (args.swaps ? M.perm[r] : r));
     }
-    C pre[P];
+    C pre[P];  // as stored: conjugated where used, as a use at the load would wait for it
     auto fetch = [&](int64_t qj) {  // this thread's entries of block (b, j)
       const int64_t c0 = (LOWER ? qj : nblk - 1 - qj) * NB;
       if (!TRANS) {
@@ -318,7 +318,6 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
         for (int e = 0; e < P; ++e) {
           const int64_t r = row0 + wid * RW + e / KL, c = c0 + lane + 32 * (e % KL);
           pre[e] = r < n && c < n ? ldv<R>(M.a, c + r * lda) : C{0, 0};
-          pre[e].y = -pre[e].y;
         }
       }
     };
@@ -370,7 +369,7 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
 #pragma unroll
           for (int i = 0; i < KL; ++i) ok = ok && await(g, c0 + lane + 32 * i, true, xv[i]);
 #pragma unroll
-          for (int e = 0; e < P; ++e) fma_c(acc[TRANS ? e / KL : 0][g], pre[e], xv[e % KL]);
+          for (int e = 0; e < P; ++e) fma_c(acc[TRANS ? e / KL : 0][g], C{pre[e].x, -pre[e].y}, xv[e % KL]);
         }
       }
       if (!ok) break;
@@ -451,7 +450,7 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
         if (kUnit ? i > j : i <= j) {
 #pragma unroll
           for (int g = 0; g < RG; ++g)
-            if (g < nr) fma_c(t[TRANS ? e / KL : 0][g], pre[e], sx[g * NB + c]);
+            if (g < nr) fma_c(t[TRANS ? e / KL : 0][g], TRANS ? C{pre[e].x, -pre[e].y} : pre[e], sx[g * NB + c]);
         }
       }
       row_sums<C, TRANS, RG, RW, KQ, NB>(t, sred, nr, tid);
