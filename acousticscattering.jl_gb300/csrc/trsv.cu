@@ -346,6 +346,23 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
         if (lane == 0) atomicExch(err, kErrTimeout);
         return false;
       };
+      auto await_row = [&](int g, int64_t c, C(&v)[KL]) {  // the entries c + 32 i
+        const int64_t i0 = (int64_t)(r0g + g) * ldx + c;
+#pragma unroll
+        for (int i = 0; i < KL; ++i) v[i] = C{0, 0};
+        for (uint32_t it = 0; it < kSpinLimit; ++it) {
+          bool missing = false;
+#pragma unroll
+          for (int i = 0; i < KL; ++i)
+            if (c + 32 * i < n) v[i] = ldv_volatile<R>(dst, i0 + 32 * i);
+#pragma unroll
+          for (int i = 0; i < KL; ++i) missing = missing || (c + 32 * i < n && unset(v[i]));
+          if (!__any_sync(0xffffffffu, missing)) return true;
+          if ((it & 1023) == 1023 && *(volatile int*)err) return false;  // another CTA gave up
+        }
+        if (lane == 0) atomicExch(err, kErrTimeout);
+        return false;
+      };
       if (!TRANS) {
 #pragma unroll
         for (int g = 0; g < RG; ++g) {
@@ -366,8 +383,8 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
         for (int g = 0; g < RG; ++g) {
           if (g >= nr) break;
           C xv[KL];
-#pragma unroll
-          for (int i = 0; i < KL; ++i) ok = ok && await(g, c0 + lane + 32 * i, true, xv[i]);
+          // all of a lane's entries in one round: the next round trip starts at the last's end
+          ok = ok && await_row(g, c0 + lane, xv);
 #pragma unroll
           for (int e = 0; e < P; ++e) fma_c(acc[TRANS ? e / KL : 0][g], C{pre[e].x, -pre[e].y}, xv[e % KL]);
         }
