@@ -662,29 +662,34 @@ __global__ void k_wide_mag(const VecInst V, float* __restrict__ xa) {
 }
 
 // den = |b| + |A||x| in FP32 magnitudes (as the row-wise products): 64 x 96 tiles, 4 x 6
-// entries per thread, K-chunks of 16 with the next chunk in registers.  FP32-issue bound, one
-// FMA per matrix entry and vector (2.1 ms for 20480 unknowns and 181 vectors at the peak rate,
-// about 11 ms measured).
+// entries per thread, K-chunks of 16 with the next chunk in registers as it was loaded (a
+// magnitude taken at the load would wait for it).  FP32-issue bound, one FMA per matrix entry and
+// vector, two of them in a paired instruction: 2.1 ms for 20480 unknowns and 181 vectors at the
+// single rate, 11 ms before the pairs, the late magnitudes and the odd row stride of sX, 5.0 ms
+// with them.
 constexpr int kWaM = 64, kWaN = 96, kWaK = 16;
 template <bool A32>
 __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* __restrict__ xa) {
+  using E = Entry<A32>;
   const int64_t r0 = (int64_t)blockIdx.x * kWaM, n = V.n;
   const int g0 = blockIdx.y * kWaN;
   __shared__ alignas(16) float sA[kWaK][kWaM];
-  __shared__ alignas(16) float sX[kWaK][kWaN];
+  __shared__ alignas(16) float sX[kWaK][kWaN + 2];  // 2 more: the 16 columns of a store apart
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   constexpr int kA = kWaM * kWaK / 256, kX = kWaN * kWaK / 256;
-  float na[kA], nx[kX], acc[4][6];
+  typename E::T na[kA];
+  float nx[kX];
+  float2 acc[4][3];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 6; ++b) acc[a][b] = 0.f;
+    for (int b = 0; b < 3; ++b) acc[a][b] = make_float2(0.f, 0.f);
   auto load = [&](int64_t k) {
 #pragma unroll
     for (int e = 0; e < kA; ++e) {
       const int t = tid + 256 * e;
       const int64_t r = r0 + t % kWaM, c = k + t / kWaM;
-      na[e] = r < n && c < n ? mag_at<A32>(V, r + c * V.lda) : 0.f;
+      na[e] = r < n && c < n ? E::at(V, r + c * V.lda) : typename E::T{};
     }
 #pragma unroll
     for (int e = 0; e < kX; ++e) {
@@ -697,7 +702,8 @@ __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* 
   load(0);
   for (int64_t k = 0; k < n; k += kWaK) {
 #pragma unroll
-    for (int e = 0; e < kA; ++e) sA[(tid + 256 * e) / kWaM][(tid + 256 * e) % kWaM] = na[e];
+    for (int e = 0; e < kA; ++e)
+      sA[(tid + 256 * e) / kWaM][(tid + 256 * e) % kWaM] = E::mag(na[e]);
 #pragma unroll
     for (int e = 0; e < kX; ++e) sX[(tid + 256 * e) % kWaK][(tid + 256 * e) / kWaK] = nx[e];
     __syncthreads();
@@ -706,13 +712,13 @@ __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* 
     for (int kk = 0; kk < kWaK; ++kk) {
       const float4 av = *reinterpret_cast<const float4*>(&sA[kk][tx * 4]);
       const float2* xp = reinterpret_cast<const float2*>(&sX[kk][ty * 6]);
-      const float2 x0 = xp[0], x1 = xp[1], x2 = xp[2];
+      const float2 xv[3] = {xp[0], xp[1], xp[2]};
       const float ar[4] = {av.x, av.y, av.z, av.w};
-      const float xv[6] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y};
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 6; ++b) acc[a][b] = fmaf(ar[a], xv[b], acc[a][b]);
+        for (int b = 0; b < 3; ++b)
+          acc[a][b] = __ffma2_rn(make_float2(ar[a], ar[a]), xv[b], acc[a][b]);
     }
     __syncthreads();
   }
@@ -723,8 +729,8 @@ __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* 
       const int64_t r = r0 + tx * 4 + a;
       const int g = g0 + ty * 6 + b;
       if (r < n && g < V.nrhs)
-        V.den[r + (int64_t)g * V.ldy] =
-            cabs(ldc(V.b, r + (int64_t)g * V.ldb)) + (double)acc[a][b];
+        V.den[r + (int64_t)g * V.ldy] = cabs(ldc(V.b, r + (int64_t)g * V.ldb)) +
+                                        (double)(b & 1 ? acc[a][b / 2].y : acc[a][b / 2].x);
     }
 }
 
