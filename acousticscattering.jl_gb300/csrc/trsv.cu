@@ -106,7 +106,8 @@ __device__ __forceinline__ cx<R> recip(cx<R> a) {
 }
 template <typename R>
 __device__ __forceinline__ void fma_c(cx<R>& s, cx<R> a, cx<R> b) {
-  s += a * b;
+  s.x = fma(-a.y, b.y, fma(a.x, b.x, s.x));
+  s.y = fma(a.y, b.x, fma(a.x, b.y, s.y));
 }
 }  // namespace
 
@@ -511,19 +512,106 @@ __global__ void k_tri_unset(const MatInst* __restrict__ insts, int of_y) {
 // ------------------------------------------------------------------ many right-hand sides
 // With many right-hand sides the work, not the chain, is the bound: the chain solves outer
 // blocks of kOuter block rows for all of them, and a tiled product takes each solved block out
-// of the rows that follow.  128 x 32 tiles, 4 x 4 entries per thread, K-chunks of 16 with the
-// next chunk in registers; every entry adds its columns in order.  One solve of 20480 unknowns
-// with 181 right-hand sides: 33 -> 20 ms against a
-// product kernel with eight right-hand sides per CTA.
+// of the rows that follow.  128 x N tiles, 4 x N / 8 entries per thread, K-chunks of 16 with the
+// next chunk in registers; every entry adds its columns in order with the same four FMAs.
+// Complex64 is bound by FP32 issue: the four FMAs of two right-hand sides go through the paired
+// instructions, and with more than 32 right-hand sides a thread takes eight of them, which halves
+// its loads of A.  One solve of 20480 unknowns with 181 right-hand sides: 33 ms with a product
+// kernel of eight right-hand sides per CTA, 23 with 128 x 32 tiles and six single operations an
+// entry, MANYNEW so (8 ms at the FP32 peak).
 constexpr int kManyRhs = 8;   // right-hand sides of a system from which this path is taken
 constexpr int kOuter = 8;
-constexpr int kUpM = 128, kUpN = 32, kUpK = 16;
+constexpr int kUpM = 128, kUpK = 16;
 
-template <typename R, bool LOWER>
-__global__ void __launch_bounds__(256) k_many_update(const MatInst* __restrict__ insts, int64_t q0,
-                                                     int64_t q1, int src_y) {
+// The tile's products in shared memory: A and the vectors' chunk, whose complex64 parts lie in
+// planes (real, imaginary, -imaginary) so that neighbouring right-hand sides make a pair.
+template <typename R, int N>
+struct UpTile {
   using C = cx<R>;
-  constexpr int NB = kTriNB<R>;
+  C a[kUpK][kUpM];
+  C x[kUpK][N + 1];
+  __device__ void put(int k, int g, C v) { x[k][g] = v; }
+};
+template <int N>
+struct UpTile<float, N> {
+  using C = cx<float>;
+  C a[kUpK][kUpM];
+  alignas(16) float re[kUpK][N + 4], im[kUpK][N + 4], ni[kUpK][N + 4];
+  __device__ void put(int k, int g, C v) {
+    re[k][g] = v.x;
+    im[k][g] = v.y;
+    ni[k][g] = -v.y;
+  }
+};
+template <typename R, int TN>
+struct UpSum {
+  using C = cx<R>;
+  C acc[4][TN];
+  __device__ void zero() {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < TN; ++b) acc[a][b] = C{0, 0};
+  }
+  __device__ void add(const UpTile<R, 8 * TN>& t, int kk, int tx, int ty) {
+    C av[4], xv[TN];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) av[a] = t.a[kk][tx + 32 * a];
+#pragma unroll
+    for (int b = 0; b < TN; ++b) xv[b] = t.x[kk][ty * TN + b];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < TN; ++b) fma_c(acc[a][b], av[a], xv[b]);
+  }
+  __device__ C get(int a, int b) const { return acc[a][b]; }
+};
+template <int TN>
+struct UpSum<float, TN> {
+  using C = cx<float>;
+  float2 re[4][TN / 2], im[4][TN / 2];
+  __device__ void zero() {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < TN / 2; ++b) re[a][b] = im[a][b] = make_float2(0.f, 0.f);
+  }
+  __device__ void add(const UpTile<float, 8 * TN>& t, int kk, int tx, int ty) {
+    C av[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) av[a] = t.a[kk][tx + 32 * a];
+#pragma unroll
+    for (int h = 0; h < TN / 4; ++h) {  // four right-hand sides at a time
+      const float4 r = *reinterpret_cast<const float4*>(&t.re[kk][ty * TN + 4 * h]);
+      const float4 i = *reinterpret_cast<const float4*>(&t.im[kk][ty * TN + 4 * h]);
+      const float4 m = *reinterpret_cast<const float4*>(&t.ni[kk][ty * TN + 4 * h]);
+      const float2 br[2] = {make_float2(r.x, r.y), make_float2(r.z, r.w)};
+      const float2 bi[2] = {make_float2(i.x, i.y), make_float2(i.z, i.w)};
+      const float2 bm[2] = {make_float2(m.x, m.y), make_float2(m.z, m.w)};
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float2 ax = make_float2(av[a].x, av[a].x), ay = make_float2(av[a].y, av[a].y);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          float2& sr = re[a][2 * h + b];
+          float2& si = im[a][2 * h + b];
+          sr = __ffma2_rn(ay, bm[b], __ffma2_rn(ax, br[b], sr));
+          si = __ffma2_rn(ay, br[b], __ffma2_rn(ax, bi[b], si));
+        }
+      }
+    }
+  }
+  __device__ C get(int a, int b) const {
+    const float2 r = re[a][b / 2], i = im[a][b / 2];
+    return b & 1 ? C{r.y, i.y} : C{r.x, i.x};
+  }
+};
+
+template <typename R, bool LOWER, int TN>
+__global__ void __launch_bounds__(256, TN == 8 ? 2 : 1)
+    k_many_update(const MatInst* __restrict__ insts, int64_t q0, int64_t q1, int src_y) {
+  using C = cx<R>;
+  constexpr int NB = kTriNB<R>, kUpN = 8 * TN;
   const MatInst& M = insts[blockIdx.z];
   const int64_t n = M.n, nblk = (n + NB - 1) / NB;
   if (!M.active || q0 >= nblk) return;
@@ -538,14 +626,10 @@ __global__ void __launch_bounds__(256) k_many_update(const MatInst* __restrict__
   const int64_t lda = M.lda, ldx = M.ldx;
   const void* sol = src_y ? M.x : M.y;   // the chain's destination
   void* rest = src_y ? M.y : M.x;
-  __shared__ C sA[kUpK][kUpM];
-  __shared__ C sX[kUpK][kUpN + 1];
+  __shared__ UpTile<R, kUpN> tile;
   const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-  C acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = C{0, 0};
+  UpSum<R, TN> sum;
+  sum.zero();
   constexpr int kA = kUpM * kUpK / 256, kX = kUpN * kUpK / 256;
   C na[kA], nx[kX];
   auto load = [&](int64_t k) {
@@ -568,39 +652,29 @@ __global__ void __launch_bounds__(256) k_many_update(const MatInst* __restrict__
 #pragma unroll
     for (int e = 0; e < kA; ++e) {
       const int t = tid + 256 * e;
-      sA[t / kUpM][t % kUpM] = na[e];
+      tile.a[t / kUpM][t % kUpM] = na[e];
     }
 #pragma unroll
     for (int e = 0; e < kX; ++e) {
       const int t = tid + 256 * e;
-      sX[t % kUpK][t / kUpK] = nx[e];
+      tile.put(t % kUpK, t / kUpK, nx[e]);
     }
     __syncthreads();
     if (k + kUpK < c1) load(k + kUpK);
 #pragma unroll
-    for (int kk = 0; kk < kUpK; ++kk) {
-      C av[4], xv[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = sA[kk][tx + 32 * a];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) xv[b] = sX[kk][ty * 4 + b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) fma_c(acc[a][b], av[a], xv[b]);
-    }
+    for (int kk = 0; kk < kUpK; ++kk) sum.add(tile, kk, tx, ty);
     __syncthreads();
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < TN; ++b) {
       const int64_t r = r0 + tx + 32 * a;
-      const int g = g0 + ty * 4 + b;
+      const int g = g0 + ty * TN + b;
       if (r < hi && g < M.nrhs) {
         const int64_t i = (int64_t)g * ldx + r;
         C v = ldv<R>(rest, i);
-        v -= acc[a][b];
+        v -= sum.get(a, b);
         stv_relaxed(rest, i, v);
       }
     }
@@ -682,10 +756,15 @@ static void triangle(const Launch& L, const MatInst* d, int ninst, int64_t nmax,
         // rows after the outer block (short instances have fewer and skip the tiles)
         const int64_t rows = nmax - q * NB;
         if (args.q1 < nblk) {
-          k_many_update<R, LOWER>
-              <<<dim3((unsigned)((rows + kUpM - 1) / kUpM), (unsigned)((max_rhs + kUpN - 1) / kUpN),
-                      (unsigned)ninst),
-                 256, 0, L.stream>>>(d, q, args.q1, src_y);
+          const int tn = sizeof(R) == 4 && max_rhs > 32 ? 8 : 4;  // right-hand sides a thread
+          const dim3 grid((unsigned)((rows + kUpM - 1) / kUpM),
+                          (unsigned)((max_rhs + 8 * tn - 1) / (8 * tn)), (unsigned)ninst);
+          if (tn == 4) {
+            k_many_update<R, LOWER, 4><<<grid, 256, 0, L.stream>>>(d, q, args.q1, src_y);
+          } else {
+            if constexpr (sizeof(R) == 4)
+              k_many_update<R, LOWER, 8><<<grid, 256, 0, L.stream>>>(d, q, args.q1, src_y);
+          }
           count_launch(1);
         }
       }
