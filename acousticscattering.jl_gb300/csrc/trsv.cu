@@ -518,7 +518,7 @@ __global__ void k_tri_unset(const MatInst* __restrict__ insts, int of_y) {
 // instructions, and with more than 32 right-hand sides a thread takes eight of them, which halves
 // its loads of A.  One solve of 20480 unknowns with 181 right-hand sides: 33 ms with a product
 // kernel of eight right-hand sides per CTA, 23 with 128 x 32 tiles and six single operations an
-// entry, MANYNEW so (8 ms at the FP32 peak).
+// entry, 18 so (8 ms at the FP32 peak).
 constexpr int kManyRhs = 8;   // right-hand sides of a system from which this path is taken
 constexpr int kOuter = 8;
 constexpr int kUpM = 128, kUpK = 16;
