@@ -2844,7 +2844,9 @@ int64_t order_of(const ServerReq& r) {
 size_t solve_bytes(const ServerReq& r) {
   const size_t N = (size_t)order_of(r);
   const size_t R = (size_t)r.nangles;
-  const size_t b = N * R * (16 * 6 + 8) + (size_t)vec_chunks((int64_t)N) * R * N * 3 * 8;
+  size_t b = N * R * (16 * 7 + 12) + (size_t)vec_chunks((int64_t)N) * R * N * 3 * 8;
+  if (r.nangles >= kWideRhs)  // slices of the vectors and of one row panel (more if there is room)
+    b += oz_pack_bytes((int64_t)R, (int)N, kOzB) + oz_pack_bytes(128, (int)N, kOzA) + N * R * 4;
   return b + b / 20;
 }
 
@@ -2858,7 +2860,9 @@ size_t item_bytes(const ServerReq& r) {
                    (r.prob.assembly == BEMGPU_ASSEMBLY_DEFAULT && mixed);
   size_t b = N * N * (a32 ? 8 : 16) + N * N * (mixed ? 8 : 16) + (fl ? 0 : n * n * (a32 ? 8 : 16));
   b += a32 ? (size_t)r.mesh->n_near * (fl ? 4 : 2) * 16 : 0;
-  b += 2 * tc_pack_bytes((int64_t)N, 128) + N * 64;
+  b += mixed ? 2 * tc_pack_bytes((int64_t)N, 128)
+             : oz_pack_bytes((int64_t)N, kOzK, kOzA) + oz_pack_bytes((int64_t)N, kOzK, kOzB);
+  b += tri_inv_bytes((int64_t)N, mixed ? 1 : 2) + N * 64;
   return b + b / 20 + solve_bytes(r);
 }
 

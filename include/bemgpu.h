@@ -522,9 +522,10 @@ int bemgpu_ctx_inject_alloc_failures(bemgpu_ctx *ctx, int32_t count);
 /* Batched-LU graphs captured and replayed by the context so far. */
 int bemgpu_ctx_graph_stats(const bemgpu_ctx *ctx, int64_t *captures, int64_t *replays);
 /*
- * Complex64 trailing updates of the mixed-precision LU on the tensor cores (split-BF16
- * tcgen05 GEMM, default 1) or on the CUDA cores (0).  No reference counterpart: a
- * switch for the precision study and for tests.
+ * Tensor cores (default 1) or CUDA cores (0) for the updates of the LU, complex64 by split-BF16
+ * products and complex128 by integer digit slices, and for the products of a system with 16
+ * right-hand sides or more (digit slices).  No reference counterpart: a switch for the
+ * precision study and for tests.
  */
 int bemgpu_ctx_set_tensor_lu(bemgpu_ctx *ctx, int32_t enable);
 
