@@ -401,18 +401,19 @@ __device__ __forceinline__ bool group_on(const GmState* st, int r0, int rb, int 
 
 // Coefficients of one column chunk of a compressed block: T[toff + c kmax + l] =
 // sum over the chunk of V[j, l] x[clo + j]; one warp per l, four independent accumulators
-// per lane and right-hand side (added in a fixed order).
+// per lane and right-hand side (added in a fixed order).  Five CTAs per SM: 73 -> 66 us a product.
 constexpr int kVtU = 4, kVtN = 3;  // coefficients per warp and values per lane in flight
 template <typename R, int RB>
-__global__ void __launch_bounds__(256) k_hm_vt(HmOp A, const void* __restrict__ X, int64_t ldx,
-                                               int32_t nr, const GmState* st, int mode,
-                                               const int32_t* jptr, int64_t jstride) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 && RB == 1 ? 5 : 1)
+    k_hm_vt(HmOp A, const void* __restrict__ X, int64_t ldx, int32_t nr, const GmState* st, int mode,
+            const int32_t* jptr, int64_t jstride) {
   using C = cx<R>;
   const int r0 = blockIdx.y * RB;
-  if (!group_on(st, r0, RB, nr, mode)) return;
+  const bool group = group_on(st, r0, RB, nr, mode);  // tested once the other loads are under way
   if (jptr) X = static_cast<const C*>(X) + (int64_t)*jptr * jstride;
   const HmItem it = A.vt_items[blockIdx.x];
   const HmLR B = A.lr[it.blk];
+  if (!group) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const C* V = static_cast<const C*>(A.V) + B.voff;
   const C* x[RB];
@@ -499,23 +500,28 @@ constexpr int kLeafSlices = 4;
 // blocks (about 40 x 40) a densified block can have thousands of rows and columns, so the
 // rows are spread over items (one CTA per block took 9 ms a product of 20480 panels with a
 // 10240-column densified block), the wide blocks' items come first in the list, and a thread
-// keeps all or kDblkU of its loads in flight.  A row is the sum of eight column chains
+// keeps all or kDblkU of its loads in flight.  Four CTAs per SM (64 registers): 152 -> 67 us a
+// product of 20480 panels with one 2560-column densified block, against three with 77 registers;
+// five spill and take 153.  A row is the sum of eight column chains
 // j = c + 8 t, in the order (0 + 4) + (1 + 5) + (2 + 6) + (3 + 7); for 64 x 64 blocks of four
 // chains j = c + 4 t.  Narrow blocks (at most kHmNarrow columns): 64 rows, a thread takes
 // chains c and c + 4 at once.  Wide ones: 32 rows, a thread takes one chain.
 template <typename R>
 constexpr int kDblkU = sizeof(R) == 4 ? 16 : 8;
 template <typename R, int RB>
-__global__ void __launch_bounds__(kLeafRows * kLeafSlices) k_hm_dblk(
+__global__ void __launch_bounds__(kLeafRows * kLeafSlices, sizeof(R) == 4 && RB == 1 ? 4 : 1)
+    k_hm_dblk(
     HmOp A, const void* __restrict__ X, int64_t ldx, int32_t nr, const GmState* st, int mode,
     const int32_t* jptr, int64_t jstride) {
   using C = cx<R>;
   const int r0 = blockIdx.y * RB;
-  if (!group_on(st, r0, RB, nr, mode)) return;
+  const bool group = group_on(st, r0, RB, nr, mode);  // tested once the other loads are under way
   if (jptr) X = static_cast<const C*>(X) + (int64_t)*jptr * jstride;
   const HmItem it = A.db_items[blockIdx.x];
   const HmDense B = A.dn[it.blk];
+  if (!group) return;
   __shared__ C part[RB][kLeafSlices * kLeafRows];
+  __shared__ C sx[RB][kHmNarrow];  // a narrow block's vectors, loaded beside its entries
   const int64_t m = B.m;
   const int n = B.n;
   const C* x[RB];
@@ -526,6 +532,11 @@ __global__ void __launch_bounds__(kLeafRows * kLeafSlices) k_hm_dblk(
   const int rows = wide ? kHmWideRows : kLeafRows;
   const int row = threadIdx.x % rows, ch = threadIdx.x / rows;
   const C* D = static_cast<const C*>(A.D) + B.off + it.lo + row;
+  static_assert(RB * kHmNarrow <= kLeafRows * kLeafSlices, "one value per thread");
+  const int xq = threadIdx.x / kHmNarrow, xj = threadIdx.x % kHmNarrow;
+  C xv = {0, 0};
+  if (!wide && xq < RB && xj < n)
+    xv = (static_cast<const C*>(X) + (int64_t)min(r0 + xq, nr - 1) * ldx + B.clo)[xj];
   if (wide) {
     constexpr int U = kDblkU<R>;
     C a[RB];
@@ -563,11 +574,13 @@ __global__ void __launch_bounds__(kLeafRows * kLeafSlices) k_hm_dblk(
     C d[kPer];
 #pragma unroll
     for (int u = 0; u < kPer; ++u) d[u] = D[(int64_t)(ch + u * kLeafSlices) * kLeafRows];
+    if (xq < RB) sx[xq][xj] = xv;
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
-      C a = d[0] * x[q][ch];
+      C a = d[0] * sx[q][ch];
 #pragma unroll
-      for (int u = 1; u < kPer; ++u) a += d[u] * x[q][ch + u * kLeafSlices];
+      for (int u = 1; u < kPer; ++u) a += d[u] * sx[q][ch + u * kLeafSlices];
       part[q][threadIdx.x] = a;
     }
   } else {
@@ -579,14 +592,16 @@ __global__ void __launch_bounds__(kLeafRows * kLeafSlices) k_hm_dblk(
       d0[u] = row < it.cnt && j < n ? D[(int64_t)j * m] : C{0, 0};
       d1[u] = row < it.cnt && j + 4 < n ? D[(int64_t)(j + 4) * m] : C{0, 0};
     }
+    if (xq < RB) sx[xq][xj] = xv;
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
       C a0 = {0, 0}, a1 = {0, 0};
 #pragma unroll
       for (int u = 0; u < kPer; ++u) {
         const int j = ch + 8 * u;
-        if (j < n) a0 += d0[u] * x[q][j];
-        if (j + 4 < n) a1 += d1[u] * x[q][j + 4];
+        if (j < n) a0 += d0[u] * sx[q][j];
+        if (j + 4 < n) a1 += d1[u] * sx[q][j + 4];
       }
       part[q][threadIdx.x] = a0 + a1;
     }
@@ -613,9 +628,10 @@ __global__ void __launch_bounds__(kHmRowChunk) k_hm_lblk(HmOp A, int32_t nr, con
                                                         int mode) {
   using C = cx<R>;
   const int r0 = blockIdx.y * RB;
-  if (!group_on(st, r0, RB, nr, mode)) return;
+  const bool group = group_on(st, r0, RB, nr, mode);  // tested once the other loads are under way
   const HmItem it = A.lb_items[blockIdx.x];
   const HmLR B = A.lr[it.blk];
+  if (!group) return;
   __shared__ C t[RB][kHmMaxRank];
   static_assert(kHmRowChunk >= kHmMaxRank, "one coefficient per thread");
   const int rank = B.rank, rank4 = rank & ~3;
