@@ -324,7 +324,8 @@ void launch_pressure(const Launch& L, const PressureInst& P) {
   if (P.nsurf > 0)
     k_pressure_regions<<<(unsigned)P.npts, kPrThreads, 0, L.stream>>>(P);
   else {
-    if (P.fluid) {
+    // the incident field has no traces (a Nystroem solution asks for it and the regions alone)
+    if (P.fluid && P.field != BEMGPU_FIELD_INCIDENT) {
       k_interior_traces<<<(unsigned)((P.n + 127) / 128), 128, 0, L.stream>>>(P);
       count_launch(1);
     }
