@@ -2288,8 +2288,8 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
 // right-hand sides: the vectors and the matrix, in row panels, are cut into digit slices and
 // multiplied on the tensor cores (gemm_oz.cu), the near corrections and the denominators are
 // added by their own kernels.  The row-wise products spend about 44 FP32 instructions per
-// complex product whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 34 ms (of
-// which 16 the products, 5 the slices of the matrix, 11 the denominators).
+// complex product whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 29 ms (of
+// which 16 the products, 4 the slices of the matrix, 5 the denominators).
 int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
   const Launch L = c->launch();
   const int64_t n = v.n, kb = (n + kOzK - 1) / kOzK;

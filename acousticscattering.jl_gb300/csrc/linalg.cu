@@ -391,8 +391,8 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
                                                      int nb, int share) {
   using C = cx<R>;
   // Columns whose code is unrolled.  All 16 of a sub-panel are 80 KB of instructions that run twice
-  // in a launch: a quarter of the cycles waited for them.  Four at a time: 74 to 58 us a panel of
-  // 1280 rows.  With more than two rows per thread the registers that take turns cost more.
+  // in a launch: a quarter of the cycles waited for them.  Four at a time: 61 to 53 us a panel of
+  // a factorisation of 1280 unknowns on average.  With more than two rows per thread the registers that take turns cost more.
   constexpr int kU = RPT > 2 || W <= 4 ? W : 4;
   const unsigned rank = cluster_rank(), cs = cluster_size();
   const MatInst& M = insts[blockIdx.x / cs];
