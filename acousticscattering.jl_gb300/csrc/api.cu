@@ -4958,7 +4958,7 @@ int bemgpu_pressure_region(bemgpu_solution* sol, int32_t rhs, int64_t npts, cons
   P.eta = s->mesh->eta;
   P.field = field;
   P.fluid = fluid ? 1 : 0;
-  if (fluid && !s->region) {
+  if (fluid && !s->region && npts >= kTracesPoints) {
     TRY(alloc(c, (size_t)s->mesh->n * 32, &dint));
     P.pi = dint.as<double>();
     P.qi = dint.as<double>() + 2 * (size_t)s->mesh->n;

@@ -13,7 +13,7 @@
 // point, fixed-order reductions, FP64 fields.
 //
 // Bound by FP64 issue.  The far panels take the shared-phase rule of quad_regular.cuh, the
-// interior traces are formed once per call, and the region test sums FP32 angles (panels
+// interior traces are formed once per call (from kTracesPoints points on), and the region test sums FP32 angles (panels
 // within two diameters in FP64), repeated in FP64 when the sum is not clearly 0 or 4 pi:
 // 2001 points of a 2880-panel fluid body 6.30 -> 4.5 ms.
 #include "bemgpu_internal.h"
@@ -83,19 +83,25 @@ __device__ __forceinline__ void far_layers(const double* rj, const double* x, do
 }
 
 // Interior traces p = p_s + p_inc, q = g (q_s + q_inc).
-__global__ void k_interior_traces(const PressureInst P) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= P.n) return;
-  const double* rj = P.panels + j * kPanelDoubles;
+__device__ __forceinline__ void interior_traces(const PressureInst& P, const double* rj, cd& p,
+                                                cd& q) {
   const double* d = P.dir;
   const double ph = P.k * (d[0] * rj[0] + d[1] * rj[1] + d[2] * rj[2]);
   double sn, cs;
   sincos(ph, &sn, &cs);
   const double dn = P.k * (d[0] * rj[3] + d[1] * rj[4] + d[2] * rj[5]);
-  P.pi[2 * j] = P.p[2 * j] + cs;
-  P.pi[2 * j + 1] = P.p[2 * j + 1] + sn;
-  P.qi[2 * j] = P.g * (P.q[2 * j] - dn * sn);
-  P.qi[2 * j + 1] = P.g * (P.q[2 * j + 1] + dn * cs);
+  p = cd{p.x + cs, p.y + sn};
+  q = cd{P.g * (q.x - dn * sn), P.g * (q.y + dn * cs)};
+}
+__global__ void k_interior_traces(const PressureInst P) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= P.n) return;
+  cd p = {P.p[2 * j], P.p[2 * j + 1]}, q = {P.q[2 * j], P.q[2 * j + 1]};
+  interior_traces(P, P.panels + j * kPanelDoubles, p, q);
+  P.pi[2 * j] = p.x;
+  P.pi[2 * j + 1] = p.y;
+  P.qi[2 * j] = q.x;
+  P.qi[2 * j + 1] = q.y;
 }
 
 __global__ void __launch_bounds__(kPrThreads) k_pressure(const PressureInst P) {
@@ -155,9 +161,11 @@ __global__ void __launch_bounds__(kPrThreads) k_pressure(const PressureInst P) {
   for (int64_t j = threadIdx.x; j < P.n; j += kPrThreads) {
     const double* rj = P.panels + j * kPanelDoubles;
     const double* nT = rj + 3;
-    const double* tp = interior ? P.pi : P.p;
-    const double* tq = interior ? P.qi : P.q;
-    const cd pj = {tp[2 * j], tp[2 * j + 1]}, qj = {tq[2 * j], tq[2 * j + 1]};
+    const bool formed = interior && P.pi;
+    const double* tp = formed ? P.pi : P.p;
+    const double* tq = formed ? P.qi : P.q;
+    cd pj = {tp[2 * j], tp[2 * j + 1]}, qj = {tq[2 * j], tq[2 * j + 1]};
+    if (interior && !formed) interior_traces(P, rj, pj, qj);
     const double dx = x[0] - rj[0], dy = x[1] - rj[1], dz = x[2] - rj[2];
     const double d2 = dx * dx + dy * dy + dz * dz;
     const double lim = P.eta * rj[7];
@@ -325,7 +333,7 @@ void launch_pressure(const Launch& L, const PressureInst& P) {
     k_pressure_regions<<<(unsigned)P.npts, kPrThreads, 0, L.stream>>>(P);
   else {
     // the incident field has no traces (a Nystroem solution asks for it and the regions alone)
-    if (P.fluid && P.field != BEMGPU_FIELD_INCIDENT) {
+    if (P.pi && P.field != BEMGPU_FIELD_INCIDENT) {
       k_interior_traces<<<(unsigned)((P.n + 127) / 128), 128, 0, L.stream>>>(P);
       count_launch(1);
     }

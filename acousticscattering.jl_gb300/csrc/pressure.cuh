@@ -5,13 +5,19 @@
 
 namespace bemgpu {
 
+// Points from which a fluid body's interior traces are formed once, by a launch of their own; with
+// fewer, two per SM at most, that launch and its scratch cost more than the sines they save (36
+// points of 364 panels: 180 us with it, 175 without).
+constexpr int64_t kTracesPoints = 256;
+
 struct PressureInst {
   const double* panels;  // FP64 panel records
   const double* verts;   // vertex records
   int64_t n;             // panels
   const double* p;       // scattered pressure trace of one rhs (complex128, n)
   const double* q;       // scattered normal-derivative trace (complex128, n)
-  double* pi;            // scratch for a fluid body's interior traces (complex128, n each)
+  double* pi;            // scratch for a fluid body's interior traces (complex128, n each), or
+                         // null: formed where they are used
   double* qi;
   const double* dir;     // incidence direction (3)
   const double* points;  // 3 x npts
