@@ -75,6 +75,13 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                    : "memory");
 }
+// The two halves of the barrier, for work in between.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t peer_smem(const void* p, unsigned rank) {
   uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
@@ -398,6 +405,9 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
   const MatInst& M = insts[blockIdx.x / cs];
   const int64_t n = M.n;
   if (!M.active || k0 >= n) return;  // the whole cluster (one instance) leaves together
+  // a CTA's shared memory exists for its peers once it has started: every CTA says so here and
+  // waits for the others before its first store to a peer, with the panel's loads in between
+  cluster_arrive();
   const int nbe = (int)min((int64_t)nb, n - k0);
   const int64_t lda = M.lda;
   void* A = M.a;
@@ -425,6 +435,7 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
 #pragma unroll
       for (int w = 0; w < W; ++w)
         a[t][w] = fz[t] >= 0 && w < wn ? ld<R>(A, (g + t * stride) + (k0 + s0 + w) * lda) : C{0, 0};
+    if (s0 == 0) cluster_wait();  // every peer has started
     if (s0 > 0) {
       // U rows of the finished pivots in these columns
       for (int e = tid; e < s0 * s0; e += T) {
