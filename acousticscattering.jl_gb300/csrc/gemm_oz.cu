@@ -16,23 +16,26 @@
 // unknowns are those of the FP64 pipe's (stopping at level 8 made them up to twice as large).
 //
 // Tile and layout: 128 x 32 complex entries of C per CTA, all eight levels of the real and
-// imaginary part in tensor memory (2 x 8 x 32 = 512 columns).  The B slices of a K-chunk are
-// stacked along N (slice 1 first), so slice p of A meets B slices 1..min(7, 9-p) in ONE
-// instruction of N = 224 .. 64 whose accumulator columns are the levels from p+1 on: 34 digit
-// pairs take 7 instructions per real product instead of 34 narrow ones, and A is read from
-// shared memory 7 times instead of 34.  K-chunks of 16: rows of 64 bytes, 16 real then 16
-// imaginary digits, in the 64-byte swizzle.  A stage is 7 slices of both operands (70 KB),
-// three stages.
+// imaginary part in tensor memory (2 x 8 x 32 = 512 columns).  The levels of a part form two
+// accumulators of N = 128, levels 2..5 and 6..9.  tcgen05.mma instructions are only ordered
+// among themselves when they share accumulator and shape, so every instruction takes a whole
+// accumulator: the B slices of a K-chunk are stacked along N (slice 1 first) between blocks of
+// zeros, and slice p of A meets the four blocks that belong to the accumulator's levels, some
+// of them zeros.  34 digit pairs take 11 instructions per real product, 1.3 times the tensor
+// work of instructions cut to the slices that exist, whose accumulators overlap.  K-chunks of
+// 16: rows of 64 bytes, 16 real then 16 imaginary digits, in the 64-byte swizzle.  A stage is 7
+// slices of both operands and the zeros (78 KB), two stages.
 //
 // Roles as in gemm_tc.cu: a producer thread (bulk copies), a tcgen05.mma issuer, eight
 // epilogue warps that move the levels of a tile to 64-bit integers in registers, release
 // the tensor memory, then convert, scale and update C while the next tile's products run.
 // Every wait is bounded.
 //
-// Bound by the tensor pipe and the shared-memory operand reads: 136 real products of K = 128
-// per tile take at least 17.4k cycles, the FP64 conversion and update of the epilogue about 8k
-// beside them, moving the levels out of tensor memory about 2k in between.  The trailing
-// updates of an LU of 5760 unknowns: 718 ms on the FP64 pipe (0.7 TFLOP/s), 12 ms here.
+// Bound by the tensor pipe and the shared-memory operand reads: 44 instructions of 64 cycles in
+// each of the 8 chunks of a tile and K-block take at least 22.5k cycles, the FP64 conversion
+// and update of the epilogue about 8k beside them, moving the levels out of tensor memory about
+// 2k in between.  The trailing updates of an LU of 5760 unknowns: 718 ms on the FP64 pipe (0.7
+// TFLOP/s), 12 ms here.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,14 +56,17 @@ constexpr int kOzABlock = kOzM * 64;        // one slice of a chunk, 64-byte row
 constexpr int kOzBBlock = kOzN * 64;
 constexpr int kOzAChunk = kOzSlices * kOzABlock;  // 56 KB
 constexpr int kOzBChunk = kOzSlices * kOzBBlock;  // 14 KB
-constexpr int kOzStage = kOzAChunk + kOzBChunk;
-constexpr int kOzStages = 3;
+constexpr int kOzLow = 3, kOzHigh = 1;      // blocks of zeros before and after the B slices
+constexpr int kOzAccN = 4 * kOzN;           // columns of an accumulator: four levels
+constexpr int kOzStage = kOzAChunk + (kOzLow + kOzHigh) * kOzBBlock + kOzBChunk;
+constexpr int kOzStages = 2;
 constexpr int kOzThreads = 320;             // producer, MMA, 8 epilogue warps
 constexpr int kOzEpiThreads = 256;
 constexpr uint32_t kOzTmem = 512;
 constexpr uint32_t kOzIm = kOzLevels * kOzN;  // first tensor-memory column of the imaginary part
 constexpr int32_t kOzNaN = INT32_MAX;       // exponent of a row with a NaN or an infinity
 static_assert(kOzStage % 1024 == 0 && kOzABlock % 1024 == 0 && kOzBBlock % 1024 == 0, "swizzle");
+static_assert(kOzLevels * kOzN == 2 * kOzAccN, "two accumulators");
 
 // ------------------------------------------------------------------ slicing
 // Fixed-point value of x in units of 2^(e - 56), e = row exponent field - 1021.
@@ -258,6 +264,15 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     }
     mbar_fence_init();
   }
+  // the zeros around the B slices of every stage, for the tensor core's reads
+  for (int e = threadIdx.x; e < kOzStages * (kOzLow + kOzHigh) * kOzBBlock / 16; e += kOzThreads) {
+    constexpr int kPer = kOzBBlock / 16;
+    const int stage = e / ((kOzLow + kOzHigh) * kPer), r = e % ((kOzLow + kOzHigh) * kPer);
+    const int block = r / kPer < kOzLow ? r / kPer : r / kPer + kOzSlices;
+    *reinterpret_cast<uint4*>(base + stage * kOzStage + kOzAChunk + block * kOzBBlock +
+                              r % kPer * 16) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) {
     asm volatile(
         "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -294,9 +309,10 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           uint8_t* dst = base + stage * kOzStage;
           armed[stage] = 1;
           armed_par[stage] = phase;
-          mbar_arrive_expect_tx(&S.full[stage], kOzStage);
+          mbar_arrive_expect_tx(&S.full[stage], kOzAChunk + kOzBChunk);
           bulk_g2s(dst, pa + (size_t)c * kOzAChunk, kOzAChunk, &S.full[stage]);
-          bulk_g2s(dst + kOzAChunk, pb + (size_t)c * kOzBChunk, kOzBChunk, &S.full[stage]);
+          bulk_g2s(dst + kOzAChunk + kOzLow * kOzBBlock, pb + (size_t)c * kOzBChunk, kOzBChunk,
+                   &S.full[stage]);
           if (++stage == kOzStages) {
             stage = 0;
             phase ^= 1;
@@ -335,32 +351,29 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             break;
           }
           tc_fence_after();
-          const uint32_t a0 = sbase + stage * kOzStage, b0 = a0 + kOzAChunk;
-          const uint64_t b_re = oz_desc(b0), b_im = oz_desc(b0 + 32);
-          // slice p + 1 of A against slices q0 + 1..q1 of B: levels p + q0 + 2..p + q1 + 1
-          auto products = [&](int p, int q0, int q1, uint32_t acc) {
-            const uint32_t n = kOzN * (q1 - q0);
-            const uint32_t dr = tmem + kOzN * (p + q0), di = dr + kOzIm;
+          const uint32_t a0 = sbase + stage * kOzStage;
+          const uint32_t b0 = a0 + kOzAChunk + kOzLow * kOzBBlock;  // B slice 1
+          const uint32_t pos = oz_idesc(kOzAccN, false), neg = oz_idesc(kOzAccN, true);
+          // slice p + 1 of A into levels 2 + 4 h .. 5 + 4 h: B slices 4 h - p + 1 .. 4 h - p + 4,
+          // those outside 1..7 zeros
+          auto products = [&](int p, int h, uint32_t acc) {
+            const uint32_t dr = tmem + h * kOzAccN, di = dr + kOzIm;
             const uint64_t a_re = oz_desc(a0 + p * kOzABlock);
             const uint64_t a_im = oz_desc(a0 + p * kOzABlock + 32);
-            const uint64_t b_re = oz_desc(b0 + q0 * kOzBBlock);
-            const uint64_t b_im = oz_desc(b0 + q0 * kOzBBlock + 32);
-            const uint32_t pos = oz_idesc(n, false), neg = oz_idesc(n, true);
+            const uint64_t b_re = oz_desc(b0 + (4 * h - p) * kOzBBlock);
+            const uint64_t b_im = oz_desc(b0 + (4 * h - p) * kOzBBlock + 32);
             mma_bf16(dr, a_re, b_re, pos, acc);
             mma_bf16(di, a_re, b_im, pos, acc);
             mma_bf16(dr, a_im, b_im, neg, 1u);
             mma_bf16(di, a_im, b_re, pos, 1u);
           };
-          if (c % kOzBlockChunks == 0) {  // slice 2 starts levels 3..9, the leading digits' product level 2
-            products(1, 0, kOzSlices, 0u);
-            products(0, 0, 1, 0u);
-            products(0, 1, kOzSlices, 1u);
-          } else {
-            products(0, 0, kOzSlices, 1u);
-            products(1, 0, kOzSlices, 1u);
-          }
+          static_assert(kOzLow >= 3 && 4 + kOzLow >= kOzSlices && 8 - kOzSlices <= kOzHigh,
+                        "every block of an accumulator lies in the stage");
+          const uint32_t more = c % kOzBlockChunks == 0 ? 0u : 1u;
 #pragma unroll
-          for (int p = 2; p < kOzSlices; ++p) products(p, 0, kOzLevels - p, 1u);
+          for (int p = 0; p < 4; ++p) products(p, 0, p == 0 ? more : 1u);
+#pragma unroll
+          for (int p = 0; p < kOzSlices; ++p) products(p, 1, p == 0 ? more : 1u);
           mma_commit(&S.empty[stage]);
           if (++stage == kOzStages) {
             stage = 0;
