@@ -8,6 +8,7 @@
 // consecutive rows of a column: coalesced), and the columns are split into vec_chunks(n)
 // chunks whose partial results are combined by a second kernel in a fixed order, so
 // every reduction here is deterministic.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -362,10 +363,10 @@ __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
 }
 
 template <int NR>
-__device__ __forceinline__ void gemv_body(const VecInst& V, int with_abs) {
+__device__ __forceinline__ void gemv_body(const VecInst& V, int grp0, int with_abs) {
   constexpr int kGemvR = NR;  // right-hand sides per pass of this instantiation
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int ch = blockIdx.y % kMaxChunks, grp = blockIdx.y / kMaxChunks;
+  const int ch = blockIdx.y % kMaxChunks, grp = grp0 + blockIdx.y / kMaxChunks;
   if (ch >= vec_chunks(V.n)) return;
   const int r0 = grp * kGemvR;
   if (i >= V.n || r0 >= V.nrhs) return;
@@ -425,14 +426,15 @@ constexpr int kA32Cols = 4, kA32Stages = 4;
 constexpr int a32_smem(int threads) { return kA32Stages * kA32Cols * 2 * 8 * threads; }
 
 template <int NR, bool ABS, int T>
-__global__ void __launch_bounds__(T, (NR == 1 ? 640 : 512) / T) k_gemv_a32(const VecInst* __restrict__ insts) {
+__global__ void __launch_bounds__(T, (NR == 1 ? 640 : 512) / T)
+    k_gemv_a32(const VecInst* __restrict__ insts, int grp0) {
   constexpr int kFold = 32, kRows = 2;
   const VecInst& V = insts[blockIdx.z];
   if (!V.a32) return;
   extern __shared__ __align__(16) unsigned char a32_ring[];
   const int64_t n = V.n, lda = V.lda;
   const int64_t i0 = (int64_t)blockIdx.x * (kRows * T) + threadIdx.x;
-  const int ch = blockIdx.y % kMaxChunks, grp = blockIdx.y / kMaxChunks;
+  const int ch = blockIdx.y % kMaxChunks, grp = grp0 + blockIdx.y / kMaxChunks;
   if (ch >= vec_chunks(n)) return;
   const int r0 = grp * NR;
   if (i0 >= n || r0 >= V.nrhs) return;
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(T, (NR == 1 ? 640 : 512) / T) k_gemv_a32(const
 }
 
 template <int NR, bool ABS, int T>
-void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int groups) {
+void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int grp0, int groups) {
   static PerDeviceOnce attr;
   attr.call([] {
     cudaFuncSetAttribute(k_gemv_a32<NR, ABS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -572,23 +574,25 @@ void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int gr
   constexpr int rows = 2 * T;
   k_gemv_a32<NR, ABS, T><<<dim3((unsigned)((nmax + rows - 1) / rows),
                                 (unsigned)(kMaxChunks * groups), (unsigned)ninst),
-                           T, a32_smem(T), L.stream>>>(d);
+                           T, a32_smem(T), L.stream>>>(d, grp0);
 }
 template <int NR, bool ABS>
-void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int groups, int rows) {
+void gemv_a32(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int grp0, int groups,
+              int rows) {
   if (rows == 1)
-    gemv_a32<NR, ABS, 64>(L, d, ninst, nmax, groups);
+    gemv_a32<NR, ABS, 64>(L, d, ninst, nmax, grp0, groups);
   else
-    gemv_a32<NR, ABS, 128>(L, d, ninst, nmax, groups);
+    gemv_a32<NR, ABS, 128>(L, d, ninst, nmax, grp0, groups);
 }
 
 // partial y = A x (and |A||x|) over a column chunk, up to kGemvR right-hand sides
-// per pass (rhs group = blockIdx.y / kMaxChunks).
+// per pass (rhs group = grp0 + blockIdx.y / kMaxChunks).
 template <int NR>
-__global__ void __launch_bounds__(256) k_gemv_part(const VecInst* __restrict__ insts, int with_abs) {
+__global__ void __launch_bounds__(256) k_gemv_part(const VecInst* __restrict__ insts, int grp0,
+                                                   int with_abs) {
   const VecInst& V = insts[blockIdx.z];
   if (V.a32) return;
-  gemv_body<NR>(V, with_abs);
+  gemv_body<NR>(V, grp0, with_abs);
 }
 
 // Lane s of the eight threads of a row: its share of the row's near corrections (FP64, every
@@ -954,21 +958,26 @@ void launch_gemv(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int
   const int groups = (max_rhs + nr - 1) / nr;
   dim3 g0((unsigned)((nmax + 255) / 256), (unsigned)max_rhs, (unsigned)ninst);
   k_split_x<<<g0, 256, 0, L.stream>>>(d); count_launch(1);
-  dim3 g1((unsigned)((nmax + 255) / 256), (unsigned)(kMaxChunks * groups), (unsigned)ninst);
-  if (nr == 1) {
-    if (mode == 1)
-      gemv_a32<1, true>(L, d, ninst, nmax, groups, rows);
-    else
-      gemv_a32<1, false>(L, d, ninst, nmax, groups, rows);
-    k_gemv_part<1><<<g1, 256, 0, L.stream>>>(d, mode == 1);
-  } else {
-    if (mode == 1)
-      gemv_a32<kGemvR, true>(L, d, ninst, nmax, groups, rows);
-    else
-      gemv_a32<kGemvR, false>(L, d, ninst, nmax, groups, rows);
-    k_gemv_part<kGemvR><<<g1, 256, 0, L.stream>>>(d, mode == 1);
+  // chunks and groups share the grid's second dimension: as many groups per launch as it holds
+  constexpr int kMaxGroups = 65535 / kMaxChunks;
+  for (int q0 = 0; q0 < groups; q0 += kMaxGroups) {
+    const int q = std::min(kMaxGroups, groups - q0);
+    const dim3 g1((unsigned)((nmax + 255) / 256), (unsigned)(kMaxChunks * q), (unsigned)ninst);
+    if (nr == 1) {
+      if (mode == 1)
+        gemv_a32<1, true>(L, d, ninst, nmax, q0, q, rows);
+      else
+        gemv_a32<1, false>(L, d, ninst, nmax, q0, q, rows);
+      k_gemv_part<1><<<g1, 256, 0, L.stream>>>(d, q0, mode == 1);
+    } else {
+      if (mode == 1)
+        gemv_a32<kGemvR, true>(L, d, ninst, nmax, q0, q, rows);
+      else
+        gemv_a32<kGemvR, false>(L, d, ninst, nmax, q0, q, rows);
+      k_gemv_part<kGemvR><<<g1, 256, 0, L.stream>>>(d, q0, mode == 1);
+    }
+    count_launch(2);
   }
-  count_launch(2);
   dim3 g2((unsigned)((nmax + 31) / 32), (unsigned)max_rhs, (unsigned)ninst);
   k_gemv_finish<<<g2, 256, 0, L.stream>>>(d, mode); count_launch(1);
 }
