@@ -2284,19 +2284,29 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
   return BEMGPU_OK;
 }
 
-// y = A x (mode 0) or y = b - A x with den = |b| + |A||x| (mode 1) of one system with many
-// right-hand sides: the vectors and the matrix, in row panels, are cut into digit slices and
-// multiplied on the tensor cores (gemm_oz.cu), the near corrections and the denominators are
-// added by their own kernels.  The row-wise products spend about 44 FP32 instructions per
+// y = A x (mode 0, den used as scratch) or y = b - A x with den = |b| + |A||x| (mode 1) of one
+// system with many right-hand sides: the vectors and the matrix, in row panels, are cut into
+// digit slices and multiplied on the tensor cores (gemm_oz.cu), the near corrections and the
+// denominators are added by their own kernels.  The slices share an exponent per row and block,
+// so the unknowns are taken in units of their sizes (columns of A times, vectors divided by, a
+// power of two per unknown), and entries whose error could still matter beside |A||x| are
+// computed again in FP64, or the whole product row by row when there are many of them (decided
+// on the device).  The row-wise products spend about 44 FP32 instructions per
 // complex product whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 29 ms (of
 // which 16 the products, 4 the slices of the matrix, 5 the denominators).
 int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
   const Launch L = c->launch();
   const int64_t n = v.n, kb = (n + kOzK - 1) / kOzK;
   const int32_t R = v.nrhs;
-  Buf xp, xe, ap, ae;
+  Buf xp, xe, ap, ae, ke, found, list;
   TRY(alloc(c, oz_pack_bytes(R, (int)n, kOzB), &xp));
   TRY(alloc(c, (size_t)kb * oz_exps(R, kOzB) * 4, &xe));
+  TRY(alloc(c, (size_t)n * 4, &ke));
+  // entries computed again at most, one in 64: their rows are read at 32 bytes an entry, 38 GB or
+  // 6 ms for 181 vectors of 20480 unknowns
+  const int32_t cap = (int32_t)std::min<int64_t>(1 << 20, std::max<int64_t>(1024, n * R / 64));
+  TRY(alloc(c, 4, &found));
+  TRY(alloc(c, (size_t)cap * sizeof(int2), &list));
   // row panels: about 8 GB of slices, at most a quarter of what the budget leaves
   const size_t tile = oz_pack_bytes(128, (int)n, kOzA);
   const uint64_t used = total_live(c), budget = root_of(c)->budget;
@@ -2305,34 +2315,50 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
   const int64_t rows = tiles * 128;
   TRY(alloc(c, tile * (size_t)tiles, &ap));
   TRY(alloc(c, (size_t)kb * (size_t)rows * 4, &ae));
+  const int32_t* kexp = ke.as<int32_t>();
   std::vector<OzPackInst> pk;
   std::vector<OzGemmInst> ge;
-  pk.push_back(OzPackInst{v.x, v.ldx, 0, 0, R, (int32_t)n, 0, xp.p, xe.as<int32_t>()});
+  pk.push_back(OzPackInst{v.x, v.ldx, 0, 0, R, (int32_t)n, 0, xp.p, xe.as<int32_t>(), kexp});
   for (int64_t r0 = 0; r0 < n; r0 += rows) {
     const int64_t m = std::min(rows, n - r0);
-    pk.push_back(OzPackInst{v.A, v.lda, r0, 0, m, (int32_t)n, v.a32, ap.p, ae.as<int32_t>()});
+    pk.push_back(
+        OzPackInst{v.A, v.lda, r0, 0, m, (int32_t)n, v.a32, ap.p, ae.as<int32_t>(), kexp});
     ge.push_back(OzGemmInst{ap.p, xp.p, ae.as<int32_t>(), xe.as<int32_t>(), v.y, v.ldy, r0, 0, m, R,
-                            (int32_t)n, 1});
+                            (int32_t)n, 1, found.as<int32_t>(), cap});
   }
-  Buf dpk, dge;
+  Buf dpk, dge, dv;
   TRY(to_device(c, pk, &dpk));
   TRY(to_device(c, ge, &dge));
+  VecInst gated = v;
+  gated.gate = found.as<int32_t>();
+  gated.gate_cap = cap;
+  TRY(to_device(c, std::vector<VecInst>{gated}, &dv));
   if (mode == 1) {
     CUDA_TRY(c, cudaMemcpy2DAsync(v.y, (size_t)v.ldy * 16, v.b, (size_t)v.ldb * 16, (size_t)n * 16,
                                   (size_t)R, cudaMemcpyDeviceToDevice, c->stream));
-    Buf xa;
-    TRY(alloc(c, (size_t)n * R * 4, &xa));
-    launch_wide_abs(L, v, xa.as<float>());
   } else {
     CUDA_TRY(c, cudaMemset2DAsync(v.y, (size_t)v.ldy * 16, 0, (size_t)n * 16, (size_t)R, c->stream));
   }
+  CUDA_TRY(c, cudaMemsetAsync(found.p, 0, 4, c->stream));
+  Buf xa;
+  TRY(alloc(c, (size_t)n * R * 4, &xa));
+  launch_wide_abs(L, v, xa.as<float>(), mode);
+  launch_wide_scale(L, v, ke.as<int32_t>());
   launch_oz_pack(L, dpk.as<OzPackInst>(), 1, R, (int)n, kOzB);
+  WideCheck ck{ae.as<int32_t>(), xe.as<int32_t>(), 0, 0, 0, (int64_t)oz_exps(R, kOzB), (int32_t)kb,
+               cap, found.as<int32_t>(), list.as<int2>()};
   for (size_t p = 0; p < ge.size(); ++p) {
     launch_oz_pack(L, dpk.as<OzPackInst>() + 1 + p, 1, ge[p].m, (int)n, kOzA, v.a32 != 0);
+    ck.r0 = ge[p].c_r0;
+    ck.m = ge[p].m;
+    ck.as = (int64_t)oz_exps(ge[p].m, kOzA);
+    launch_wide_check(L, v, ck, mode);
     const int64_t t = oz_tiles(ge[p].m, R);
     launch_oz_gemm(L, dge.as<OzGemmInst>() + p, 1, &t);
   }
+  launch_wide_redo(L, v, ck, mode);
   launch_wide_finish(L, v, mode);
+  launch_gemv(L, dv.as<VecInst>(), 1, n, R, mode);
   CUDA_TRY(c, cudaGetLastError());
   return BEMGPU_OK;
 }

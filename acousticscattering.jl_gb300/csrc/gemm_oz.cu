@@ -11,9 +11,11 @@
 // up to d = 5 for any operands, and a few units of 2^(-8d) in the worst case beyond, below
 // 2^-53 of the largest possible result).  The levels are added in 64-bit integers and
 // rounded to FP64 once.  What is dropped (digits beyond the seventh, levels above 9) is about
-// 2^-55 of sqrt(K) (largest |a| of the row) x (largest |b| of the column), below the
-// accumulated rounding errors of 4 K FP64 operations: backward errors of LUs of 128 to 2049
-// unknowns are those of the FP64 pipe's (stopping at level 8 made them up to twice as large).
+// 2^-55 of sqrt(K) (largest |a| of the row) x (largest |b| of the column) of the K-block, below
+// the accumulated rounding errors of 4 K FP64 operations when no index k stands out: backward
+// errors of LUs of 128 to 2049 unknowns are those of the FP64 pipe's (stopping at level 8 made
+// them up to twice as large).  It is not relative to sum_k |a||b|: where the sizes differ along
+// k, the caller gives a power of two per k that moves between the operands (kexp).
 //
 // Tile and layout: 128 x 32 complex entries of C per CTA, all eight levels of the real and
 // imaginary part in tensor memory (2 x 8 x 32 = 512 columns).  The levels of a part form two
@@ -64,26 +66,27 @@ constexpr int kOzThreads = 320;             // producer, MMA, 8 epilogue warps
 constexpr int kOzEpiThreads = 256;
 constexpr uint32_t kOzTmem = 512;
 constexpr uint32_t kOzIm = kOzLevels * kOzN;  // first tensor-memory column of the imaginary part
-constexpr int32_t kOzNaN = INT32_MAX;       // exponent of a row with a NaN or an infinity
+constexpr int kOzMark = 1 << 20;            // exponent field of such a row while it is packed
+constexpr int kOzDrop = -200000;            // shift of a column that is taken as zeros
 static_assert(kOzStage % 1024 == 0 && kOzABlock % 1024 == 0 && kOzBBlock % 1024 == 0, "swizzle");
 static_assert(kOzLevels * kOzN == 2 * kOzAccN, "two accumulators");
 
 // ------------------------------------------------------------------ slicing
-// Fixed-point value of x in units of 2^(e - 56), e = row exponent field - 1021.
-__device__ __forceinline__ long long oz_fixed(double x, int erow) {
+// Fixed-point value of x 2^sh in units of 2^(e - 56), e = row exponent field - 1021.
+__device__ __forceinline__ long long oz_fixed(double x, int sh, int erow) {
   const long long b = __double_as_longlong(x);
   const int ex = (int)((b >> 52) & 0x7FF);
   long long m = (b & 0xFFFFFFFFFFFFFLL) | 0x10000000000000LL;
-  const int s = ex - erow + 2;  // <= 2
+  const int s = ex + sh - erow + 2;  // <= 2
   if (ex == 0 || s < -53) return 0;
   m = s >= 0 ? m << s : (m + (1LL << (-s - 1))) >> -s;
   return b < 0 ? -m : m;
 }
-__device__ __forceinline__ long long oz_fixed(float x, int erow) {  // zero when subnormal
+__device__ __forceinline__ long long oz_fixed(float x, int sh, int erow) {  // zero when subnormal
   const uint32_t b = __float_as_uint(x);
   const int ex = (int)((b >> 23) & 0xFF);
   long long m = (long long)((b & 0x7FFFFFu) | 0x800000u) << 29;
-  const int s = ex + 896 - erow + 2;  // exponent field of the same value in FP64
+  const int s = ex + 896 + sh - erow + 2;  // exponent field of the same value in FP64
   if (ex == 0 || s < -53) return 0;
   m = s >= 0 ? m << s : (m + (1LL << (-s - 1))) >> -s;
   return (int32_t)b < 0 ? -m : m;
@@ -105,6 +108,12 @@ __device__ __forceinline__ uint32_t oz_bf16x2(uint32_t d0, uint32_t d1) {
   return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
 
+// The field of an entry shifted by its column's scale, kOzMark for a NaN or an infinity, far
+// below every field for a zero or a column taken as zeros.
+__device__ __forceinline__ int oz_shifted(int field, int sh) {
+  return field == 0x7FF ? kOzMark : field == 0 ? kOzDrop : field + sh;
+}
+
 // One CTA per R rows of an operand tile of T rows and K-block: the rows' exponents, then the
 // slices, eight K values of one row per work item (14 vector stores of eight digits).  Integer
 // work on small pieces: R is a quarter of the tile so that an operand of a few thousand rows
@@ -120,26 +129,35 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackInst* __restrict__ 
   const int64_t k0 = P.k0 + kb;
   constexpr int kBlock = T * 64, kChunk = kOzSlices * kBlock;
   constexpr int kPer = 256 / R;  // threads per row in the exponent pass
-  __shared__ int s_exp[R];
+  __shared__ int s_exp[R], s_sh[kOzK];  // row exponents, column scales
   const V2* A = static_cast<const V2*>(P.a);
   const int tid = threadIdx.x;
-  for (int r = tid; r < R; r += 256) s_exp[r] = 0;
+  for (int r = tid; r < R; r += 256) s_exp[r] = kOzNone + 1021;
+  if (tid < kOzK) {
+    int sh = 0;
+    if (P.kexp && tid < kk) {
+      const int f = P.kexp[kb + tid];
+      sh = f == 0 ? (TRANS ? 0 : kOzDrop) : TRANS ? 1023 - f : f - 1023;
+    }
+    s_sh[tid] = sh;
+  }
   __syncthreads();
   {
     const int r = TRANS ? tid / kPer : tid % R, g = TRANS ? tid % kPer : tid / R;
     const int64_t gr = row0 + r;
-    int mx = 0;
+    int mx = kOzNone + 1021;
     if (gr < P.rows)
       for (int k = g; k < kk; k += kPer)
-        mx = max(mx, oz_expo(A[TRANS ? (k0 + k) + (P.r0 + gr) * P.lda
-                                     : (P.r0 + gr) + (k0 + k) * P.lda]));
+        mx = max(mx, oz_shifted(oz_expo(A[TRANS ? (k0 + k) + (P.r0 + gr) * P.lda
+                                                : (P.r0 + gr) + (k0 + k) * P.lda]),
+                                s_sh[k]));
     atomicMax(&s_exp[r], mx);
   }
   __syncthreads();
   int32_t* exps = P.exps + (int64_t)blockIdx.z * ((P.rows + T - 1) / T * T);
   for (int r = tid; r < R; r += 256) {
     const int e = s_exp[r];
-    exps[row0 + r] = e == 0x7FF ? kOzNaN : e - 1021;
+    exps[row0 + r] = e == kOzMark ? kOzNaN : e - 1021;
   }
   const int all = (P.kk + kOzKC - 1) / kOzKC, chunks = (kk + kOzKC - 1) / kOzKC;
   uint8_t* out = static_cast<uint8_t*>(P.out) + ((size_t)(row0 / T) * all + kb / kOzKC) * kChunk;
@@ -157,8 +175,9 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackInst* __restrict__ 
       if (gr < P.rows && k < kk)
         v = A[TRANS ? (k0 + k) + (P.r0 + gr) * P.lda : (P.r0 + gr) + (k0 + k) * P.lda];
       // digits + 128 in the bytes (byte 6 keeps a carry into bit 8)
-      zr[e] = (unsigned long long)(oz_fixed(v.x, erow) + 0x0080808080808080LL);
-      zi[e] = (unsigned long long)(oz_fixed(v.y, erow) + 0x0080808080808080LL);
+      const int sh = s_sh[k];
+      zr[e] = (unsigned long long)(oz_fixed(v.x, sh, erow) + 0x0080808080808080LL);
+      zi[e] = (unsigned long long)(oz_fixed(v.y, sh, erow) + 0x0080808080808080LL);
     }
     const int sw = ((rt + r) >> 1) & 3, half = g & 1;
     uint8_t* base = out + (size_t)(g >> 1) * kChunk + (rt + r) * 64;
@@ -231,12 +250,11 @@ __device__ __forceinline__ void oz_coords(const OzShared& S, const OzGemmInst* i
   }
 }
 
-// 2^(e - 28), exact (subnormal at the lower end); NaN for a row with a NaN or an infinity
-__device__ __forceinline__ double oz_scale(int32_t e) {
-  if (e == kOzNaN) return __longlong_as_double(0x7FF8000000000000LL);
-  const int x = e - 28 + 1023;  // e in [-1021, 1025]
-  return x > 0 ? __longlong_as_double((long long)x << 52)
-               : __longlong_as_double(1LL << (51 + x));
+// v 2^t where 2^t is no normal number
+__device__ __noinline__ double oz_scaled_far(double v, int t) { return scalbn(v, t); }
+__device__ __forceinline__ double oz_scaled(long long v, int t) {
+  if (t < -1022 || t > 1023) return oz_scaled_far((double)v, t);
+  return (double)v * __longlong_as_double((long long)(t + 1023) << 52);
 }
 
 __global__ void __launch_bounds__(kOzThreads, 1)
@@ -246,6 +264,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   OzShared& S = *reinterpret_cast<OzShared*>(base + kOzStages * kOzStage);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (insts[0].gate && *insts[0].gate > insts[0].gate_cap) return;  // uniform over the grid
   if (threadIdx.x == 0) {
     for (int s = 0; s < kOzStages; ++s) {
       mbar_init(&S.full[s], 1);
@@ -408,7 +427,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       const int blocks = (G.kk + kOzK - 1) / kOzK;
       bool gone = false;
       for (int kb = 0; kb < blocks; ++kb) {
-        const double sr = gr < G.m ? oz_scale(G.aexp[kb * as + gr]) : 0.0;
+        const int32_t er = gr < G.m ? G.aexp[kb * as + gr] : kOzNone;
         const int32_t* be = G.bexp + kb * bs;
         const bool ok = tc_wait(&S.tfull, tphase, err, abort_flag);
         if (!__all_sync(0xffffffffu, ok)) {
@@ -450,9 +469,13 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j)
           if (j < ncol) {
-            const double sc = sr * oz_scale(be[gc + j]);  // 2^(e + f - 56)
-            x[j].x -= (double)v[0][j] * sc;
-            x[j].y -= (double)v[1][j] * sc;
+            const int32_t ec = be[gc + j];
+            if (er == kOzNaN || ec == kOzNaN) {
+              x[j].x = x[j].y = __longlong_as_double(0x7FF8000000000000LL);
+            } else {
+              x[j].x -= oz_scaled(v[0][j], er + ec - 56);
+              x[j].y -= oz_scaled(v[1][j], er + ec - 56);
+            }
             C[(int64_t)j * G.ldc] = x[j];
           }
       }

@@ -20,7 +20,12 @@ struct OzPackInst {
   void* out;       // slice images, oz_pack_bytes(rows, kk, side)
   int32_t* exps;   // exponent of every operand row and block of kOzK columns, block by block:
                    // oz_exps(rows, side) values each
+  const int32_t* kexp;  // or null: an exponent field (of FP64, 1..2046) per K index, by which
+                   // side A is multiplied and side B divided (relative to 1023, the field of
+                   // one); 0: side A takes the column as zeros
 };
+// Stored exponents of a row with a NaN or an infinity, and of one without nonzero entries.
+constexpr int32_t kOzNaN = INT32_MAX, kOzNone = -101021;
 
 // One C -= A B update: C block rows [c_r0, c_r0 + m), columns [c_c0, c_c0 + n).
 struct OzGemmInst {
@@ -34,6 +39,8 @@ struct OzGemmInst {
   int64_t m, n;    // 0: nothing to do
   int32_t kk;
   int32_t n_first;  // 1: neighbouring CTAs take neighbouring columns (A larger than L2)
+  const int32_t* gate;  // or null: nothing to do when *gate > gate_cap (one instance per launch)
+  int32_t gate_cap;
 };
 
 enum OzSide { kOzA = 0, kOzB = 1 };

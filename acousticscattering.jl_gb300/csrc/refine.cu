@@ -13,6 +13,7 @@
 #include <cmath>
 
 #include "bemgpu_internal.h"
+#include "gemm_oz.cuh"
 #include "linalg.cuh"
 #include "refine.cuh"
 
@@ -65,6 +66,8 @@ struct Entry<true> {
   static __device__ __forceinline__ T at(const VecInst& V, int64_t idx) { return ldf(V.A, idx); }
   static __device__ __forceinline__ float mag(T a) { return sqrtf(fmaf(a.x, a.x, a.y * a.y)); }
 };
+// Row-wise products of a system whose digit products were good enough (VecInst::gate).
+__device__ __forceinline__ bool closed(const VecInst& V) { return V.gate && *V.gate <= V.gate_cap; }
 template <bool A32>
 __device__ __forceinline__ float mag_at(const VecInst& V, int64_t idx) {
   return Entry<A32>::mag(Entry<A32>::at(V, idx));
@@ -315,7 +318,7 @@ __global__ void k_split_x(const VecInst* __restrict__ insts) {
   const VecInst& V = insts[blockIdx.z];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int r = blockIdx.y;
-  if (!V.a32 || i >= V.n || r >= V.nrhs) return;
+  if (!V.a32 || i >= V.n || r >= V.nrhs || closed(V)) return;
   const cd x = ldc(V.x, i + (int64_t)r * V.ldx);
   const float hr = (float)x.x, hi = (float)x.y;
   const float lr = (float)(x.x - (double)hr), li = (float)(x.y - (double)hi);
@@ -430,7 +433,7 @@ __global__ void __launch_bounds__(T, (NR == 1 ? 640 : 512) / T)
     k_gemv_a32(const VecInst* __restrict__ insts, int grp0) {
   constexpr int kFold = 32, kRows = 2;
   const VecInst& V = insts[blockIdx.z];
-  if (!V.a32) return;
+  if (!V.a32 || closed(V)) return;
   extern __shared__ __align__(16) unsigned char a32_ring[];
   const int64_t n = V.n, lda = V.lda;
   const int64_t i0 = (int64_t)blockIdx.x * (kRows * T) + threadIdx.x;
@@ -591,7 +594,7 @@ template <int NR>
 __global__ void __launch_bounds__(256) k_gemv_part(const VecInst* __restrict__ insts, int grp0,
                                                    int with_abs) {
   const VecInst& V = insts[blockIdx.z];
-  if (V.a32) return;
+  if (V.a32 || closed(V)) return;
   gemv_body<NR>(V, grp0, with_abs);
 }
 
@@ -625,7 +628,7 @@ __global__ void k_gemv_finish(const VecInst* __restrict__ insts, int mode) {
   const VecInst& V = insts[blockIdx.z];
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   const int r = blockIdx.y, s = threadIdx.x & 7;
-  if (r >= V.nrhs) return;
+  if (r >= V.nrhs || closed(V)) return;
   const bool on = i < V.n;
   double re = 0.0, im = 0.0, ab = 0.0;
   if (on) {
@@ -658,6 +661,153 @@ __global__ void k_gemv_finish(const VecInst* __restrict__ insts, int mode) {
 }
 
 // ---------------------------------------------------------------- many right-hand sides
+// kexp[j]: the largest FP64 exponent field (0: none) of the finite x_jr over the vectors r, 32
+// unknowns per CTA, eight threads each
+__global__ void __launch_bounds__(256) k_wide_scale(const VecInst V, int32_t* __restrict__ kexp) {
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t j = (int64_t)blockIdx.x * 32 + tx;
+  int mx = 0;
+  if (j < V.n)
+    for (int r = ty; r < V.nrhs; r += 8) {
+      const cd x = ldc(V.x, j + (int64_t)r * V.ldx);
+      const int ex = (__double2hiint(x.x) >> 20) & 0x7FF, ey = (__double2hiint(x.y) >> 20) & 0x7FF;
+      if (ex != 0x7FF) mx = max(mx, ex);
+      if (ey != 0x7FF) mx = max(mx, ey);
+    }
+  __shared__ int sh[8][32];
+  sh[ty][tx] = mx;
+  __syncthreads();
+  if (ty == 0 && j < V.n) {
+    for (int u = 1; u < 8; ++u) mx = max(mx, sh[u][tx]);
+    kexp[j] = mx;
+  }
+}
+
+void launch_wide_scale(const Launch& L, const VecInst& v, int32_t* kexp) {
+  k_wide_scale<<<(unsigned)((v.n + 31) / 32), 256, 0, L.stream>>>(v, kexp);
+  count_launch(1);
+}
+
+// The digit products' error bound.  With one exponent per row of A and per vector in a block of
+// 128 columns, the error of y_ir is a few times 2^-56 E_ir, E_ir = sum over the blocks of
+// 2^(aexp + bexp), about 16 max|a| max|x| of the block (up to 8 times for entries of mixed signs
+// and 30 for equal ones, whose E is about |A||x|; random, Burton-Miller and fluid systems of up
+// to 640 unknowns on the CPU).  Entries with E above a multiple of |A||x| (large x meet small a)
+// are listed for k_wide_redo.  The multiple: 32 for right-hand sides, whose E stays below it for
+// bodies of 560 to 20480 panels; 64 for residuals of complex128 systems (up to 1 % of the
+// entries of rigid bodies are above it, those in the shadow of a direction); 256 for those of
+// compact ones (one entry in 64000), which leaves errors below 3e-14 of |A||x|, half of what
+// the paired FP32 products may reach.
+__device__ __forceinline__ double wide_spread(const VecInst& V, int mode) {
+  return mode == 0 ? 32.0 : V.a32 ? 256.0 : 64.0;
+}
+constexpr int kChkRows = 128, kChkN = 8;
+__device__ __forceinline__ float chk_pow2(int e) {  // 2^e of e <= 0, not below 2^-63
+  return __int_as_float((max(e, -63) + 127) << 23);
+}
+__global__ void __launch_bounds__(kChkRows) k_wide_check(const VecInst V, const WideCheck K,
+                                                         int mode) {
+  constexpr int kSeg = 16;  // blocks of the vectors' exponents at a time
+  const int64_t i = (int64_t)blockIdx.x * kChkRows + threadIdx.x;
+  const int g0 = blockIdx.y * kChkN;
+  const bool on = i < K.m;
+  __shared__ float sb[kSeg][kChkN];
+  __shared__ int smax[kChkN];
+  if (threadIdx.x < kChkN) {
+    int mx = kOzNone;
+    if (g0 + threadIdx.x < V.nrhs)
+      for (int b = 0; b < K.kb; ++b) mx = max(mx, K.bexp[b * K.bs + g0 + threadIdx.x]);
+    smax[threadIdx.x] = mx;
+  }
+  int amax = kOzNone;
+  if (on)
+    for (int b = 0; b < K.kb; ++b) amax = max(amax, K.aexp[b * K.as + i]);
+  float sum[kChkN];
+#pragma unroll
+  for (int g = 0; g < kChkN; ++g) sum[g] = 0.f;
+  for (int b0 = 0; b0 < K.kb; b0 += kSeg) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < kSeg * kChkN; e += kChkRows) {
+      const int b = b0 + e / kChkN, g = e % kChkN;
+      const bool some = b < K.kb && g0 + g < V.nrhs && smax[g] != kOzNaN;
+      sb[e / kChkN][g] = some ? chk_pow2(K.bexp[b * K.bs + g0 + g] - smax[g]) : 0.f;
+    }
+    __syncthreads();
+    if (on && amax != kOzNaN)
+      for (int b = b0; b < min(K.kb, b0 + kSeg); ++b) {
+        const float fa = chk_pow2(K.aexp[b * K.as + i] - amax);
+#pragma unroll
+        for (int g = 0; g < kChkN; ++g) sum[g] = fmaf(fa, sb[b - b0][g], sum[g]);
+      }
+  }
+  if (!on || amax == kOzNaN) return;
+#pragma unroll
+  for (int g = 0; g < kChkN; ++g) {
+    if (g0 + g >= V.nrhs || smax[g] == kOzNaN) continue;
+    const double den = V.den[K.r0 + i + (int64_t)(g0 + g) * V.ldy];
+    if (isfinite(den) && scalbn((double)sum[g], amax + smax[g]) > wide_spread(V, mode) * den) {
+      const int at = atomicAdd(K.count, 1);
+      if (at < K.cap) K.list[at] = make_int2((int)(K.r0 + i), g0 + g);
+    }
+  }
+}
+
+void launch_wide_check(const Launch& L, const VecInst& v, const WideCheck& k, int mode) {
+  k_wide_check<<<dim3((unsigned)((k.m + kChkRows - 1) / kChkRows),
+                      (unsigned)((v.nrhs + kChkN - 1) / kChkN)),
+                 kChkRows, 0, L.stream>>>(v, k, mode);
+  count_launch(1);
+}
+
+// The listed entries of y in FP64, one warp each.  The list's order varies, its entries do not
+// depend on one another.
+template <bool A32>
+__global__ void __launch_bounds__(256) k_wide_redo(const VecInst V, const WideCheck K, int mode) {
+  const int count = *K.count;
+  if (count > K.cap) return;  // the row-wise products do them all
+  const int lane = threadIdx.x & 31;
+  for (int e = blockIdx.x * 8 + (threadIdx.x >> 5); e < count; e += gridDim.x * 8) {
+    const int2 at = K.list[e];
+    const int64_t i = at.x, n = V.n;
+    const double* x = V.x + 2 * (int64_t)at.y * V.ldx;
+    cd t = {0.0, 0.0};
+    constexpr int kB = 8;
+    for (int64_t j0 = lane; j0 < n; j0 += 32 * kB) {
+      typename Entry<A32>::T a[kB];
+#pragma unroll
+      for (int q = 0; q < kB; ++q) {
+        const int64_t j = j0 + 32 * q;
+        a[q] = j < n ? Entry<A32>::at(V, i + j * V.lda) : typename Entry<A32>::T{};
+      }
+#pragma unroll
+      for (int q = 0; q < kB; ++q) {
+        const int64_t j = j0 + 32 * q;
+        const cd v = j < n ? ldc(x, j) : cd{0.0, 0.0};
+        t.x = fma((double)a[q].x, v.x, fma(-(double)a[q].y, v.y, t.x));
+        t.y = fma((double)a[q].x, v.y, fma((double)a[q].y, v.x, t.y));
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    if (lane == 0) {
+      const cd b = mode == 1 ? ldc(V.b, i + (int64_t)at.y * V.ldb) : cd{0.0, 0.0};
+      stc(V.y, i + (int64_t)at.y * V.ldy, cd{b.x - t.x, b.y - t.y});
+    }
+  }
+}
+
+void launch_wide_redo(const Launch& L, const VecInst& v, const WideCheck& k, int mode) {
+  const unsigned grid = (unsigned)std::min<int64_t>((k.cap + 7) / 8, 4 * (int64_t)device_sm_count());
+  if (v.a32)
+    k_wide_redo<true><<<grid, 256, 0, L.stream>>>(v, k, mode);
+  else
+    k_wide_redo<false><<<grid, 256, 0, L.stream>>>(v, k, mode);
+  count_launch(1);
+}
+
 // |x| of every vector in FP32 (ld n)
 __global__ void k_wide_mag(const VecInst V, float* __restrict__ xa) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -665,7 +815,7 @@ __global__ void k_wide_mag(const VecInst V, float* __restrict__ xa) {
   if (i < V.n) xa[i + (int64_t)r * V.n] = fabs_c(ldc(V.x, i + (int64_t)r * V.ldx));
 }
 
-// den = |b| + |A||x| in FP32 magnitudes (as the row-wise products): 64 x 96 tiles, 4 x 6
+// den = |A||x| (mode 1: + |b|) in FP32 magnitudes (as the row-wise products): 64 x 96 tiles, 4 x 6
 // entries per thread, K-chunks of 16 with the next chunk in registers as it was loaded (a
 // magnitude taken at the load would wait for it).  FP32-issue bound, one FMA per matrix entry and
 // vector, two of them in a paired instruction: 2.1 ms for 20480 unknowns and 181 vectors at the
@@ -673,7 +823,8 @@ __global__ void k_wide_mag(const VecInst V, float* __restrict__ xa) {
 // with them.
 constexpr int kWaM = 64, kWaN = 96, kWaK = 16;
 template <bool A32>
-__global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* __restrict__ xa) {
+__global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* __restrict__ xa,
+                                                  int mode) {
   using E = Entry<A32>;
   const int64_t r0 = (int64_t)blockIdx.x * kWaM, n = V.n;
   const int g0 = blockIdx.y * kWaN;
@@ -732,19 +883,20 @@ __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* 
     for (int b = 0; b < 6; ++b) {
       const int64_t r = r0 + tx * 4 + a;
       const int g = g0 + ty * 6 + b;
-      if (r < n && g < V.nrhs)
-        V.den[r + (int64_t)g * V.ldy] = cabs(ldc(V.b, r + (int64_t)g * V.ldb)) +
-                                        (double)(b & 1 ? acc[a][b / 2].y : acc[a][b / 2].x);
+      if (r < n && g < V.nrhs) {
+        const double ab = mode == 1 ? cabs(ldc(V.b, r + (int64_t)g * V.ldb)) : 0.0;
+        V.den[r + (int64_t)g * V.ldy] = ab + (double)(b & 1 ? acc[a][b / 2].y : acc[a][b / 2].x);
+      }
     }
 }
 
-void launch_wide_abs(const Launch& L, const VecInst& v, float* xa) {
+void launch_wide_abs(const Launch& L, const VecInst& v, float* xa, int mode) {
   k_wide_mag<<<dim3((unsigned)((v.n + 255) / 256), (unsigned)v.nrhs), 256, 0, L.stream>>>(v, xa);
   const dim3 g((unsigned)((v.n + kWaM - 1) / kWaM), (unsigned)((v.nrhs + kWaN - 1) / kWaN));
   if (v.a32)
-    k_wide_abs<true><<<g, 256, 0, L.stream>>>(v, xa);
+    k_wide_abs<true><<<g, 256, 0, L.stream>>>(v, xa, mode);
   else
-    k_wide_abs<false><<<g, 256, 0, L.stream>>>(v, xa);
+    k_wide_abs<false><<<g, 256, 0, L.stream>>>(v, xa, mode);
   count_launch(2);
 }
 

@@ -51,6 +51,8 @@ struct VecInst {
   float* xa;                 // |x| in FP32, n x nrhs
   float* cols_inv32;         // 1 / cols in FP32 (n)
   double norm_floor;         // equilibration: lower bound of the row and column scales
+  const int32_t* gate;       // or null: the row-wise products do nothing unless *gate > gate_cap
+  int32_t gate_cap;
 };
 
 #ifdef __CUDACC__
@@ -60,11 +62,26 @@ void launch_scale_copy(const Launch& L, const VecInst* d, int ninst, int64_t nma
 // 256 (2) rows in the compact-storage product (results identical)
 void launch_gemv(const Launch& L, const VecInst* d, int ninst, int64_t nmax, int32_t max_rhs,
                  int mode, int rows = 2);
-// Products of one system with many vectors (api.cu:wide_product): den = |b| + |A||x|, and the
-// end of a product whose sum the tensor-core kernel left in y (mode 0: y = -A x without the
-// near corrections, mode 1: y = b - A x without them).
+// Products of one system with many vectors (api.cu:wide_product).  scale: kexp[j] = largest
+// exponent field of x_j over the vectors (n values); abs: den = |A||x| (mode 1: + |b|), xa: n x
+// nrhs scratch; check: entries whose digit product may be off by more than its share of den, at
+// most cap of them listed; redo: those entries in FP64; finish: the end of a product whose sum
+// the tensor-core kernel left in y (mode 0: y = -A x without the near corrections, mode 1:
+// y = b - A x without them).
 constexpr int kWideRhs = 16;  // right-hand sides of a system from which they are used
-void launch_wide_abs(const Launch& L, const VecInst& v, float* xa);  // xa: n x nrhs scratch
+struct WideCheck {
+  const int32_t* aexp;  // exponents of rows [r0, r0 + m) of A and of the vectors, kb blocks
+  const int32_t* bexp;
+  int64_t r0, m;
+  int64_t as, bs;       // entries of a block of aexp, bexp
+  int32_t kb, cap;
+  int32_t* count;       // entries found so far (more than cap: the row-wise products take over)
+  int2* list;           // (row, vector)
+};
+void launch_wide_scale(const Launch& L, const VecInst& v, int32_t* kexp);
+void launch_wide_abs(const Launch& L, const VecInst& v, float* xa, int mode);
+void launch_wide_check(const Launch& L, const VecInst& v, const WideCheck& k, int mode);
+void launch_wide_redo(const Launch& L, const VecInst& v, const WideCheck& k, int mode);
 void launch_wide_finish(const Launch& L, const VecInst& v, int mode);
 // compact instances: out (complex128, ld n) += the near corrections, each scaled by
 // 1 / (rows_i cols_j) (unit_scales = 0) or unscaled (unit_scales = 1)
