@@ -1697,6 +1697,11 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
   enum { kU12 = kInner, kTrail, kPhases };
   const int64_t blocks = (nmax + B - 1) / B;
   const size_t count = (size_t)blocks * kPhases * ni;
+  // the scale of every update's K index, from the rows of its right operand: with rows of
+  // different sizes (no equilibration) l_ik goes with 1 / d_k and u_kj with d_k
+  Buf kexp;
+  TRY(alloc(c, count * B * 4, &kexp));
+  CUDA_TRY(c, cudaMemsetAsync(kexp.p, 0, count * B * 4, c->stream));
   std::vector<OzPackInst> pa(count), pb(count);
   std::vector<OzGemmInst> ge(count);
   std::vector<int64_t> tiles(count), ra((size_t)blocks * kPhases, 0), rb((size_t)blocks * kPhases, 0);
@@ -1723,9 +1728,10 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
         a = OzPackInst{u12 ? negn[t].p : mi[t].a, u12 ? (int64_t)B : mi[t].lda, u12 ? 0 : r0,
                        u12 ? 0 : k0, on ? r1 - r0 : 0, on ? kk : 0, 0,
                        u12 ? npack[t].p : apack[t].p,
-                       u12 ? nexp[t].as<int32_t>() : aexp[t].as<int32_t>()};
+                       u12 ? nexp[t].as<int32_t>() : aexp[t].as<int32_t>(),
+                       kexp.as<int32_t>() + q * B};
         pb[q] = OzPackInst{mi[t].a, mi[t].lda, c0, k0, on ? c1 - c0 : 0, on ? kk : 0, 0,
-                           bpack[t].p, bexp[t].as<int32_t>()};
+                           bpack[t].p, bexp[t].as<int32_t>(), a.kexp};
         ge[q] = OzGemmInst{a.out, bpack[t].p, a.exps, bexp[t].as<int32_t>(), mi[t].a, mi[t].lda,
                            r0, c0, on ? r1 - r0 : 0, on ? c1 - c0 : 0, on ? kk : 0, 0};
         tiles[q] = on ? oz_tiles(r1 - r0, c1 - c0) : 0;
@@ -1745,6 +1751,7 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
     if (ra[q] <= 0 || rb[q] <= 0) return;
     {
       Prof pr(c, "oz_pack");
+      launch_oz_kexp(L, dpb.as<OzPackInst>() + q * ni, ni, rb[q], B);
       launch_oz_pack(L, dpa.as<OzPackInst>() + q * ni, ni, ra[q], B, kOzA);
       launch_oz_pack(L, dpb.as<OzPackInst>() + q * ni, ni, rb[q], B, kOzB);
     }
@@ -2315,7 +2322,7 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
   const int64_t rows = tiles * 128;
   TRY(alloc(c, tile * (size_t)tiles, &ap));
   TRY(alloc(c, (size_t)kb * (size_t)rows * 4, &ae));
-  const int32_t* kexp = ke.as<int32_t>();
+  int32_t* kexp = ke.as<int32_t>();
   std::vector<OzPackInst> pk;
   std::vector<OzGemmInst> ge;
   pk.push_back(OzPackInst{v.x, v.ldx, 0, 0, R, (int32_t)n, 0, xp.p, xe.as<int32_t>(), kexp});

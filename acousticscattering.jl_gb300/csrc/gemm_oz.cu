@@ -201,6 +201,44 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackInst* __restrict__ 
   }
 }
 
+// The scales of the K index from side B (complex128, at most kOzK of them): lanes along k,
+// kKexpRows operand rows per CTA.  The largest of integers, whatever the order.
+constexpr int kKexpRows = 64;
+__global__ void __launch_bounds__(256) k_oz_kexp(const OzPackInst* __restrict__ insts) {
+  const OzPackInst& P = insts[blockIdx.y];
+  const int64_t row0 = (int64_t)blockIdx.x * kKexpRows;
+  if (row0 >= P.rows || P.kk <= 0) return;  // uniform over the CTA
+  const int width = P.kk <= 32 ? 32 : kOzK, step = 256 / width;
+  const int k = threadIdx.x % width;
+  const int64_t end = min(row0 + kKexpRows, P.rows);
+  const double2* A = static_cast<const double2*>(P.a) + P.k0 + k + P.r0 * P.lda;
+  int mx = 0;
+  if (k < P.kk) {
+    constexpr int kFly = 8;
+    for (int64_t r0 = row0 + threadIdx.x / width; r0 < end; r0 += kFly * step) {
+      double2 v[kFly];
+#pragma unroll
+      for (int u = 0; u < kFly; ++u) {
+        const int64_t r = r0 + u * step;
+        v[u] = r < end ? A[r * P.lda] : double2{0.0, 0.0};
+      }
+#pragma unroll
+      for (int u = 0; u < kFly; ++u) {
+        const int x = (__double2hiint(v[u].x) >> 20) & 0x7FF;
+        const int y = (__double2hiint(v[u].y) >> 20) & 0x7FF;
+        mx = max(mx, max(x == 0x7FF ? 0 : x, y == 0x7FF ? 0 : y));
+      }
+    }
+  }
+  __shared__ int sh[256];
+  sh[threadIdx.x] = mx;
+  __syncthreads();
+  if (threadIdx.x < width && k < P.kk) {
+    for (int u = 1; u < step; ++u) mx = max(mx, sh[threadIdx.x + u * width]);
+    atomicMax(P.kexp + k, mx);
+  }
+}
+
 // ------------------------------------------------------------------ the GEMM
 // Shared-memory descriptor: K-major operand, 64-byte swizzle, 8-row groups 512 bytes apart.
 __device__ __forceinline__ uint64_t oz_desc(uint32_t saddr) {
@@ -505,6 +543,13 @@ size_t oz_exps(int64_t rows, OzSide side) {
 }
 int64_t oz_tiles(int64_t m, int64_t n) {
   return m > 0 && n > 0 ? ((m + kOzM - 1) / kOzM) * ((n + kOzN - 1) / kOzN) : 0;
+}
+
+void launch_oz_kexp(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows, int max_kk) {
+  if (ninst <= 0 || max_rows <= 0 || max_kk <= 0) return;
+  k_oz_kexp<<<dim3((unsigned)((max_rows + kKexpRows - 1) / kKexpRows), (unsigned)ninst), 256, 0,
+              L.stream>>>(d);
+  count_launch(1);
 }
 
 void launch_oz_pack(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows, int max_kk,

@@ -20,9 +20,9 @@ struct OzPackInst {
   void* out;       // slice images, oz_pack_bytes(rows, kk, side)
   int32_t* exps;   // exponent of every operand row and block of kOzK columns, block by block:
                    // oz_exps(rows, side) values each
-  const int32_t* kexp;  // or null: an exponent field (of FP64, 1..2046) per K index, by which
-                   // side A is multiplied and side B divided (relative to 1023, the field of
-                   // one); 0: side A takes the column as zeros
+  int32_t* kexp;   // or null: an exponent field (of FP64, 1..2046) per K index, by which side A is
+                   // multiplied and side B divided (relative to 1023, the field of one); 0: side
+                   // A takes the column as zeros
 };
 // Stored exponents of a row with a NaN or an infinity, and of one without nonzero entries.
 constexpr int32_t kOzNaN = INT32_MAX, kOzNone = -101021;
@@ -49,6 +49,9 @@ size_t oz_exps(int64_t rows, OzSide side);
 int64_t oz_tiles(int64_t m, int64_t n);  // tiles of one update
 
 #ifdef __CUDACC__
+// kexp of side B: kexp[k] = max(kexp[k], largest field of the operand's finite entries at k) over
+// its rows (zeros before the first call)
+void launch_oz_kexp(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows, int max_kk);
 // side A: element (r, k) at r + k lda, single: the complex64 instances (the others are
 // skipped); side B: at k + r lda, complex128
 void launch_oz_pack(const Launch& L, const OzPackInst* d, int ninst, int64_t max_rows, int max_kk,
