@@ -202,8 +202,9 @@ __global__ void __launch_bounds__(256) k_oz_pack(const OzPackInst* __restrict__ 
 }
 
 // The scales of the K index from side B (complex128, at most kOzK of them): lanes along k,
-// kKexpRows operand rows per CTA.  The largest of integers, whatever the order.
-constexpr int kKexpRows = 64;
+// kKexpRows operand rows per CTA.  The largest of integers, whatever the order.  Bound by latency:
+// a CTA's loads are one round.
+constexpr int kKexpRows = 16;
 __global__ void __launch_bounds__(256) k_oz_kexp(const OzPackInst* __restrict__ insts) {
   const OzPackInst& P = insts[blockIdx.y];
   const int64_t row0 = (int64_t)blockIdx.x * kKexpRows;
