@@ -820,8 +820,9 @@ __global__ void k_wide_mag(const VecInst V, float* __restrict__ xa) {
 // magnitude taken at the load would wait for it).  FP32-issue bound, one FMA per matrix entry and
 // vector, two of them in a paired instruction: 2.1 ms for 20480 unknowns and 181 vectors at the
 // single rate, 11 ms before the pairs, the late magnitudes and the odd row stride of sX, 5.0 ms
-// with them.
-constexpr int kWaM = 64, kWaN = 96, kWaK = 16;
+// with them.  FP32 sums of kWaFold columns are added in FP64 (the row-wise products': n / 8 to n
+// / 32 columns).
+constexpr int kWaM = 64, kWaN = 96, kWaK = 16, kWaFold = 2048;
 template <bool A32>
 __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* __restrict__ xa,
                                                   int mode) {
@@ -854,8 +855,29 @@ __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* 
       nx[e] = g < V.nrhs && c < n ? xa[c + (int64_t)g * n] : 0.f;
     }
   };
+  // the sums so far into den, the first time with |b|
+  auto fold = [&](bool first) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 6; ++b) {
+        const int64_t r = r0 + tx * 4 + a;
+        const int g = g0 + ty * 6 + b;
+        if (r < n && g < V.nrhs) {
+          double* at = V.den + r + (int64_t)g * V.ldy;
+          const double old =
+              !first ? *at : mode == 1 ? cabs(ldc(V.b, r + (int64_t)g * V.ldb)) : 0.0;
+          *at = old + (double)(b & 1 ? acc[a][b / 2].y : acc[a][b / 2].x);
+        }
+      }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) acc[a][b] = make_float2(0.f, 0.f);
+  };
   load(0);
   for (int64_t k = 0; k < n; k += kWaK) {
+    if (k > 0 && k % kWaFold == 0) fold(k == kWaFold);
 #pragma unroll
     for (int e = 0; e < kA; ++e)
       sA[(tid + 256 * e) / kWaM][(tid + 256 * e) % kWaM] = E::mag(na[e]);
@@ -877,17 +899,7 @@ __global__ void __launch_bounds__(256) k_wide_abs(const VecInst V, const float* 
     }
     __syncthreads();
   }
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 6; ++b) {
-      const int64_t r = r0 + tx * 4 + a;
-      const int g = g0 + ty * 6 + b;
-      if (r < n && g < V.nrhs) {
-        const double ab = mode == 1 ? cabs(ldc(V.b, r + (int64_t)g * V.ldb)) : 0.0;
-        V.den[r + (int64_t)g * V.ldy] = ab + (double)(b & 1 ? acc[a][b / 2].y : acc[a][b / 2].x);
-      }
-    }
+  fold(n <= kWaFold);
 }
 
 void launch_wide_abs(const Launch& L, const VecInst& v, float* xa, int mode) {
