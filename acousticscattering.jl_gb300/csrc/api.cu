@@ -418,6 +418,21 @@ int alloc(bemgpu_ctx* c, size_t bytes, Buf* out) {
   return BEMGPU_OK;
 }
 
+// The same for scratch a call can do without: *got false (and no error left behind) when the
+// budget or the device has no room.
+int try_alloc(bemgpu_ctx* c, size_t bytes, Buf* out, bool* got) {
+  const std::string err = c->err;
+  const cudaError_t last = c->last_cuda;
+  const int s = alloc(c, bytes, out);
+  *got = s == BEMGPU_OK;
+  if (s == BEMGPU_ENOMEM_BUDGET || (s == BEMGPU_ECUDA && c->last_cuda == cudaErrorMemoryAllocation)) {
+    c->err = err;
+    c->last_cuda = last;
+    return BEMGPU_OK;
+  }
+  return s;
+}
+
 template <class T>
 int upload(bemgpu_ctx* c, const std::vector<T>& h, Buf* out) {
   TRY(alloc(c, h.size() * sizeof(T), out));
@@ -2291,6 +2306,23 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
   return BEMGPU_OK;
 }
 
+// Entries of a product with many right-hand sides that are computed again at most, one in 64: their
+// rows are read at 32 bytes an entry, 38 GB or 6 ms for 181 vectors of 20480 unknowns.
+int32_t wide_cap(int64_t n, int64_t R) {
+  return (int32_t)std::min<int64_t>(1 << 20, std::max<int64_t>(1024, n * R / 64));
+}
+// Slices of A held at a time at most: all of them or about 8 GB.
+size_t wide_panel_bytes(int64_t n) {
+  const size_t tile = oz_pack_bytes(128, (int)n, kOzA);
+  return tile * std::max<size_t>(1, std::min<size_t>((size_t)(n + 127) / 128, (8ull << 30) / tile));
+}
+// Scratch of one such product (they run one at a time).
+size_t wide_scratch(int64_t n, int64_t R) {
+  const size_t kb = (size_t)(n + kOzK - 1) / kOzK;
+  return oz_pack_bytes(R, (int)n, kOzB) + kb * oz_exps(R, kOzB) * 4 + wide_panel_bytes(n) +
+         kb * (size_t)(n + 127) * 4 + (size_t)wide_cap(n, R) * 8 + (size_t)n * (4 + 4 * R);
+}
+
 // y = A x (mode 0, den used as scratch) or y = b - A x with den = |b| + |A||x| (mode 1) of one
 // system with many right-hand sides: the vectors and the matrix, in row panels, are cut into
 // digit slices and multiplied on the tensor cores (gemm_oz.cu), the near corrections and the
@@ -2301,27 +2333,39 @@ int correction_pass(bemgpu_ctx* c, std::vector<SolveInst*>& ss, bool from_b,
 // on the device).  The row-wise products spend about 44 FP32 instructions per
 // complex product whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 29 ms (of
 // which 16 the products, 4 the slices of the matrix, 5 the denominators).
-int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
+//
+// Scratch (wide_scratch) is taken if it is there: fewer row panels when the allocation fails, and
+// the row-wise products when not even one panel can be had (*done false).
+int wide_product(bemgpu_ctx* c, const VecInst& v, int mode, bool* done) {
   const Launch L = c->launch();
   const int64_t n = v.n, kb = (n + kOzK - 1) / kOzK;
   const int32_t R = v.nrhs;
-  Buf xp, xe, ap, ae, ke, found, list;
-  TRY(alloc(c, oz_pack_bytes(R, (int)n, kOzB), &xp));
-  TRY(alloc(c, (size_t)kb * oz_exps(R, kOzB) * 4, &xe));
-  TRY(alloc(c, (size_t)n * 4, &ke));
-  // entries computed again at most, one in 64: their rows are read at 32 bytes an entry, 38 GB or
-  // 6 ms for 181 vectors of 20480 unknowns
-  const int32_t cap = (int32_t)std::min<int64_t>(1 << 20, std::max<int64_t>(1024, n * R / 64));
-  TRY(alloc(c, 4, &found));
-  TRY(alloc(c, (size_t)cap * sizeof(int2), &list));
-  // row panels: about 8 GB of slices, at most a quarter of what the budget leaves
+  *done = false;
+  Buf xp, xe, ap, ae, ke, found, list, xa;
+  const int32_t cap = wide_cap(n, R);
+  bool got = true;
+  auto scratch = [&](size_t bytes, Buf* b) { return got ? try_alloc(c, bytes, b, &got) : BEMGPU_OK; };
+  TRY(scratch(oz_pack_bytes(R, (int)n, kOzB), &xp));
+  TRY(scratch((size_t)kb * oz_exps(R, kOzB) * 4, &xe));
+  TRY(scratch((size_t)n * 4, &ke));
+  TRY(scratch(4, &found));
+  TRY(scratch((size_t)cap * sizeof(int2), &list));
+  TRY(scratch((size_t)n * R * 4, &xa));
+  if (!got) return BEMGPU_OK;
+  // row panels: at most a quarter of what the budget leaves
   const size_t tile = oz_pack_bytes(128, (int)n, kOzA);
   const uint64_t used = total_live(c), budget = root_of(c)->budget;
-  const uint64_t room = std::min<uint64_t>(8ull << 30, budget > used ? (budget - used) / 4 : 0);
-  const int64_t tiles = std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, (int64_t)(room / tile)));
+  const uint64_t room = std::min<uint64_t>(wide_panel_bytes(n), budget > used ? (budget - used) / 4 : 0);
+  int64_t tiles = std::max<int64_t>(1, (int64_t)(room / tile));
+  for (;; tiles = (tiles + 1) / 2) {
+    got = true;
+    TRY(scratch((size_t)kb * (size_t)tiles * 128 * 4, &ae));
+    TRY(scratch(tile * (size_t)tiles, &ap));
+    if (got) break;
+    if (tiles == 1) return BEMGPU_OK;
+  }
+  *done = true;
   const int64_t rows = tiles * 128;
-  TRY(alloc(c, tile * (size_t)tiles, &ap));
-  TRY(alloc(c, (size_t)kb * (size_t)rows * 4, &ae));
   int32_t* kexp = ke.as<int32_t>();
   std::vector<OzPackInst> pk;
   std::vector<OzGemmInst> ge;
@@ -2347,8 +2391,6 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode) {
     CUDA_TRY(c, cudaMemset2DAsync(v.y, (size_t)v.ldy * 16, 0, (size_t)n * 16, (size_t)R, c->stream));
   }
   CUDA_TRY(c, cudaMemsetAsync(found.p, 0, 4, c->stream));
-  Buf xa;
-  TRY(alloc(c, (size_t)n * R * 4, &xa));
   launch_wide_abs(L, v, xa.as<float>(), mode);
   launch_wide_scale(L, v, ke.as<int32_t>());
   launch_oz_pack(L, dpk.as<OzPackInst>(), 1, R, (int)n, kOzB);
@@ -2379,8 +2421,9 @@ int products(bemgpu_ctx* c, const std::vector<VecInst>& all, int mode, int rows)
   int32_t rmax = 0;
   for (const VecInst& v : all) {
     if (v.nrhs >= kWideRhs && c->tensor_lu) {
-      TRY(wide_product(c, v, mode));
-      continue;
+      bool done = false;
+      TRY(wide_product(c, v, mode, &done));
+      if (done) continue;
     }
     few.push_back(v);
     nmax = std::max(nmax, v.n);
@@ -2878,8 +2921,7 @@ size_t solve_bytes(const ServerReq& r) {
   const size_t N = (size_t)order_of(r);
   const size_t R = (size_t)r.nangles;
   size_t b = N * R * (16 * 7 + 12) + (size_t)vec_chunks((int64_t)N) * R * N * 3 * 8;
-  if (r.nangles >= kWideRhs)  // slices of the vectors and of one row panel (more if there is room)
-    b += oz_pack_bytes((int64_t)R, (int)N, kOzB) + oz_pack_bytes(128, (int)N, kOzA) + N * R * 4;
+  if (r.nangles >= kWideRhs) b += wide_scratch((int64_t)N, (int64_t)R);
   return b + b / 20;
 }
 
