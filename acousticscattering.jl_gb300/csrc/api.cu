@@ -2206,6 +2206,11 @@ struct SolveInst {
   std::vector<RhsState> rs;
 };
 
+// VecInst::part of a solve: the products' partial sums
+size_t part_bytes(int64_t n, int32_t nrhs) {
+  return (size_t)vec_chunks(n, nrhs) * (size_t)nrhs * (size_t)n * 3 * 8;
+}
+
 void fill_vec(VecInst& v, SolveInst& s, const void* A, int64_t N) {
   std::memset(&v, 0, sizeof v);
   v.A = A;
@@ -2559,8 +2564,7 @@ int solve_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<i
     }
     TRY(alloc(c, (size_t)N * s.R * 16, &s.work));
     TRY(alloc(c, (size_t)kStats * s.R * 8, &s.stats));
-    TRY(alloc(c, (size_t)vec_chunks(N) * (int64_t)s.R * N * 3 * 8,
-              &s.part));
+    TRY(alloc(c, part_bytes(N, s.R), &s.part));
     TRY(alloc(c, (size_t)s.R * 4, &s.active));
     TRY(alloc(c, (size_t)s.R * 4, &s.changed));
     TRY(alloc(c, (size_t)n * s.R * 16, &out[t]->ps));
@@ -2920,7 +2924,7 @@ int64_t order_of(const ServerReq& r) {
 size_t solve_bytes(const ServerReq& r) {
   const size_t N = (size_t)order_of(r);
   const size_t R = (size_t)r.nangles;
-  size_t b = N * R * (16 * 7 + 12) + (size_t)vec_chunks((int64_t)N) * R * N * 3 * 8;
+  size_t b = N * R * (16 * 7 + 12) + part_bytes((int64_t)N, r.nangles);
   if (r.nangles >= kWideRhs) b += wide_scratch((int64_t)N, (int64_t)R);
   return b + b / 20;
 }
@@ -5257,8 +5261,7 @@ int bemgpu_dense_solve(bemgpu_ctx* c, int64_t n, const double* A, int32_t nrhs, 
   TRY(alloc(c, (size_t)n * nrhs * 8, &s.den));
   TRY(alloc(c, (size_t)n * nrhs * 16, &s.work));
   TRY(alloc(c, (size_t)kStats * nrhs * 8, &s.stats));
-  TRY(alloc(c, (size_t)vec_chunks(n) * (int64_t)nrhs * n * 3 * 8,
-            &s.part));
+  TRY(alloc(c, part_bytes(n, nrhs), &s.part));
   TRY(alloc(c, (size_t)nrhs * 4, &s.active));
   TRY(alloc(c, (size_t)nrhs * 4, &s.changed));
   CUDA_TRY(c, cudaMemcpyAsync(s.b.p, B, (size_t)n * nrhs * 16, cudaMemcpyHostToDevice, c->stream));

@@ -370,12 +370,12 @@ __device__ __forceinline__ void gemv_body(const VecInst& V, int grp0, int with_a
   constexpr int kGemvR = NR;  // right-hand sides per pass of this instantiation
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int ch = blockIdx.y % kMaxChunks, grp = grp0 + blockIdx.y / kMaxChunks;
-  if (ch >= vec_chunks(V.n)) return;
+  if (ch >= vec_chunks(V.n, V.nrhs)) return;
   const int r0 = grp * kGemvR;
   if (i >= V.n || r0 >= V.nrhs) return;
   const int nr = min(kGemvR, V.nrhs - r0);
   int64_t j0, j1;
-  chunk_range(V.n, ch, vec_chunks(V.n), &j0, &j1);
+  chunk_range(V.n, ch, vec_chunks(V.n, V.nrhs), &j0, &j1);
   cd acc[kGemvR];
   float aacc[kGemvR];
 #pragma unroll
@@ -438,12 +438,12 @@ __global__ void __launch_bounds__(T, (NR == 1 ? 640 : 512) / T)
   const int64_t n = V.n, lda = V.lda;
   const int64_t i0 = (int64_t)blockIdx.x * (kRows * T) + threadIdx.x;
   const int ch = blockIdx.y % kMaxChunks, grp = grp0 + blockIdx.y / kMaxChunks;
-  if (ch >= vec_chunks(n)) return;
+  if (ch >= vec_chunks(n, V.nrhs)) return;
   const int r0 = grp * NR;
   if (i0 >= n || r0 >= V.nrhs) return;
   const int nr = min(NR, V.nrhs - r0);
   int64_t j0, j1;
-  chunk_range(n, ch, vec_chunks(n), &j0, &j1);
+  chunk_range(n, ch, vec_chunks(n, V.nrhs), &j0, &j1);
   const int cols = (int)(j1 - j0), groups = cols / kA32Cols;  // whole groups
   const float2* A[kRows];  // rows past the last: the first one again
 #pragma unroll
@@ -632,7 +632,7 @@ __global__ void k_gemv_finish(const VecInst* __restrict__ insts, int mode) {
   const bool on = i < V.n;
   double re = 0.0, im = 0.0, ab = 0.0;
   if (on) {
-    const int chunks = vec_chunks(V.n);
+    const int chunks = vec_chunks(V.n, V.nrhs);
     for (int c = s; c < chunks; c += 8) {
       const int64_t o = 3 * (((int64_t)c * V.nrhs + r) * V.n + i);
       re += V.part[o];

@@ -7,9 +7,13 @@ namespace bemgpu {
 
 // Column chunks of the row-wise sweeps, by the system's own order: a thread takes a row, so
 // small systems need more chunks to fill the GPU (1280 unknowns: 24 CTAs with 8 chunks, 76 us
-// a residual; 19 us with 32).
+// a residual; 19 us with 32).  Products of many right-hand sides fill it by these, and their
+// partial sums are a chunk's worth of memory per right-hand side: 8 chunks.
 constexpr int kMaxChunks = 32;
-__host__ __device__ inline int vec_chunks(int64_t n) { return n <= 2560 ? 32 : n <= 5120 ? 16 : 8; }
+constexpr int kManyChunksRhs = 16;
+__host__ __device__ inline int vec_chunks(int64_t n, int32_t nrhs = 1) {
+  return nrhs >= kManyChunksRhs || n > 5120 ? 8 : n <= 2560 ? 32 : 16;
+}
 constexpr int kGemvR = 4;    // right-hand sides per gemv pass
 constexpr int kStats = 9;    // residual statistics per right-hand side
 
@@ -22,7 +26,7 @@ struct VecInst {
   double* rowsum;    // row sums of |A| (n)
   double* cols_inv;  // 1 / cols (n), filled by the scaled-copy launch
   float* rows_inv;   // 1 / rows (n), filled by the row-statistics launch
-  double* part;      // scratch: vec_chunks(n) * nrhs * n * 3 doubles (>= vec_chunks(n) * n * 2)
+  double* part;      // scratch: vec_chunks(n, nrhs) * nrhs * n * 3 doubles
   void* out;         // scaled copy / correction work buffer (ld n)
   int32_t out_single;
   int32_t nrhs;

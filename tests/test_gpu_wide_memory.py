@@ -46,6 +46,17 @@ def test_least_budget_is_that_of_the_row_wise_products(ctx):
         assert d["normwise_backward_error"] <= (5 * np.sqrt(n) + 1) * eps
 
 
+def test_partial_sums_of_many_right_hand_sides(ctx):
+    """Eight chunks of partial sums per right-hand side (of 24 bytes an unknown), the seven other
+    vectors and the few MB of a system of 300 unknowns are enough."""
+    n, nrhs = 300, 400
+    rng = np.random.default_rng(4)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 2 * np.eye(n)
+    B = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    need = n * nrhs * (8 * 24 + 7 * 16) + 16 * MB
+    assert _solve(need, A, B, True) is not None
+
+
 def test_server_under_a_budget_with_many_angles(ctx):
     """Requests whose slices count in the admission: all complete, none runs out of memory."""
     from bemgpu import meshes
