@@ -13,8 +13,9 @@
 // point, fixed-order reductions, FP64 fields.
 //
 // Bound by FP64 issue.  The far panels take the shared-phase rule of quad_regular.cuh, the
-// interior traces are formed once per call (from kTracesPoints points on), and the region test sums FP32 angles (panels
-// within two diameters in FP64), repeated in FP64 when the sum is not clearly 0 or 4 pi:
+// interior traces are formed once per call (from kTracesPoints points on), and the region test
+// sums FP32 angles (panels within two diameters, or at distances whose cubes FP32 does not
+// hold, in FP64), repeated in FP64 when the sum is not clearly 0 or 4 pi:
 // 2001 points of a 2880-panel fluid body 6.30 -> 4.5 ms.
 #include "bemgpu_internal.h"
 #include "pressure.cuh"
@@ -37,8 +38,10 @@ __device__ __forceinline__ double solid_angle(const double* v, const double* x) 
   return 2.0 * atan2(num, den);
 }
 
-// Solid angle of a panel in FP32, for the region test: records relative to the mesh's centre
-// lose nothing that matters at a distance of a few panels.
+// Solid angle of a panel in FP32, for the region test: records relative to the point lose nothing
+// that matters at a distance of a few panels.  Its products are of the third degree in the
+// distances, so it is for panels whose squared distance is within kAngleMin2 and kAngleMax2.
+constexpr float kAngleMin2 = 1e-20f, kAngleMax2 = 1e20f;
 __device__ __forceinline__ float solid_angle_f(const double* v, const double* x) {
   float R[3][3];
 #pragma unroll
@@ -117,8 +120,8 @@ __global__ void __launch_bounds__(kPrThreads) k_pressure(const PressureInst P) {
   for (int64_t j = threadIdx.x; j < P.n; j += kPrThreads) {
     const double* rj = P.panels + j * kPanelDoubles;
     const float dx = (float)(x[0] - rj[0]), dy = (float)(x[1] - rj[1]), dz = (float)(x[2] - rj[2]);
-    const float lim = 2.0f * (float)rj[7];
-    if (dx * dx + dy * dy + dz * dz < lim * lim)
+    const float lim = 2.0f * (float)rj[7], d2 = dx * dx + dy * dy + dz * dz;
+    if (!(d2 >= lim * lim && d2 > kAngleMin2 && d2 < kAngleMax2))
       om += solid_angle(P.verts + j * kVertDoubles, x);
     else
       omf += solid_angle_f(P.verts + j * kVertDoubles, x);
