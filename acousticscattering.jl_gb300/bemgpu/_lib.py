@@ -174,6 +174,8 @@ SIGNATURES = {
     "bemgpu_schwarz_neighbourhoods": (ctypes.c_int, [_dp, _i64, _i64p, _i64, _i32,
                                                      ctypes.POINTER(ctypes.c_int32)]),
     "bemgpu_ctx_graph_stats": (ctypes.c_int, [_vp, _i64p, _i64p]),
+    "bemgpu_debug_panel": (ctypes.c_int, [_vp, _i64, _i32, _i32, _i32, _dp,
+                                          ctypes.POINTER(ctypes.c_int32)]),
     "bemgpu_debug_cgemm": (ctypes.c_int, [_vp, _i64, _i64, _i32,
                                           ctypes.POINTER(ctypes.c_float),
                                           ctypes.POINTER(ctypes.c_float),

@@ -156,6 +156,17 @@ class Context:
         """Complex64 LU trailing updates on the tensor cores (default) or CUDA cores."""
         _check(C.lib().bemgpu_ctx_set_tensor_lu(self.handle, int(enable)), self.handle)
 
+    def debug_panel(self, A, precision="double", cluster=0, streaming=False):
+        """Factors and row interchanges of an n x 32 LU panel with the given launch shape
+        (testing hook)."""
+        out = np.asfortranarray(np.array(A, dtype=np.complex128))
+        piv = np.zeros(32, dtype=np.int32)
+        _check(C.lib().bemgpu_debug_panel(
+            self.handle, out.shape[0], C.MIXED if precision == "mixed" else C.DOUBLE, int(cluster),
+            int(streaming), C.dptr(out), piv.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))),
+            self.handle)
+        return out, piv
+
     def debug_cgemm(self, A, B, C_):
         """C - A B through the split-BF16 tensor-core update (complex64 testing hook)."""
         A = np.asfortranarray(A, dtype=np.complex64)

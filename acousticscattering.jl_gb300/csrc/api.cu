@@ -5520,6 +5520,51 @@ int bemgpu_ctx_set_tensor_lu(bemgpu_ctx* c, int32_t enable) {
   return BEMGPU_OK;
 }
 
+int bemgpu_debug_panel(bemgpu_ctx* c, int64_t n, int32_t precision, int32_t cluster,
+                       int32_t streaming, double* A, int32_t* pivots) {
+  if (!c || !A || !pivots || n < kPanelNB || n >= INT32_MAX ||
+      (precision != BEMGPU_MIXED && precision != BEMGPU_DOUBLE) ||
+      !(cluster == 0 || cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8 ||
+        cluster == 16))
+    return fail(c, BEMGPU_EINVAL, "invalid arguments");
+  std::lock_guard<std::recursive_mutex> lk(c->mu);
+  cudaSetDevice(c->device);
+  const bool single = precision == BEMGPU_MIXED;
+  const size_t count = (size_t)n * kPanelNB * 2;  // reals
+  std::vector<float> a32;
+  if (single) a32.assign(A, A + count);
+  Buf dA, dpiv, dinfo, d;
+  TRY(alloc(c, count * (single ? 4 : 8), &dA));
+  TRY(alloc(c, kPanelNB * 4, &dpiv));
+  TRY(alloc(c, 4, &dinfo));
+  CUDA_TRY(c, cudaMemcpyAsync(dA.p, single ? (const void*)a32.data() : (const void*)A,
+                              count * (single ? 4 : 8), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(c, cudaMemsetAsync(dinfo.p, 0, 4, c->stream));
+  MatInst m{};
+  m.a = dA.p;
+  m.n = n;
+  m.lda = n;
+  m.ipiv = dpiv.as<int32_t>();
+  m.info = dinfo.as<int32_t>();
+  m.active = 1;
+  TRY(to_device(c, std::vector<MatInst>{m}, &d));
+  const Launch L = c->launch();
+  PanelShape shape;
+  shape.cluster = cluster;
+  shape.streaming = streaming != 0;
+  const int prec = single ? 1 : 0;
+  if (!launch_getf2(L, d.as<MatInst>(), 1, 1, n, 0, kPanelNB, prec, shape))
+    launch_laswp(L, d.as<MatInst>(), 1, 0, kPanelNB, 0, kPanelNB, 0, 0, prec);
+  CUDA_TRY(c, cudaGetLastError());
+  CUDA_TRY(c, cudaMemcpyAsync(single ? (void*)a32.data() : (void*)A, dA.p,
+                              count * (single ? 4 : 8), cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaMemcpyAsync(pivots, dpiv.p, kPanelNB * 4, cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  TRY(check_device_error(c));
+  if (single) std::copy(a32.begin(), a32.end(), A);
+  return BEMGPU_OK;
+}
+
 int bemgpu_debug_cgemm(bemgpu_ctx* c, int64_t m, int64_t n, int32_t k, const float* A,
                        const float* B, float* C) {
   if (!c || !A || !B || !C || m <= 0 || n <= 0 || k <= 0)

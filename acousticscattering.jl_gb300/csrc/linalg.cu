@@ -14,6 +14,7 @@
 //           uses the tensor-core kernel in gemm_tc.cu instead).
 // The triangular solves are in trsv.cu.
 #include <cfloat>
+#include <climits>
 #include <cstdio>
 
 #include "bemgpu_internal.h"
@@ -52,17 +53,18 @@ __device__ __forceinline__ cx<R> cinv(cx<R> a) {
   R d = (ar * ar + ai * ai) * s;
   return {ar / d, -ai / d};
 }
-// ------------------------------------------------------------------ getf2, left-looking
-// Complex64 panel factorisation for the LU driver: column c is brought up to date only
+// ------------------------------------------------------------------ getf2, streaming
+// The panel factorisation for more rows than k_getf2_reg below holds: the panel stays in global
+// memory (L2).  Column c is brought up to date only
 // when it is reached (U[0:c, c] by one warp from the finished L11 rows cached in shared
 // memory, then a[r, c] -= sum_j L[r, j] u_j for the rows below), and the pivot search is
 // fused into that pass, as is the scaling of column c - 1 by its pivot's reciprocal.
-// Each row of the panel is read about c + 2 times at column c instead of the
-// right-looking 2 (31 - c) + 1, and a cluster of CS CTAs shares an instance's rows
-// (fixed ownership: row k0 + g + t CS T belongs to cluster thread g), exchanging
-// the pivot candidates through distributed shared memory.  Two cluster barriers per
-// column order the global writes of one CTA before the reads of the other.  Pivoting
-// rule, interchanges and the singular marker are those of the right-looking kernel.
+// A cluster of CTAs shares an instance's rows (fixed ownership: row k0 + g + t CS T belongs to
+// cluster thread g), exchanging the pivot candidates through distributed shared memory.  Two
+// cluster barriers per column order the global writes of one CTA before the reads of the other.
+// Every entry takes the operations of k_getf2_reg in the same order, so both give the same
+// factor.
+constexpr int kRegMaxCS = 16;   // CTAs per cluster at most
 constexpr int kGetf2T = 1024;
 constexpr int kLLBatch = 16;  // L values per row in flight
 
@@ -116,25 +118,44 @@ __device__ __forceinline__ R ld_peer_real(uint32_t a) {
   else
     return ld_peer_f32(a);
 }
-__device__ __forceinline__ long long ld_peer_s64(uint32_t a) {
-  long long v;
-  asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
-  return v;
+__device__ __forceinline__ unsigned cluster_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
 }
-
-__device__ __forceinline__ void better(float& bv, int64_t& bi, float ov, int64_t oi) {
-  if (ov > bv || (ov == bv && oi < bi)) {
-    bv = ov;
-    bi = oi;
-  }
+// x -= a b and a b, the one form every panel kernel uses
+__device__ __forceinline__ void cfnma(cx<float>& x, cx<float> a, cx<float> b) {
+  x.x = __fmaf_rn(a.y, b.y, __fmaf_rn(-a.x, b.x, x.x));
+  x.y = __fmaf_rn(-a.y, b.x, __fmaf_rn(-a.x, b.y, x.y));
 }
+__device__ __forceinline__ void cfnma(cx<double>& x, cx<double> a, cx<double> b) {
+  x.x = __fma_rn(a.y, b.y, __fma_rn(-a.x, b.x, x.x));
+  x.y = __fma_rn(-a.y, b.x, __fma_rn(-a.x, b.y, x.y));
+}
+__device__ __forceinline__ cx<float> cmul(cx<float> a, cx<float> b) {
+  return {__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x))};
+}
+__device__ __forceinline__ cx<double> cmul(cx<double> a, cx<double> b) {
+  return {__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x))};
+}
+// reciprocal with one division: scaled by a power of two so that the squares neither
+// overflow nor vanish
+__device__ __forceinline__ cx<double> cinv_fast(cx<double> a) {
+  const int e = (max(__double2hiint(a.x) & 0x7FFFFFFF, __double2hiint(a.y) & 0x7FFFFFFF)) >> 20;
+  if (e < 2 || e > 2044) return cinv(a);
+  const double sc = __hiloint2double((2046 - e) << 20, 0);
+  const double x = a.x * sc, y = a.y * sc;
+  const double q = sc / (x * x + y * y);
+  return {x * q, -y * q};
+}
+__device__ __forceinline__ cx<float> cinv_fast(cx<float> a) { return cinv(a); }
 
-template <typename R, int CS, int T, int BATCH>
+template <typename R, int T, int BATCH>
 __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ insts, int64_t k0,
                                                 int nb) {
   using C = cx<R>;
-  const unsigned rank = CS > 1 ? cluster_rank() : 0u;
-  const MatInst& M = insts[blockIdx.x / CS];
+  const unsigned rank = cluster_rank(), cs = cluster_size();
+  const MatInst& M = insts[blockIdx.x / cs];
   const int64_t n = M.n;
   if (!M.active || k0 >= n) return;  // the whole cluster (one instance) leaves together
   const int nbe = (int)min((int64_t)nb, n - k0);
@@ -149,7 +170,7 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
   __shared__ C s_inv;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int64_t g = (int64_t)rank * T + tid;
-  constexpr int64_t stride = (int64_t)CS * T;
+  const int64_t stride = (int64_t)cs * T;
   C inv_prev = {(R)1, (R)0};
   for (int c = 0; c < nbe; ++c) {
     const int64_t col = k0 + c;
@@ -161,7 +182,7 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
         C ui;
         ui.x = __shfl_sync(0xffffffffu, x.x, i);
         ui.y = __shfl_sync(0xffffffffu, x.y, i);
-        if (lane > i && lane < c) x -= sL[lane][i] * ui;
+        if (lane > i && lane < c) cfnma(x, sL[lane][i], ui);
       }
       if (lane < c) su[lane] = x;  // stored after the first cluster barrier (peers read
                                    // the original values of these rows first)
@@ -185,10 +206,10 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
         for (int e = 0; e < BATCH; ++e) {
           if (j0 + e < c) {
             if (j0 + e == c - 1) {
-              lv[e] = lv[e] * inv_prev;
+              lv[e] = cmul(lv[e], inv_prev);
               st<R>(A, r + (k0 + j0 + e) * lda, lv[e]);
             }
-            acc -= lv[e] * su[j0 + e];
+            cfnma(acc, lv[e], su[j0 + e]);
           }
         }
       }
@@ -222,15 +243,12 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
     }
     // (3) pivot of the cluster: only warp 0 needs it (the U row, the interchange over the
     // panel's <= 32 columns, the singular marker and the pivot's reciprocal are its work)
-    if (CS > 1)
-      cluster_sync_all();
-    else
-      __syncthreads();
+    cluster_sync_all();
     R pv = (R)-1;
     int32_t piv32 = INT32_MAX;
     if (wid == 0) {  // one lane per CTA of the cluster, all peer loads in flight
-      if (lane < CS) {
-        if (CS > 1 && (unsigned)lane != rank) {
+      if (lane < (int)cs) {
+        if ((unsigned)lane != rank) {
           pv = ld_peer_real<R>(peer_smem(&c_val, (unsigned)lane));
           piv32 = ld_peer_s32(peer_smem(&c_idx, (unsigned)lane));
         } else {
@@ -261,13 +279,10 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
         st<R>(A, piv + cc * lda, a);
       }
     }
-    if (CS > 1)
-      cluster_sync_all();
-    else
-      __syncthreads();
+    cluster_sync_all();
     // (4) reciprocal of the pivot; cache the finished row of L11
     if (tid < c) sL[c][tid] = ld<R>(A, col + (k0 + tid) * lda);
-    if (tid == 0) s_inv = nonzero ? cinv(ld<R>(A, col + col * lda)) : C{(R)1, (R)0};
+    if (tid == 0) s_inv = nonzero ? cinv_fast(ld<R>(A, col + col * lda)) : C{(R)1, (R)0};
     __syncthreads();
     inv_prev = s_inv;
   }
@@ -275,7 +290,7 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
   const int64_t colL = k0 + nbe - 1;
   int64_t r = k0 + g;
   if (r <= colL) r += ((colL + 1 - r + stride - 1) / stride) * stride;
-  for (; r < n; r += stride) st<R>(A, r + colL * lda, ld<R>(A, r + colL * lda) * inv_prev);
+  for (; r < n; r += stride) st<R>(A, r + colL * lda, cmul(ld<R>(A, r + colL * lda), inv_prev));
 }
 
 // ------------------------------------------------------------------ getf2, in registers
@@ -294,36 +309,9 @@ __global__ void __launch_bounds__(T) k_getf2_ll(const MatInst* __restrict__ inst
 // on the batch.  Measured, one instance of 8960 unknowns, complex64: 7.0 us a column with the
 // streaming kernel above, see the launcher for this one's; complex128 (FP64 issue: two FMAs
 // per clock and SM beside the latency) of 5760 unknowns: 27 us a column before.
-constexpr int kRegMaxCS = 16;   // CTAs per cluster at most
-__device__ __forceinline__ unsigned cluster_size() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ void st_peer_b32(uint32_t a, uint32_t v) {
   asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
-// x -= a b, the one form every kernel path of the panel uses
-__device__ __forceinline__ void cfnma(cx<float>& x, cx<float> a, cx<float> b) {
-  x.x = __fmaf_rn(a.y, b.y, __fmaf_rn(-a.x, b.x, x.x));
-  x.y = __fmaf_rn(-a.y, b.x, __fmaf_rn(-a.x, b.y, x.y));
-}
-__device__ __forceinline__ void cfnma(cx<double>& x, cx<double> a, cx<double> b) {
-  x.x = __fma_rn(a.y, b.y, __fma_rn(-a.x, b.x, x.x));
-  x.y = __fma_rn(-a.y, b.x, __fma_rn(-a.x, b.y, x.y));
-}
-// reciprocal with one division: scaled by a power of two so that the squares neither
-// overflow nor vanish
-__device__ __forceinline__ cx<double> cinv_fast(cx<double> a) {
-  const int e = (max(__double2hiint(a.x) & 0x7FFFFFFF, __double2hiint(a.y) & 0x7FFFFFFF)) >> 20;
-  if (e < 2 || e > 2044) return cinv(a);
-  const double sc = __hiloint2double((2046 - e) << 20, 0);
-  const double x = a.x * sc, y = a.y * sc;
-  const double q = sc / (x * x + y * y);
-  return {x * q, -y * q};
-}
-__device__ __forceinline__ cx<float> cinv_fast(cx<float> a) { return cinv(a); }
-
 // Ordered key of a pivot candidate: |re| + |im| as bits, 0 for a NaN (never a candidate).
 struct PivKey {
   uint32_t hi, lo;   // value bits (lo: 0 for complex64)
@@ -549,7 +537,7 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
               pos[t] = col;
             } else {
               if (pos[t] == col) pos[t] = piv;
-              const C l = a[t][w] * inv;
+              const C l = cmul(a[t][w], inv);
               a[t][w] = l;
 #pragma unroll
               for (int q = w + 1; q < W; ++q) {
@@ -1049,6 +1037,16 @@ static void cluster_launch(const Launch& L, K kernel, int ninst, int cs, int thr
   count_launch(1);
 }
 
+template <typename R>
+static void getf2_ll_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int cs) {
+  auto kernel = k_getf2_ll<R, LLCfg<R>::kT, LLCfg<R>::kBatch>;
+  static PerDeviceOnce attr;
+  attr.call([&] {  // clusters of 16 are beyond the portable size
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  cluster_launch(L, kernel, ninst, cs, LLCfg<R>::kT, d, k0, nb);
+}
+
 template <typename R, int W, int RPT, int T = 512>
 static void getf2_reg_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int cs,
                         int threads, int share) {
@@ -1085,32 +1083,31 @@ static int panel_cluster(int nact, int64_t rows, bool single) {
   return best;
 }
 
-// Columns in registers: as many as the rows per thread leave room for.
+// Columns in registers: as many as the rows per thread leave room for.  The streaming kernel takes
+// one complex64 system beyond 81920 rows, one complex128 system beyond 40960.
 bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_t nmax, int64_t k0,
-                  int nb, int prec) {
+                  int nb, int prec, const PanelShape& shape) {
   const bool single = prec_is_single(prec);
   const int64_t rows = nmax - k0;
-  const int cs = panel_cluster(std::max(1, nact), rows, single);
+  const int cs = shape.cluster > 0 ? shape.cluster : panel_cluster(std::max(1, nact), rows, single);
   const int share = (int)(((rows + cs - 1) / cs + 31) / 32 * 32);  // rows per CTA
   // complex128: at least eight warps, which solve the U rows of a sub-panel's columns
   const int threads =
       std::min(512, std::max(single ? 64 : 256, share));
-  const int q = (share + threads - 1) / threads;  // rows per thread
+  const int q = shape.streaming ? INT_MAX : (share + threads - 1) / threads;  // rows per thread
   if (single) {
     if (q <= 1) return getf2_reg_t<float, 16, 1>(L, d, ninst, k0, nb, cs, threads, share), false;
     if (q <= 2) return getf2_reg_t<float, 16, 2>(L, d, ninst, k0, nb, cs, threads, share), false;
     if (q <= 5) return getf2_reg_t<float, 8, 5>(L, d, ninst, k0, nb, cs, threads, share), false;
     if (q <= 10) return getf2_reg_t<float, 4, 10>(L, d, ninst, k0, nb, cs, threads, share), false;
-    cluster_launch(L, k_getf2_ll<float, 2, LLCfg<float>::kT, LLCfg<float>::kBatch>, ninst, 2,
-                   LLCfg<float>::kT, d, k0, nb);
+    getf2_ll_t<float>(L, d, ninst, k0, nb, cs);
   } else {
     if (threads <= 256 && q <= 1)
       return getf2_reg_t<double, 16, 1, 256>(L, d, ninst, k0, nb, cs, threads, share), false;
     if (q <= 1) return getf2_reg_t<double, 8, 1>(L, d, ninst, k0, nb, cs, threads, share), false;
     if (q <= 2) return getf2_reg_t<double, 8, 2>(L, d, ninst, k0, nb, cs, threads, share), false;
     if (q <= 5) return getf2_reg_t<double, 4, 5>(L, d, ninst, k0, nb, cs, threads, share), false;
-    cluster_launch(L, k_getf2_ll<double, 2, LLCfg<double>::kT, LLCfg<double>::kBatch>, ninst, 2,
-                   LLCfg<double>::kT, d, k0, nb);
+    getf2_ll_t<double>(L, d, ninst, k0, nb, cs);
   }
   return true;
 }

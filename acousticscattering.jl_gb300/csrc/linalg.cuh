@@ -11,8 +11,13 @@ constexpr int kPanelNB = 32;  // LU panel width (columns factored per getf2 laun
 // Factors the panel [k0, k0 + nb) of every instance; nmax: largest order, nact: instances
 // with rows left (the launch shape; the factor does not depend on it).  Returns whether the
 // interchanges were applied to the panel's own columns (if not, they are the caller's).
+// shape: a launch shape other than the one chosen by size (bemgpu_debug_panel).
+struct PanelShape {
+  int cluster = 0;         // CTAs per instance, a power of two up to 16 (0: by size)
+  bool streaming = false;  // the kernel that keeps the panel in global memory
+};
 bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_t nmax, int64_t k0,
-                  int nb, int prec);
+                  int nb, int prec, const PanelShape& shape = {});
 // row interchanges k0 .. k0 + nb - 1 on columns [c_lo, c_hi) \ [s_lo, s_hi)
 void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int64_t c_lo,
                   int64_t c_hi, int64_t s_lo, int64_t s_hi, int prec);

@@ -530,6 +530,16 @@ int bemgpu_ctx_graph_stats(const bemgpu_ctx *ctx, int64_t *captures, int64_t *re
 int bemgpu_ctx_set_tensor_lu(bemgpu_ctx *ctx, int32_t enable);
 
 /*
+ * LU panel of the first 32 columns of a matrix of order n (A: n x 32 complex128, column-major;
+ * rounded to complex64 with BEMGPU_MIXED): A receives the factors, pivots the 32 row
+ * interchanges.  cluster: thread blocks that share the panel (1, 2, 4, 8 or 16; 0 chosen by
+ * size), streaming: 1 keeps the panel in memory whatever its size.  Every choice gives the same
+ * bits (testing hook).
+ */
+int bemgpu_debug_panel(bemgpu_ctx *ctx, int64_t n, int32_t precision, int32_t cluster,
+                       int32_t streaming, double *A, int32_t *pivots);
+
+/*
  * C -= A B for complex64 column-major A (m x k), B (k x n), C (m x n) through the
  * tensor-core update used by the mixed-precision LU (testing hook).
  */
