@@ -120,8 +120,8 @@ class Context:
         _check(C.lib().bemgpu_ctx_synchronize(self.handle), self.handle)
 
     def set_autotune(self, enable: bool = True):
-        """Measured launch shapes (panel cluster size, residual CTA size); every
-        choice gives bit-identical results."""
+        """Measured launch shapes (residual CTA size); every choice gives bit-identical
+        results."""
         _check(C.lib().bemgpu_ctx_set_autotune(self.handle, int(enable)), self.handle)
 
     def profile(self, enable: bool = True):

@@ -53,7 +53,7 @@ void bemgpu_set_process_error(const char* msg) { g_err = msg ? msg : ""; }
 }  // namespace bemgpu
 
 // ===================================================================== context + memory
-constexpr int kEventPool = 512;  // ordering events of the two-stream triangular solves
+constexpr int kEventPool = 2;  // ordering events of the two-stream cross approximation
 
 struct bemgpu_ctx {
   int device = 0;
@@ -94,8 +94,8 @@ struct bemgpu_ctx {
   int64_t lu_captures = 0, lu_replays = 0;
 
   std::recursive_mutex mu;
-  cudaStream_t side = nullptr;           // look-ahead stream of the triangular solves
-  std::vector<cudaEvent_t> evpool;       // their ordering events
+  cudaStream_t side = nullptr;           // second stream of the cross approximation
+  std::vector<cudaEvent_t> evpool;       // its ordering events
   Launch launch() const {
     return Launch{stream, d_err, side, const_cast<cudaEvent_t*>(evpool.data()),
                   (int)evpool.size()};
@@ -263,8 +263,8 @@ cudaError_t init_streams(bemgpu_ctx* c) {
     return e;
   }
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-  // look-ahead stream and events of the blocked triangular solves (optional: without them
-  // the solves run on the main stream alone)
+  // second stream and events of the cross approximation (optional: without them its large
+  // blocks run on the main stream after the others)
   if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) == cudaSuccess) {
     c->evpool.resize(kEventPool, nullptr);
     for (auto& ev : c->evpool)
@@ -425,7 +425,8 @@ int try_alloc(bemgpu_ctx* c, size_t bytes, Buf* out, bool* got) {
   const cudaError_t last = c->last_cuda;
   const int s = alloc(c, bytes, out);
   *got = s == BEMGPU_OK;
-  if (s == BEMGPU_ENOMEM_BUDGET || (s == BEMGPU_ECUDA && c->last_cuda == cudaErrorMemoryAllocation)) {
+  if (s == BEMGPU_ENOMEM_BUDGET ||
+      (s == BEMGPU_ECUDA && c->last_cuda == cudaErrorMemoryAllocation)) {
     c->err = err;
     c->last_cuda = last;
     return BEMGPU_OK;
@@ -830,8 +831,8 @@ struct FactorData {
   int32_t* info_ptr() const { return single ? info.as<int32_t>() : (mixed ? info64.as<int32_t>() : info.as<int32_t>()); }
   int32_t* perm_ptr() const { return single ? perm.as<int32_t>() : (mixed ? perm64.as<int32_t>() : perm.as<int32_t>()); }
   size_t bytes() const {
-    return A.bytes + dinv.bytes + dnear.bytes + dnear_rhs.bytes + Mrhs.bytes + LU.bytes + LU64.bytes + ipiv.bytes +
-           ipiv64.bytes + rows.bytes + cols.bytes + rowsum.bytes;
+    return A.bytes + dinv.bytes + dnear.bytes + dnear_rhs.bytes + Mrhs.bytes + LU.bytes +
+           LU64.bytes + ipiv.bytes + ipiv64.bytes + rows.bytes + cols.bytes + rowsum.bytes;
   }
 };
 }  // namespace
@@ -1587,7 +1588,7 @@ int getrf_tc(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<MatI
       }
       {
         Prof pr(c, "trsm");
-        launch_trsm_panel(L, dm, ni, k0, kPanelNB, k0 + kPanelNB, H + HB, 1);
+        launch_trsm_panel(L, dm, ni, k0, k0 + kPanelNB, H + HB, 1);
       }
       const int q = (int)((k0 - H) / kPanelNB);
       if (q < kInner) {
@@ -1719,7 +1720,8 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
   CUDA_TRY(c, cudaMemsetAsync(kexp.p, 0, count * B * 4, c->stream));
   std::vector<OzPackInst> pa(count), pb(count);
   std::vector<OzGemmInst> ge(count);
-  std::vector<int64_t> tiles(count), ra((size_t)blocks * kPhases, 0), rb((size_t)blocks * kPhases, 0);
+  std::vector<int64_t> tiles(count);
+  std::vector<int64_t> ra((size_t)blocks * kPhases, 0), rb((size_t)blocks * kPhases, 0);
   for (int64_t b = 0; b < blocks; ++b)
     for (int ph = 0; ph < kPhases; ++ph)
       for (int t = 0; t < ni; ++t) {
@@ -1786,7 +1788,7 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
       if (q == kInner) break;
       {
         Prof pr(c, "trsm");
-        launch_trsm_panel(L, dm, ni, k0, kPanelNB, k0 + kPanelNB, K1, 0);
+        launch_trsm_panel(L, dm, ni, k0, k0 + kPanelNB, K1, 0);
       }
       update(b, q);
     }
@@ -1849,7 +1851,7 @@ int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool prom
       }
       {
         Prof pr(c, "trsm");
-        launch_trsm_panel(L, dm, ni, k0, kPanelNB, k0 + kPanelNB, nmax, prec);
+        launch_trsm_panel(L, dm, ni, k0, k0 + kPanelNB, nmax, prec);
       }
       {
         Prof pr(c, prec ? "gemm_c64" : "gemm_c128");
@@ -2349,7 +2351,9 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode, bool* done) {
   Buf xp, xe, ap, ae, ke, found, list, xa;
   const int32_t cap = wide_cap(n, R);
   bool got = true;
-  auto scratch = [&](size_t bytes, Buf* b) { return got ? try_alloc(c, bytes, b, &got) : BEMGPU_OK; };
+  auto scratch = [&](size_t bytes, Buf* b) {
+    return got ? try_alloc(c, bytes, b, &got) : BEMGPU_OK;
+  };
   TRY(scratch(oz_pack_bytes(R, (int)n, kOzB), &xp));
   TRY(scratch((size_t)kb * oz_exps(R, kOzB) * 4, &xe));
   TRY(scratch((size_t)n * 4, &ke));
@@ -2360,7 +2364,8 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode, bool* done) {
   // row panels: at most a quarter of what the budget leaves
   const size_t tile = oz_pack_bytes(128, (int)n, kOzA);
   const uint64_t used = total_live(c), budget = root_of(c)->budget;
-  const uint64_t room = std::min<uint64_t>(wide_panel_bytes(n), budget > used ? (budget - used) / 4 : 0);
+  const uint64_t room =
+      std::min<uint64_t>(wide_panel_bytes(n), budget > used ? (budget - used) / 4 : 0);
   int64_t tiles = std::max<int64_t>(1, (int64_t)(room / tile));
   for (;; tiles = (tiles + 1) / 2) {
     got = true;
@@ -2393,7 +2398,8 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode, bool* done) {
     CUDA_TRY(c, cudaMemcpy2DAsync(v.y, (size_t)v.ldy * 16, v.b, (size_t)v.ldb * 16, (size_t)n * 16,
                                   (size_t)R, cudaMemcpyDeviceToDevice, c->stream));
   } else {
-    CUDA_TRY(c, cudaMemset2DAsync(v.y, (size_t)v.ldy * 16, 0, (size_t)n * 16, (size_t)R, c->stream));
+    CUDA_TRY(c, cudaMemset2DAsync(v.y, (size_t)v.ldy * 16, 0, (size_t)n * 16, (size_t)R,
+                                  c->stream));
   }
   CUDA_TRY(c, cudaMemsetAsync(found.p, 0, 4, c->stream));
   launch_wide_abs(L, v, xa.as<float>(), mode);
@@ -4099,8 +4105,8 @@ int hm_build(bemgpu_ctx* c, MeshData* m, const bemgpu_problem& p, int kind,
   for (int op = 0; op < 2; ++op) TRY(upload(c, keep[op], &H->lr[op]));
   {
     Prof pr(c, "hm_dense");
-    launch_hm_dense(L, H->dn.as<HmDense>(), d_dei.as<HmItem>(), (int32_t)dei.size(), H->D1.p, H->D2.p, recs, H->f32,
-                    H->pc->perm.as<int32_t>(), kind, k, a_re, a_im);
+    launch_hm_dense(L, H->dn.as<HmDense>(), d_dei.as<HmItem>(), (int32_t)dei.size(), H->D1.p,
+                    H->D2.p, recs, H->f32, H->pc->perm.as<int32_t>(), kind, k, a_re, a_im);
   }
   // near pairs (the mesh's list, same order) into their full leaf blocks
   if (m->n_near > 0) {

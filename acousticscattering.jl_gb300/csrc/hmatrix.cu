@@ -362,22 +362,26 @@ __global__ void __launch_bounds__(256) k_hm_dense(const HmDense* __restrict__ dn
 }
 
 void launch_hm_dense(const Launch& L, const HmDense* dn, const HmItem* items, int32_t n_items,
-                     void* D1, void* D2, const void* recs, bool f32, const int32_t* perm, int kind, double k,
-                     double a_re, double a_im) {
+                     void* D1, void* D2, const void* recs, bool f32, const int32_t* perm, int kind,
+                     double k, double a_re, double a_im) {
   if (n_items <= 0) return;
   const unsigned g = (unsigned)n_items;
   const float* rf = static_cast<const float*>(recs);
   const double* rd = static_cast<const double*>(recs);
   if (f32) {
     if (kind == kAsmBM)
-      k_hm_dense<float, kAsmBM><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rf, perm, k, a_re, a_im);
+      k_hm_dense<float, kAsmBM>
+          <<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rf, perm, k, a_re, a_im);
     else
-      k_hm_dense<float, kAsmCBIE><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rf, perm, k, a_re, a_im);
+      k_hm_dense<float, kAsmCBIE>
+          <<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rf, perm, k, a_re, a_im);
   } else {
     if (kind == kAsmBM)
-      k_hm_dense<double, kAsmBM><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rd, perm, k, a_re, a_im);
+      k_hm_dense<double, kAsmBM>
+          <<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rd, perm, k, a_re, a_im);
     else
-      k_hm_dense<double, kAsmCBIE><<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rd, perm, k, a_re, a_im);
+      k_hm_dense<double, kAsmCBIE>
+          <<<g, 256, 0, L.stream>>>(dn, items, D1, D2, rd, perm, k, a_re, a_im);
   }
   count_launch(1);
 }
@@ -405,8 +409,8 @@ __device__ __forceinline__ bool group_on(const GmState* st, int r0, int rb, int 
 constexpr int kVtU = 4, kVtN = 3;  // coefficients per warp and values per lane in flight
 template <typename R, int RB>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 && RB == 1 ? 5 : 1)
-    k_hm_vt(HmOp A, const void* __restrict__ X, int64_t ldx, int32_t nr, const GmState* st, int mode,
-            const int32_t* jptr, int64_t jstride) {
+    k_hm_vt(HmOp A, const void* __restrict__ X, int64_t ldx, int32_t nr, const GmState* st,
+            int mode, const int32_t* jptr, int64_t jstride) {
   using C = cx<R>;
   const int r0 = blockIdx.y * RB;
   const bool group = group_on(st, r0, RB, nr, mode);  // tested once the other loads are under way
@@ -563,7 +567,8 @@ __global__ void __launch_bounds__(kLeafRows * kLeafSlices, sizeof(R) == 4 && RB 
     __syncthreads();
     if (ch < kLeafSlices) {
 #pragma unroll
-      for (int q = 0; q < RB; ++q) a[q] = part[q][threadIdx.x] + part[q][threadIdx.x + 4 * kHmWideRows];
+      for (int q = 0; q < RB; ++q)
+        a[q] = part[q][threadIdx.x] + part[q][threadIdx.x + 4 * kHmWideRows];
     }
     __syncthreads();
 #pragma unroll

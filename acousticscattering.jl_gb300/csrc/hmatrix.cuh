@@ -123,8 +123,8 @@ void launch_hm_compact(const Launch& L, const HmCopy* d, int32_t count, const vo
 // entries each.
 constexpr int kHmDenseChunk = 1024;
 void launch_hm_dense(const Launch& L, const HmDense* dn, const HmItem* items, int32_t n_items,
-                     void* D1, void* D2, const void* recs, bool f32, const int32_t* perm, int kind, double k,
-                     double a_re, double a_im);
+                     void* D1, void* D2, const void* recs, bool f32, const int32_t* perm, int kind,
+                     double k, double a_re, double a_im);
 // Y[:, r] = sb B[:, r] + sa (A X)[:, r] for every right-hand side r < nr with
 // (act == null or act[r].active), the operands in permuted order.
 // jptr (optional): X is offset by (*jptr) * jstride complex entries, read on the device

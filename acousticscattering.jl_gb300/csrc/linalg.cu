@@ -387,7 +387,8 @@ __global__ void __launch_bounds__(T_) k_getf2_reg(const MatInst* __restrict__ in
   using C = cx<R>;
   // Columns whose code is unrolled.  All 16 of a sub-panel are 80 KB of instructions that run twice
   // in a launch: a quarter of the cycles waited for them.  Four at a time: 61 to 53 us a panel of
-  // a factorisation of 1280 unknowns on average.  With more than two rows per thread the registers that take turns cost more.
+  // a factorisation of 1280 unknowns on average.  With more than two rows per thread the registers
+  // that take turns cost more.
   constexpr int kU = RPT > 2 || W <= 4 ? W : 4;
   const unsigned rank = cluster_rank(), cs = cluster_size();
   const MatInst& M = insts[blockIdx.x / cs];
@@ -670,62 +671,43 @@ __global__ void __launch_bounds__(kSwpWarps * 32) k_laswp(const MatInst* __restr
 // ------------------------------------------------------------------ trsm (U12)
 // U12 = L11^{-1} A12 for the columns [c_lo, min(c_hi, n)); L11 = unit lower nbe x nbe
 // block at (k0, k0), staged once per CTA in shared memory; each warp solves per_warp columns
-// (column = warp + kTrsmWarps * t), lane r holding rows r, r + 32, ...
-// The columns are the at most 96 to the right of a 32-column panel inside a 128-column block.
+// (column = warp + kTrsmWarps * t), lane r holding row r.  The columns are the at most 96 to the
+// right of a 32-column panel inside a 128-column block (all of them without the tensor cores).
 // A warp takes per_warp of them, one after the other (32 dependent steps each): few for one
 // system, where 16 made one CTA do all the work (8 us a launch, 2 us with two), 16 in a large
 // batch, whose CTAs then stage the block once (see the launcher).
 constexpr int kTrsmWarps = 8;
-template <typename R, int NB>
+template <typename R>
 __global__ void __launch_bounds__(kTrsmWarps * 32) k_trsm_panel(const MatInst* __restrict__ insts,
                                                                int64_t k0, int64_t c_lo,
                                                                int64_t c_hi, int per_warp) {
   const MatInst& M = insts[blockIdx.y];
   const int64_t n = M.n;
   if (!M.active || k0 >= n) return;
-  const int nbe = (int)min((int64_t)NB, n - k0);
+  const int nbe = (int)min((int64_t)kPanelNB, n - k0);
   const int64_t lda = M.lda;
   const int64_t c_end = min(c_hi, n);
   const int64_t cta0 = c_lo + (int64_t)blockIdx.x * kTrsmWarps * per_warp;
   if (cta0 >= c_end) return;  // uniform per CTA
-  extern __shared__ __align__(16) unsigned char trsm_smem[];
-  cx<R>* sL = reinterpret_cast<cx<R>*>(trsm_smem);  // [NB][NB + 1]
+  static_assert(kPanelNB == 32, "a lane holds a row");
+  __shared__ cx<R> sL[kPanelNB][kPanelNB + 1];
   for (int t = threadIdx.x; t < nbe * nbe; t += blockDim.x) {
-    int r = t % nbe, c = t / nbe;
-    sL[r * (NB + 1) + c] = ld<R>(M.a, (k0 + r) + (k0 + c) * lda);
+    const int r = t % nbe, c = t / nbe;
+    sL[r][c] = ld<R>(M.a, (k0 + r) + (k0 + c) * lda);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int kPer = NB / 32;
   for (int tcol = 0; tcol < per_warp; ++tcol) {
     const int64_t j = cta0 + wid + (int64_t)kTrsmWarps * tcol;
     if (j >= c_end) break;
-    cx<R> x[kPer];
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      int r = lane + 32 * t;
-      x[t] = r < nbe ? ld<R>(M.a, (k0 + r) + j * lda) : cx<R>{0, 0};
+    cx<R> x = lane < nbe ? ld<R>(M.a, (k0 + lane) + j * lda) : cx<R>{0, 0};
+    for (int c = 0; c < nbe; ++c) {
+      cx<R> xc;
+      xc.x = __shfl_sync(0xffffffffu, x.x, c);
+      xc.y = __shfl_sync(0xffffffffu, x.y, c);
+      if (lane > c && lane < nbe) x -= sL[lane][c] * xc;
     }
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      for (int cl = 0; cl < 32; ++cl) {
-        const int c = 32 * t + cl;
-        if (c >= nbe) break;
-        cx<R> xc;
-        xc.x = __shfl_sync(0xffffffffu, x[t].x, cl);
-        xc.y = __shfl_sync(0xffffffffu, x[t].y, cl);
-#pragma unroll
-        for (int u = t; u < kPer; ++u) {
-          int r = lane + 32 * u;
-          if (r > c && r < nbe) x[u] -= sL[r * (NB + 1) + c] * xc;
-        }
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      int r = lane + 32 * t;
-      if (r < nbe) st<R>(M.a, (k0 + r) + j * lda, x[t]);
-    }
+    if (lane < nbe) st<R>(M.a, (k0 + lane) + j * lda, x);
   }
 }
 
@@ -802,15 +784,14 @@ __global__ void __launch_bounds__(kGThreads) k_gemm_update(const MatInst* __rest
 
 // ------------------------------------------------------------------ -(L11^{-1} - I)
 // For the tensor-core U12 solve: with L11^{-1} = I + N (N strictly lower),
-// U12 = L11^{-1} A12 = A12 - (-N) A12.  One CTA per instance stages the unit lower
-// block L11 (nbe x nbe at (k0, k0)) in shared memory and solves L11 x = e_j for every
-// column j (one warp per column); out (ld kLinvB, complex64) receives -N.
+// U12 = L11^{-1} A12 = A12 - (-N) A12.  Each CTA stages the unit lower block L11 (nbe x nbe at
+// (k0, k0)) in shared memory and solves L11 x = e_j for its columns j (one warp per column); out (ld kLinvB, complex64) receives -N.
 constexpr int kLinvB = 128;
 
 // gridDim.x CTAs per instance take the columns j = blockIdx.x + gridDim.x i (spread over the
 // triangle for balance), a warp one column after the other.  A launch for one instance took 68 us
-// with 32 CTAs whose loads waited for one another and takes 23 with 16; each CTA stages the block, so
-// a batch uses fewer (linv_ctas).
+// with 32 CTAs whose loads waited for one another and takes 23 with 16; each CTA stages the block,
+// so a batch uses fewer (linv_ctas).
 constexpr int kLinvWarps = 8;
 static int linv_ctas(int ninst) {
   int n = 16;
@@ -955,7 +936,8 @@ __global__ void __launch_bounds__(kLinvWarps * 32) k_linv_neg_c128(
     for (int t = 0; t < kPer; ++t) {
       const int r = lane + 32 * t;
       const bool strict = r > j && r < nbe && j < nbe;
-      out[r + (int64_t)j * kLinvB] = strict ? make_double2(-x[t].x, -x[t].y) : make_double2(0.0, 0.0);
+      out[r + (int64_t)j * kLinvB] =
+          strict ? make_double2(-x[t].x, -x[t].y) : make_double2(0.0, 0.0);
     }
   }
 }
@@ -1052,7 +1034,8 @@ static void getf2_reg_t(const Launch& L, const MatInst* d, int ninst, int64_t k0
                         int threads, int share) {
   static PerDeviceOnce attr;
   attr.call([] {  // clusters of 16 are beyond the portable size
-    cudaFuncSetAttribute(k_getf2_reg<R, W, RPT, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k_getf2_reg<R, W, RPT, T>,
+                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   });
   cluster_launch(L, k_getf2_reg<R, W, RPT, T>, ninst, cs, threads, d, k0, nb, share);
 }
@@ -1137,38 +1120,24 @@ void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int 
   }
 }
 
-template <typename R, int NB>
+template <typename R>
 static void trsm_t(const Launch& L, const MatInst* d, int ninst, int64_t k0, int64_t c_lo,
                    int64_t c_hi) {
-  const size_t smem = (size_t)NB * (NB + 1) * sizeof(cx<R>);
-  static PerDeviceOnce attr;
-  if (smem > 48 * 1024)
-    attr.call([&] {
-      cudaFuncSetAttribute(k_trsm_panel<R, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-    });
   // complex128 columns are FP64-bound: one per warp in a small batch
   const int per_warp = ninst >= 32 ? 16 : sizeof(R) == 4 ? 2 : 1;
   const int64_t per = (int64_t)kTrsmWarps * per_warp;
   dim3 grid((unsigned)((c_hi - c_lo + per - 1) / per), (unsigned)ninst);
-  k_trsm_panel<R, NB><<<grid, kTrsmWarps * 32, smem, L.stream>>>(d, k0, c_lo, c_hi, per_warp);
+  k_trsm_panel<R><<<grid, kTrsmWarps * 32, 0, L.stream>>>(d, k0, c_lo, c_hi, per_warp);
   count_launch(1);
 }
 
-void launch_trsm_panel(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb,
-                       int64_t c_lo, int64_t c_hi, int prec) {
+void launch_trsm_panel(const Launch& L, const MatInst* d, int ninst, int64_t k0, int64_t c_lo,
+                       int64_t c_hi, int prec) {
   if (c_hi <= c_lo) return;
-  if (nb <= 32) {
-    if (prec_is_single(prec))
-      trsm_t<float, 32>(L, d, ninst, k0, c_lo, c_hi);
-    else
-      trsm_t<double, 32>(L, d, ninst, k0, c_lo, c_hi);
-  } else {
-    if (prec_is_single(prec))
-      trsm_t<float, 128>(L, d, ninst, k0, c_lo, c_hi);
-    else
-      trsm_t<double, 128>(L, d, ninst, k0, c_lo, c_hi);
-  }
+  if (prec_is_single(prec))
+    trsm_t<float>(L, d, ninst, k0, c_lo, c_hi);
+  else
+    trsm_t<double>(L, d, ninst, k0, c_lo, c_hi);
 }
 
 void launch_gemm_update(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb,

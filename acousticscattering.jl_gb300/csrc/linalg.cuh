@@ -21,9 +21,9 @@ bool launch_getf2(const Launch& L, const MatInst* d, int ninst, int nact, int64_
 // row interchanges k0 .. k0 + nb - 1 on columns [c_lo, c_hi) \ [s_lo, s_hi)
 void launch_laswp(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb, int64_t c_lo,
                   int64_t c_hi, int64_t s_lo, int64_t s_hi, int prec);
-// U12 = L11^{-1} A12 on columns [c_lo, c_hi); nb <= 32 or <= 128
-void launch_trsm_panel(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb,
-                       int64_t c_lo, int64_t c_hi, int prec);
+// U12 = L11^{-1} A12 of the panel at k0 on columns [c_lo, c_hi)
+void launch_trsm_panel(const Launch& L, const MatInst* d, int ninst, int64_t k0, int64_t c_lo,
+                       int64_t c_hi, int prec);
 // rows [k0 + nb, n) x columns [c_lo, c_hi) -= L21 U12 (SIMT)
 void launch_gemm_update(const Launch& L, const MatInst* d, int ninst, int64_t k0, int nb,
                         int64_t nmax, int64_t c_lo, int64_t c_hi, int prec);
@@ -44,7 +44,7 @@ void launch_linv_neg(const Launch& L, const MatInst* d, int ninst, int64_t k0, f
 // The same for complex128 factors.
 void launch_linv_neg_c128(const Launch& L, const MatInst* d, int ninst, int64_t k0,
                           double2* const* outs);
-// Row permutation of each factor from its pivots (one CTA per instance).
+// Row permutation of each factor from its pivots.
 void launch_make_perm(const Launch& L, const MatInst* d, int ninst, int64_t nmax);
 
 }  // namespace bemgpu

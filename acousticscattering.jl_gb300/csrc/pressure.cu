@@ -53,7 +53,8 @@ __device__ __forceinline__ float solid_angle_f(const double* v, const double* x)
   const float t[3] = {R[1][1] * R[2][2] - R[1][2] * R[2][1], R[1][2] * R[2][0] - R[1][0] * R[2][2],
                       R[1][0] * R[2][1] - R[1][1] * R[2][0]};
   const float num = dot(R[0], t);
-  const float den = r0 * r1 * r2 + dot(R[0], R[1]) * r2 + dot(R[0], R[2]) * r1 + dot(R[1], R[2]) * r0;
+  const float den =
+      r0 * r1 * r2 + dot(R[0], R[1]) * r2 + dot(R[0], R[2]) * r1 + dot(R[1], R[2]) * r0;
   return 2.0f * atan2f(num, den);
 }
 

@@ -196,8 +196,8 @@ __device__ __forceinline__ void regular_panel(const R* rec, const R x[3], const 
 
 // The same at two wavenumbers.
 template <typename R, bool NEED_KH>
-__device__ __forceinline__ void regular_panel2(const R* rec, const R x[3], const R nx[3], R k0, R k1,
-                                               Acc<R>& a0, Acc<R>& a1) {
+__device__ __forceinline__ void regular_panel2(const R* rec, const R x[3], const R nx[3], R k0,
+                                               R k1, Acc<R>& a0, Acc<R>& a1) {
   if constexpr (sizeof(R) == 8) {
     const double k[2] = {k0, k1};
     Acc<double> a[2] = {a0, a1};

@@ -800,7 +800,8 @@ __global__ void __launch_bounds__(256) k_wide_redo(const VecInst V, const WideCh
 }
 
 void launch_wide_redo(const Launch& L, const VecInst& v, const WideCheck& k, int mode) {
-  const unsigned grid = (unsigned)std::min<int64_t>((k.cap + 7) / 8, 4 * (int64_t)device_sm_count());
+  const unsigned grid =
+      (unsigned)std::min<int64_t>((k.cap + 7) / 8, 4 * (int64_t)device_sm_count());
   if (v.a32)
     k_wide_redo<true><<<grid, 256, 0, L.stream>>>(v, k, mode);
   else
@@ -1168,7 +1169,8 @@ void launch_resid_stats(const Launch& L, const VecInst* d, int ninst, int32_t ma
 
 void launch_corr_prep(const Launch& L, const VecInst* d, int ninst, int64_t nmax,
                       int32_t max_rhs) {
-  k_scaled_absmax<<<dim3((unsigned)max_rhs, (unsigned)ninst, kMaxStatSplit), 256, 0, L.stream>>>(d); count_launch(1);
+  k_scaled_absmax<<<dim3((unsigned)max_rhs, (unsigned)ninst, kMaxStatSplit), 256, 0, L.stream>>>(
+      d); count_launch(1);
   k_corr_prep<<<dim3((unsigned)((nmax + 255) / 256), (unsigned)max_rhs, (unsigned)ninst), 256, 0,
                 L.stream>>>(d); count_launch(1);
 }

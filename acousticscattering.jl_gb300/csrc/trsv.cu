@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_inv(const MatInst* __restri
             const int c = 32 * t + cl;
             if (c >= nbe) break;
             if (c < j) continue;
-            const C xc = {__shfl_sync(0xffffffffu, x[t].x, cl), __shfl_sync(0xffffffffu, x[t].y, cl)};
+            const C xc = {__shfl_sync(0xffffffffu, x[t].x, cl),
+                          __shfl_sync(0xffffffffu, x[t].y, cl)};
 #pragma unroll
             for (int u = t; u < kPer; ++u) {
               const int r = lane + 32 * u;
@@ -169,7 +170,8 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_inv(const MatInst* __restri
             const int c = 32 * t + cl;
             if (c > j) continue;
             if (lane == cl) x[t] = x[t] * di[c];
-            const C xc = {__shfl_sync(0xffffffffu, x[t].x, cl), __shfl_sync(0xffffffffu, x[t].y, cl)};
+            const C xc = {__shfl_sync(0xffffffffu, x[t].x, cl),
+                          __shfl_sync(0xffffffffu, x[t].y, cl)};
 #pragma unroll
             for (int u = 0; u <= t; ++u) {
               const int r = lane + 32 * u;
@@ -208,7 +210,8 @@ void launch_tri_inv(const Launch& L, const MatInst* d, int ninst, int64_t nmax, 
 // Partial sums of the block's rows to shared memory (op(A) = A: one per row and thread of the
 // row; A^H: the warp's sum), and the sum of a row; all threads take part in row_sums.
 template <class C, bool TRANS, int RG, int RW, int KQ, int NB>
-__device__ __forceinline__ void row_sums(const C (&s)[TRANS ? RW : 1][RG], C* sred, int nr, int tid) {
+__device__ __forceinline__ void row_sums(const C (&s)[TRANS ? RW : 1][RG], C* sred, int nr,
+                                         int tid) {
   if (!TRANS) {
 #pragma unroll
     for (int g = 0; g < RG; ++g)
@@ -387,7 +390,8 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
           // all of a lane's entries in one round: the next round trip starts at the last's end
           ok = ok && await_row(g, c0 + lane, xv);
 #pragma unroll
-          for (int e = 0; e < P; ++e) fma_c(acc[TRANS ? e / KL : 0][g], C{pre[e].x, -pre[e].y}, xv[e % KL]);
+          for (int e = 0; e < P; ++e)
+            fma_c(acc[TRANS ? e / KL : 0][g], C{pre[e].x, -pre[e].y}, xv[e % KL]);
         }
       }
       if (!ok) break;
@@ -468,7 +472,9 @@ __global__ void __launch_bounds__(kTriThreads, kTriCtas<RG>)
         if (kUnit ? i > j : i <= j) {
 #pragma unroll
           for (int g = 0; g < RG; ++g)
-            if (g < nr) fma_c(t[TRANS ? e / KL : 0][g], TRANS ? C{pre[e].x, -pre[e].y} : pre[e], sx[g * NB + c]);
+            if (g < nr)
+              fma_c(t[TRANS ? e / KL : 0][g], TRANS ? C{pre[e].x, -pre[e].y} : pre[e],
+                    sx[g * NB + c]);
         }
       }
       row_sums<C, TRANS, RG, RW, KQ, NB>(t, sred, nr, tid);
