@@ -434,6 +434,14 @@ int try_alloc(bemgpu_ctx* c, size_t bytes, Buf* out, bool* got) {
   return s;
 }
 
+// Scratch whose lack changes the path and with it the last bits.  A server's lane fails instead: its
+// batch runs again when no other is on the device, with the bits it would have had.
+int path_alloc(bemgpu_ctx* c, size_t bytes, Buf* out, bool* got) {
+  if (!c->parent) return try_alloc(c, bytes, out, got);
+  *got = true;
+  return alloc(c, bytes, out);
+}
+
 template <class T>
 int upload(bemgpu_ctx* c, const std::vector<T>& h, Buf* out) {
   TRY(alloc(c, h.size() * sizeof(T), out));
@@ -1690,22 +1698,30 @@ int getrf_tc(bemgpu_ctx* c, std::vector<FactorData*>& fs, const std::vector<MatI
 // Complex128 LU in 128-column blocks of four 32-column SIMT panels; the updates inside a
 // block (K = 32), the U12 solve (through -(L11^{-1} - I)) and the trailing update (K = 128)
 // run on the tensor cores from integer digit slices (gemm_oz.cu).
-int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax) {
+// *done false: no room for the slices (28 bytes per unknown and column of a block, for both
+// operands), nothing done.
+int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax, bool* done) {
   const Launch L = c->launch();
   const int ni = (int)mi.size();
   constexpr int B = kOzK;
   constexpr int kInner = B / kPanelNB - 1;  // panels of a block with columns to their right
   std::vector<Buf> apack(ni), bpack(ni), npack(ni), negn(ni), aexp(ni), bexp(ni), nexp(ni);
   std::vector<double2*> np(ni);
+  *done = false;
   for (int t = 0; t < ni; ++t) {
     const int64_t n = mi[t].n;
-    TRY(alloc(c, oz_pack_bytes(n, B, kOzA), &apack[t]));
-    TRY(alloc(c, oz_pack_bytes(n, B, kOzB), &bpack[t]));
-    TRY(alloc(c, oz_pack_bytes(B, B, kOzA), &npack[t]));
-    TRY(alloc(c, (size_t)B * B * 16, &negn[t]));
-    TRY(alloc(c, oz_exps(n, kOzA) * 4, &aexp[t]));
-    TRY(alloc(c, oz_exps(n, kOzB) * 4, &bexp[t]));
-    TRY(alloc(c, oz_exps(B, kOzA) * 4, &nexp[t]));
+    bool got = true;
+    auto scratch = [&](size_t bytes, Buf* b) {
+      return got ? path_alloc(c, bytes, b, &got) : BEMGPU_OK;
+    };
+    TRY(scratch(oz_pack_bytes(n, B, kOzA), &apack[t]));
+    TRY(scratch(oz_pack_bytes(n, B, kOzB), &bpack[t]));
+    TRY(scratch(oz_pack_bytes(B, B, kOzA), &npack[t]));
+    TRY(scratch((size_t)B * B * 16, &negn[t]));
+    TRY(scratch(oz_exps(n, kOzA) * 4, &aexp[t]));
+    TRY(scratch(oz_exps(n, kOzB) * 4, &bexp[t]));
+    TRY(scratch(oz_exps(B, kOzA) * 4, &nexp[t]));
+    if (!got) return BEMGPU_OK;
     np[t] = negn[t].as<double2>();
   }
   // descriptors of every update, uploaded once: per block and inner panel, then the U12
@@ -1716,7 +1732,10 @@ int getrf_oz(bemgpu_ctx* c, const std::vector<MatInst>& mi, Buf& d, int64_t nmax
   // the scale of every update's K index, from the rows of its right operand: with rows of
   // different sizes (no equilibration) l_ik goes with 1 / d_k and u_kj with d_k
   Buf kexp;
-  TRY(alloc(c, count * B * 4, &kexp));
+  bool got = false;
+  TRY(path_alloc(c, count * B * 4, &kexp, &got));
+  if (!got) return BEMGPU_OK;
+  *done = true;
   CUDA_TRY(c, cudaMemsetAsync(kexp.p, 0, count * B * 4, c->stream));
   std::vector<OzPackInst> pa(count), pb(count);
   std::vector<OzGemmInst> ge(count);
@@ -1835,11 +1854,14 @@ int getrf_batch(bemgpu_ctx* c, std::vector<FactorData*>& fs, int prec, bool prom
   }
   Buf d;
   TRY(to_device(c, mi, &d));
+  bool done = false;
   if (prec == 1 && c->tensor_lu) {
     TRY(getrf_tc(c, fs, mi, d, nmax));
+    done = true;
   } else if (prec == 0 && c->tensor_lu) {
-    TRY(getrf_oz(c, mi, d, nmax));
-  } else {
+    TRY(getrf_oz(c, mi, d, nmax, &done));
+  }
+  if (!done) {
     // right-looking blocked LU, 32-column panels; each kernel family timed on its own
     const MatInst* dm = d.as<MatInst>();
     const int ni = (int)fs.size();
@@ -2352,7 +2374,7 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode, bool* done) {
   const int32_t cap = wide_cap(n, R);
   bool got = true;
   auto scratch = [&](size_t bytes, Buf* b) {
-    return got ? try_alloc(c, bytes, b, &got) : BEMGPU_OK;
+    return got ? path_alloc(c, bytes, b, &got) : BEMGPU_OK;
   };
   TRY(scratch(oz_pack_bytes(R, (int)n, kOzB), &xp));
   TRY(scratch((size_t)kb * oz_exps(R, kOzB) * 4, &xe));
@@ -2367,12 +2389,18 @@ int wide_product(bemgpu_ctx* c, const VecInst& v, int mode, bool* done) {
   const uint64_t room =
       std::min<uint64_t>(wide_panel_bytes(n), budget > used ? (budget - used) / 4 : 0);
   int64_t tiles = std::max<int64_t>(1, (int64_t)(room / tile));
-  for (;; tiles = (tiles + 1) / 2) {
+  for (;; tiles = (tiles + 1) / 2) {  // the number of panels does not change the bits
+    const size_t exps = (size_t)kb * (size_t)tiles * 128 * 4, slices = tile * (size_t)tiles;
     got = true;
-    TRY(scratch((size_t)kb * (size_t)tiles * 128 * 4, &ae));
-    TRY(scratch(tile * (size_t)tiles, &ap));
+    if (tiles == 1) {
+      TRY(scratch(exps, &ae));
+      TRY(scratch(slices, &ap));
+      if (!got) return BEMGPU_OK;
+      break;
+    }
+    TRY(try_alloc(c, exps, &ae, &got));
+    if (got) TRY(try_alloc(c, slices, &ap, &got));
     if (got) break;
-    if (tiles == 1) return BEMGPU_OK;
   }
   *done = true;
   const int64_t rows = tiles * 128;

@@ -46,6 +46,29 @@ def test_least_budget_is_that_of_the_row_wise_products(ctx):
         assert d["normwise_backward_error"] <= (5 * np.sqrt(n) + 1) * eps
 
 
+def test_least_budget_of_a_double_factorisation(ctx):
+    """The slices of its updates are taken if there is room: the least budget is that of the FP64
+    pipe and the descriptors."""
+    n = 900
+    rng = np.random.default_rng(5)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 2 * np.eye(n)
+    B = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    lo, hi = 1, 512
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        if _solve(mid * MB, A, B, False) is None:
+            lo = mid
+        else:
+            hi = mid
+    eps = 2.0 ** -53
+    for budget in (hi + 1, 512):
+        got = _solve(budget * MB, A, B, True)
+        assert got is not None, budget
+        r = np.abs(B - A @ got[0]).max(axis=0)
+        scale = np.abs(A).sum(axis=1).max() * np.abs(got[0]).max(axis=0) + np.abs(B).max(axis=0)
+        assert np.all(r <= (5 * np.sqrt(n) + 1) * eps * scale)
+
+
 def test_partial_sums_of_many_right_hand_sides(ctx):
     """Eight chunks of partial sums per right-hand side (of 24 bytes an unknown), the seven other
     vectors and the few MB of a system of 300 unknowns are enough."""
