@@ -153,7 +153,8 @@ class Context:
         return {"captures": cap.value, "replays": rep.value}
 
     def set_tensor_lu(self, enable: bool):
-        """Complex64 LU trailing updates on the tensor cores (default) or CUDA cores."""
+        """Tensor cores (default) or CUDA cores for the LU's updates and for the products of a
+        system with 16 right-hand sides or more."""
         _check(C.lib().bemgpu_ctx_set_tensor_lu(self.handle, int(enable)), self.handle)
 
     def debug_panel(self, A, precision="double", cluster=0, streaming=False):
@@ -468,6 +469,8 @@ class BEMSolution:
         return len(self.incidence_angles)
 
     def far_field(self, directions=None, rhs: int = 0) -> np.ndarray:
+        """Far-field amplitudes at unit directions (None: backscatter).  From 32 directions on
+        the panels are added in another order, which may change a value's last bits."""
         if directions is None:
             out = np.zeros(1, dtype=np.complex128)
             _check(C.lib().bemgpu_far_field(self.handle, rhs, 1, None, C.dptr(out)),

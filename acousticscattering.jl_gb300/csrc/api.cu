@@ -2359,9 +2359,10 @@ size_t wide_scratch(int64_t n, int64_t R) {
 // so the unknowns are taken in units of their sizes (columns of A times, vectors divided by, a
 // power of two per unknown), and entries whose error could still matter beside |A||x| are
 // computed again in FP64, or the whole product row by row when there are many of them (decided
-// on the device).  The row-wise products spend about 44 FP32 instructions per
-// complex product whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 29 ms (of
-// which 16 the products, 4 the slices of the matrix, 5 the denominators).
+// on the device).  The row-wise products spend about 44 FP32 instructions per complex product
+// whatever the number of vectors; 181 vectors of 20480 unknowns: 175 -> 31 ms (of which 17 the
+// products, 4.5 the slices of the matrix, 5.3 the denominators, 3.4 the near corrections, 0.5 the
+// check and the entries again).
 //
 // Scratch (wide_scratch) is taken if it is there: fewer row panels when the allocation fails, and
 // the row-wise products when not even one panel can be had (*done false).

@@ -37,7 +37,7 @@
 // each of the 8 chunks of a tile and K-block take at least 22.5k cycles, the FP64 conversion
 // and update of the epilogue about 8k beside them, moving the levels out of tensor memory about
 // 2k in between.  The trailing updates of an LU of 5760 unknowns: 718 ms on the FP64 pipe (0.7
-// TFLOP/s), 12 ms here.
+// TFLOP/s), 13 ms here (12 with instructions cut to the slices that exist).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -820,7 +820,7 @@ __global__ void k_wide_mag(const VecInst V, float* __restrict__ xa) {
 // entries per thread, K-chunks of 16 with the next chunk in registers as it was loaded (a
 // magnitude taken at the load would wait for it).  FP32-issue bound, one FMA per matrix entry and
 // vector, two of them in a paired instruction: 2.1 ms for 20480 unknowns and 181 vectors at the
-// single rate, 11 ms before the pairs, the late magnitudes and the odd row stride of sX, 5.0 ms
+// single rate, 11 ms before the pairs, the late magnitudes and the odd row stride of sX, 5.3 ms
 // with them.  FP32 sums of kWaFold columns are added in FP64 (the row-wise products': n / 8 to n
 // / 32 columns).
 constexpr int kWaM = 64, kWaN = 96, kWaK = 16, kWaFold = 2048;

@@ -381,6 +381,8 @@ int bemgpu_gmres_history(const bemgpu_solution *sol, int32_t rhs, double *out, i
  * Far-field amplitude f(x_hat) of right-hand side `rhs` at ndir unit directions
  * (3 * ndir doubles); out receives 2 * ndir doubles.  dirs == NULL means backscatter.
  * Replaces far_field (full.jl:509-519) / scattering_amplitude (postprocessing.jl:1-13).
+ * From 32 directions on the panels are added in another order: a direction's value may differ
+ * in its last bits from that of a call with fewer.
  */
 int bemgpu_far_field(bemgpu_solution *sol, int32_t rhs, int64_t ndir, const double *dirs,
                      double *out);
@@ -393,7 +395,9 @@ int bemgpu_solution_diagnostics(const bemgpu_solution *sol, bemgpu_diagnostics *
 /*
  * Pressure at npts points (3 * npts doubles, out 2 * npts doubles) by the layer
  * potentials of the surface traces, fields/pressure.jl:404-471.  Points on the
- * surface or on the wrong side for `field` give BEMGPU_EINVAL.
+ * surface or on the wrong side for `field` give BEMGPU_EINVAL.  For a fluid body the interior
+ * traces are formed by a launch of their own from 256 points on, which may change a value's
+ * last bits against that of a call with fewer.
  */
 int bemgpu_pressure(bemgpu_solution *sol, int32_t rhs, int64_t npts, const double *points,
                     int32_t field, double *out);
